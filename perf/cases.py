@@ -43,7 +43,7 @@ def listed():
         # the smallest runs of a parameter scan: 65 k particles, where launches and latency count
         dict(name="es 64x64", kind="es", nx=64, ny=64, dx=1.0, ppc=16, vth=0.03, vd=0.2, bz=0.0, dt=0.1, steps=50),
         # the electrostatic two-stream benchmark (4.2 M particles)
-        dict(name="es 256x256", kind="es", nx=256, ny=256, dx=1.0, ppc=64, vth=0.01, vd=0.2, bz=0.0, dt=0.1, steps=50),
+        dict(name="es 256x256", kind="es", nx=256, ny=256, dx=1.0, ppc=64, vth=0.01, vd=0.2, bz=0.0, dt=0.1, steps=20),
         # an electrostatic run off the powers of two: odd grid, cell size 0.3, magnetised, ragged count
         dict(name="es 375x225 magnetised", kind="es", nx=375, ny=225, dx=0.3, ppc=50, vth=0.05, vd=0.1, bz=0.5, dt=0.1,
              steps=20),
@@ -104,7 +104,7 @@ def draw(rng):
         nx, ny = _grid(rng, 512 * 512)
         ppc = _ppc(rng, nx * ny, TOTAL // 2) & ~1
         return dict(kind=kind, nx=nx, ny=ny, dx=dx, ppc=ppc, vth=vth, vd=round(rng.uniform(0.0, 0.3), 3),
-                    bz=rng.choice((0.0, round(rng.uniform(0.2, 1.0), 3))), dt=0.1, steps=rng.choice((20, 30, 40)))
+                    bz=rng.choice((0.0, round(rng.uniform(0.2, 1.0), 3))), dt=0.1, steps=rng.choice((10, 15, 20)))
     if kind in ("darwin", "operators", "resort"):
         nx, ny = _grid(rng, 512 * 512)
         if kind == "darwin" and rng.random() < 0.15:
