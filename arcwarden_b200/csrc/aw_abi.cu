@@ -330,7 +330,8 @@ double grad_es_impl(Ctx& c, long long nsteps, int every, float* dux, float* duy,
     prep_adj_scatter();
     if (!c.gexec) c.gexec = capture_exec(c, [&] { step_body(c); });
     const AdjK kf = adj_constants(c, 1.0f);
-    AdjP a{w.traj_xy, w.lam, w.lam + n, w.lam + 2 * n, w.lam + 3 * n, w.lam + 4 * n, n, (n % 4 == 0) ? 1 : 0};
+    AdjP a{w.traj_xy, w.lam, w.lam + n, w.lam + 2 * n, w.lam + 3 * n, w.lam + 4 * n, n, (n % 4 == 0) ? 1 : 0,
+           aw::chunk_size(n, 3 * c.sms)};
     // The recording step: the ES step whose kernels also write x_n, y_n and E_n
     // into the trajectory slot they advance; with the end-of-step reduction for
     // the forward run's last segment, without it (diagnostics only) for the
@@ -478,6 +479,7 @@ int aw_ctx_create(const aw_grid* g, const aw_params* p, int32_t model, void* str
         c.grid = *g;
         c.prm = *p;
         c.model = model;
+        c.parts.cs = aw::kChunk;
         c.resort_every = (model == AW_MODEL_DARWIN || model == AW_MODEL_YEE) ? 50 : 0;
         c.geo.nx = g->nx; c.geo.ny = g->ny;
         c.geo.nxf = static_cast<float>(g->nx); c.geo.nyf = static_cast<float>(g->ny);
@@ -487,6 +489,9 @@ int aw_ctx_create(const aw_grid* g, const aw_params* p, int32_t model, void* str
         c.sg.dkx = 6.28318530717958647692 / g->Lx;
         c.sg.dky = 6.28318530717958647692 / g->Ly;
         c.sg.invN = 1.0f / static_cast<float>(c.geo.ncell);
+        int dev = 0;
+        AW_CUDA(cudaGetDevice(&dev));
+        AW_CUDA(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
         if (stream) {
             c.stream = static_cast<cudaStream_t>(stream);
         } else {
@@ -589,7 +594,10 @@ int aw_particles_bind(aw_ctx* ctx, float* x, float* y, float* ux, float* uy, flo
         c.parts_bound = true;
         auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
         c.parts.vec_ok = (al(x) && al(y) && al(ux) && al(uy) && al(uz) && al(w) && (!cell || al(cell))) ? 1 : 0;
-        const int nb = static_cast<int>(std::max<long long>(1, (n + aw::kChunk - 1) / aw::kChunk));
+        // resident CTAs of the model's particle kernels (the ES kernel's small window leaves room for four per SM)
+        const bool four = c.model == AW_MODEL_ES && n >= 32LL * c.geo.ncell;
+        c.parts.cs = aw::chunk_size(n, (four ? 4 : 3) * c.sms);
+        const int nb = static_cast<int>(std::max<long long>(1, (n + c.parts.cs - 1) / c.parts.cs));
         if (nb > c.npart_p) {
             if (c.part_p) cudaFree(c.part_p);
             if (c.part_c) cudaFree(c.part_c);

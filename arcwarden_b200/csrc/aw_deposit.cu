@@ -43,6 +43,7 @@
 #include <cmath>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace aw {
@@ -191,24 +192,48 @@ __device__ __forceinline__ bool scale_fast(const float (&cf)[NF], const float (&
     return fast;
 }
 
-// Block-wide fixed-order sum of 4 doubles into part[blk*5 + 0..3] (blk: the chunk).
-__device__ void block_sum4(double a, double b, double c, double d, double* __restrict__ part,
-                           double* sh /* 4 * warps */, int blk) {
+// Warp sums with halving: at each of the first levels a lane gives away half of
+// its values and keeps the sums of the other half, so n values take about n
+// shuffles instead of 5 n. Fixed order. On return lanes 0, 8, 16, 24 hold the
+// sums of v[0], v[1], v[2], v[3].
+template <class T>
+__device__ __forceinline__ T warp_sum4(T v0, T v1, T v2, T v3) {
+    const int lane = threadIdx.x & 31;
+    const bool h = lane & 16, q = lane & 8;
+    const T a0 = h ? v2 : v0, a1 = h ? v3 : v1, g0 = h ? v0 : v2, g1 = h ? v1 : v3;
+    const T b0 = a0 + __shfl_xor_sync(0xffffffffu, g0, 16), b1 = a1 + __shfl_xor_sync(0xffffffffu, g1, 16);
+    T c = (q ? b1 : b0) + __shfl_xor_sync(0xffffffffu, q ? b0 : b1, 8);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-        c += __shfl_down_sync(0xffffffffu, c, o);
-        d += __shfl_down_sync(0xffffffffu, d, o);
-    }
-    const int warp = threadIdx.x >> 5;
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+// The same for 8 values: lanes 0, 4, 8, .., 28 hold the sums of v[0..8).
+__device__ __forceinline__ float warp_sum8(const float (&v)[8]) {
+    const int lane = threadIdx.x & 31;
+    const bool h = lane & 16, q = lane & 8, e = lane & 4;
+    float a[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] = (h ? v[4 + k] : v[k]) + __shfl_xor_sync(0xffffffffu, h ? v[k] : v[4 + k], 16);
+    const float b0 = (q ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, q ? a[0] : a[2], 8);
+    const float b1 = (q ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, q ? a[1] : a[3], 8);
+    float c = (e ? b1 : b0) + __shfl_xor_sync(0xffffffffu, e ? b0 : b1, 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    return c;
+}
+
+// Block-wide fixed-order sum of 4 doubles into part[blk*5 + 0..3] (blk: the chunk).
+__device__ __forceinline__ void block_sum4(double a, double b, double c, double d, double* __restrict__ part,
+                                           double* sh /* 4 * warps */, int blk) {
     constexpr int NW = kThreads / 32;
-    if ((threadIdx.x & 31) == 0) { sh[warp] = a; sh[NW + warp] = b; sh[2 * NW + warp] = c; sh[3 * NW + warp] = d; }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double w = warp_sum4(a, b, c, d);
+    if ((lane & 7) == 0) sh[(lane >> 3) * NW + warp] = w;
     __syncthreads();
     if (threadIdx.x < 4) {
         double s = 0;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) s += sh[threadIdx.x * NW + w];
+        for (int k = 0; k < NW; ++k) s += sh[threadIdx.x * NW + k];
         part[blk * 5 + threadIdx.x] = s;
     }
     if (threadIdx.x == 4) part[blk * 5 + 4] = 0.0;
@@ -216,23 +241,22 @@ __device__ void block_sum4(double a, double b, double c, double d, double* __res
 
 // Block-wide fixed-order sum of NF floats (plus the valid-particle count in
 // slot NF) into part[blk * (NF + 1) + f]. Deterministic for a fixed
-// launch shape.
+// launch shape. 1, 3, 4 or 8 fields.
 template <int NF>
-__device__ void block_sumsq(float (&sq)[NF], float cnt, float* __restrict__ part, float* sh /* (NF+1) * warps */,
-                            int blk) {
+__device__ __forceinline__ void block_sumsq(const float (&sq)[NF], float cnt, float* __restrict__ part,
+                                            float* sh /* (NF+1) * warps */, int blk) {
     constexpr int NW = kThreads / 32;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int f = 0; f < NF; ++f) sq[f] += __shfl_down_sync(0xffffffffu, sq[f], o);
-        cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (NF == 8) {
+        const float w = warp_sum8(sq);
+        if ((lane & 3) == 0) sh[(lane >> 2) * NW + warp] = w;
+    } else {
+        const float w = warp_sum4(sq[0], NF > 1 ? sq[NF > 1 ? 1 : 0] : 0.f, NF > 2 ? sq[NF > 2 ? 2 : 0] : 0.f,
+                                  NF > 3 ? sq[NF > 3 ? 3 : 0] : 0.f);
+        if ((lane & 7) == 0 && (lane >> 3) < NF) sh[(lane >> 3) * NW + warp] = w;
     }
-    const int warp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int f = 0; f < NF; ++f) sh[f * NW + warp] = sq[f];
-        sh[NF * NW + warp] = cnt;
-    }
+    const unsigned n = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(cnt));   // a count: exact
+    if (lane == 0) sh[NF * NW + warp] = static_cast<float>(n);
     __syncthreads();
     if (threadIdx.x <= NF) {
         float s = 0.f;
@@ -270,11 +294,11 @@ __device__ __forceinline__ Win open_window(const BBox& bb, int ir, int jr, int w
 // Block tail shared by every kernel: window flush, slow list, counters.
 template <int NF, int NS, bool T0, int PC = 0, class CoefFn>
 __device__ __forceinline__ void close_window(const Smem& m, const Win& wn, int nlist,
-                                             unsigned long long* __restrict__ acc, const Geo& g, DevState* st,
+                                             int cs_, unsigned long long* __restrict__ acc, const Geo& g, DevState* st,
                                              CoefFn coef) {
     __syncthreads();
     if (wn.nb == 1) win_flush<NF, T0, PC>(m.win, wn, acc, g);
-    slow_pass<NF, NS>(m.stage, m.slow, nlist, !wn.use, acc, g, st, coef);
+    slow_pass<NF, NS>(m.stage, m.slow, nlist, !wn.use, cs_, acc, g, st, coef);
     if (threadIdx.x == 0) {
         atomicAdd(&st->chunks, 1ull);
         if (!wn.use || wn.nb > 1) atomicAdd(&st->overflow, 1ull);
@@ -283,7 +307,7 @@ __device__ __forceinline__ void close_window(const Smem& m, const Win& wn, int n
 
 // ---------------------------------------------------------------------------
 // Standalone source deposit at the current positions.
-template <int SET>
+template <int SET, bool FULL>
 __global__ void __launch_bounds__(kThreads, 3)
 k_deposit_src(Parts p, Geo g, double qoa, const float* __restrict__ Sdev,
               unsigned long long* __restrict__ acc, int wmaxc, DevState* st, float* __restrict__ psq) {
@@ -295,8 +319,10 @@ k_deposit_src(Parts p, Geo g, double qoa, const float* __restrict__ Sdev,
     __shared__ int nlist;
     __shared__ float ssq[(NF + 1) * (kThreads / 32)];
 
-    const long long c0 = static_cast<long long>(blockIdx.x) * kChunk;
-    const int cnt = static_cast<int>(min(static_cast<long long>(kChunk), p.n - c0));
+    const int cs_ = FULL ? kChunk : p.cs;
+    const long long c0 = static_cast<long long>(blockIdx.x) * cs_;
+    const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
+    const int ppt = cs_ / kThreads;               // particles per thread
     if (threadIdx.x == 0) nlist = 0;
     const ChunkSrc src{{p.x, p.y, p.w, p.ux, p.uy, p.uz}};
     float x0, y0;
@@ -313,7 +339,7 @@ k_deposit_src(Parts p, Geo g, double qoa, const float* __restrict__ Sdev,
     float sq[NF] = {};
     float nval = 0.f;
 #pragma unroll 1
-    for (int it = 0; it < kPPT; ++it) {
+    for (int it = 0; it < ppt; ++it) {
         const int s = it * kThreads + threadIdx.x;
         float a[NS];
 #pragma unroll
@@ -352,8 +378,8 @@ k_deposit_src(Parts p, Geo g, double qoa, const float* __restrict__ Sdev,
 #pragma unroll
         for (int f = 0; f < NF; ++f) cs[f] = __fmul_rn(cf[f], S[f]);
     };
-    window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, g, coef, acc);
-    close_window<NF, NS, T0, PC>(m, wn, nlist, acc, g, st, coef);
+    window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);
+    close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
     if (psq) block_sumsq<NF>(sq, nval, psq, ssq, blockIdx.x);
 }
 
@@ -460,19 +486,6 @@ __device__ __forceinline__ bool load_tile8(float* tile, const float* __restrict_
     return mbar_wait_block(bar, st);
 }
 
-// ---------------------------------------------------------------------------
-// Single-pass chunks. When a chunk's deposit window - the box of its CURRENT
-// base cells, widened on every side by the cells a particle can cross in one
-// step, plus the +1 CIC corner - fits the shared capacity next to its gather
-// tile, the kernel pushes and deposits each particle in the same pass, from
-// registers: no second pass over the staged chunk, no per-particle re-read or
-// recomputation of the weights and coefficients. The new state is written back
-// into the stage in place and leaves with one bulk copy per array. A particle
-// that lands outside the window (it moved further than the margin) or whose
-// coefficients leave the fast range takes the exact slow path, as in the two-pass
-// kernels, so the sums are the same bits either way. Chunks that do not fit take
-// the two-pass path.
-
 // Block-wide box of the threads' BBoxes (empty: lo > hi). Ends with a barrier
 // after the scratch `red` is read.
 struct Box { int lo_i, hi_i, lo_j, hi_j; };
@@ -495,99 +508,280 @@ __device__ __forceinline__ Box box_reduce(const BBox& bb, int* red) {
     return b;
 }
 
-// True (block-uniformly) when some untracked field's chunk bound
-// sum_p (|cs_p| + 1) may reach 2^31 (win_setup's test): its biased int32 window
-// words may then have wrapped, and the chunk is deposited through the exact
-// slow path instead. Ends with a barrier after `red` is read.
-template <int NF, bool T0>
-__device__ __forceinline__ bool chunk_overflows(const float (&l1)[NF], int* red) {
+// ---------------------------------------------------------------------------
+// Single-pass windows. A chunk whose particles are all in the grid and whose
+// deposit window - the box of their CURRENT base cells, widened on every side by
+// the cells a particle can cross in one step, plus the +1 CIC corner - fits the
+// shared capacity is pushed and deposited in one pass, from registers: no second
+// pass over the staged chunk, no re-read or recomputation of weights and
+// coefficients. The gather fields of the box are staged beside the window. A
+// particle that lands outside the window (it moved further than the margin) or
+// whose coefficients leave the fast range takes the exact slow path, as in the
+// two-pass kernels, so the sums are the same bits either way.
+//
+// Planes of P1 int32 words: NF biased sums (M + q per contribution, one native
+// shared atomic each); with HI (field 0 is the charge density, whose chunk sums
+// exceed int32) two more of field 0's coarse parts, packed: the base cell's
+// (corner 0 | corner 1 << 16) and (corner 2 | corner 3 << 16) sums of
+// (q + 2^22) >> 19; and the particle counts of the base cells. A chunk has at
+// most 2048 particles, so a coarse sum is at most 2^15 and the fine sum modulo
+// 2^32 plus the coarse one (short by less than 2^30) give the exact 64-bit sum:
+// 6 atomics and 6 more instructions per particle in place of four read-back
+// atomics with their compares (whistler1024: see k_push_deposit_em).
+//
+// Lanes sit 8 m particles apart, so where a cell holds more particles than that
+// neighbouring lanes meet in it: the window is then kept in up to 16 copies
+// (lane l adds to copy l mod rep), CS cells apart, CS congruent to 32 / rep
+// modulo 32: the copies of a cell fall in different banks.
+struct Win1 {
+    int oi, oj;      // grid cell of window cell (0, 0)
+    int W, H, WH;
+    int rep, CS;
+};
+// The box of the chunk's base cells: nI x nJ cells from grid cell (i0, j0).
+struct Box1 { int i0, j0, nI, nJ; };
+
+// Block-wide box; false (block-uniformly) when some particle is not in the grid.
+// First without regard to the periodic edges (positions in the grid are
+// non-negative floats, so integer order of the bits is their order, and anything
+// else - negative, NaN, too large - shows at one of the two ends); a box wider
+// than `cap_i` x `cap_j` cells is taken again as wrapped offsets from the first
+// particle's cell, which is exact for chunks that straddle an edge. Slots past
+// cnt are filled with the first particle's position by the threads that read
+// them. `red` is 32 ints of scratch. Ends with every warp past its reads of `red`
+// only after the caller's next barrier.
+__device__ __forceinline__ bool chunk_box(float* stage, int cs, int cnt, float x0, float y0, const Geo& g, int* red,
+                                          int cap_cells, int mg, Box1& b) {
     constexpr int NW = kThreads / 32;
     const int warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int f = T0 ? 1 : 0; f < NF; ++f) {
-        const float b = fminf(ceilf(__fmul_rn(l1[f], 1.00000095367431640625f)), 33554432.0f);
-        const unsigned w = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(b) + static_cast<unsigned>(kPPT));
-        if ((threadIdx.x & 31) == 0) red[f * NW + warp] = static_cast<int>(w);
+    if (cnt < cs)
+        for (int s = threadIdx.x; s < cs; s += kThreads)
+            if (s >= cnt) { stage[s] = x0; stage[kChunk + s] = y0; }
+    const int* xb = reinterpret_cast<const int*>(stage);
+    int lx = xb[threadIdx.x], hx = lx, ly = xb[kChunk + threadIdx.x], hy = ly;
+#pragma unroll 7
+    for (int s = kThreads + threadIdx.x; s < cs; s += kThreads) {
+        const int x = xb[s], y = xb[kChunk + s];
+        lx = min(lx, x); hx = max(hx, x);
+        ly = min(ly, y); hy = max(hy, y);
     }
+    lx = __reduce_min_sync(0xffffffffu, lx); hx = __reduce_max_sync(0xffffffffu, hx);
+    ly = __reduce_min_sync(0xffffffffu, ly); hy = __reduce_max_sync(0xffffffffu, hy);
+    if ((threadIdx.x & 31) == 0) { red[warp] = lx; red[NW + warp] = hx; red[2 * NW + warp] = ly; red[3 * NW + warp] = hy; }
     __syncthreads();
-    bool over = false;
+    lx = red[0]; hx = red[NW]; ly = red[2 * NW]; hy = red[3 * NW];
 #pragma unroll
-    for (int f = T0 ? 1 : 0; f < NF; ++f) {
-        unsigned long long t = 0;
-#pragma unroll
-        for (int k = 0; k < NW; ++k) t += static_cast<unsigned>(red[f * NW + k]);
-        over = over || (t >= 2147483648ull);
+    for (int k = 1; k < NW; ++k) {
+        lx = min(lx, red[k]); hx = max(hx, red[NW + k]);
+        ly = min(ly, red[2 * NW + k]); hy = max(hy, red[3 * NW + k]);
     }
-    __syncthreads();
-    return over;
-}
-
-// The window of a single-pass chunk: the box widened by `mg` cells, plus the
-// corner; biased, one band, plane stride P1. False when it does not fit, or
-// when it spans more than n + 1 cells of a grid dimension n (a margin too wide
-// for the grid, e.g. ny = 1): the origin and the flush wrap each index once,
-// which is exact while W <= nx + 1 and H <= ny + 1.
-template <int NF, bool T0, int P1>
-__device__ __forceinline__ bool one_pass_window(Win& w, const Box& b, int ir, int jr, int mg, const Geo& g) {
-    if (b.hi_i < b.lo_i) return false;
-    w.ir = ir; w.jr = jr;
-    w.mi = b.lo_i - mg; w.mj = b.lo_j - mg;
-    w.W = b.hi_i - b.lo_i + 2 + 2 * mg;
-    w.H = b.hi_j - b.lo_j + 2 + 2 * mg;
-    if (w.W > g.nx + 1 || w.H > g.ny + 1) return false;
-    if (static_cast<long long>(w.W) * w.H > P1) return false;
-    w.Hb = w.H; w.nb = 1;
-    w.WH = w.W * w.H;
-    w.P = P1;
-    // as many copies (4, 2, 1) as fit, each rep copies CS cells apart, CS the
-    // first stride >= WH congruent to 32 / rep modulo 32: a cell's copies then
-    // fall in banks 32 / rep apart
-    const int cs4 = w.WH + (((8 - w.WH) % 32) + 32) % 32, cs2 = w.WH + (((16 - w.WH) % 32) + 32) % 32;
-    if (4 * cs4 <= P1) { w.rep = 4; w.CS = cs4; }
-    else if (2 * cs2 <= P1) { w.rep = 2; w.CS = cs2; }
-    else { w.rep = 1; w.CS = w.WH; }
-    w.use = true;
-    w.track_all = false;
-    w.biased = NF > (T0 ? 1 : 0);
+    const float xhi = __int_as_float(hx), yhi = __int_as_float(hy);
+    if (lx < 0 || ly < 0 || !(xhi < g.nxf) || !(yhi < g.nyf)) return false;
+    b.i0 = static_cast<int>(__int_as_float(lx)); b.nI = static_cast<int>(xhi) - b.i0 + 1;
+    b.j0 = static_cast<int>(__int_as_float(ly)); b.nJ = static_cast<int>(yhi) - b.j0 + 1;
+    if (static_cast<long long>(min(b.nI + 1 + 2 * mg, g.nx + 1)) * min(b.nJ + 1 + 2 * mg, g.ny + 1) <= cap_cells) return true;
+    // the chunk straddles an edge, or is simply large: wrapped offsets
+    const int ir = static_cast<int>(x0), jr = static_cast<int>(y0);
+    BBox bb;
+    for (int s = threadIdx.x; s < cs; s += kThreads)
+        bb.add(static_cast<int>(stage[s]), static_cast<int>(stage[kChunk + s]), ir, jr, g);
+    __syncthreads();                          // `red` has been read
+    const Box w = box_reduce(bb, red);
+    b.i0 = ir + w.lo_i; if (b.i0 < 0) b.i0 += g.nx; if (b.i0 >= g.nx) b.i0 -= g.nx;
+    b.j0 = jr + w.lo_j; if (b.j0 < 0) b.j0 += g.ny; if (b.j0 >= g.ny) b.j0 -= g.ny;
+    b.nI = w.hi_i - w.lo_i + 1;
+    b.nJ = w.hi_j - w.lo_j + 1;
     return true;
 }
 
-// The gather tile of the box (its base cells plus the corner), from the
-// wrapped origin; use = false when it does not fit `cap` cells.
-__device__ __forceinline__ Tile box_tile(const Box& b, int ir, int jr, const Geo& g, int cap) {
-    Tile t;
-    t.i0 = ir + b.lo_i; if (t.i0 < 0) t.i0 += g.nx; if (t.i0 >= g.nx) t.i0 -= g.nx;
-    t.j0 = jr + b.lo_j; if (t.j0 < 0) t.j0 += g.ny; if (t.j0 >= g.ny) t.j0 -= g.ny;
-    t.W = b.hi_i - b.lo_i + 2;
-    t.H = b.hi_j - b.lo_j + 2;
-    t.use = b.hi_i >= b.lo_i && t.W <= g.nx && t.H <= g.ny && t.W * t.H <= cap;
-    return t;
+// The window of box b widened by mg cells; false when it does not fit P1 cells.
+// A dimension the window would span whole (a margin wider than the grid, e.g.
+// ny = 1) is taken from cell 0 with its n + 1 cells: the flush wraps each index
+// once. rep_need: the copies asked for (a power of two, at most 16).
+template <int P1>
+__device__ __forceinline__ bool window1(Win1& w, const Box1& b, int mg, int rep_need, const Geo& g) {
+    w.oi = b.i0 - mg; w.W = b.nI + 1 + 2 * mg;
+    w.oj = b.j0 - mg; w.H = b.nJ + 1 + 2 * mg;
+    if (w.W > g.nx) { w.W = g.nx + 1; w.oi = 0; }
+    else if (w.oi < 0) w.oi += g.nx;
+    if (w.H > g.ny) { w.H = g.ny + 1; w.oj = 0; }
+    else if (w.oj < 0) w.oj += g.ny;
+    if (static_cast<long long>(w.W) * w.H > P1) return false;
+    w.WH = w.W * w.H;
+    w.rep = 1; w.CS = w.WH;
+    for (int r = rep_need; r > 1; r >>= 1) {
+        const int cs = w.WH + ((32 / r - w.WH) & 31);
+        if (r * cs <= P1) { w.rep = r; w.CS = cs; break; }
+    }
+    return true;
 }
 
-// Write stage planes pl[0..NP) back to their arrays dst[0..NP) for the chunk
+// Zero the window's planes (rep copies); the caller syncs.
+template <int PLANES, int P1>
+__device__ __forceinline__ void win1_zero(int* __restrict__ s, const Win1& w) {
+    for (int c = threadIdx.x; c < w.CS * w.rep; c += kThreads)
+#pragma unroll
+        for (int f = 0; f < PLANES; ++f) s[f * P1 + c] = 0;
+}
+
+// The contributions of one particle whose base cell is window cell (di, dj).
+template <int NF, bool HI, int P1>
+__device__ __forceinline__ void win1_add(int* __restrict__ win, const Win1& w, int di, int dj, float x, float y,
+                                         const float (&cs)[NF]) {
+    const Cic2 c2 = cic2(x, y);
+    int b[NF][4];
+    quant_bits<NF>(cs, c2, b);
+    int* e0 = win + (threadIdx.x & (w.rep - 1)) * w.CS + dj * w.W + di;   // this lane's copy
+    int* e2 = e0 + w.W;
+    constexpr int NC = NF + (HI ? 2 : 0);
+    atomicAdd(e0 + NC * P1, 1);
+    if (HI) {
+        atomicAdd(e0 + NF * P1, (static_cast<int>(__byte_perm(b[0][0], b[0][1], 0x7632)) >> 3) & 0x001F001F);
+        atomicAdd(e0 + (NF + 1) * P1, (static_cast<int>(__byte_perm(b[0][2], b[0][3], 0x7632)) >> 3) & 0x001F001F);
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        atomicAdd(e0 + f * P1, b[f][0]);
+        atomicAdd(e0 + f * P1 + 1, b[f][1]);
+        atomicAdd(e2 + f * P1, b[f][2]);
+        atomicAdd(e2 + f * P1 + 1, b[f][3]);
+    }
+}
+
+// Flush into the global int64 accumulators, TPC threads per window cell (each
+// takes every TPC-th field); the caller has synced.
+template <int NF, bool HI, int P1, int TPC>
+__device__ __forceinline__ void win1_flush(const int* __restrict__ s, const Win1& w,
+                                           unsigned long long* __restrict__ acc, const Geo& g) {
+    constexpr int NC = NF + (HI ? 2 : 0);
+    const int f0 = threadIdx.x % TPC;
+    for (int c = threadIdx.x / TPC; c < w.WH; c += kThreads / TPC) {
+        const int wj = c / w.W, wi = c - wj * w.W;
+        const int cl = wi > 0 ? 1 : 0, cd = wj > 0 ? w.W : 0;    // offsets of the neighbours that exist
+        int n = 0;
+        long long A = 0;
+        for (int r = 0; r < w.rep; ++r) {
+            const int* q = s + NC * P1 + r * w.CS + c;
+            n += q[0];
+            if (cl) n += q[-1];
+            if (cd) n += q[-cd];
+            if (cl && cd) n += q[-cd - 1];
+        }
+        if (n == 0) continue;
+        int gi = w.oi + wi, gj = w.oj + wj;
+        if (gi >= g.nx) gi -= g.nx;
+        if (gj >= g.ny) gj -= g.ny;
+        unsigned long long* a = acc + (static_cast<size_t>(gj) * g.nx + gi);
+        const unsigned nM = static_cast<unsigned>(n) * kMagicU;
+#pragma unroll
+        for (int f = f0; f < NF; f += TPC) {
+            unsigned u = 0;
+            for (int r = 0; r < w.rep; ++r) u += static_cast<unsigned>(s[f * P1 + r * w.CS + c]);
+            long long v;
+            if (HI && f == 0) {
+                for (int r = 0; r < w.rep; ++r) {
+                    const int* h = s + NF * P1 + r * w.CS + c;
+                    A += h[0] & 0xFFFF;
+                    if (cl) A += static_cast<unsigned>(h[-1]) >> 16;
+                    if (cd) A += h[P1 - cd] & 0xFFFF;
+                    if (cl && cd) A += static_cast<unsigned>(h[P1 - cd - 1]) >> 16;
+                }
+                A <<= 19;
+                // sum of q + 2^22: A plus what the fine sum adds modulo 2^32 (less than n 2^19)
+                const unsigned fine = u - static_cast<unsigned>(n) * (kMagicU - 4194304u);
+                v = A + static_cast<long long>(fine - static_cast<unsigned>(A)) - static_cast<long long>(n) * 4194304ll;
+            } else {
+                v = static_cast<int>(u - nM);          // the copies' true sums add up to the chunk's, < 2^31
+            }
+            if (v != 0) atomicAdd(a + static_cast<size_t>(f) * g.ncell, static_cast<unsigned long long>(v));
+        }
+    }
+}
+
+// True (block-uniformly) when some biased field's chunk sum may reach 2^31. Each
+// thread brings the largest of its fields' sums of cs^2 over its m fast
+// particles: sum |cs| + 1 <= sqrt(m l2) + m there (Cauchy), the sum over the
+// threads of the largest bounds every field. `red` is NW ints of scratch; the
+// barrier inside also ends the pass.
+__device__ __forceinline__ bool chunk_overflows1(float l2max, int ppt, int* red) {
+    constexpr int NW = kThreads / 32;
+    const float t = fminf(ceilf(__fmul_ru(__fsqrt_ru(__fmul_ru(l2max, static_cast<float>(ppt))), 1.00001f)), 33554432.0f);
+    const unsigned s = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(t) + static_cast<unsigned>(ppt));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = static_cast<int>(s);
+    __syncthreads();
+    unsigned long long tot = 0;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) tot += static_cast<unsigned>(red[k]);
+    return tot >= 2147483648ull;
+}
+
+// The gather fields of a box, staged from the interleaved [ncell][8] buffer as
+// two planes: float4 (Ex Ey Ez Bx) and float2 (By Bz) of the nI + 1 by nJ + 1
+// cells from (i0, j0), T cells at most. Two planes, because lanes gather from
+// neighbouring cells: 16- and 8-byte strides spread them over the banks.
+struct Tile1 {
+    const float4* a;
+    const float2* b;
+    int i0, j0, W;
+};
+template <int T>
+__device__ __forceinline__ void tile1_load(Tile1& t, float* area, const Box1& bx, const float* __restrict__ gb,
+                                           const Geo& g) {
+    float4* A = reinterpret_cast<float4*>(area);
+    float2* B = reinterpret_cast<float2*>(area + 4 * T);
+    t.a = A; t.b = B; t.i0 = bx.i0; t.j0 = bx.j0; t.W = bx.nI + 1;
+    const int cells = t.W * (bx.nJ + 1);
+    const float4* q = reinterpret_cast<const float4*>(gb);
+    for (int c = threadIdx.x; c < cells; c += kThreads) {
+        const int r = c / t.W;
+        int gi = t.i0 + (c - r * t.W), gj = t.j0 + r;
+        if (gi >= g.nx) gi -= g.nx;
+        if (gj >= g.ny) gj -= g.ny;
+        const size_t k = 2 * (static_cast<size_t>(gj) * g.nx + gi);
+        A[c] = __ldg(q + k);
+        B[c] = __ldg(reinterpret_cast<const float2*>(q + k + 1));
+    }
+}
+__device__ __forceinline__ EB2 tile1_gather(const Tile1& t, const Cic& s, const Geo& g) {
+    int li = s.i0 - t.i0, lj = s.j0 - t.j0;
+    if (li < 0) li += g.nx;
+    if (lj < 0) lj += g.ny;
+    const int c0 = lj * t.W + li, c2 = c0 + t.W;
+    const float4 a[4] = {t.a[c0], t.a[c0 + 1], t.a[c2], t.a[c2 + 1]};
+    const float2 b0 = t.b[c0], b1 = t.b[c0 + 1], b2 = t.b[c2], b3 = t.b[c2 + 1];
+    const float2 W[4] = {bc2(s.w0), bc2(s.w1), bc2(s.w2), bc2(s.w3)};
+    EB2 r;
+    r.exy  = gather4_tile2(W, lo2(a[0]), lo2(a[1]), lo2(a[2]), lo2(a[3]));
+    r.ezbx = gather4_tile2(W, hi2(a[0]), hi2(a[1]), hi2(a[2]), hi2(a[3]));
+    r.byz  = gather4_tile2(W, b0, b1, b2, b3);
+    return r;
+}
+
+// Write stage planes pl[0..np) back to their arrays dst[0..np) for the chunk
 // [c0, c0 + cnt): one bulk shared->global copy per plane for the 16-byte
 // aligned body (issued by thread 0, evict-first), plain stores for the ragged
-// tail and unaligned arrays. The caller has synced after writing the stage;
-// thread 0 must call bulk_store_wait before the block exits.
+// tail and unaligned arrays. Every thread has fenced its stage writes
+// (stage_fence) and synced since; thread 0 must call bulk_store_wait before the
+// block exits.
+__device__ __forceinline__ void stage_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 template <int NP>
 __device__ __forceinline__ void bulk_store_planes(const float* stage, const int (&pl)[NP], float* const (&dst)[NP],
-                                                  long long c0, int cnt, bool vec) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
+                                                  int np, long long c0, int cnt, bool vec) {
     const int nbulk = vec ? (cnt & ~3) : 0;
     if (threadIdx.x == 0 && nbulk > 0) {
         unsigned long long pol;
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
 #pragma unroll
         for (int k = 0; k < NP; ++k)
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;"
-                         :: "l"(dst[k] + c0), "r"(smem_u32(stage + pl[k] * kChunk)),
-                            "r"(static_cast<unsigned>(nbulk) * 4u), "l"(pol) : "memory");
+            if (k < np)
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;"
+                             :: "l"(dst[k] + c0), "r"(smem_u32(stage + pl[k] * kChunk)),
+                                "r"(static_cast<unsigned>(nbulk) * 4u), "l"(pol) : "memory");
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
     const int rem = cnt - nbulk;
     if (rem > 0)
-        for (int idx = threadIdx.x; idx < rem * NP; idx += blockDim.x) {
+        for (int idx = threadIdx.x; idx < rem * np; idx += blockDim.x) {
             const int k = idx / rem, sl = nbulk + idx % rem;
 #pragma unroll
             for (int q = 0; q < NP; ++q)
@@ -625,34 +819,6 @@ __device__ __forceinline__ void slow_pass_linear(const float* __restrict__ stage
     if (n) atomicAdd(&st->slow, static_cast<unsigned long long>(n));
 }
 
-// The NF x 4 contributions of one particle into a single-pass window (plane
-// stride P1): the count of its base cell, field 0 tracked when T0, the others
-// as biased words.
-template <int NF, bool T0, int P1>
-__device__ __forceinline__ void one_pass_deposit(int* __restrict__ win, const Win& w, int di, int dj, float x, float y,
-                                                 const float (&cs)[NF]) {
-    const Cic2 c2 = cic2(x, y);
-    int b[NF][4];
-    quant_bits<NF>(cs, c2, b);
-    int* e0 = win + (threadIdx.x & (w.rep - 1)) * w.CS + dj * w.W + di;   // this lane's copy
-    int* e2 = e0 + w.W;
-    if (NF > (T0 ? 1 : 0)) atomicAdd(e0 + 2 * NF * P1, 1);
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        if (T0 && f == 0) {
-            add_tracked(e0, NF * P1, b[0][0] - kMagicBits);
-            add_tracked(e0 + 1, NF * P1, b[0][1] - kMagicBits);
-            add_tracked(e2, NF * P1, b[0][2] - kMagicBits);
-            add_tracked(e2 + 1, NF * P1, b[0][3] - kMagicBits);
-        } else {
-            atomicAdd(e0 + f * P1, b[f][0]);
-            atomicAdd(e0 + f * P1 + 1, b[f][1]);
-            atomicAdd(e2 + f * P1, b[f][2]);
-            atomicAdd(e2 + f * P1 + 1, b[f][3]);
-        }
-    }
-}
-
 // dcu scales: |coef_dcu (E + v x B)| <= |qm| coef_max (Emax + 2 Umax Bmax); in
 // the fused step the bound per component is also capped at 8 x the rms the
 // previous step's dcu coefficients had.
@@ -674,8 +840,10 @@ __device__ __forceinline__ void dcu_scales(const DevState* st, float abs_qm, boo
 // dcu deposit: input x y w ux uy uz; stage = x, y, ax, ay, az (scaled coefficients).
 struct DcuArgs {
     Parts p; Geo g; double qm2oa; float abs_qm; const float* gb; unsigned long long* acc; int wmaxc;
-    DevState* st; int use_rms; float* psq; int use_tile; int one_pass;
+    DevState* st; int use_rms; float* psq; int use_tile; int one_pass; int rep_need;
 };
+// FULL: chunks of kChunk particles (the trip counts are compile-time constants).
+template <bool FULL>
 __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int chunk) {
     const Parts& p = A.p; const Geo& g = A.g;
     const double qm2oa = A.qm2oa; const float abs_qm = A.abs_qm;
@@ -690,8 +858,11 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     __shared__ int nlist;
     __shared__ float ssq[(NF + 1) * (kThreads / 32)];
 
-    const long long c0 = static_cast<long long>(chunk) * kChunk;
-    const int cnt = static_cast<int>(min(static_cast<long long>(kChunk), p.n - c0));
+    const int cs_ = FULL ? kChunk : p.cs;
+    const long long c0 = static_cast<long long>(chunk) * cs_;
+    const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
+    const int ppt = cs_ / kThreads;               // particles per thread
+    const Spread sp(cs_);
     float S[3];
     dcu_scales(st, abs_qm, use_rms != 0, S);
     if (chunk == 0 && threadIdx.x == 0) { st->S_dcu[0] = S[0]; st->S_dcu[1] = S[1]; st->S_dcu[2] = S[2]; }
@@ -702,64 +873,66 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     int ir, jr;
     ref_of(x0, y0, g, ir, jr);
 
-    // ---- single pass when the window fits: the particles do not move, so the
-    // window is the box of their base cells plus the corner - the gather tile's box
-    constexpr int P1 = 352, kTileCap1 = (PC - P1) * win_planes(NF) / 8;
-    static_assert(kTileCap1 >= P1, "the tile of a single-pass window must fit beside it");
+    // ---- single pass: the particles do not move, so the window is the box of
+    // their base cells plus the corner - the gather tile's box
     if (A.one_pass) {
-        BBox cb;
-#pragma unroll 4
-        for (int it = 0; it < kPPT; ++it) {
-            const int sl = it * kThreads + threadIdx.x;
-            const float x = m.stage[sl], y = m.stage[kChunk + sl];
-            if (sl < cnt && in_grid(x, y, g)) cb.add(static_cast<int>(x), static_cast<int>(y), ir, jr, g);
-        }
-        const Box bx = box_reduce(cb, m.red);
-        Win w1;
-        if (A.one_pass && one_pass_window<NF, T0, P1>(w1, bx, ir, jr, 0, g)) {
-            float* const tile1 = reinterpret_cast<float*>(m.win + P1 * win_planes(NF));
-            const Tile tl = box_tile(bx, ir, jr, g, kTileCap1);
-            if (tl.use && !load_tile8(tile1, gb, tl, g, &tbar, st)) return;
-            win_zero<NF, T0, P1>(m.win, w1);
+        constexpr int P1 = 640, T1 = ((PC * win_planes(NF) - P1 * (NF + 1)) / 6) & ~3;     // 24 bytes per tile cell
+        Box1 bx;
+        Win1 w1;
+        if (chunk_box(m.stage, cs_, cnt, x0, y0, g, m.red, T1, 0, bx) && window1<P1>(w1, bx, 0, A.rep_need, g) &&
+            (bx.nI + 1) * (bx.nJ + 1) <= T1) {
+            Tile1 tl;
+            tile1_load<T1>(tl, reinterpret_cast<float*>(m.win + P1 * (NF + 1)), bx, gb, g);
+            win1_zero<NF + 1, P1>(m.win, w1);
             __syncthreads();
-            const int oi = win_origin(ir, w1.mi, g.nx), oj = win_origin(jr, w1.mj, g.ny);
-            float l1[NF] = {}, sq[NF] = {};
-            float nval = 0.f;
-#pragma unroll 1
-            for (int k = 0; k < kPPT; ++k) {
-                const int sl = spread_slot(k);
-                if (sl >= cnt) continue;
-                const float x = m.stage[sl], y = m.stage[kChunk + sl];
-                if (!in_grid(x, y, g)) { set_err(st, AW_DEV_OUT_OF_GRID); continue; }
+            // slot sl's coefficients (unscaled)
+            auto coefs = [&](int sl, float x, float y, const Cic& c, float (&cf)[NF]) {
                 const float w = m.stage[2 * kChunk + sl];
                 const float vx = m.stage[3 * kChunk + sl], vy = m.stage[4 * kChunk + sl], vz = m.stage[5 * kChunk + sl];
-                const Cic c = cic(x, y);
-                const EB2 eb = tl.use ? gather_em_tile2(tile1, c, win_col(c.i0, tl.i0, g.nx), win_col(c.j0, tl.j0, g.ny), tl.W)
-                                      : gather_em2(gb, c, g);
+                const EB2 eb = tile1_gather(tl, c, g);
                 const float bxf = eb.ezbx.y, by = eb.byz.x, bz = eb.byz.y;
                 const float coef = __double2float_rn(qm2oa * static_cast<double>(w));
+                // v x B: (cx, cy) = (vy bz - vz by, vz bx - vx bz) paired, cz = vx by - vy bx
                 const float2 nxy = __fmul2_rn(make_float2(vz, vx), make_float2(-by, -bz));
                 const float2 cxy = __ffma2_rn(make_float2(vy, vz), make_float2(bz, bxf), nxy);
                 const float cz = __fmaf_rn(vx, by, -__fmul_rn(vy, bxf));
                 const float2 cfxy = __fmul2_rn(bc2(coef), __fadd2_rn(eb.exy, cxy));
-                const float cf[NF] = {cfxy.x, cfxy.y, __fmul_rn(coef, __fadd_rn(eb.ezbx.x, cz))};
-                float cs[NF];
-                const bool fast = scale_fast<NF>(cf, S, cs, l1);
+                cf[0] = cfxy.x; cf[1] = cfxy.y; cf[2] = __fmul_rn(coef, __fadd_rn(eb.ezbx.x, cz));
+            };
+            float l2[NF] = {}, sq[NF] = {};
+            float nval = 0.f;
+#pragma unroll 1
+            for (int k = 0; k < ppt; ++k) {
+                const int sl = sp.slot(k);
+                if (sl >= cnt) continue;
+                const float x = m.stage[sl], y = m.stage[kChunk + sl];
+                const Cic c = cic(x, y);
+                float cf[NF], cs[NF];
+                coefs(sl, x, y, c, cf);
+#pragma unroll
+                for (int f = 0; f < NF; ++f) cs[f] = __fmul_rn(cf[f], S[f]);
                 if (((c.i0 + c.j0) & 7) == 0) {   // rms sample: the particles of one cell in 8, any order
 #pragma unroll
                     for (int f = 0; f < NF; ++f) sq[f] = __fmaf_rn(cf[f], cf[f], sq[f]);
                     nval += 1.0f;
                 }
-                // the scaled coefficients replace w, vx, vy in the stage for the slow path
-                m.stage[2 * kChunk + sl] = cs[0]; m.stage[3 * kChunk + sl] = cs[1]; m.stage[4 * kChunk + sl] = cs[2];
-                const int di = win_col(c.i0, oi, g.nx), dj = win_col(c.j0, oj, g.ny);
-                if (fast && di <= w1.W - 2 && dj <= w1.H - 2) one_pass_deposit<NF, T0, P1>(m.win, w1, di, dj, x, y, cs);
-                else list_slow(m.slow, &nlist, sl);
+                // (a NaN fails the test: fmaxf would drop it)
+                if (fabsf(cs[0]) < kFastLim && fabsf(cs[1]) < kFastLim && fabsf(cs[2]) < kFastLim) {
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) l2[f] = __fmaf_rn(cs[f], cs[f], l2[f]);
+                    win1_add<NF, false, P1>(m.win, w1, win_col(c.i0, w1.oi, g.nx), win_col(c.j0, w1.oj, g.ny), x, y, cs);
+                } else {
+                    list_slow(m.slow, &nlist, sl);
+                }
             }
-            const bool redo = chunk_overflows<NF, T0>(l1, m.red);     // (its barrier also ends the pass)
-            if (!redo) win_flush<NF, T0, P1>(m.win, w1, acc, g);
+            const bool redo = chunk_overflows1(fmaxf(l2[0], fmaxf(l2[1], l2[2])), ppt, m.red);   // (its barrier ends the pass)
+            if (!redo) win1_flush<NF, false, P1, 4>(m.win, w1, acc, g);
             slow_pass_linear<NF>(m.stage, m.slow, nlist, redo, cnt, acc, g, st, [&](int sl, float (&cs)[NF]) {
-                cs[0] = m.stage[2 * kChunk + sl]; cs[1] = m.stage[3 * kChunk + sl]; cs[2] = m.stage[4 * kChunk + sl];
+                float cf[NF];
+                const float x = m.stage[sl], y = m.stage[kChunk + sl];
+                coefs(sl, x, y, cic(x, y), cf);
+#pragma unroll
+                for (int f = 0; f < NF; ++f) cs[f] = __fmul_rn(cf[f], S[f]);
             });
             if (threadIdx.x == 0) {
                 atomicAdd(&st->chunks, 1ull);
@@ -769,6 +942,7 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
             if (psq) block_sumsq<NF>(sq, nval, psq, ssq, chunk);
             return;
         }
+        __syncthreads();           // the box scratch has been read
     }
 
     // ---- two passes --------------------------------------------------------
@@ -777,7 +951,7 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     if (A.use_tile) {
         float xmin = 3.0e38f, xmax = -1.0f, ymin = 3.0e38f, ymax = -1.0f;
 #pragma unroll 4
-        for (int it = 0; it < kPPT; ++it) {
+        for (int it = 0; it < ppt; ++it) {
             const int s = it * kThreads + threadIdx.x;
             const float x = m.stage[s], y = m.stage[kChunk + s];
             if (s < cnt && in_grid(x, y, g)) {
@@ -797,7 +971,7 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     BBox bb;
     float l1[NF] = {};
 #pragma unroll 2
-    for (int it = 0; it < kPPT; ++it) {
+    for (int it = 0; it < ppt; ++it) {
         const int s = it * kThreads + threadIdx.x;
         const float x = m.stage[s], y = m.stage[kChunk + s], w = m.stage[2 * kChunk + s];
         const float vx = m.stage[3 * kChunk + s], vy = m.stage[4 * kChunk + s], vz = m.stage[5 * kChunk + s];
@@ -850,22 +1024,23 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
         }
     };
     if (wn.use && wn.nb == 1) {
-        if (wn.track_all) window_particles<NF, NS, T0, true, PC>(m.stage, m.win, wn, g, coef, stats);
-        else window_particles<NF, NS, T0, false, PC>(m.stage, m.win, wn, g, coef, stats);
+        if (wn.track_all) window_particles<NF, NS, T0, true, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
+        else window_particles<NF, NS, T0, false, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
     } else {
 #pragma unroll 1
-        for (int k = 0; k < kPPT; ++k) {
-            const int d = spread_slot(k);
+        for (int k = 0; k < ppt; ++k) {
+            const int d = sp.slot(k);
             float a[NS];
 #pragma unroll
             for (int f = 0; f < NS; ++f) a[f] = m.stage[f * kChunk + d];
             stats(a);
         }
-        window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, g, coef, acc);   // bands (or the slow path alone)
+        window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);   // bands (or the slow path alone)
     }
-    close_window<NF, NS, T0, PC>(m, wn, nlist, acc, g, st, coef);
+    close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
     if (psq) block_sumsq<NF>(sq, nval, psq, ssq, chunk);}
-__global__ void __launch_bounds__(kThreads, 3) k_deposit_dcu(DcuArgs A) { deposit_dcu_chunk(A, blockIdx.x); }
+template <bool FULL>
+__global__ void __launch_bounds__(kThreads, 3) k_deposit_dcu(DcuArgs A) { deposit_dcu_chunk<FULL>(A, blockIdx.x); }
 
 // ---------------------------------------------------------------------------
 // Backward step A of the ES adjoint (the transpose of k_push_deposit_es's push
@@ -897,8 +1072,9 @@ k_adj_scatter(AdjP a, Geo g, AdjK k, const float2* __restrict__ trajE, AdjDev* a
     __shared__ unsigned long long bar;
     __shared__ int nlist;
 
-    const long long c0 = static_cast<long long>(blockIdx.x) * kChunk;
-    const int cnt = static_cast<int>(min(static_cast<long long>(kChunk), a.n - c0));
+    const long long c0 = static_cast<long long>(blockIdx.x) * a.cs;
+    const int cnt = static_cast<int>(min(static_cast<long long>(a.cs), a.n - c0));
+    const int ppt = a.cs / kThreads;               // particles per thread
     const int slot = ad->slot;
     const float* xn = a.traj + static_cast<size_t>(slot) * 2 * a.n;
     const float2* __restrict__ E = trajE + static_cast<size_t>(slot) * g.ncell;
@@ -916,7 +1092,7 @@ k_adj_scatter(AdjP a, Geo g, AdjK k, const float2* __restrict__ trajE, AdjDev* a
     BBox bb;
     float l1[NF] = {};
 #pragma unroll 1
-    for (int it = 0; it < kPPT; ++it) {
+    for (int it = 0; it < ppt; ++it) {
         const int s = it * kThreads + threadIdx.x;
         const long long i = c0 + s;
         const float x = m.stage[s], y = m.stage[kChunk + s];
@@ -966,8 +1142,8 @@ k_adj_scatter(AdjP a, Geo g, AdjK k, const float2* __restrict__ trajE, AdjDev* a
     }
     const Win wn = open_window<NF, T0, PC>(bb, ir, jr, wmaxc, m, l1);
     auto coef = [&](const float (&q)[NS], float (&c2)[NF]) { c2[0] = q[2]; c2[1] = q[3]; };
-    window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, g, coef, acc);
-    close_window<NF, NS, T0, PC>(m, wn, nlist, acc, g, st, coef);
+    window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, a.cs, g, coef, acc);
+    close_window<NF, NS, T0, PC>(m, wn, nlist, a.cs, acc, g, st, coef);
 }
 
 // ---------------------------------------------------------------------------
@@ -991,13 +1167,30 @@ __device__ __forceinline__ void move_xy(float& x, float& y, float ux, float uy, 
     }
 }
 
+// Move and wrap; true when the new position is in the grid. A particle that stays
+// between the edges needs no wrap (wrap_pos would return it unchanged).
+template <bool POW2>
+__device__ __forceinline__ bool step_xy(float& x, float& y, float ux, float uy, const PushP& pp, const Geo& g) {
+    if constexpr (POW2) {
+        x = move1_pow2(x, ux, pp.dtx);
+        y = move1_pow2(y, uy, pp.dty);
+    } else {
+        x = move1(x, ux, pp.dt, g.dx);
+        y = move1(y, uy, pp.dt, g.dy);
+    }
+    if (in_grid(x, y, g)) return true;
+    x = wrap_pos(x, g.nxf);
+    y = wrap_pos(y, g.nyf);
+    return in_grid(x, y, g);
+}
+
 // Fused ES step kernel: input x y w ux uy uz; stage = new x, y, coefficient q w / (dx dy).
 struct EsArgs {
     Parts p; Geo g; PushP pp; const float* gb; double qoa; unsigned long long* acc; int wmaxc;
     double* part; DevState* st;
     float* traj; const AdjDev* rec;   // trajectory recording (x_n, y_n into slot rec->rec_slot), or null
 };
-template <bool POW2, bool RECORD = false>
+template <bool POW2, bool FULL, bool RECORD = false>
 __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int chunk) {
     const Parts& p = A.p; const Geo& g = A.g; const PushP& pp = A.pp;
     const float* __restrict__ gb = A.gb; const double qoa = A.qoa; unsigned long long* __restrict__ acc = A.acc;
@@ -1010,8 +1203,10 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     __shared__ int nlist;
     __shared__ double dsh[4 * (kThreads / 32)];
 
-    const long long c0 = static_cast<long long>(chunk) * kChunk;
-    const int cnt = static_cast<int>(min(static_cast<long long>(kChunk), p.n - c0));
+    const int cs_ = FULL ? kChunk : p.cs;
+    const long long c0 = static_cast<long long>(chunk) * cs_;
+    const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
+    const int ppt = cs_ / kThreads;               // particles per thread
     const float S1[1] = {st->S_next[0]};
     if (threadIdx.x == 0) nlist = 0;
     const ChunkSrc src{{p.x, p.y, p.ux, p.uy, p.uz, nullptr}};
@@ -1026,7 +1221,7 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     float l1[NF] = {};
     double ke = 0, px = 0, py = 0, pz = 0;
 #pragma unroll 2
-    for (int it = 0; it < kPPT; ++it) {
+    for (int it = 0; it < ppt; ++it) {
         const int s = it * kThreads + threadIdx.x;
         const long long i = c0 + s;
         float x = m.stage[s], y = m.stage[kChunk + s];
@@ -1085,24 +1280,24 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     auto coef = [&](const float (&a)[NS], float (&cs)[NF]) {
         cs[0] = __fmul_rn(a[2], S1[0]);
     };
-    window_pass<NF, NS, T0>(m.stage, m.win, wn, g, coef, acc);
-    close_window<NF, NS, T0>(m, wn, nlist, acc, g, st, coef);
+    window_pass<NF, NS, T0>(m.stage, m.win, wn, cs_, g, coef, acc);
+    close_window<NF, NS, T0>(m, wn, nlist, cs_, acc, g, st, coef);
     block_sum4(ke, px, py, pz, part, dsh, chunk);
     if (threadIdx.x == 0 && chunk == 0) {
         st->S_pend[0] = S1[0];
         st->step += 1;
     }}
-template <bool POW2, bool RECORD>
+template <bool POW2, bool FULL, bool RECORD>
 __global__ void __launch_bounds__(kThreads, 4) k_push_deposit_es(EsArgs A) {
-    push_deposit_es_chunk<POW2, RECORD>(A, blockIdx.x);
+    push_deposit_es_chunk<POW2, FULL, RECORD>(A, blockIdx.x);
 }
 
 // Fused Darwin step kernel: input x y w ux uy uz; stage = new x, y, coefficient, ux, uy, uz.
 struct EmArgs {
     Parts p; Geo g; PushP pp; const float* gb; double qoa; unsigned long long* acc; int wmaxc;
-    double* part; DevState* st; float* psq; int use_tile; int one_pass;
+    double* part; DevState* st; float* psq; int use_tile; int one_pass; int rep_need;
 };
-template <bool POW2>
+template <bool POW2, bool FULL>
 __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int chunk) {
     const Parts& p = A.p; const Geo& g = A.g; const PushP& pp = A.pp;
     const float* __restrict__ gb = A.gb; const double qoa = A.qoa; unsigned long long* __restrict__ acc = A.acc;
@@ -1119,8 +1314,11 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     __shared__ unsigned umx[3][kThreads / 32];
     __shared__ float ssq[(NF + 1) * (kThreads / 32)];
 
-    const long long c0 = static_cast<long long>(chunk) * kChunk;
-    const int cnt = static_cast<int>(min(static_cast<long long>(kChunk), p.n - c0));
+    const int cs_ = FULL ? kChunk : p.cs;
+    const long long c0 = static_cast<long long>(chunk) * cs_;
+    const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
+    const int ppt = cs_ / kThreads;               // particles per thread
+    const Spread sp(cs_);
     float S[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) S[f] = st->S_next[f];
@@ -1133,78 +1331,77 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     int ir, jr;
     ref_of(x0, y0, g, ir, jr);
 
-    // ---- single pass when the window fits ----------------------------------
-    // Window planes of stride P1 (window capacity P1 cells), the gather tile after them.
-    constexpr int P1 = 288, kTileCap1 = (PC - P1) * win_planes(NF) / 8;
+    // ---- single pass -------------------------------------------------------
     if (A.one_pass) {
-        BBox cb;
-#pragma unroll 4
-        for (int it = 0; it < kPPT; ++it) {
-            const int sl = it * kThreads + threadIdx.x;
-            const float x = m.stage[sl], y = m.stage[kChunk + sl];
-            if (sl < cnt && in_grid(x, y, g)) cb.add(static_cast<int>(x), static_cast<int>(y), ir, jr, g);
-        }
-        const Box bx = box_reduce(cb, m.red);
+        constexpr int P1 = 384, T1 = ((PC * win_planes(NF) - P1 * (NF + 3)) / 6) & ~3;     // 24 bytes per tile cell
         // the cells a particle can cross in one step: twice the largest in-plane |u| of
         // the current state times dt/dx (one further cell for the rounding)
         const float uxy_max = fmaxf(__uint_as_float(st->ucur_bits[0]), __uint_as_float(st->ucur_bits[1]));
         const float dmv = __fmul_rn(2.0f * uxy_max, static_cast<float>(fmax(pp.dtx, pp.dty)));
         const int mg = (dmv >= 0.0f && dmv < 8.0f) ? 1 + static_cast<int>(dmv) : -1;
-        Win w1;
-        if (A.one_pass && mg > 0 && one_pass_window<NF, T0, P1>(w1, bx, ir, jr, mg, g)) {
-            float* const tile1 = reinterpret_cast<float*>(m.win + P1 * win_planes(NF));
-            const Tile tl = box_tile(bx, ir, jr, g, kTileCap1);
-            if (tl.use && !load_tile8(tile1, gb, tl, g, &tbar, st)) return;
-            win_zero<NF, T0, P1>(m.win, w1);
+        Box1 bx;
+        Win1 w1;
+        if (mg > 0 && chunk_box(m.stage, cs_, cnt, x0, y0, g, m.red, P1, mg, bx) &&
+            window1<P1>(w1, bx, mg, A.rep_need, g) && (bx.nI + 1) * (bx.nJ + 1) <= T1) {
+            Tile1 tl;
+            tile1_load<T1>(tl, reinterpret_cast<float*>(m.win + P1 * (NF + 3)), bx, gb, g);
+            win1_zero<NF + 3, P1>(m.win, w1);
             __syncthreads();
-            const int oi = win_origin(ir, w1.mi, g.nx), oj = win_origin(jr, w1.mj, g.ny);
-            float2 l1p[4] = {}, sqp[4] = {};
+            const bool cells = pp.write_cell && p.cell;
+            float2 l2p[4] = {}, sqp[4] = {};
             double ke = 0, px = 0, py = 0, pz = 0;
             float m0 = 0.f, m1 = 0.f, m2 = 0.f, nval = 0.f;
 #pragma unroll 1
-            for (int k = 0; k < kPPT; ++k) {
-                const int sl = spread_slot(k);
+            for (int k = 0; k < ppt; ++k) {
+                const int sl = sp.slot(k);
                 if (sl >= cnt) continue;
                 float x = m.stage[sl], y = m.stage[kChunk + sl];
-                if (!in_grid(x, y, g)) { set_err(st, AW_DEV_OUT_OF_GRID); continue; }
                 const float w = m.stage[2 * kChunk + sl];
-                float ux = m.stage[3 * kChunk + sl], uy = m.stage[4 * kChunk + sl], uz = m.stage[5 * kChunk + sl];
-                const Cic c = cic(x, y);
-                const EB2 eb = tl.use ? gather_em_tile2(tile1, c, win_col(c.i0, tl.i0, g.nx), win_col(c.j0, tl.j0, g.ny), tl.W)
-                                      : gather_em2(gb, c, g);
-                float2 uxy = make_float2(ux, uy);
-                boris_em2(uxy, uz, eb.exy, eb.ezbx.x, eb.ezbx.y, eb.byz, pp.qmh);
-                ux = uxy.x; uy = uxy.y;
-                move_xy<POW2>(x, y, ux, uy, pp, g);
-                int ci, cj;
-                cell_ij(x, y, g, ci, cj);
+                float2 uxy = make_float2(m.stage[3 * kChunk + sl], m.stage[4 * kChunk + sl]);
+                float uz = m.stage[5 * kChunk + sl];
+                {
+                    const EB2 eb = tile1_gather(tl, cic(x, y), g);
+                    boris_em2(uxy, uz, eb.exy, eb.ezbx.x, eb.ezbx.y, eb.byz, pp.qmh);
+                }
+                const float ux = uxy.x, uy = uxy.y;
+                bool ok = step_xy<POW2>(x, y, ux, uy, pp, g);
+                const double dw = w, du = ux, dv = uy, dz = uz;
+                ke += dw * (du * du + dv * dv + dz * dz);
+                px += dw * du; py += dw * dv; pz += dw * dz;
                 m.stage[sl] = x; m.stage[kChunk + sl] = y;
                 m.stage[3 * kChunk + sl] = ux; m.stage[4 * kChunk + sl] = uy; m.stage[5 * kChunk + sl] = uz;
                 m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy)); m2 = fmaxf(m2, fabsf(uz));
-                if (in_grid(x, y, g)) {
+                int cell;
+                if (ok) {
+                    const int ci = static_cast<int>(x), cj = static_cast<int>(y);
+                    cell = cj * g.nx + ci;
                     float2 cp[4], csp[4];
-                    const float cf0 = __double2float_rn(qoa * static_cast<double>(w));
-                    src_coefs8(cf0, ux, uy, uz, cp);
-                    const bool fast = scale_fast2<4>(cp, Sp, csp, l1p);
+                    src_coefs8(__double2float_rn(qoa * dw), ux, uy, uz, cp);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) csp[i] = __fmul2_rn(cp[i], Sp[i]);
                     if (((ci + cj) & 7) == 0) {   // rms sample: the particles of one cell in 8, any order
 #pragma unroll
                         for (int i = 0; i < 4; ++i) sqp[i] = __ffma2_rn(cp[i], cp[i], sqp[i]);
                         nval += 1.0f;
                     }
-                    const int di = win_col(ci, oi, g.nx), dj = win_col(cj, oj, g.ny);
+                    bool fast = true;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) fast = fast && fabsf(csp[i].x) < kFastLim && fabsf(csp[i].y) < kFastLim;
+                    const int di = win_col(ci, w1.oi, g.nx), dj = win_col(cj, w1.oj, g.ny);
                     if (fast && di <= w1.W - 2 && dj <= w1.H - 2) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) l2p[i] = __ffma2_rn(csp[i], csp[i], l2p[i]);
                         const float cs[NF] = {csp[0].x, csp[0].y, csp[1].x, csp[1].y,
                                               csp[2].x, csp[2].y, csp[3].x, csp[3].y};
-                        one_pass_deposit<NF, T0, P1>(m.win, w1, di, dj, x, y, cs);
+                        win1_add<NF, true, P1>(m.win, w1, di, dj, x, y, cs);
                     } else {
                         list_slow(m.slow, &nlist, sl);
                     }
                 } else {
                     set_err(st, AW_DEV_OUT_OF_GRID);
+                    cell = cells ? p.cell[c0 + sl] : 0;          // stays as it is
                 }
-                const double dw = w, du = ux, dv = uy, dz = uz;
-                ke += dw * (du * du + dv * dv + dz * dz);
-                px += dw * du; py += dw * dv; pz += dw * dz;
+                m.stage[2 * kChunk + sl] = __int_as_float(cell);  // w is read again from the caller's array
             }
             m0 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m0)));
             m1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m1)));
@@ -1214,32 +1411,19 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
                 umx[1][threadIdx.x >> 5] = __float_as_uint(m1);
                 umx[2][threadIdx.x >> 5] = __float_as_uint(m2);
             }
-            // the new state leaves by bulk copy (x y ux uy uz: stage planes 0 1 3 4 5)
-            const int pl[5] = {0, 1, 3, 4, 5};
-            float* const dst[5] = {p.x, p.y, p.ux, p.uy, p.uz};
-            bulk_store_planes<5>(m.stage, pl, dst, c0, cnt, p.vec_ok != 0);
-            if (pp.write_cell && p.cell)      // the owning cells, coalesced, from the staged new positions
-                for (int sl = threadIdx.x; sl < cnt; sl += kThreads) {
-                    const float x = m.stage[sl], y = m.stage[kChunk + sl];
-                    if (in_grid(x, y, g)) {
-                        int ci, cj;
-                        cell_ij(x, y, g, ci, cj);
-                        __stcs(p.cell + c0 + sl, cj * g.nx + ci);
-                    }
-                }
-            if (threadIdx.x < 3) {
-                unsigned mx = 0;
-                for (int k = 0; k < kThreads / 32; ++k) mx = max(mx, umx[threadIdx.x][k]);
-                atomicMax(&st->umax_bits[threadIdx.x], mx);
-            }
-            float l1[NF], sq[NF];
+            stage_fence();
+            float l2m = l2p[0].y;                                // field 0 is carried exactly (coarse planes)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { l1[2 * i] = l1p[i].x; l1[2 * i + 1] = l1p[i].y; sq[2 * i] = sqp[i].x; sq[2 * i + 1] = sqp[i].y; }
-            const bool redo = chunk_overflows<NF, T0>(l1, m.red);
-            if (!redo) win_flush<NF, T0, P1>(m.win, w1, acc, g);
+            for (int i = 1; i < 4; ++i) l2m = fmaxf(l2m, fmaxf(l2p[i].x, l2p[i].y));
+            const bool redo = chunk_overflows1(l2m, ppt, m.red);    // (its barrier ends the pass)
+            // the new state leaves by bulk copy (x y ux uy uz and the cells: stage planes 0 1 3 4 5 2)
+            const int pl[6] = {0, 1, 3, 4, 5, 2};
+            float* const dst[6] = {p.x, p.y, p.ux, p.uy, p.uz, reinterpret_cast<float*>(p.cell)};
+            bulk_store_planes<6>(m.stage, pl, dst, cells ? 6 : 5, c0, cnt, p.vec_ok != 0);
+            if (!redo) win1_flush<NF, true, P1, 4>(m.win, w1, acc, g);
             slow_pass_linear<NF>(m.stage, m.slow, nlist, redo, cnt, acc, g, st, [&](int sl, float (&cs)[NF]) {
                 float2 cp[4];
-                src_coefs8(__double2float_rn(qoa * static_cast<double>(m.stage[2 * kChunk + sl])),
+                src_coefs8(__double2float_rn(qoa * static_cast<double>(p.w[c0 + sl])),
                            m.stage[3 * kChunk + sl], m.stage[4 * kChunk + sl], m.stage[5 * kChunk + sl], cp);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -1247,11 +1431,17 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
                     cs[2 * i] = cc.x; cs[2 * i + 1] = cc.y;
                 }
             });
+            if (threadIdx.x < 3) {
+                unsigned mx = 0;
+                for (int k = 0; k < kThreads / 32; ++k) mx = max(mx, umx[threadIdx.x][k]);
+                atomicMax(&st->umax_bits[threadIdx.x], mx);
+            }
             if (threadIdx.x == 0) {
                 atomicAdd(&st->chunks, 1ull);
                 atomicAdd(&st->one_pass, 1ull);
                 if (redo) atomicAdd(&st->overflow, 1ull);
             }
+            const float sq[NF] = {sqp[0].x, sqp[0].y, sqp[1].x, sqp[1].y, sqp[2].x, sqp[2].y, sqp[3].x, sqp[3].y};
             block_sumsq<NF>(sq, nval, psq, ssq, chunk);
             block_sum4(ke, px, py, pz, part, dsh, chunk);
             if (threadIdx.x == 0 && chunk == 0) {
@@ -1262,6 +1452,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
             bulk_store_wait();
             return;
         }
+        __syncthreads();           // the box scratch has been read
     }
 
     // ---- two passes --------------------------------------------------------
@@ -1278,7 +1469,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     if (A.use_tile) {
         float xmin = 3.0e38f, xmax = -1.0f, ymin = 3.0e38f, ymax = -1.0f;
 #pragma unroll 4
-        for (int it = 0; it < kPPT; ++it) {
+        for (int it = 0; it < ppt; ++it) {
             const int s = it * kThreads + threadIdx.x;
             const float x = m.stage[s], y = m.stage[kChunk + s];
             if (s < cnt && in_grid(x, y, g)) {
@@ -1295,7 +1486,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     float2 l1p[4] = {};
     float m0 = 0.f, m1 = 0.f, m2 = 0.f;
 #pragma unroll 2
-    for (int it = 0; it < kPPT; ++it) {
+    for (int it = 0; it < ppt; ++it) {
         const int s = it * kThreads + threadIdx.x;
         const long long i = c0 + s;
         float x = m.stage[s], y = m.stage[kChunk + s];
@@ -1390,20 +1581,20 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
         }
     };
     if (wn.use && wn.nb == 1) {
-        if (wn.track_all) window_particles<NF, NS, T0, true, PC>(m.stage, m.win, wn, g, coef, stats);
-        else window_particles<NF, NS, T0, false, PC>(m.stage, m.win, wn, g, coef, stats);
+        if (wn.track_all) window_particles<NF, NS, T0, true, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
+        else window_particles<NF, NS, T0, false, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
     } else {
 #pragma unroll 1
-        for (int k = 0; k < kPPT; ++k) {
-            const int d = spread_slot(k);
+        for (int k = 0; k < ppt; ++k) {
+            const int d = sp.slot(k);
             float a[NS];
 #pragma unroll
             for (int f = 0; f < NS; ++f) a[f] = m.stage[f * kChunk + d];
             stats(a);
         }
-        window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, g, coef, acc);   // bands (or the slow path alone)
+        window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);   // bands (or the slow path alone)
     }
-    close_window<NF, NS, T0, PC>(m, wn, nlist, acc, g, st, coef);
+    close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
     float sq[NF];
 #pragma unroll
     for (int i = 0; i < 4; ++i) { sq[2 * i] = sqp[i].x; sq[2 * i + 1] = sqp[i].y; }
@@ -1414,8 +1605,10 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
         for (int f = 0; f < NF; ++f) st->S_pend[f] = S[f];
         st->step += 1;
     }}
-template <bool POW2>
-__global__ void __launch_bounds__(kThreads, 3) k_push_deposit_em(EmArgs A) { push_deposit_em_chunk<POW2>(A, blockIdx.x); }
+template <bool POW2, bool FULL>
+__global__ void __launch_bounds__(kThreads, 3) k_push_deposit_em(EmArgs A) {
+    push_deposit_em_chunk<POW2, FULL>(A, blockIdx.x);
+}
 
 // ---------------------------------------------------------------------------
 // Multi-run launches (batched ensembles): one grid over the chunks of several
@@ -1437,7 +1630,7 @@ k_deposit_dcu_multi(const DcuArgs* __restrict__ runs, const int* __restrict__ fi
     __shared__ int chunk;
     if (threadIdx.x == 0) { const int r = find_run(first, nruns); A = runs[r]; chunk = blockIdx.x - first[r]; }
     __syncthreads();
-    deposit_dcu_chunk(A, chunk);
+    deposit_dcu_chunk<false>(A, chunk);
 }
 template <bool POW2>
 __global__ void __launch_bounds__(kThreads, 4)
@@ -1446,7 +1639,7 @@ k_push_deposit_es_multi(const EsArgs* __restrict__ runs, const int* __restrict__
     __shared__ int chunk;
     if (threadIdx.x == 0) { const int r = find_run(first, nruns); A = runs[r]; chunk = blockIdx.x - first[r]; }
     __syncthreads();
-    push_deposit_es_chunk<POW2>(A, chunk);
+    push_deposit_es_chunk<POW2, false>(A, chunk);
 }
 template <bool POW2>
 __global__ void __launch_bounds__(kThreads, 3)
@@ -1455,10 +1648,11 @@ k_push_deposit_em_multi(const EmArgs* __restrict__ runs, const int* __restrict__
     __shared__ int chunk;
     if (threadIdx.x == 0) { const int r = find_run(first, nruns); A = runs[r]; chunk = blockIdx.x - first[r]; }
     __syncthreads();
-    push_deposit_em_chunk<POW2>(A, chunk);
+    push_deposit_em_chunk<POW2, false>(A, chunk);
 }
 
-inline int nchunks(long long n) { return static_cast<int>(std::max<long long>(1, (n + kChunk - 1) / kChunk)); }
+inline int nchunks(long long n, int cs) { return static_cast<int>(std::max<long long>(1, (n + cs - 1) / cs)); }
+inline int nchunks(const Parts& p) { return nchunks(p.n, p.cs); }
 
 // Opt a kernel into its dynamic shared-memory size (never inside a stream
 // capture: aw_init launches every kernel before any capture). The attribute
@@ -1473,9 +1667,10 @@ template <int SET>
 void launch_src(Ctx& c, unsigned long long* acc) {
     constexpr int NF = SetNF<SET>::NF, NS = SetNF<SET>::NS;
     const size_t sh = smem_bytes(NF, NS);
-    prep_smem(k_deposit_src<SET>, sh);
+    auto kern = c.parts.cs == kChunk ? k_deposit_src<SET, true> : k_deposit_src<SET, false>;
+    prep_smem(kern, sh);
     const double qoa = c.prm.qm / (c.geo.dx * c.geo.dy);
-    k_deposit_src<SET><<<nchunks(c.parts.n), kThreads, sh, c.stream>>>(c.parts, c.geo, qoa, c.st->S_pend, acc,
+    kern<<<nchunks(c.parts), kThreads, sh, c.stream>>>(c.parts, c.geo, qoa, c.st->S_pend, acc,
                                                                         wmax_cells(NF), c.st,
                                                                         SET == SET_ALL ? c.part_c : nullptr);
     AW_LAUNCH();
@@ -1505,12 +1700,16 @@ PushP push_params(const Ctx& c) {
 bool use_tile(const Ctx& c) {
     return c.plan.tile >= 0 ? c.plan.tile != 0 : c.parts.n <= 128LL * c.geo.ncell;
 }
-// The single pass pays where chunks are dense (few cells, the spread lanes of the
-// deposit share cells anyway); where a chunk spans many cells the two-pass
-// kernels gather with lanes on neighbouring particles, which read the same tile
-// cells.
-bool one_pass(const Ctx& c) {
-    return c.plan.one_pass >= 0 ? c.plan.one_pass != 0 : c.parts.n > 128LL * c.geo.ncell;
+// The single pass is the default wherever a chunk's window fits (the kernels fall
+// back to two passes by themselves where it does not).
+bool one_pass(const Ctx& c) { return c.plan.one_pass != 0; }
+// Window copies of the single pass: the lanes that meet in a cell, lanes sitting
+// 8 m particles apart (a power of two, at most 16).
+int rep_need(const Ctx& c) {
+    const double lanes = static_cast<double>(c.parts.n) / c.geo.ncell / (c.parts.cs / 32);
+    int r = 1;
+    while (r < 16 && r < lanes) r <<= 1;
+    return r;
 }
 DcuArgs dcu_args(const Ctx& c, const float* gb, bool fused) {
     DcuArgs a{};
@@ -1521,6 +1720,7 @@ DcuArgs dcu_args(const Ctx& c, const float* gb, bool fused) {
     a.use_rms = fused ? 1 : 0; a.psq = fused ? c.part_d : nullptr;
     a.use_tile = use_tile(c) ? 1 : 0;
     a.one_pass = one_pass(c) ? 1 : 0;
+    a.rep_need = rep_need(c);
     return a;
 }
 int es_window(const Ctx& c) {
@@ -1542,6 +1742,7 @@ EmArgs em_args(const Ctx& c) {
     a.acc = c.acc_src; a.wmaxc = wmax_cells(8); a.part = c.part_p; a.st = c.st; a.psq = c.part_c;
     a.use_tile = use_tile(c) ? 1 : 0;
     a.one_pass = one_pass(c) ? 1 : 0;
+    a.rep_need = rep_need(c);
     return a;
 }
 bool pow2_geo(const Ctx& c) { return is_pow2(c.geo.dx) && is_pow2(c.geo.dy); }
@@ -1555,7 +1756,7 @@ constexpr int kScatterNF = 6;
 __global__ void __launch_bounds__(kThreads, 2)
 k_scatter6(const float* __restrict__ xs, const float* __restrict__ ys, const float* __restrict__ vals, long long n,
            Geo g, const unsigned* __restrict__ vmax, float* __restrict__ Sout,
-           unsigned long long* __restrict__ acc, DevState* st, int vec_ok) {
+           unsigned long long* __restrict__ acc, DevState* st, int vec_ok, int cs_) {
     constexpr int NF = kScatterNF, NS = 2 + NF;
     constexpr bool T0 = false;
     constexpr int PC = wmax_cells(NF);
@@ -1563,8 +1764,9 @@ k_scatter6(const float* __restrict__ xs, const float* __restrict__ ys, const flo
     const Smem m = carve(smem, NS, win_planes(NF), PC);
     __shared__ unsigned long long bar;
     __shared__ int nlist;
-    const long long c0 = static_cast<long long>(blockIdx.x) * kChunk;
-    const int cnt = static_cast<int>(min(static_cast<long long>(kChunk), n - c0));
+    const long long c0 = static_cast<long long>(blockIdx.x) * cs_;
+    const int cnt = static_cast<int>(min(static_cast<long long>(cs_), n - c0));
+    const int ppt = cs_ / kThreads;               // particles per thread
     float S[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) S[f] = scale_for_bound(__fmul_rn(__uint_as_float(vmax[f]), 1.0001f));
@@ -1581,7 +1783,7 @@ k_scatter6(const float* __restrict__ xs, const float* __restrict__ ys, const flo
     BBox bb;
     float l1[NF] = {};
 #pragma unroll 1
-    for (int it = 0; it < kPPT; ++it) {
+    for (int it = 0; it < ppt; ++it) {
         const int sl = it * kThreads + threadIdx.x;
         const float x = m.stage[sl], y = m.stage[kChunk + sl];
         float xsv = -1.0f, cs[NF];
@@ -1609,8 +1811,8 @@ k_scatter6(const float* __restrict__ xs, const float* __restrict__ ys, const flo
 #pragma unroll
         for (int f = 0; f < NF; ++f) c[f] = a[2 + f];
     };
-    window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, g, coef, acc);
-    close_window<NF, NS, T0, PC>(m, wn, nlist, acc, g, st, coef);
+    window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);
+    close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
 }
 
 }  // namespace
@@ -1637,7 +1839,8 @@ void launch_scatter6(Ctx& c, cudaStream_t s, const float* xs, const float* ys, c
     prep_smem(k_scatter6, sh);
     const int vec = (n % 4 == 0 && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(ys) & 15) == 0 && (reinterpret_cast<uintptr_t>(vals) & 15) == 0) ? 1 : 0;
-    k_scatter6<<<nchunks(n), kThreads, sh, s>>>(xs, ys, vals, n, c.geo, vmax, Sout, acc, st, vec);
+    const int cs = chunk_size(n, 2 * c.sms);        // two CTAs per SM
+    k_scatter6<<<nchunks(n, cs), kThreads, sh, s>>>(xs, ys, vals, n, c.geo, vmax, Sout, acc, st, vec, cs);
     AW_LAUNCH();
 }
 
@@ -1646,7 +1849,7 @@ void launch_adj_scatter(Ctx& c, const AdjP& a, const AdjK& k, const float* trajE
     if (a.n == 0) return;
     const size_t sh = smem_bytes(2, 4);
     prep_smem(k_adj_scatter, sh);
-    k_adj_scatter<<<nchunks(a.n), kThreads, sh, c.stream>>>(a, c.geo, k, reinterpret_cast<const float2*>(trajE),
+    k_adj_scatter<<<nchunks(a.n, a.cs), kThreads, sh, c.stream>>>(a, c.geo, k, reinterpret_cast<const float2*>(trajE),
                                                              ad, acc, kAdjWindow, st);
     AW_LAUNCH();
 }
@@ -1759,11 +1962,13 @@ __device__ __forceinline__ int wrap_node(int i, int n) {
 // Stage planes: 0 x0 (sign set: skipped, listed for the slow pass), 1 y0, 2 x1,
 // 3 y1 (unwrapped), 4..6 the scaled coefficients ax ay az.
 __device__ __forceinline__ void yee_window_pass(const float* __restrict__ stage, int* __restrict__ win,
-                                                const Win& wn, const Geo& g) {
+                                                const Win& wn, int csz, const Geo& g) {
     if (!wn.use) return;
+    const Spread sp(csz);
+    const int ppt = csz / kThreads;
 #pragma unroll 1
-    for (int k = 0; k < kPPT; ++k) {
-        const int d = spread_slot(k);
+    for (int k = 0; k < ppt; ++k) {
+        const int d = sp.slot(k);
         const float x0 = stage[d];
         if (__float_as_int(x0) < 0) continue;
         const float y0 = stage[kChunk + d], x1 = stage[2 * kChunk + d], y1 = stage[3 * kChunk + d];
@@ -1784,9 +1989,9 @@ __device__ __forceinline__ void yee_window_pass(const float* __restrict__ stage,
 // The exact slow path: the same rounded contributions (the double product of
 // two floats is exact), straight into the global int64 planes.
 __device__ __forceinline__ void yee_slow_pass(const float* __restrict__ stage, const unsigned short* __restrict__ list,
-                                              int nlist, bool all_slots, unsigned long long* __restrict__ gacc,
+                                              int nlist, bool all_slots, int csz, unsigned long long* __restrict__ gacc,
                                               const Geo& g, DevState* st) {
-    const int total = nlist + (all_slots ? kChunk : 0);
+    const int total = nlist + (all_slots ? csz : 0);
     unsigned n = 0;
     for (int k = threadIdx.x; k < total; k += kThreads) {
         const bool listed = k < nlist;
@@ -1821,6 +2026,7 @@ __device__ __forceinline__ double yee_ramp(double t, double trmp, double toff) {
     return 1.0;
 }
 
+template <bool FULL>
 __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
     const Parts& p = A.p; const Geo& g = A.g;
     unsigned long long* __restrict__ acc = A.acc;
@@ -1834,8 +2040,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
     __shared__ unsigned umx[3][kThreads / 32];
 
     const int chunk = blockIdx.x;
-    const long long c0 = static_cast<long long>(chunk) * kChunk;
-    const int cnt = static_cast<int>(min(static_cast<long long>(kChunk), p.n - c0));
+    const int cs_ = FULL ? kChunk : p.cs;
+    const long long c0 = static_cast<long long>(chunk) * cs_;
+    const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
+    const int ppt = cs_ / kThreads;               // particles per thread
     const float S[3] = {st->S_next[1], st->S_next[2], st->S_next[3]};
     const double tnow = st->t;
     const bool pump = A.pump.on && tnow < A.pump.toff;
@@ -1852,7 +2060,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
     double ke = 0, px = 0, py = 0, pz = 0;
     float m0 = 0.f, m1 = 0.f, m2 = 0.f;
 #pragma unroll 1
-    for (int it = 0; it < kPPT; ++it) {
+    for (int it = 0; it < ppt; ++it) {
         const int s = it * kThreads + threadIdx.x;
         const long long i = c0 + s;
         const float x0 = m.stage[s], y0 = m.stage[kChunk + s];
@@ -1943,10 +2151,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
         atomicMax(&st->umax_bits[threadIdx.x], mx);
     }
     __syncthreads();
-    yee_window_pass(m.stage, m.win, wn, g);
+    yee_window_pass(m.stage, m.win, wn, cs_, g);
     __syncthreads();
     win_flush<NF, false>(m.win, wn, acc, g);
-    yee_slow_pass(m.stage, m.slow, nlist, !wn.use, acc, g, st);
+    yee_slow_pass(m.stage, m.slow, nlist, !wn.use, cs_, acc, g, st);
     if (threadIdx.x == 0) {
         atomicAdd(&st->chunks, 1ull);
         if (!wn.use) atomicAdd(&st->overflow, 1ull);
@@ -1971,7 +2179,7 @@ MultiPhase* multi_create(int kind, Ctx* const* runs, int nruns) {
     m->kind = kind;
     m->nruns = nruns;
     std::vector<int> first(nruns + 1, 0);
-    for (int r = 0; r < nruns; ++r) first[r + 1] = first[r] + (runs[r]->parts.n > 0 ? nchunks(runs[r]->parts.n) : 0);
+    for (int r = 0; r < nruns; ++r) first[r + 1] = first[r] + (runs[r]->parts.n > 0 ? nchunks(runs[r]->parts) : 0);
     m->nblocks = first[nruns];
     m->pow2 = pow2_geo(*runs[0]);
     for (int r = 1; r < nruns; ++r)
@@ -2036,8 +2244,9 @@ void multi_free(MultiPhase* m) {
 void launch_deposit_dcu(Ctx& c, const float* gb, bool fused) {
     if (c.parts.n == 0) return;
     const size_t sh = smem_bytes(3, 6);
-    prep_smem(k_deposit_dcu, sh);
-    k_deposit_dcu<<<nchunks(c.parts.n), kThreads, sh, c.stream>>>(dcu_args(c, gb, fused));
+    auto kern = c.parts.cs == kChunk ? k_deposit_dcu<true> : k_deposit_dcu<false>;
+    prep_smem(kern, sh);
+    kern<<<nchunks(c.parts), kThreads, sh, c.stream>>>(dcu_args(c, gb, fused));
     AW_LAUNCH();
 }
 
@@ -2046,10 +2255,14 @@ void launch_push_deposit_es(Ctx& c) {
     const size_t sh = es_smem_bytes(es_window(c));
     const bool p2 = pow2_geo(c);
     const bool rec = c.rec_xy != nullptr;
-    auto kern = p2 ? (rec ? k_push_deposit_es<true, true> : k_push_deposit_es<true, false>)
-                   : (rec ? k_push_deposit_es<false, true> : k_push_deposit_es<false, false>);
+    auto pick = [&](auto full) {
+        constexpr bool F = decltype(full)::value;
+        return p2 ? (rec ? k_push_deposit_es<true, F, true> : k_push_deposit_es<true, F, false>)
+                  : (rec ? k_push_deposit_es<false, F, true> : k_push_deposit_es<false, F, false>);
+    };
+    auto kern = c.parts.cs == kChunk ? pick(std::true_type{}) : pick(std::false_type{});
     prep_smem(kern, sh);
-    kern<<<nchunks(c.parts.n), kThreads, sh, c.stream>>>(es_args(c));
+    kern<<<nchunks(c.parts), kThreads, sh, c.stream>>>(es_args(c));
     AW_LAUNCH();
 }
 
@@ -2072,8 +2285,9 @@ void launch_push_esirkepov(Ctx& c) {
     a.pump.k0 = c.prm.pump_k0; a.pump.w0 = c.prm.pump_w0; a.pump.trmp = c.prm.pump_trmp; a.pump.toff = c.prm.pump_toff;
     a.acc = c.acc_src; a.wmaxc = kYeeWindow; a.part = c.part_p; a.st = c.st; a.write_cell = c.write_cell;
     const size_t sh = smem_bytes_w(3, kYeePlanes, kYeeWindow, 6);
-    prep_smem(k_push_esirkepov, sh);
-    k_push_esirkepov<<<nchunks(c.parts.n), kThreads, sh, c.stream>>>(a);
+    auto kern = c.parts.cs == kChunk ? k_push_esirkepov<true> : k_push_esirkepov<false>;
+    prep_smem(kern, sh);
+    kern<<<nchunks(c.parts), kThreads, sh, c.stream>>>(a);
     AW_LAUNCH();
 }
 
@@ -2081,9 +2295,11 @@ void launch_push_deposit_em(Ctx& c) {
     if (c.parts.n == 0) return;
     const size_t sh = smem_bytes(8, 6);
     const bool p2 = pow2_geo(c);
-    auto kern = p2 ? k_push_deposit_em<true> : k_push_deposit_em<false>;
+    const bool full = c.parts.cs == kChunk;
+    auto kern = p2 ? (full ? k_push_deposit_em<true, true> : k_push_deposit_em<true, false>)
+                   : (full ? k_push_deposit_em<false, true> : k_push_deposit_em<false, false>);
     prep_smem(kern, sh);
-    kern<<<nchunks(c.parts.n), kThreads, sh, c.stream>>>(em_args(c));
+    kern<<<nchunks(c.parts), kThreads, sh, c.stream>>>(em_args(c));
     AW_LAUNCH();
 }
 

@@ -37,7 +37,8 @@ namespace aw {
 
 constexpr int kThreads = 256;          // CTA size of every particle kernel
 constexpr int kPPT     = 8;            // particles per thread per chunk
-constexpr int kChunk   = kThreads * kPPT;   // particles per CTA chunk (2048)
+constexpr int kChunk   = kThreads * kPPT;   // particles per CTA chunk (2048) at most: the stage
+                                       // planes' stride; a launch's chunks hold Parts::cs
 
 // Fast-path range of one quantised contribution: |v*S| < 2^22 rounds exactly
 // with one FFMA against 1.5*2^23. The shared window words are int32: plain adds
@@ -306,6 +307,7 @@ struct Parts {
     int*   cell;
     long long n;
     int   vec_ok;     // all arrays 16-byte aligned
+    int   cs;         // particles per chunk: a multiple of kThreads, at most kChunk (chunk_size)
 };
 
 // ---------------------------------------------------------------------------
@@ -520,14 +522,24 @@ __device__ __forceinline__ int win_off(int c, int r, int n) { return wrap_signed
 // The stage is linear: chunk slot s of plane f is stage[f * kChunk + s]. Pass 1
 // takes slots it * kThreads + t (lanes on neighbouring particles: coalesced
 // global accesses, and the gathers of a warp fall on few cells); the deposit
-// takes this thread's k-th slot below. Lanes sit 64 particles apart (in loader
-// order a warp's atomics then fall on different cells) and read the linear
-// stage without bank conflicts (lane l's slot is congruent to 8 w + k + l
-// modulo 32). Over k = 0..7 the 256 threads take every slot exactly once.
-__device__ __forceinline__ int spread_slot(int k) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    return 64 * lane + ((8 * warp + k + lane) & 63);
-}
+// takes the slots below. With chunks of cs = m * kThreads particles, lanes sit
+// 8 m particles apart (64 in a full chunk: in loader order a warp's atomics then
+// fall on different cells) and read the linear stage without bank conflicts
+// (lane l's slot is l (8 m + 1) + m w + k before the wrap, an odd multiple of l).
+// Over k = 0..m-1 the 256 threads take every slot exactly once.
+struct Spread {
+    int base, r, stride;
+    __device__ __forceinline__ explicit Spread(int cs) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        stride = cs >> 5;
+        base = stride * lane;
+        r = (cs / kThreads) * warp + (lane >= stride ? lane % stride : lane);
+    }
+    __device__ __forceinline__ int slot(int k) const {
+        const int o = r + k;
+        return base + (o >= stride ? o - stride : o);
+    }
+};
 
 // Exact quantisation of a contribution: rint(a*b) with one FFMA against
 // 1.5*2^23 (exact for |a*b| < 2^22), read back as an integer.
@@ -689,15 +701,16 @@ __device__ __forceinline__ void store_chunk(const float* stage, float* const (&d
 
 // Exact slow path after the window pass: the particles pass 1 listed (a
 // coefficient outside the fast range or non-finite; their staged x carries a
-// flipped sign) and, when the window did not fit, every valid particle. Each
+// flipped sign) and, when the window did not fit, every valid particle of the
+// chunk's cs_ slots. Each
 // contribution is rounded exactly from the double product and added to the
 // global int64 planes. coef(a, cs) maps the staged values a[0..NS) of one
 // particle (a[0] = x, a[1] = y) to its NF scaled coefficients.
 template <int NF, int NS, class CoefFn>
 __device__ __forceinline__ void slow_pass(const float* __restrict__ stage, const unsigned short* __restrict__ list,
-                                          int nlist, bool all_slots, unsigned long long* __restrict__ gacc,
+                                          int nlist, bool all_slots, int cs_, unsigned long long* __restrict__ gacc,
                                           const Geo& g, DevState* st, CoefFn coef) {
-    const int total = nlist + (all_slots ? kChunk : 0);
+    const int total = nlist + (all_slots ? cs_ : 0);
     unsigned n = 0;
     for (int k = threadIdx.x; k < total; k += kThreads) {
         const bool listed = k < nlist;
@@ -753,9 +766,8 @@ __device__ __forceinline__ void quant_bits(const float (&cs)[NF], const Cic2& c,
     }
 }
 
-// Window pass of a one-band chunk: lane l of warp w deposits the chunk slots
-// 64 l + 8 w + k, k = 0..7, one particle at a time (lanes sit 64 particles
-// apart, so a warp's atomics fall on different cells). TRACK_ALL: every
+// Window pass of a one-band chunk of csz particles: each thread deposits its
+// spread slots (Spread), one particle at a time. TRACK_ALL: every
 // contribution is a tracked add. Otherwise field 0 is tracked when T0 and the
 // other fields add the FMA's biased bits, one native 32-bit shared atomic per
 // contribution, and the particle counts itself in its base cell. Particles whose
@@ -766,13 +778,15 @@ struct NoHook {
 };
 template <int NF, int NS, bool T0, bool TRACK_ALL, int PC, class CoefFn, class Hook = NoHook>
 __device__ __forceinline__ void window_particles(const float* __restrict__ stage, int* __restrict__ win,
-                                                 const Win& wn, const Geo& g, CoefFn coef, Hook hook = Hook{}) {
+                                                 const Win& wn, int csz, const Geo& g, CoefFn coef, Hook hook = Hook{}) {
     constexpr bool kBiased = !TRACK_ALL && NF > (T0 ? 1 : 0);
     const int P = PC ? PC : wn.P;
     const int oi = win_origin(wn.ir, wn.mi, g.nx), oj = win_origin(wn.jr, wn.mj, g.ny);
+    const Spread sp(csz);
+    const int ppt = csz / kThreads;
 #pragma unroll 1
-    for (int k = 0; k < kPPT; ++k) {
-        const int d = spread_slot(k);
+    for (int k = 0; k < ppt; ++k) {
+        const int d = sp.slot(k);
         float a[NS];
 #pragma unroll
         for (int f = 0; f < NS; ++f) a[f] = stage[f * kChunk + d];
@@ -809,12 +823,14 @@ __device__ __forceinline__ void window_particles(const float* __restrict__ stage
 // integer sums per cell as one window); unbiased adds.
 template <int NF, int NS, bool T0, bool TRACK_ALL, int PC, class CoefFn>
 __device__ __forceinline__ void window_band(const float* __restrict__ stage, int* __restrict__ win,
-                                            const Win& wn, int r0, const Geo& g, CoefFn coef) {
+                                            const Win& wn, int csz, int r0, const Geo& g, CoefFn coef) {
     const int P = PC ? PC : wn.P;
     const int oi = win_origin(wn.ir, wn.mi, g.nx), oj = win_origin(wn.jr, wn.mj, g.ny);
+    const Spread sp(csz);
+    const int ppt = csz / kThreads;
 #pragma unroll 1
-    for (int k = 0; k < kPPT; ++k) {
-        const int d = spread_slot(k);
+    for (int k = 0; k < ppt; ++k) {
+        const int d = sp.slot(k);
         const float x = stage[d];
         if (__float_as_int(x) < 0) continue;
         const float y = stage[kChunk + d];
@@ -849,12 +865,12 @@ __device__ __forceinline__ void window_band(const float* __restrict__ stage, int
 // several, each band is flushed here, and the window is zeroed for the next.
 template <int NF, int NS, bool T0, int PC = 0, class CoefFn>
 __device__ __forceinline__ void window_pass(const float* __restrict__ stage, int* __restrict__ win,
-                                            const Win& wn, const Geo& g, CoefFn coef,
+                                            const Win& wn, int csz, const Geo& g, CoefFn coef,
                                             unsigned long long* __restrict__ acc) {
     if (!wn.use) return;
     if (wn.nb == 1) {
-        if (wn.track_all) window_particles<NF, NS, T0, true, PC>(stage, win, wn, g, coef);
-        else window_particles<NF, NS, T0, false, PC>(stage, win, wn, g, coef);
+        if (wn.track_all) window_particles<NF, NS, T0, true, PC>(stage, win, wn, csz, g, coef);
+        else window_particles<NF, NS, T0, false, PC>(stage, win, wn, csz, g, coef);
         return;
     }
 #pragma unroll 1
@@ -863,8 +879,8 @@ __device__ __forceinline__ void window_pass(const float* __restrict__ stage, int
             win_zero<NF, T0, PC>(win, wn);
             __syncthreads();
         }
-        if (wn.track_all) window_band<NF, NS, T0, true, PC>(stage, win, wn, b * wn.Hb, g, coef);
-        else window_band<NF, NS, T0, false, PC>(stage, win, wn, b * wn.Hb, g, coef);
+        if (wn.track_all) window_band<NF, NS, T0, true, PC>(stage, win, wn, csz, b * wn.Hb, g, coef);
+        else window_band<NF, NS, T0, false, PC>(stage, win, wn, csz, b * wn.Hb, g, coef);
         __syncthreads();
         win_flush<NF, T0, PC>(win, wn, acc, g, b);
         __syncthreads();

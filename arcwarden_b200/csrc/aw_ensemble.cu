@@ -142,12 +142,6 @@ void make_run(aw_ensemble::Run& r, const aw_run_spec& s, cudaStream_t stream) {
     r.n4 = (r.n + 3) & ~3LL;     // keeps every array 16-byte aligned (bulk-copy chunk loads)
     int rc = aw_ctx_create(&s.grid, &s.params, s.model, stream, &r.ctx);
     if (rc != AW_OK) throw Error(rc, "ensemble: context creation failed");
-    // every run takes the two-pass particle kernels: the ensemble's step is
-    // faster that way than with the single pass that lone runs above 128
-    // particles per cell default to (ensemble64: 22.2 against 31.3 ms)
-    const aw_kernel_plan two_pass{0, -1, 0};
-    rc = aw_set_kernel_plan(r.ctx, &two_pass);
-    if (rc != AW_OK) throw Error(rc, "ensemble: kernel plan");
     AW_CUDA(cudaMalloc(&r.buf, sizeof(float) * 7 * static_cast<size_t>(r.n4)));
     rc = aw_particles_bind(r.ctx, arr(r, 0), arr(r, 1), arr(r, 2), arr(r, 3), arr(r, 4), arr(r, 5),
                            reinterpret_cast<int32_t*>(arr(r, 6)), r.n);

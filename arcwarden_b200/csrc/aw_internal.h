@@ -76,6 +76,28 @@ struct PumpP {
 // EM path ([Ex Ey Ez Bx | By Bz 0 0]) and 2 floats per cell for ES ([Ex Ey]).
 // One 32-byte sector per cell, read with two LDG.128 per CIC corner.
 
+// Particles per chunk (a multiple of kThreads) of a launch over n particles on
+// `slots` resident CTAs. A launch of two or more waves of full chunks takes full
+// chunks (its CTAs drift apart, so its last wave is not felt: balancing it made
+// es256, 3.5 waves, 4% slower). Below that the size whose waves take the least
+// time, counting a chunk as its m iterations per thread plus kChunkFixed
+// iterations' worth of work that does not shrink with it (load latency, window
+// set-up, flush, sums): 1.05 M particles (512 full chunks on 444 slots) take 820
+// chunks of 1280, 65 k take 256 of 256 instead of 32 full ones (es 64x64: 2.56 ->
+// 2.22 ms).
+constexpr int kChunkFixed = 3;
+inline int chunk_size(long long n, int slots) {
+    if (n >= 2LL * slots * kChunk) return kChunk;
+    int best = kPPT;
+    long long cost = -1;
+    for (int m = kPPT; m >= 1; --m) {
+        const long long chunks = (n + m * kThreads - 1) / (m * kThreads);
+        const long long t = (chunks + slots - 1) / slots * (m + kChunkFixed);
+        if (cost < 0 || t < cost) { cost = t; best = m; }
+    }
+    return best * kThreads;
+}
+
 struct Ctx {
     // configuration
     aw_grid   grid{};
@@ -153,6 +175,7 @@ struct Ctx {
     bool pending_valid = false;       // acc_src holds the deposit of the current state
     long long host_step = 0;
     int write_cell = 1;
+    int sms = 148;                    // multiprocessors of the context's device
 
     // k-space form factor table (aw_set_form_factor), c.sg.ff points at it
     double* ffac = nullptr;
@@ -198,6 +221,7 @@ struct AdjP {
     float *lx, *ly, *lux, *luy, *luz;
     long long n;
     int vec_ok;
+    int cs;           // particles per chunk
 };
 // Device scalars of the backward sweep.
 struct AdjDev {

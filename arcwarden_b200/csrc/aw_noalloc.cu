@@ -100,6 +100,7 @@ extern "C" int aw_deposit_rho_noalloc(const aw_grid* g, double qm, const float* 
         c.parts.uz = const_cast<float*>(uz); c.parts.w = const_cast<float*>(w);
         c.parts.cell = nullptr;
         c.parts.n = n;
+        c.parts.cs = kChunk;
         c.parts.vec_ok = (aligned16(x) && aligned16(y) && aligned16(ux) && aligned16(uy) && aligned16(uz) &&
                           aligned16(w)) ? 1 : 0;
         c.st = reinterpret_cast<DevState*>(base);
