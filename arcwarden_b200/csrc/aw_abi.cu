@@ -594,9 +594,8 @@ int aw_particles_bind(aw_ctx* ctx, float* x, float* y, float* ux, float* uy, flo
         c.parts_bound = true;
         auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
         c.parts.vec_ok = (al(x) && al(y) && al(ux) && al(uy) && al(uz) && al(w) && (!cell || al(cell))) ? 1 : 0;
-        // resident CTAs of the model's particle kernels (the ES kernel's small window leaves room for four per SM)
-        const bool four = c.model == AW_MODEL_ES && n >= 32LL * c.geo.ncell;
-        c.parts.cs = aw::chunk_size(n, (four ? 4 : 3) * c.sms);
+        // resident CTAs of the particle kernels: four per SM (electrostatic), three (Darwin, Yee)
+        c.parts.cs = aw::chunk_size(n, (c.model == AW_MODEL_ES ? 4 : 3) * c.sms);
         const int nb = static_cast<int>(std::max<long long>(1, (n + c.parts.cs - 1) / c.parts.cs));
         if (nb > c.npart_p) {
             if (c.part_p) cudaFree(c.part_p);

@@ -65,13 +65,18 @@ constexpr int wmax_cells(int nf) {
     return nf == 1 ? 2048 : (nf == 2 ? 1920 : (nf == 3 ? 800 : (nf == 4 ? 1536 : 320)));
 }
 constexpr int kRedInts = kThreads / 32 * (4 + 8);
-// The fused ES kernel stages 5 planes and takes one of two rho windows. The ES
-// path keeps the particle order, so a chunk covers kChunk / ppc consecutive
-// cells of the load order plus their drift: at 32 or more particles per cell a
-// short row segment (the 1024-cell window: 4 CTAs per SM at <= 64 registers),
-// below that whole grid rows and their spread in y (3584 cells: 14 rows of 256,
-// 3 CTAs per SM).
-constexpr int kEsPlanes = 5, kEsWindowSmall = 1024, kEsWindowLarge = 3584;
+// The fused ES kernel: four CTAs per SM (56 KB each, at most 64 registers), so its
+// stage holds x y ux uy uz and not the weights: a chunk's weights are usually equal
+// (one species), and where they are not the kernel reads them from global memory.
+// stage | red | area, the area holding either the single pass's window of kEsP1
+// cells (4 planes), its gather tile of kEsT1 cells and the slow slots' bit map, or the
+// two-pass fallback's window (2 planes, up to kEsWinMax cells) and its slow list.
+// The ES path keeps the particle order, so a chunk covers cs / ppc consecutive cells
+// of the load order plus their drift.
+constexpr int kEsP1 = 800, kEsT1 = 304;
+constexpr int kEsArea = kEsP1 * 4 * 4 + kEsT1 * 8 + kChunk / 8;
+constexpr int kEsWinMax = 1408;
+static_assert(kEsWinMax * 8 + kChunk * 2 <= kEsArea, "the fallback's window and list must fit the area");
 // stage [np][kChunk] f32 | window [planes][wmax] i32 | red ints | slow list u16[kChunk]
 constexpr size_t win_offset(int np) { return static_cast<size_t>(np) * kChunk * 4; }
 constexpr size_t smem_bytes_w(int nf, int np, int wmax, int planes) {
@@ -79,7 +84,8 @@ constexpr size_t smem_bytes_w(int nf, int np, int wmax, int planes) {
            + kChunk * sizeof(unsigned short);
 }
 constexpr size_t smem_bytes(int nf, int np) { return smem_bytes_w(nf, np, wmax_cells(nf), win_planes(nf)); }
-constexpr size_t es_smem_bytes(int wmax) { return smem_bytes_w(1, kEsPlanes, wmax, win_planes(1)); }
+constexpr size_t es_smem_bytes() { return win_offset(5) + kRedInts * sizeof(int) + kEsArea; }
+static_assert(4 * (es_smem_bytes() + 1024 + 400) <= 228 * 1024, "four ES CTAs per SM");
 
 struct Smem {
     float* stage;
@@ -222,29 +228,26 @@ __device__ __forceinline__ float warp_sum8(const float (&v)[8]) {
     return c;
 }
 
-// Block-wide fixed-order sum of 4 doubles into part[blk*5 + 0..3] (blk: the chunk).
-__device__ __forceinline__ void block_sum4(double a, double b, double c, double d, double* __restrict__ part,
-                                           double* sh /* 4 * warps */, int blk) {
-    constexpr int NW = kThreads / 32;
+// Block-wide fixed-order sums of a chunk: 4 doubles into part[blk*5 + 0..3]
+// (warp halves by block_sum4_put, a barrier, block_sum4_get) and NF floats plus
+// the valid-particle count into psq[blk*(NF+1) + f] (block_sumsq_put, barrier,
+// block_sumsq_get). Deterministic for a fixed launch shape. NF = 1, 3, 4 or 8.
+__device__ __forceinline__ void block_sum4_put(double a, double b, double c, double d, double* sh /* 4 * warps */) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double w = warp_sum4(a, b, c, d);
-    if ((lane & 7) == 0) sh[(lane >> 3) * NW + warp] = w;
-    __syncthreads();
+    if ((lane & 7) == 0) sh[(lane >> 3) * (kThreads / 32) + warp] = w;
+}
+__device__ __forceinline__ void block_sum4_get(double* __restrict__ part, const double* sh, int blk) {   // warp 0
     if (threadIdx.x < 4) {
         double s = 0;
 #pragma unroll
-        for (int k = 0; k < NW; ++k) s += sh[threadIdx.x * NW + k];
+        for (int k = 0; k < kThreads / 32; ++k) s += sh[threadIdx.x * (kThreads / 32) + k];
         part[blk * 5 + threadIdx.x] = s;
     }
     if (threadIdx.x == 4) part[blk * 5 + 4] = 0.0;
 }
-
-// Block-wide fixed-order sum of NF floats (plus the valid-particle count in
-// slot NF) into part[blk * (NF + 1) + f]. Deterministic for a fixed
-// launch shape. 1, 3, 4 or 8 fields.
 template <int NF>
-__device__ __forceinline__ void block_sumsq(const float (&sq)[NF], float cnt, float* __restrict__ part,
-                                            float* sh /* (NF+1) * warps */, int blk) {
+__device__ __forceinline__ void block_sumsq_put(const float (&sq)[NF], float cnt, float* sh /* (NF+1) * warps */) {
     constexpr int NW = kThreads / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if constexpr (NF == 8) {
@@ -257,11 +260,15 @@ __device__ __forceinline__ void block_sumsq(const float (&sq)[NF], float cnt, fl
     }
     const unsigned n = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(cnt));   // a count: exact
     if (lane == 0) sh[NF * NW + warp] = static_cast<float>(n);
-    __syncthreads();
-    if (threadIdx.x <= NF) {
+}
+template <int NF>
+__device__ __forceinline__ void block_sumsq_get(float* __restrict__ psq, const float* sh, int blk, int first = 0) {
+    const int t = static_cast<int>(threadIdx.x) - first;     // threads first .. first + NF
+    if (t >= 0 && t <= NF) {
         float s = 0.f;
-        for (int w = 0; w < NW; ++w) s += sh[threadIdx.x * NW + w];
-        part[blk * (NF + 1) + threadIdx.x] = s;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) s += sh[t * (kThreads / 32) + w];
+        psq[blk * (NF + 1) + t] = s;
     }
 }
 
@@ -380,7 +387,11 @@ k_deposit_src(Parts p, Geo g, double qoa, const float* __restrict__ Sdev,
     };
     window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);
     close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
-    if (psq) block_sumsq<NF>(sq, nval, psq, ssq, blockIdx.x);
+    if (psq) {
+        block_sumsq_put<NF>(sq, nval, ssq);
+        __syncthreads();
+        block_sumsq_get<NF>(psq, ssq, blockIdx.x);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -544,48 +555,57 @@ struct Box1 { int i0, j0, nI, nJ; };
 // Block-wide box; false (block-uniformly) when some particle is not in the grid.
 // First without regard to the periodic edges (positions in the grid are
 // non-negative floats, so integer order of the bits is their order, and anything
-// else - negative, NaN, too large - shows at one of the two ends); a box wider
-// than `cap_i` x `cap_j` cells is taken again as wrapped offsets from the first
-// particle's cell, which is exact for chunks that straddle an edge. Slots past
-// cnt are filled with the first particle's position by the threads that read
-// them. `red` is 32 ints of scratch. Ends with every warp past its reads of `red`
-// only after the caller's next barrier.
-__device__ __forceinline__ bool chunk_box(float* stage, int cs, int cnt, float x0, float y0, const Geo& g, int* red,
-                                          int cap_cells, int mg, Box1& b) {
-    constexpr int NW = kThreads / 32;
-    const int warp = threadIdx.x >> 5;
+// else - negative, NaN, too large - shows at one of the two ends); a box too large
+// for `cap` cells with its margin is taken again as wrapped offsets from the first
+// particle's cell, which is exact for chunks that straddle an edge. Slots past cnt
+// are filled with the first particle's position by the threads that read them.
+// `ends` (shared, 16-byte aligned) was set by box_reset before the block's last
+// barrier; `red` is scratch of the second way.
+__device__ __forceinline__ void box_reset(int* ends) {      // one thread
+    ends[0] = 0x7fffffff; ends[1] = static_cast<int>(0x80000000u);
+    ends[2] = 0x7fffffff; ends[3] = static_cast<int>(0x80000000u);
+}
+template <bool FULL>
+__device__ __forceinline__ bool chunk_box(float* stage, int cs, int cnt, float x0, float y0, const Geo& g, int* ends,
+                                          int* red, int cap, int mg, Box1& b) {
     if (cnt < cs)
         for (int s = threadIdx.x; s < cs; s += kThreads)
             if (s >= cnt) { stage[s] = x0; stage[kChunk + s] = y0; }
-    const int* xb = reinterpret_cast<const int*>(stage);
-    int lx = xb[threadIdx.x], hx = lx, ly = xb[kChunk + threadIdx.x], hy = ly;
-#pragma unroll 7
-    for (int s = kThreads + threadIdx.x; s < cs; s += kThreads) {
-        const int x = xb[s], y = xb[kChunk + s];
-        lx = min(lx, x); hx = max(hx, x);
-        ly = min(ly, y); hy = max(hy, y);
+    const int* xb = reinterpret_cast<const int*>(stage) + threadIdx.x;
+    int lx = xb[0], hx = lx, ly = xb[kChunk], hy = ly;
+    if constexpr (FULL) {
+#pragma unroll
+        for (int k = 1; k < kPPT; ++k) {
+            const int x = xb[k * kThreads], y = xb[kChunk + k * kThreads];
+            lx = min(lx, x); hx = max(hx, x);
+            ly = min(ly, y); hy = max(hy, y);
+        }
+    } else {
+        for (int s = kThreads; s < cs; s += kThreads) {
+            const int x = xb[s], y = xb[kChunk + s];
+            lx = min(lx, x); hx = max(hx, x);
+            ly = min(ly, y); hy = max(hy, y);
+        }
     }
     lx = __reduce_min_sync(0xffffffffu, lx); hx = __reduce_max_sync(0xffffffffu, hx);
     ly = __reduce_min_sync(0xffffffffu, ly); hy = __reduce_max_sync(0xffffffffu, hy);
-    if ((threadIdx.x & 31) == 0) { red[warp] = lx; red[NW + warp] = hx; red[2 * NW + warp] = ly; red[3 * NW + warp] = hy; }
-    __syncthreads();
-    lx = red[0]; hx = red[NW]; ly = red[2 * NW]; hy = red[3 * NW];
-#pragma unroll
-    for (int k = 1; k < NW; ++k) {
-        lx = min(lx, red[k]); hx = max(hx, red[NW + k]);
-        ly = min(ly, red[2 * NW + k]); hy = max(hy, red[3 * NW + k]);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(ends, lx); atomicMax(ends + 1, hx);
+        atomicMin(ends + 2, ly); atomicMax(ends + 3, hy);
     }
-    const float xhi = __int_as_float(hx), yhi = __int_as_float(hy);
-    if (lx < 0 || ly < 0 || !(xhi < g.nxf) || !(yhi < g.nyf)) return false;
-    b.i0 = static_cast<int>(__int_as_float(lx)); b.nI = static_cast<int>(xhi) - b.i0 + 1;
-    b.j0 = static_cast<int>(__int_as_float(ly)); b.nJ = static_cast<int>(yhi) - b.j0 + 1;
-    if (static_cast<long long>(min(b.nI + 1 + 2 * mg, g.nx + 1)) * min(b.nJ + 1 + 2 * mg, g.ny + 1) <= cap_cells) return true;
+    __syncthreads();
+    const int4 e = *reinterpret_cast<const int4*>(ends);
+    const float xhi = __int_as_float(e.y), yhi = __int_as_float(e.w);
+    if (e.x < 0 || e.z < 0 || !(xhi < g.nxf) || !(yhi < g.nyf)) return false;
+    b.i0 = static_cast<int>(__int_as_float(e.x)); b.nI = static_cast<int>(xhi) - b.i0 + 1;
+    b.j0 = static_cast<int>(__int_as_float(e.z)); b.nJ = static_cast<int>(yhi) - b.j0 + 1;
+    // (a grid has at most 2^28 cells: the products fit)
+    if (min(b.nI + 1 + 2 * mg, g.nx + 1) * min(b.nJ + 1 + 2 * mg, g.ny + 1) <= cap) return true;
     // the chunk straddles an edge, or is simply large: wrapped offsets
     const int ir = static_cast<int>(x0), jr = static_cast<int>(y0);
     BBox bb;
     for (int s = threadIdx.x; s < cs; s += kThreads)
         bb.add(static_cast<int>(stage[s]), static_cast<int>(stage[kChunk + s]), ir, jr, g);
-    __syncthreads();                          // `red` has been read
     const Box w = box_reduce(bb, red);
     b.i0 = ir + w.lo_i; if (b.i0 < 0) b.i0 += g.nx; if (b.i0 >= g.nx) b.i0 -= g.nx;
     b.j0 = jr + w.lo_j; if (b.j0 < 0) b.j0 += g.ny; if (b.j0 >= g.ny) b.j0 -= g.ny;
@@ -593,6 +613,9 @@ __device__ __forceinline__ bool chunk_box(float* stage, int cs, int cnt, float x
     b.nJ = w.hi_j - w.lo_j + 1;
     return true;
 }
+// Row of cell c in a box of rows of W cells, r = 1 / W: the half keeps the product
+// off the integers by more than its rounding for any c below 2^21.
+__device__ __forceinline__ int row_of(int c, float r) { return static_cast<int>((static_cast<float>(c) + 0.5f) * r); }
 
 // The window of box b widened by mg cells; false when it does not fit P1 cells.
 // A dimension the window would span whole (a margin wider than the grid, e.g.
@@ -606,8 +629,8 @@ __device__ __forceinline__ bool window1(Win1& w, const Box1& b, int mg, int rep_
     else if (w.oi < 0) w.oi += g.nx;
     if (w.H > g.ny) { w.H = g.ny + 1; w.oj = 0; }
     else if (w.oj < 0) w.oj += g.ny;
-    if (static_cast<long long>(w.W) * w.H > P1) return false;
     w.WH = w.W * w.H;
+    if (w.WH > P1) return false;
     w.rep = 1; w.CS = w.WH;
     for (int r = rep_need; r > 1; r >>= 1) {
         const int cs = w.WH + ((32 / r - w.WH) & 31);
@@ -648,50 +671,52 @@ __device__ __forceinline__ void win1_add(int* __restrict__ win, const Win1& w, i
     }
 }
 
-// Flush into the global int64 accumulators, TPC threads per window cell (each
-// takes every TPC-th field); the caller has synced.
-template <int NF, bool HI, int P1, int TPC>
+// Flush into the global int64 accumulators, one thread per window cell; the
+// caller has synced. (Sharing a cell among threads repeats the count and the
+// address work: the flush is bound by instructions, not by its latency.)
+template <int NF, bool HI, int P1>
 __device__ __forceinline__ void win1_flush(const int* __restrict__ s, const Win1& w,
                                            unsigned long long* __restrict__ acc, const Geo& g) {
     constexpr int NC = NF + (HI ? 2 : 0);
-    const int f0 = threadIdx.x % TPC;
-    for (int c = threadIdx.x / TPC; c < w.WH; c += kThreads / TPC) {
-        const int wj = c / w.W, wi = c - wj * w.W;
-        const int cl = wi > 0 ? 1 : 0, cd = wj > 0 ? w.W : 0;    // offsets of the neighbours that exist
+    const float rW = 1.0f / static_cast<float>(w.W);
+    for (int c = threadIdx.x; c < w.WH; c += kThreads) {
+        const int wj = row_of(c, rW), wi = c - wj * w.W;
+        const bool L = wi > 0, D = wj > 0;                  // the neighbours that exist
         int n = 0;
-        long long A = 0;
+        unsigned h = 0u, u[NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) u[f] = 0u;
         for (int r = 0; r < w.rep; ++r) {
-            const int* q = s + NC * P1 + r * w.CS + c;
-            n += q[0];
-            if (cl) n += q[-1];
-            if (cd) n += q[-cd];
-            if (cl && cd) n += q[-cd - 1];
+            const int* q = s + r * w.CS + c;
+            n += q[NC * P1];
+            if (L) n += q[NC * P1 - 1];
+            if (D) n += q[NC * P1 - w.W];
+            if (L && D) n += q[NC * P1 - w.W - 1];
+            if (HI) {     // at most 2048 contributions of at most 16 to a node: fits
+                h += q[NF * P1] & 0xFFFF;
+                if (L) h += static_cast<unsigned>(q[NF * P1 - 1]) >> 16;
+                if (D) h += q[(NF + 1) * P1 - w.W] & 0xFFFF;
+                if (L && D) h += static_cast<unsigned>(q[(NF + 1) * P1 - w.W - 1]) >> 16;
+            }
+#pragma unroll
+            for (int f = 0; f < NF; ++f) u[f] += static_cast<unsigned>(q[f * P1]);
         }
         if (n == 0) continue;
         int gi = w.oi + wi, gj = w.oj + wj;
         if (gi >= g.nx) gi -= g.nx;
         if (gj >= g.ny) gj -= g.ny;
-        unsigned long long* a = acc + (static_cast<size_t>(gj) * g.nx + gi);
+        unsigned long long* a = acc + (gj * g.nx + gi);
         const unsigned nM = static_cast<unsigned>(n) * kMagicU;
 #pragma unroll
-        for (int f = f0; f < NF; f += TPC) {
-            unsigned u = 0;
-            for (int r = 0; r < w.rep; ++r) u += static_cast<unsigned>(s[f * P1 + r * w.CS + c]);
+        for (int f = 0; f < NF; ++f) {
             long long v;
             if (HI && f == 0) {
-                for (int r = 0; r < w.rep; ++r) {
-                    const int* h = s + NF * P1 + r * w.CS + c;
-                    A += h[0] & 0xFFFF;
-                    if (cl) A += static_cast<unsigned>(h[-1]) >> 16;
-                    if (cd) A += h[P1 - cd] & 0xFFFF;
-                    if (cl && cd) A += static_cast<unsigned>(h[P1 - cd - 1]) >> 16;
-                }
-                A <<= 19;
-                // sum of q + 2^22: A plus what the fine sum adds modulo 2^32 (less than n 2^19)
-                const unsigned fine = u - static_cast<unsigned>(n) * (kMagicU - 4194304u);
+                // sum of q + 2^22: the coarse sum plus what the fine one adds modulo 2^32 (less than n 2^19)
+                const long long A = static_cast<long long>(h) << 19;
+                const unsigned fine = u[0] - static_cast<unsigned>(n) * (kMagicU - 4194304u);
                 v = A + static_cast<long long>(fine - static_cast<unsigned>(A)) - static_cast<long long>(n) * 4194304ll;
             } else {
-                v = static_cast<int>(u - nM);          // the copies' true sums add up to the chunk's, < 2^31
+                v = static_cast<int>(u[f] - nM);       // the copies' true sums add up to the chunk's, < 2^31
             }
             if (v != 0) atomicAdd(a + static_cast<size_t>(f) * g.ncell, static_cast<unsigned long long>(v));
         }
@@ -731,15 +756,30 @@ __device__ __forceinline__ void tile1_load(Tile1& t, float* area, const Box1& bx
     float2* B = reinterpret_cast<float2*>(area + 4 * T);
     t.a = A; t.b = B; t.i0 = bx.i0; t.j0 = bx.j0; t.W = bx.nI + 1;
     const int cells = t.W * (bx.nJ + 1);
+    const float rW = 1.0f / static_cast<float>(t.W);
     const float4* q = reinterpret_cast<const float4*>(gb);
     for (int c = threadIdx.x; c < cells; c += kThreads) {
-        const int r = c / t.W;
+        const int r = row_of(c, rW);
         int gi = t.i0 + (c - r * t.W), gj = t.j0 + r;
         if (gi >= g.nx) gi -= g.nx;
         if (gj >= g.ny) gj -= g.ny;
-        const size_t k = 2 * (static_cast<size_t>(gj) * g.nx + gi);
+        const int k = 2 * (gj * g.nx + gi);          // (at most 2^28 cells)
         A[c] = __ldg(q + k);
         B[c] = __ldg(reinterpret_cast<const float2*>(q + k + 1));
+    }
+}
+// The (Ex, Ey) pairs of a box from the [ncell][2] buffer of the ES path.
+template <int T>
+__device__ __forceinline__ void tile1_load_es(float2* area, int W, const Box1& bx, const float2* __restrict__ gb,
+                                              const Geo& g) {
+    const int cells = W * (bx.nJ + 1);
+    const float rW = 1.0f / static_cast<float>(W);
+    for (int c = threadIdx.x; c < cells; c += kThreads) {
+        const int r = row_of(c, rW);
+        int gi = bx.i0 + (c - r * W), gj = bx.j0 + r;
+        if (gi >= g.nx) gi -= g.nx;
+        if (gj >= g.ny) gj -= g.ny;
+        area[c] = __ldg(gb + gj * g.nx + gi);
     }
 }
 __device__ __forceinline__ EB2 tile1_gather(const Tile1& t, const Cic& s, const Geo& g) {
@@ -866,7 +906,8 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     float S[3];
     dcu_scales(st, abs_qm, use_rms != 0, S);
     if (chunk == 0 && threadIdx.x == 0) { st->S_dcu[0] = S[0]; st->S_dcu[1] = S[1]; st->S_dcu[2] = S[2]; }
-    if (threadIdx.x == 0) nlist = 0;
+    __shared__ __align__(16) int ends[4];
+    if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
     const ChunkSrc src{{p.x, p.y, p.w, p.ux, p.uy, p.uz}};
     float x0, y0;
     if (!load_chunk(m.stage, src, NIN, c0, cnt, p.vec_ok != 0, &bar, st, &x0, &y0)) return;
@@ -879,7 +920,7 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
         constexpr int P1 = 640, T1 = ((PC * win_planes(NF) - P1 * (NF + 1)) / 6) & ~3;     // 24 bytes per tile cell
         Box1 bx;
         Win1 w1;
-        if (chunk_box(m.stage, cs_, cnt, x0, y0, g, m.red, T1, 0, bx) && window1<P1>(w1, bx, 0, A.rep_need, g) &&
+        if (chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, T1, 0, bx) && window1<P1>(w1, bx, 0, A.rep_need, g) &&
             (bx.nI + 1) * (bx.nJ + 1) <= T1) {
             Tile1 tl;
             tile1_load<T1>(tl, reinterpret_cast<float*>(m.win + P1 * (NF + 1)), bx, gb, g);
@@ -926,7 +967,7 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
                 }
             }
             const bool redo = chunk_overflows1(fmaxf(l2[0], fmaxf(l2[1], l2[2])), ppt, m.red);   // (its barrier ends the pass)
-            if (!redo) win1_flush<NF, false, P1, 4>(m.win, w1, acc, g);
+            if (!redo) win1_flush<NF, false, P1>(m.win, w1, acc, g);
             slow_pass_linear<NF>(m.stage, m.slow, nlist, redo, cnt, acc, g, st, [&](int sl, float (&cs)[NF]) {
                 float cf[NF];
                 const float x = m.stage[sl], y = m.stage[kChunk + sl];
@@ -939,7 +980,11 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
                 atomicAdd(&st->one_pass, 1ull);
                 if (redo) atomicAdd(&st->overflow, 1ull);
             }
-            if (psq) block_sumsq<NF>(sq, nval, psq, ssq, chunk);
+            if (psq) {
+                block_sumsq_put<NF>(sq, nval, ssq);
+                __syncthreads();
+                block_sumsq_get<NF>(psq, ssq, chunk);
+            }
             return;
         }
         __syncthreads();           // the box scratch has been read
@@ -1038,7 +1083,11 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
         window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);   // bands (or the slow path alone)
     }
     close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
-    if (psq) block_sumsq<NF>(sq, nval, psq, ssq, chunk);}
+    if (psq) {
+                block_sumsq_put<NF>(sq, nval, ssq);
+                __syncthreads();
+                block_sumsq_get<NF>(psq, ssq, chunk);
+            }}
 template <bool FULL>
 __global__ void __launch_bounds__(kThreads, 3) k_deposit_dcu(DcuArgs A) { deposit_dcu_chunk<FULL>(A, blockIdx.x); }
 
@@ -1153,6 +1202,8 @@ struct PushP {
     float  b0x, b0y, b0z;
     double dt;
     double dtx, dty;      // dt/dx, dt/dy (exact when dx, dy are powers of two)
+    double rdx, rdy;      // fl(1/dx), fl(1/dy)
+    float  dtmax;         // max(dt/dx, dt/dy): cells moved per unit of u
     int    write_cell;
 };
 
@@ -1175,8 +1226,8 @@ __device__ __forceinline__ bool step_xy(float& x, float& y, float ux, float uy, 
         x = move1_pow2(x, ux, pp.dtx);
         y = move1_pow2(y, uy, pp.dty);
     } else {
-        x = move1(x, ux, pp.dt, g.dx);
-        y = move1(y, uy, pp.dt, g.dy);
+        x = move1_by(x, ux, pp.dt, g.dx, pp.rdx);
+        y = move1_by(y, uy, pp.dt, g.dy, pp.rdy);
     }
     if (in_grid(x, y, g)) return true;
     x = wrap_pos(x, g.nxf);
@@ -1184,109 +1235,251 @@ __device__ __forceinline__ bool step_xy(float& x, float& y, float ux, float uy, 
     return in_grid(x, y, g);
 }
 
-// Fused ES step kernel: input x y w ux uy uz; stage = new x, y, coefficient q w / (dx dy).
+// Fused ES step kernel. Single pass where the chunk's window fits (one read of the
+// staged particle, 7 shared atomics); else two passes through the stage: new x, y,
+// coefficient q w / (dx dy). Bound by instruction issue and by the latency of a
+// chunk's fixed phases (load, box, window, flush, sums): es256, 4.2 M particles, 390 ->
+// 250 instructions a particle, 73.7 -> 55.3 us (28 us of HBM time).
 struct EsArgs {
     Parts p; Geo g; PushP pp; const float* gb; double qoa; unsigned long long* acc; int wmaxc;
     double* part; DevState* st;
     float* traj; const AdjDev* rec;   // trajectory recording (x_n, y_n into slot rec->rec_slot), or null
+    int one_pass, rep_need;
 };
 template <bool POW2, bool FULL, bool RECORD = false>
 __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int chunk) {
     const Parts& p = A.p; const Geo& g = A.g; const PushP& pp = A.pp;
     const float* __restrict__ gb = A.gb; const double qoa = A.qoa; unsigned long long* __restrict__ acc = A.acc;
     const int wmaxc = A.wmaxc; double* __restrict__ part = A.part; DevState* st = A.st;
-    constexpr int NF = 1, NS = 3, NIN = 5;          // stage in: x y ux uy uz (w read from global)
+    constexpr int NF = 1, NS = 3, NIN = 5;
     constexpr bool T0 = true;
     extern __shared__ __align__(16) unsigned char smem[];
-    const Smem m = carve(smem, NIN, win_planes(NF), wmaxc);
+    Smem m;
+    m.stage = reinterpret_cast<float*>(smem);
+    m.red = reinterpret_cast<int*>(smem + win_offset(NIN));
+    m.win = m.red + kRedInts;
+    m.slow = reinterpret_cast<unsigned short*>(m.win + 2 * kEsWinMax);
     __shared__ unsigned long long bar;
     __shared__ int nlist;
     __shared__ double dsh[4 * (kThreads / 32)];
+    __shared__ unsigned umx[2][kThreads / 32];
 
     const int cs_ = FULL ? kChunk : p.cs;
     const long long c0 = static_cast<long long>(chunk) * cs_;
     const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
     const int ppt = cs_ / kThreads;               // particles per thread
+    const Spread sp(cs_);
     const float S1[1] = {st->S_next[0]};
-    if (threadIdx.x == 0) nlist = 0;
+    __shared__ __align__(16) int ends[4];
+    if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
+    const float uxy_max = fmaxf(__uint_as_float(st->ucur_bits[0]), __uint_as_float(st->ucur_bits[1]));
     const ChunkSrc src{{p.x, p.y, p.ux, p.uy, p.uz, nullptr}};
+    // the chunk's weights, while its state is on the way: all equal?
+    int wlo = 0x7fffffff, whi = static_cast<int>(0x80000000u);
+#pragma unroll 8
+    for (int s = threadIdx.x; s < cnt; s += kThreads) {
+        const int b = __float_as_int(__ldg(p.w + c0 + s));
+        wlo = min(wlo, b); whi = max(whi, b);
+    }
+    wlo = __reduce_min_sync(0xffffffffu, wlo); whi = __reduce_max_sync(0xffffffffu, whi);
+    int* const wred = m.red + 64;             // (chunk_box uses the first 32)
+    if ((threadIdx.x & 31) == 0) { wred[threadIdx.x >> 5] = wlo; wred[8 + (threadIdx.x >> 5)] = whi; }
     float x0, y0;
     if (!load_chunk(m.stage, src, NIN, c0, cnt, p.vec_ok != 0, &bar, st, &x0, &y0)) return;
-    int ir, jr;
-    ref_of(x0, y0, g, ir, jr);
-    const float2* q = reinterpret_cast<const float2*>(gb);
-    float* __restrict__ tr = RECORD ? A.traj + static_cast<size_t>(A.rec->rec_slot) * 2 * p.n : nullptr;
-
-    BBox bb;
-    float l1[NF] = {};
-    double ke = 0, px = 0, py = 0, pz = 0;
-#pragma unroll 2
-    for (int it = 0; it < ppt; ++it) {
-        const int s = it * kThreads + threadIdx.x;
-        const long long i = c0 + s;
-        float x = m.stage[s], y = m.stage[kChunk + s];
-        float ux = m.stage[2 * kChunk + s], uy = m.stage[3 * kChunk + s], uz = m.stage[4 * kChunk + s];
-        const float w = s < cnt ? __ldcs(p.w + i) : 0.0f;
-        if (RECORD && s < cnt) { tr[i] = x; tr[p.n + i] = y; }
-        float xs = -1.0f, cf0 = 0.0f;
-        if (s < cnt) {
-            if (in_grid(x, y, g)) {
-                const Cic c = cic(x, y);
-                const int i1 = wrap_once(c.i0 + 1, g.nx);
-                const int r0 = c.j0 * g.nx, r1 = wrap_once(c.j0 + 1, g.ny) * g.nx;
-                const float2 e0 = __ldg(q + r0 + c.i0), e1 = __ldg(q + r0 + i1);
-                const float2 e2 = __ldg(q + r1 + c.i0), e3 = __ldg(q + r1 + i1);
-                // gather4 on the (Ex, Ey) pair, then the half kicks paired
-                float2 exy = __fmul2_rn(bc2(c.w0), e0);
-                exy = __ffma2_rn(bc2(c.w1), e1, exy);
-                exy = __ffma2_rn(bc2(c.w2), e2, exy);
-                exy = __ffma2_rn(bc2(c.w3), e3, exy);
-                const float2 Q = bc2(pp.qmh);
-                float2 uxy = __ffma2_rn(Q, exy, make_float2(ux, uy));
-                ux = uxy.x; uy = uxy.y;
-                if (pp.has_b0) boris_rotate(ux, uy, uz, pp.b0x, pp.b0y, pp.b0z, pp.qmh);
-                uxy = __ffma2_rn(Q, exy, make_float2(ux, uy));
-                ux = uxy.x; uy = uxy.y;
-                move_xy<POW2>(x, y, ux, uy, pp, g);
-                int ci, cj;
-                cell_ij(x, y, g, ci, cj);
-                // streaming stores: the new state is not read again this step
-                __stcs(p.x + i, x); __stcs(p.y + i, y); __stcs(p.ux + i, ux); __stcs(p.uy + i, uy); __stcs(p.uz + i, uz);
-                if (pp.write_cell && p.cell) __stcs(p.cell + i, cj * g.nx + ci);
-                if (in_grid(x, y, g)) {
-                    bb.add(ci, cj, ir, jr, g);
-                    cf0 = __double2float_rn(qoa * static_cast<double>(w));
-                    const float cf[1] = {cf0};
-                    float cs[1];
-                    const bool fast = scale_fast<1>(cf, S1, cs, l1);
-                    xs = __fadd_rn(x, 0.0f);
-                    if (!fast) { xs = -xs; list_slow(m.slow, &nlist, s); }
-                } else {
-                    set_err(st, AW_DEV_OUT_OF_GRID);
-                }
-                const double dw = w, du = ux, dv = uy, dz = uz;
-                ke += dw * (du * du + dv * dv + dz * dz);
-                px += dw * du; py += dw * dv; pz += dw * dz;
-            } else {
-                set_err(st, AW_DEV_OUT_OF_GRID);
-            }
-        }
-        const int d = s;                     // in place: this thread's own slot
-        m.stage[d] = xs;
-        m.stage[kChunk + d] = y;
-        m.stage[2 * kChunk + d] = cf0;
-    }
-    const Win wn = open_window<NF, T0>(bb, ir, jr, wmaxc, m, l1);
-    auto coef = [&](const float (&a)[NS], float (&cs)[NF]) {
-        cs[0] = __fmul_rn(a[2], S1[0]);
-    };
-    window_pass<NF, NS, T0>(m.stage, m.win, wn, cs_, g, coef, acc);
-    close_window<NF, NS, T0>(m, wn, nlist, cs_, acc, g, st, coef);
-    block_sum4(ke, px, py, pz, part, dsh, chunk);
     if (threadIdx.x == 0 && chunk == 0) {
         st->S_pend[0] = S1[0];
         st->step += 1;
-    }}
+    }
+    const float2* q = reinterpret_cast<const float2*>(gb);
+    if constexpr (RECORD) {
+        float* __restrict__ tr = A.traj + static_cast<size_t>(A.rec->rec_slot) * 2 * p.n;
+        for (int s = threadIdx.x; s < cnt; s += kThreads) { tr[c0 + s] = m.stage[s]; tr[p.n + c0 + s] = m.stage[kChunk + s]; }
+    }
+    // the rotation about the uniform B0 (boris_rotate's t and s; without B0 it would
+    // return every finite u unchanged)
+    const bool rot = pp.has_b0 && (pp.b0x != 0.0f || pp.b0y != 0.0f || pp.b0z != 0.0f);
+    const BorisRot R(pp.b0x, pp.b0y, pp.b0z, pp.qmh);
+    const float2 Q = bc2(pp.qmh);
+    // gather4 on the (Ex, Ey) pair, then the half kicks paired
+    auto push = [&](const Cic& c, float2 e0, float2 e1, float2 e2, float2 e3, float& ux, float& uy, float& uz) {
+        float2 exy = __fmul2_rn(bc2(c.w0), e0);
+        exy = __ffma2_rn(bc2(c.w1), e1, exy);
+        exy = __ffma2_rn(bc2(c.w2), e2, exy);
+        exy = __ffma2_rn(bc2(c.w3), e3, exy);
+        float2 uxy = __ffma2_rn(Q, exy, make_float2(ux, uy));
+        if (rot) R.apply(uxy.x, uxy.y, uz);
+        uxy = __ffma2_rn(Q, exy, uxy);
+        ux = uxy.x; uy = uxy.y;
+    };
+    double ke = 0, px = 0, py = 0, pz = 0;
+    float m0 = 0.f, m1 = 0.f;
+    bool done = false;
+
+    // ---- single pass -------------------------------------------------------
+    if (A.one_pass) {
+        const float dmv = __fmul_rn(2.0f * uxy_max, pp.dtmax);
+        const int mg = (dmv >= 0.0f && dmv < 8.0f) ? 1 + static_cast<int>(dmv) : -1;
+        Box1 bx;
+        Win1 w1;
+        if (mg > 0 && chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, kEsP1, mg, bx) &&
+            window1<kEsP1>(w1, bx, mg, A.rep_need, g) && (bx.nI + 1) * (bx.nJ + 1) <= kEsT1) {
+            done = true;
+            wlo = wred[0]; whi = wred[8];
+#pragma unroll
+            for (int k = 1; k < kThreads / 32; ++k) { wlo = min(wlo, wred[k]); whi = max(whi, wred[8 + k]); }
+            const bool wsame = wlo == whi;
+            float w = __int_as_float(wlo);
+            float cf0 = __double2float_rn(qoa * static_cast<double>(w));
+            float2* const tile = reinterpret_cast<float2*>(m.win + 4 * kEsP1);
+            unsigned* const slow = reinterpret_cast<unsigned*>(tile + kEsT1);      // bit map of slots
+            if (threadIdx.x < kChunk / 32) slow[threadIdx.x] = 0u;
+            const int TW = bx.nI + 1;
+            tile1_load_es<kEsT1>(tile, TW, bx, q, g);
+            win1_zero<4, kEsP1>(m.win, w1);
+            __syncthreads();
+            const bool cells = pp.write_cell && p.cell;
+#pragma unroll 1
+            for (int k = 0; k < ppt; ++k) {
+                const int sl = sp.slot(k);
+                if (sl >= cnt) continue;
+                float x = m.stage[sl], y = m.stage[kChunk + sl];
+                float ux = m.stage[2 * kChunk + sl], uy = m.stage[3 * kChunk + sl], uz = m.stage[4 * kChunk + sl];
+                if (!wsame) {
+                    w = __ldg(p.w + c0 + sl);
+                    cf0 = __double2float_rn(qoa * static_cast<double>(w));
+                }
+                {
+                    const Cic c = cic(x, y);
+                    int li = c.i0 - bx.i0, lj = c.j0 - bx.j0;
+                    if (li < 0) li += g.nx;
+                    if (lj < 0) lj += g.ny;
+                    const float2* e = tile + lj * TW + li;
+                    push(c, e[0], e[1], e[TW], e[TW + 1], ux, uy, uz);
+                }
+                const bool ok = step_xy<POW2>(x, y, ux, uy, pp, g);
+                const double dw = w, du = ux, dv = uy, dz = uz;
+                ke += dw * (du * du + dv * dv + dz * dz);
+                px += dw * du; py += dw * dv; pz += dw * dz;
+                m.stage[sl] = x; m.stage[kChunk + sl] = y;
+                m.stage[2 * kChunk + sl] = ux; m.stage[3 * kChunk + sl] = uy; m.stage[4 * kChunk + sl] = uz;
+                m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy));
+                if (ok) {
+                    const float cs[1] = {__fmul_rn(cf0, S1[0])};
+                    const int di = win_col(static_cast<int>(x), w1.oi, g.nx), dj = win_col(static_cast<int>(y), w1.oj, g.ny);
+                    if (fabsf(cs[0]) < kFastLim && di <= w1.W - 2 && dj <= w1.H - 2)
+                        win1_add<1, true, kEsP1>(m.win, w1, di, dj, x, y, cs);
+                    else { atomicOr(slow + (sl >> 5), 1u << (sl & 31)); nlist = 1; }
+                } else {
+                    set_err(st, AW_DEV_OUT_OF_GRID);
+                }
+            }
+            stage_fence();
+            __syncthreads();
+            const int pl[5] = {0, 1, 2, 3, 4};
+            float* const dst[5] = {p.x, p.y, p.ux, p.uy, p.uz};
+            bulk_store_planes<5>(m.stage, pl, dst, 5, c0, cnt, p.vec_ok != 0);
+            win1_flush<1, true, kEsP1>(m.win, w1, acc, g);
+            if (cells)                        // the owning cells, from the staged new positions
+#pragma unroll 4
+                for (int s = threadIdx.x; s < cnt; s += kThreads) {
+                    const float x = m.stage[s], y = m.stage[kChunk + s];
+                    if (in_grid(x, y, g)) __stcs(p.cell + c0 + s, static_cast<int>(y) * g.nx + static_cast<int>(x));
+                }
+            if (nlist)
+                for (int s = threadIdx.x; s < cnt; s += kThreads) {
+                    if (!(slow[s >> 5] >> (s & 31) & 1u)) continue;
+                    const float x = m.stage[s], y = m.stage[kChunk + s];
+                    const float cs[1] = {__fmul_rn(__double2float_rn(qoa * static_cast<double>(__ldg(p.w + c0 + s))), S1[0])};
+                    if (!isfinite(cs[0])) { set_err(st, AW_DEV_NONFINITE); continue; }
+                    const Cic c = cic(x, y);
+                    const float wv[4] = {c.w0, c.w1, c.w2, c.w3};
+                    deposit_global<1>(c.i0, c.j0, wv, cs, acc, g);
+                    atomicAdd(&st->slow, 1ull);
+                }
+            if (threadIdx.x == 0) {
+                atomicAdd(&st->chunks, 1ull);
+                atomicAdd(&st->one_pass, 1ull);
+            }
+        } else {
+            __syncthreads();           // the box scratch has been read
+        }
+    }
+
+    // ---- two passes --------------------------------------------------------
+    if (!done) {
+        int ir, jr;
+        ref_of(x0, y0, g, ir, jr);
+        BBox bb;
+        float l1[NF] = {};
+#pragma unroll 2
+        for (int it = 0; it < ppt; ++it) {
+            const int s = it * kThreads + threadIdx.x;
+            const long long i = c0 + s;
+            float x = m.stage[s], y = m.stage[kChunk + s];
+            float ux = m.stage[2 * kChunk + s], uy = m.stage[3 * kChunk + s], uz = m.stage[4 * kChunk + s];
+            const float w = s < cnt ? __ldcs(p.w + i) : 0.0f;
+            float xs = -1.0f, cf0 = 0.0f;
+            if (s < cnt) {
+                if (in_grid(x, y, g)) {
+                    const Cic c = cic(x, y);
+                    const int i1 = wrap_once(c.i0 + 1, g.nx);
+                    const int r0 = c.j0 * g.nx, r1 = wrap_once(c.j0 + 1, g.ny) * g.nx;
+                    push(c, __ldg(q + r0 + c.i0), __ldg(q + r0 + i1), __ldg(q + r1 + c.i0), __ldg(q + r1 + i1), ux, uy, uz);
+                    const bool ok = step_xy<POW2>(x, y, ux, uy, pp, g);
+                    int ci, cj;
+                    cell_ij(x, y, g, ci, cj);
+                    // streaming stores: the new state is not read again this step
+                    __stcs(p.x + i, x); __stcs(p.y + i, y); __stcs(p.ux + i, ux); __stcs(p.uy + i, uy); __stcs(p.uz + i, uz);
+                    if (pp.write_cell && p.cell) __stcs(p.cell + i, cj * g.nx + ci);
+                    m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy));
+                    if (ok) {
+                        bb.add(ci, cj, ir, jr, g);
+                        cf0 = __double2float_rn(qoa * static_cast<double>(w));
+                        const float cf[1] = {cf0};
+                        float cs[1];
+                        const bool fast = scale_fast<1>(cf, S1, cs, l1);
+                        xs = __fadd_rn(x, 0.0f);
+                        if (!fast) { xs = -xs; list_slow(m.slow, &nlist, s); }
+                    } else {
+                        set_err(st, AW_DEV_OUT_OF_GRID);
+                    }
+                    const double dw = w, du = ux, dv = uy, dz = uz;
+                    ke += dw * (du * du + dv * dv + dz * dz);
+                    px += dw * du; py += dw * dv; pz += dw * dz;
+                } else {
+                    set_err(st, AW_DEV_OUT_OF_GRID);
+                }
+            }
+            const int d = s;                     // in place: this thread's own slot
+            m.stage[d] = xs;
+            m.stage[kChunk + d] = y;
+            m.stage[2 * kChunk + d] = cf0;
+        }
+        const Win wn = open_window<NF, T0>(bb, ir, jr, wmaxc, m, l1);
+        auto coef = [&](const float (&a)[NS], float (&cs)[NF]) {
+            cs[0] = __fmul_rn(a[2], S1[0]);
+        };
+        window_pass<NF, NS, T0>(m.stage, m.win, wn, cs_, g, coef, acc);
+        close_window<NF, NS, T0>(m, wn, nlist, cs_, acc, g, st, coef);
+    }
+    // the in-plane |u| maxima bound the next step's moves (the single pass's margin)
+    m0 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m0)));
+    m1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m1)));
+    if ((threadIdx.x & 31) == 0) {
+        umx[0][threadIdx.x >> 5] = __float_as_uint(m0);
+        umx[1][threadIdx.x >> 5] = __float_as_uint(m1);
+    }
+    block_sum4_put(ke, px, py, pz, dsh);
+    __syncthreads();
+    block_sum4_get(part, dsh, chunk);
+    if (threadIdx.x >= 32 && threadIdx.x < 34) {
+        const int d = threadIdx.x - 32;
+        unsigned mx = 0;
+        for (int k = 0; k < kThreads / 32; ++k) mx = max(mx, umx[d][k]);
+        atomicMax(&st->umax_bits[d], mx);
+    }
+    if (done) bulk_store_wait();
+}
 template <bool POW2, bool FULL, bool RECORD>
 __global__ void __launch_bounds__(kThreads, 4) k_push_deposit_es(EsArgs A) {
     push_deposit_es_chunk<POW2, FULL, RECORD>(A, blockIdx.x);
@@ -1324,7 +1517,9 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     for (int f = 0; f < NF; ++f) S[f] = st->S_next[f];
     const float2 Sp[4] = {make_float2(S[0], S[1]), make_float2(S[2], S[3]), make_float2(S[4], S[5]),
                           make_float2(S[6], S[7])};
-    if (threadIdx.x == 0) nlist = 0;
+    __shared__ __align__(16) int ends[4];
+    if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
+    const float uxy_max = fmaxf(__uint_as_float(st->ucur_bits[0]), __uint_as_float(st->ucur_bits[1]));
     const ChunkSrc src{{p.x, p.y, p.w, p.ux, p.uy, p.uz}};
     float x0, y0;
     if (!load_chunk(m.stage, src, NS, c0, cnt, p.vec_ok != 0, &bar, st, &x0, &y0)) return;
@@ -1336,12 +1531,11 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
         constexpr int P1 = 384, T1 = ((PC * win_planes(NF) - P1 * (NF + 3)) / 6) & ~3;     // 24 bytes per tile cell
         // the cells a particle can cross in one step: twice the largest in-plane |u| of
         // the current state times dt/dx (one further cell for the rounding)
-        const float uxy_max = fmaxf(__uint_as_float(st->ucur_bits[0]), __uint_as_float(st->ucur_bits[1]));
-        const float dmv = __fmul_rn(2.0f * uxy_max, static_cast<float>(fmax(pp.dtx, pp.dty)));
+        const float dmv = __fmul_rn(2.0f * uxy_max, pp.dtmax);
         const int mg = (dmv >= 0.0f && dmv < 8.0f) ? 1 + static_cast<int>(dmv) : -1;
         Box1 bx;
         Win1 w1;
-        if (mg > 0 && chunk_box(m.stage, cs_, cnt, x0, y0, g, m.red, P1, mg, bx) &&
+        if (mg > 0 && chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, P1, mg, bx) &&
             window1<P1>(w1, bx, mg, A.rep_need, g) && (bx.nI + 1) * (bx.nJ + 1) <= T1) {
             Tile1 tl;
             tile1_load<T1>(tl, reinterpret_cast<float*>(m.win + P1 * (NF + 3)), bx, gb, g);
@@ -1420,7 +1614,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
             const int pl[6] = {0, 1, 3, 4, 5, 2};
             float* const dst[6] = {p.x, p.y, p.ux, p.uy, p.uz, reinterpret_cast<float*>(p.cell)};
             bulk_store_planes<6>(m.stage, pl, dst, cells ? 6 : 5, c0, cnt, p.vec_ok != 0);
-            if (!redo) win1_flush<NF, true, P1, 4>(m.win, w1, acc, g);
+            if (!redo) win1_flush<NF, true, P1>(m.win, w1, acc, g);
             slow_pass_linear<NF>(m.stage, m.slow, nlist, redo, cnt, acc, g, st, [&](int sl, float (&cs)[NF]) {
                 float2 cp[4];
                 src_coefs8(__double2float_rn(qoa * static_cast<double>(p.w[c0 + sl])),
@@ -1442,8 +1636,11 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
                 if (redo) atomicAdd(&st->overflow, 1ull);
             }
             const float sq[NF] = {sqp[0].x, sqp[0].y, sqp[1].x, sqp[1].y, sqp[2].x, sqp[2].y, sqp[3].x, sqp[3].y};
-            block_sumsq<NF>(sq, nval, psq, ssq, chunk);
-            block_sum4(ke, px, py, pz, part, dsh, chunk);
+            block_sumsq_put<NF>(sq, nval, ssq);
+            block_sum4_put(ke, px, py, pz, dsh);
+            __syncthreads();
+            block_sumsq_get<NF>(psq, ssq, chunk, 32);
+            block_sum4_get(part, dsh, chunk);
             if (threadIdx.x == 0 && chunk == 0) {
 #pragma unroll
                 for (int f = 0; f < NF; ++f) st->S_pend[f] = S[f];
@@ -1598,8 +1795,11 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     float sq[NF];
 #pragma unroll
     for (int i = 0; i < 4; ++i) { sq[2 * i] = sqp[i].x; sq[2 * i + 1] = sqp[i].y; }
-    block_sumsq<NF>(sq, nval, psq, ssq, chunk);
-    block_sum4(ke, px, py, pz, part, dsh, chunk);
+    block_sumsq_put<NF>(sq, nval, ssq);
+    block_sum4_put(ke, px, py, pz, dsh);
+    __syncthreads();
+    block_sumsq_get<NF>(psq, ssq, chunk, 32);
+    block_sum4_get(part, dsh, chunk);
     if (threadIdx.x == 0 && chunk == 0) {
 #pragma unroll
         for (int f = 0; f < NF; ++f) st->S_pend[f] = S[f];
@@ -1689,6 +1889,9 @@ PushP push_params(const Ctx& c) {
     pp.dt = c.prm.dt;
     pp.dtx = c.prm.dt / c.geo.dx;
     pp.dty = c.prm.dt / c.geo.dy;
+    pp.rdx = 1.0 / c.geo.dx;
+    pp.rdy = 1.0 / c.geo.dy;
+    pp.dtmax = static_cast<float>(std::max(pp.dtx, pp.dty));
     pp.write_cell = c.write_cell;
     return pp;
 }
@@ -1723,16 +1926,17 @@ DcuArgs dcu_args(const Ctx& c, const float* gb, bool fused) {
     a.rep_need = rep_need(c);
     return a;
 }
-int es_window(const Ctx& c) {
-    if (c.plan.es_window > 0) return c.plan.es_window;
-    return c.parts.n >= 32LL * c.geo.ncell ? kEsWindowSmall : kEsWindowLarge;
-}
+// Capacity of the two-pass fallback's window in cells (aw_kernel_plan::es_window;
+// results do not depend on it).
+int es_window(const Ctx& c) { return c.plan.es_window > 0 ? std::min(c.plan.es_window, kEsWinMax) : kEsWinMax; }
 EsArgs es_args(const Ctx& c) {
     EsArgs a{};
     a.p = c.parts; a.g = c.geo; a.pp = push_params(c); a.gb = c.gb_es;
     a.qoa = c.prm.qm / (c.geo.dx * c.geo.dy);
     a.acc = c.acc_src; a.wmaxc = es_window(c); a.part = c.part_p; a.st = c.st;
     a.traj = c.rec_xy; a.rec = c.rec_ad;
+    a.one_pass = one_pass(c) ? 1 : 0;
+    a.rep_need = rep_need(c);
     return a;
 }
 EmArgs em_args(const Ctx& c) {
@@ -2159,7 +2363,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
         atomicAdd(&st->chunks, 1ull);
         if (!wn.use) atomicAdd(&st->overflow, 1ull);
     }
-    block_sum4(ke, px, py, pz, A.part, dsh, chunk);
+    block_sum4_put(ke, px, py, pz, dsh);
+    __syncthreads();
+    block_sum4_get(A.part, dsh, chunk);
     if (threadIdx.x == 0 && chunk == 0) st->step += 1;
 }
 
@@ -2194,7 +2400,7 @@ MultiPhase* multi_create(int kind, Ctx* const* runs, int nruns) {
         if (kind == kMultiEsPush) {
             const EsArgs a = es_args(*runs[r]);
             put(&a, sizeof a);
-            m->smem = std::max(m->smem, es_smem_bytes(a.wmaxc));
+            m->smem = es_smem_bytes();
         }
         else if (kind == kMultiDcu) { const DcuArgs a = dcu_args(*runs[r], runs[r]->gb_dcu, true); put(&a, sizeof a); }
         else { const EmArgs a = em_args(*runs[r]); put(&a, sizeof a); }
@@ -2252,7 +2458,7 @@ void launch_deposit_dcu(Ctx& c, const float* gb, bool fused) {
 
 void launch_push_deposit_es(Ctx& c) {
     if (c.parts.n == 0) return;
-    const size_t sh = es_smem_bytes(es_window(c));
+    const size_t sh = es_smem_bytes();
     const bool p2 = pow2_geo(c);
     const bool rec = c.rec_xy != nullptr;
     auto pick = [&](auto full) {

@@ -221,6 +221,23 @@ __device__ __forceinline__ void boris_rotate(float& ux, float& uy, float& uz,
     uy = __fadd_rn(uy, __fmaf_rn(upz, sx, -__fmul_rn(upx, sz)));
     uz = __fadd_rn(uz, __fmaf_rn(upx, sy, -__fmul_rn(upy, sx)));
 }
+// boris_rotate about a uniform B, its t and s taken once.
+struct BorisRot {
+    float tx, ty, tz, sx, sy, sz;
+    __device__ __forceinline__ BorisRot(float bx, float by, float bz, float qmh) {
+        tx = __fmul_rn(qmh, bx); ty = __fmul_rn(qmh, by); tz = __fmul_rn(qmh, bz);
+        const float sf = boris_sf(__fmaf_rn(tz, tz, __fmaf_rn(ty, ty, __fmul_rn(tx, tx))));
+        sx = __fmul_rn(sf, tx); sy = __fmul_rn(sf, ty); sz = __fmul_rn(sf, tz);
+    }
+    __device__ __forceinline__ void apply(float& ux, float& uy, float& uz) const {
+        const float upx = __fadd_rn(ux, __fmaf_rn(uy, tz, -__fmul_rn(uz, ty)));
+        const float upy = __fadd_rn(uy, __fmaf_rn(uz, tx, -__fmul_rn(ux, tz)));
+        const float upz = __fadd_rn(uz, __fmaf_rn(ux, ty, -__fmul_rn(uy, tx)));
+        ux = __fadd_rn(ux, __fmaf_rn(upy, sz, -__fmul_rn(upz, sy)));
+        uy = __fadd_rn(uy, __fmaf_rn(upz, sx, -__fmul_rn(upx, sz)));
+        uz = __fadd_rn(uz, __fmaf_rn(upx, sy, -__fmul_rn(upy, sx)));
+    }
+};
 // ES velocity update over dt_eff with uniform B0 — pusher.hpp:47-80 (Ez = 0).
 __device__ __forceinline__ void boris_es(float& ux, float& uy, float& uz, float ex, float ey,
                                          float qmh, bool has_b0, float b0x, float b0y, float b0z) {
@@ -271,6 +288,16 @@ __device__ __forceinline__ float move1(float x, float u, double dt, double d) {
 // the rounded product by 2^k is exact, so RN(u*dt)/d == RN(u*dtd) bit for bit.
 __device__ __forceinline__ float move1_pow2(float x, float u, double dtd) {
     return __fadd_rn(x, __double2float_rn(__dmul_rn(static_cast<double>(u), dtd)));
+}
+// The same move for any d, with r = fl(1/d): the correctly rounded quotient from a
+// multiplication and two fused multiply-adds (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990: with
+// r = fl(1/d) and q = fl(a r), fl(q + r (a - q d)) is fl(a/d)). 3 instructions
+// in place of the general division.
+__device__ __forceinline__ float move1_by(float x, float u, double dt, double d, double r) {
+    const double a = __dmul_rn(static_cast<double>(u), dt);
+    const double q = __dmul_rn(a, r);
+    return __fadd_rn(x, __double2float_rn(__fma_rn(__fma_rn(-q, d, a), r, q)));
 }
 // Periodic wrap of a position — particles.hpp:301-306: x = fmodf(x, n);
 // x < 0 -> x + n; x >= n -> 0. The three common cases are answered exactly
@@ -653,10 +680,11 @@ __device__ __forceinline__ bool load_chunk(float* stage, const ChunkSrc& src, in
     const int nbulk = vec ? (cnt & ~3) : 0;
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
-        mbar_arrive_expect_tx(bar, static_cast<unsigned>(np * nbulk) * 4u + st->dbg_extra_tx);
+        // the copies first; the phase cannot complete before this thread's arrival
         if (nbulk > 0)
             for (int k = 0; k < np; ++k)
                 bulk_load(stage + k * kChunk, src.at(k) + c0, static_cast<unsigned>(nbulk) * 4u, bar);
+        mbar_arrive_expect_tx(bar, static_cast<unsigned>(np * nbulk) * 4u + st->dbg_extra_tx);
     }
     const int rem = cnt - nbulk;
     if (rem > 0)

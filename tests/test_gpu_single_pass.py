@@ -1,0 +1,59 @@
+"""The single-pass particle kernels against the two-pass ones: the same particles,
+cells, densities and fields, bit for bit, over the chunk and window shapes the
+single pass meets - chunks of one to eight iterations, windows of one copy to
+sixteen, boxes that straddle an edge or span a whole dimension, rows one cell high,
+cell sizes off the powers of two, odd grids, weights of both signs and weights so
+uneven that some particles leave the fast range (the exact slow path)."""
+import numpy as np
+import pytest
+
+from gpu_helpers import PARTICLE_KEYS, Setup
+
+pytestmark = pytest.mark.gpu
+
+#        model nx  ny  Lx    Ly    ppc  weights
+CASES = [(0, 64, 64, 64.0, 64.0, 16, "one"),      # chunks of 256: four rows' worth of one species
+         (0, 48, 20, 14.4, 6.0, 50, "mixed"),     # dx = 0.3
+         (0, 33, 7, 33.0, 7.0, 700, "uneven"),    # odd grid, 11 copies' worth of lanes per cell
+         (0, 256, 8, 256.0, 8.0, 300, "one"),
+         (1, 48, 20, 14.4, 6.0, 25, "mixed"),
+         (1, 16, 1, 32.0, 2.0, 512, "one"),       # one row: the window spans the dimension
+         (1, 8, 8, 8.0, 8.0, 2048, "uneven"),     # one cell per chunk, 16 copies
+         (1, 37, 5, 18.5, 2.5, 64, "uneven"),
+         (1, 128, 64, 64.0, 32.0, 130, "mixed")]
+
+
+@pytest.mark.parametrize("model,nx,ny,Lx,Ly,ppc,weights", CASES)
+def test_single_pass_equals_two_passes(torch_cuda, aw, model, nx, ny, Lx, Ly, ppc, weights):
+    n = nx * ny * ppc - 3                                # a ragged last chunk
+    rng = np.random.default_rng(nx * 1000 + ny)
+    cell = np.repeat(np.arange(nx * ny), ppc)[:n]
+    edge = lambda v, top: np.minimum(v.astype(np.float32), np.nextafter(np.float32(top), np.float32(0)))  # noqa: E731
+    P = {"x": edge(cell % nx + rng.random(n), nx), "y": edge(cell // nx + rng.random(n), ny),
+         "ux": rng.normal(0, 0.3, n), "uy": rng.normal(0, 0.3, n), "uz": rng.normal(0, 0.2, n)}
+    w = np.full(n, Lx * Ly / (nx * ny) / ppc)
+    if weights != "one":
+        w *= np.where(rng.random(n) < 0.4, -1.0, 1.0) * rng.random(n)
+    if weights == "uneven":
+        w[rng.random(n) < 0.999] *= 1e-3
+    P["w"] = w
+    out = []
+    for one_pass in (0, 1):
+        s = Setup(torch_cuda, aw, nx, ny, Lx, Ly, n, model, dt=0.05, B0=(0.1, 0.0, 0.3))
+        try:
+            s.ctx.set_kernel_plan(one_pass=one_pass)
+            for k in PARTICLE_KEYS:
+                s.put(k, P[k].astype(np.float32))
+            s.ctx.init()
+            s.ctx.run(0, 3)
+            r = s.parts()
+            for k in ("rho", "Ex", "Ey") + (("Jx", "Jz", "Ez", "Bz") if model else ()):
+                r[k] = s.grid(k)
+            assert s.ctx.error_word() == 0
+            st = s.ctx.stats()
+            assert (st["one_pass_chunks"] > 0) == bool(one_pass), st
+            out.append(r)
+        finally:
+            s.close()
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
