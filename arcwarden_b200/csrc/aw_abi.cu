@@ -86,6 +86,7 @@ void free_all(Ctx& c) {
     free_checkpoint(c);
     free_adjoint(c);
     free_dadj(c);
+    gridfft_free(c);
     if (c.gexec) cudaGraphExecDestroy(c.gexec);
     if (c.graph) cudaGraphDestroy(c.graph);
     cufftHandle* plans[] = {&c.p_r2c1, &c.p_c2r1, &c.p_r2cS, &c.p_c2rO, &c.p_r2c3, &c.p_c2r3, &c.p_r2c4};
@@ -145,6 +146,12 @@ struct NoMark { void operator()(int) const {} };
 template <class Mark>
 void es_fields_from_pending(Ctx& c, bool step_begin, Mark mark) {
     float* api[1] = {c.src.rho};
+    if (c.gf) {
+        gridfft_rows_acc(c, c.acc_src, 0, 1, c.st->S_pend, api, true, step_begin, true, c.k_src); mark(0); mark(1);
+        gridfft_cols_es(c, c.k_src, c.k_out); mark(2); mark(3);
+        gridfft_fields_es(c, c.k_out, !step_begin); mark(4);        // aw_init's rollback reads the planes
+        return;
+    }
     launch_finalize(c, c.acc_src, 0, 1, c.st->S_pend, c.r_src, api, false, true, step_begin, true); mark(0);
     AW_CUFFT(cufftExecR2C(c.p_r2cS, c.r_src, c.k_src)); mark(1);
     launch_kspace_es(c, c.k_src, c.k_out); mark(2);
@@ -158,6 +165,12 @@ void es_fields_from_pending(Ctx& c, bool step_begin) { es_fields_from_pending(c,
 template <class Mark>
 void darwin_fields_a(Ctx& c, bool step_begin, Mark mark) {
     float* api[8] = {c.src.rho, c.src.Jx, c.src.Jy, c.src.Jz, c.src.amu0, c.src.amu1, c.src.amu2, c.src.amu3};
+    if (c.gf) {
+        gridfft_rows_acc(c, c.acc_src, 0, 8, c.st->S_pend, api, true, step_begin, true, c.k_src); mark(0); mark(1);
+        gridfft_cols_elb(c, c.k_src, c.k_out); mark(2); mark(3);
+        gridfft_fields_dcu(c, c.k_out); mark(4);
+        return;
+    }
     launch_finalize(c, c.acc_src, 0, 8, c.st->S_pend, c.r_src, api, false, true, step_begin, true); mark(0);
     AW_CUFFT(cufftExecR2C(c.p_r2cS, c.r_src, c.k_src)); mark(1);
     launch_kspace_elb(c, c.k_src, c.k_out); mark(2);
@@ -167,6 +180,12 @@ void darwin_fields_a(Ctx& c, bool step_begin, Mark mark) {
 template <class Mark>
 void darwin_fields_b(Ctx& c, Mark mark) {
     float* apid[3] = {c.src.dcux, c.src.dcuy, c.src.dcuz};
+    if (c.gf) {      // amu waits in k_src, transformed along x
+        gridfft_rows_acc(c, c.acc_dcu, 0, 3, c.st->S_dcu, apid, false, false, false, c.k_dcu); mark(6); mark(7);
+        gridfft_cols_et(c, c.k_dcu, c.k_src + static_cast<size_t>(4) * c.sg.nk, c.k_et); mark(8); mark(9);
+        gridfft_fields_push(c, c.k_et); mark(10);
+        return;
+    }
     launch_finalize(c, c.acc_dcu, 0, 3, c.st->S_dcu, c.r_dcu, apid, false, false, false); mark(6);
     AW_CUFFT(cufftExecR2C(c.p_r2c3, c.r_dcu, c.k_dcu)); mark(7);
     launch_kspace_et(c, c.k_dcu, c.k_src + static_cast<size_t>(4) * c.sg.nk, c.k_et); mark(8);
@@ -542,6 +561,7 @@ int aw_ctx_create(const aw_grid* g, const aw_params* p, int32_t model, void* str
             for (cufftHandle ph : plans) if (ph) AW_CUFFT(cufftSetWorkArea(ph, c.fft_work));
             c.plans_made = true;
             aw::set_fft_stream(c);
+            if (model != AW_MODEL_YEE) aw::gridfft_make(c);
         } catch (...) {
             aw::free_all(c);
             throw;
@@ -810,6 +830,14 @@ int aw_solve_es(aw_ctx* ctx) {
         aw::need(ctx != nullptr, AW_ERR_ARG, "null ctx");
         Ctx& c = ctx->c;
         aw::need(c.src.rho && c.fld.Ex && c.fld.Ey, AW_ERR_STATE, "solve_es: rho/Ex/Ey not bound");
+        if (c.gf) {
+            const float* in[1] = {c.src.rho};
+            float* out[2] = {c.fld.Ex, c.fld.Ey};
+            aw::gridfft_rows_real(c, in, 1, c.k_src);
+            aw::gridfft_cols_es(c, c.k_src, c.k_out);
+            aw::gridfft_rows_planes(c, c.k_out, out, 2);
+            return;
+        }
         AW_CUFFT(cufftExecR2C(c.p_r2c1, c.src.rho, c.k_src));
         aw::launch_es_solve_k(c, c.k_src, c.k_out, c.k_out + c.sg.nk);
         AW_CUFFT(cufftExecC2R(c.p_c2r1, c.k_out, c.fld.Ex));
@@ -823,6 +851,14 @@ static void solve_el_b_into(Ctx& c, float* ex, float* ey) {
     aw::need(s.rho && s.Jx && s.Jy && s.Jz, AW_ERR_STATE, "rho/J not bound");
     aw::need(ex && ey && c.fld.Bx && c.fld.By && c.fld.Bz, AW_ERR_STATE, "E/B fields not bound");
     const size_t nk = c.sg.nk;
+    if (c.gf) {
+        const float* in[4] = {s.rho, s.Jx, s.Jy, s.Jz};
+        float* out[5] = {ex, ey, c.fld.Bx, c.fld.By, c.fld.Bz};
+        aw::gridfft_rows_real(c, in, 4, c.k_src);
+        aw::gridfft_cols_elb(c, c.k_src, c.k_out);
+        aw::gridfft_rows_planes(c, c.k_out, out, 5);
+        return;
+    }
     AW_CUFFT(cufftExecR2C(c.p_r2c1, s.rho, c.k_src));
     AW_CUFFT(cufftExecR2C(c.p_r2c1, s.Jx, c.k_src + nk));
     AW_CUFFT(cufftExecR2C(c.p_r2c1, s.Jy, c.k_src + 2 * nk));
@@ -859,6 +895,14 @@ int aw_solve_darwin_et(aw_ctx* ctx) {
                  "solve_darwin_et: dcu/amu not bound");
         aw::need(c.fld.ETx && c.fld.ETy && c.fld.ETz, AW_ERR_STATE, "solve_darwin_et: ET not bound");
         const size_t nk = c.sg.nk;
+        if (c.gf) {
+            const float* in[7] = {s.dcux, s.dcuy, s.dcuz, s.amu0, s.amu1, s.amu2, s.amu3};
+            float* out[3] = {c.fld.ETx, c.fld.ETy, c.fld.ETz};
+            aw::gridfft_rows_real(c, in, 7, c.k_src);
+            aw::gridfft_cols_et(c, c.k_src, c.k_src + 3 * nk, c.k_et);
+            aw::gridfft_rows_planes(c, c.k_et, out, 3);
+            return;
+        }
         const float* ins[3] = {s.dcux, s.dcuy, s.dcuz};
         for (int f = 0; f < 3; ++f) AW_CUFFT(cufftExecR2C(c.p_r2c1, const_cast<float*>(ins[f]), c.k_dcu + f * nk));
         const float* am[4] = {s.amu0, s.amu1, s.amu2, s.amu3};

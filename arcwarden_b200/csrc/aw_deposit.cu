@@ -613,10 +613,6 @@ __device__ __forceinline__ bool chunk_box(float* stage, int cs, int cnt, float x
     b.nJ = w.hi_j - w.lo_j + 1;
     return true;
 }
-// Row of cell c in a box of rows of W cells, r = 1 / W: the half keeps the product
-// off the integers by more than its rounding for any c below 2^21.
-__device__ __forceinline__ int row_of(int c, float r) { return static_cast<int>((static_cast<float>(c) + 0.5f) * r); }
-
 // The window of box b widened by mg cells; false when it does not fit P1 cells.
 // A dimension the window would span whole (a margin wider than the grid, e.g.
 // ny = 1) is taken from cell 0 with its n + 1 cells: the flush wraps each index

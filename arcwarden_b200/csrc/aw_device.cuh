@@ -110,6 +110,10 @@ __device__ __forceinline__ void set_err(DevState* st, unsigned bits) {
     atomicOr(&st->err, bits);
 }
 
+// c / W for r = 1 / W: the half keeps the product off the integers by more than its
+// rounding for any c below 2^21.
+__device__ __forceinline__ int row_of(int c, float r) { return static_cast<int>((static_cast<float>(c) + 0.5f) * r); }
+
 // Power-of-two scale S such that bound * S < 2^top (the fast path uses
 // top = 22), from a positive bound. Deterministic: a pure function of the bound.
 __host__ __device__ inline float scale_for_bound(float bound, int top = 22) {

@@ -1,0 +1,566 @@
+// aw_gridfft.cuh — the grid solves as three kernels each (included by
+// aw_spectral.cu inside its anonymous namespace).
+//
+//   k_rows_fwd   rows in, real -> complex along x. The rows come from the int64
+//                accumulators (the finalisation: scale, reset, caller's arrays,
+//                charge partial, the step's opening) or from real planes.
+//   k_cols       complex along y, the solve's multiplier in k-space, and back.
+//   k_rows_inv   complex -> real along x, and what the fields are for: gather
+//                buffers, caller's arrays, maxima and energy partials.
+//
+// A solve through the library transforms takes seven launches and writes every
+// plane to memory between them; on grids of this path (up to 1024 on a side, a few
+// MB) the launches and the latency of seven dependent kernels are its time, not the
+// bytes or the arithmetic. Here a row or column lives in shared memory from its
+// load to its last use.
+//
+// Two rows share one complex transform (z = a + i b, a and b of one field, so their
+// magnitudes are alike). Between the kernels a field is stored transposed,
+// [k][j], so that the columns are contiguous and a block of PR row pairs reads and
+// writes 16 PR bytes at a time. The transforms are Stockham passes of radix 8, 4,
+// 2, 3, 5, 7 between two shared buffers, padded by one element in 16 so that a pass's
+// strided writes spread over the banks; the twiddles are rounded from double.
+
+constexpr int kFftMax = 1024;          // longest row or column
+struct FftPlan {
+    int n, np;
+    int r[12];
+    float rnb[12], rl[12];             // 1 / (n / r), 1 / (product of the radices before)
+};
+__device__ __forceinline__ int fpad(int i) { return i + (i >> 4); }
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// a * (SIGN i)
+template <int SIGN> __device__ __forceinline__ float2 cimul(float2 a) {
+    return SIGN < 0 ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
+}
+
+// In-register transforms of R values, kernel exp(SIGN 2 pi i p q / R).
+template <int R, int SIGN> struct Dft;
+template <int SIGN> struct Dft<2, SIGN> {
+    static __device__ __forceinline__ void run(float2 (&v)[2]) {
+        const float2 a = v[0];
+        v[0] = cadd(a, v[1]); v[1] = csub(a, v[1]);
+    }
+};
+template <int SIGN> struct Dft<4, SIGN> {
+    static __device__ __forceinline__ void run(float2 (&v)[4]) {
+        const float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]), d = cimul<SIGN>(csub(v[1], v[3]));
+        v[0] = cadd(a, c); v[1] = cadd(b, d); v[2] = csub(a, c); v[3] = csub(b, d);
+    }
+};
+template <int SIGN> struct Dft<8, SIGN> {
+    static __device__ __forceinline__ void run(float2 (&v)[8]) {
+        float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        Dft<4, SIGN>::run(e);
+        Dft<4, SIGN>::run(o);
+        constexpr float h = 0.70710678118654752440f;
+        const float2 i1 = cimul<SIGN>(o[1]), i3 = cimul<SIGN>(o[3]);
+        o[1] = make_float2(h * (o[1].x + i1.x), h * (o[1].y + i1.y));
+        o[2] = cimul<SIGN>(o[2]);
+        o[3] = make_float2(h * (i3.x - o[3].x), h * (i3.y - o[3].y));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { v[k] = cadd(e[k], o[k]); v[k + 4] = csub(e[k], o[k]); }
+    }
+};
+// Odd R: with s_p = v_p + v_(R-p), d_p = v_p - v_(R-p),
+// V_q = v_0 + sum_p cos(2 pi p q / R) s_p + SIGN i sum_p sin(2 pi p q / R) d_p.
+template <int R> struct OddTab;
+template <> struct OddTab<3> {
+    static __device__ __forceinline__ float c(int) { return -0.5f; }
+    static __device__ __forceinline__ float s(int m) { return m == 1 ? 0.86602540378443864676f : -0.86602540378443864676f; }
+};
+template <> struct OddTab<5> {
+    static __device__ __forceinline__ float c(int m) { return (m == 1 || m == 4) ? 0.30901699437494742410f : -0.80901699437494742410f; }
+    static __device__ __forceinline__ float s(int m) {
+        return m == 1 ? 0.95105651629515357212f : m == 2 ? 0.58778525229247312917f
+             : m == 3 ? -0.58778525229247312917f : -0.95105651629515357212f;
+    }
+};
+template <> struct OddTab<7> {
+    static __device__ __forceinline__ float c(int m) {
+        return (m == 1 || m == 6) ? 0.62348980185873353053f : (m == 2 || m == 5) ? -0.22252093395631440429f
+                                                                                 : -0.90096886790241912624f;
+    }
+    static __device__ __forceinline__ float s(int m) {
+        return m == 1 ? 0.78183148246802980871f : m == 2 ? 0.97492791218182360702f : m == 3 ? 0.43388373911755812048f
+             : m == 4 ? -0.43388373911755812048f : m == 5 ? -0.97492791218182360702f : -0.78183148246802980871f;
+    }
+};
+template <int R, int SIGN> struct Dft {
+    static __device__ __forceinline__ void run(float2 (&v)[R]) {
+        constexpr int H = R / 2;
+        float2 s[H], d[H], V[R];
+        float2 t = v[0];
+#pragma unroll
+        for (int p = 0; p < H; ++p) {
+            s[p] = cadd(v[p + 1], v[R - 1 - p]);
+            d[p] = csub(v[p + 1], v[R - 1 - p]);
+            t = cadd(t, s[p]);
+        }
+        V[0] = t;
+#pragma unroll
+        for (int q = 1; q <= H; ++q) {
+            float2 a = v[0], b = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int p = 0; p < H; ++p) {
+                const int m = ((p + 1) * q) % R;
+                const float c = OddTab<R>::c(m), w = OddTab<R>::s(m);
+                a.x = __fmaf_rn(c, s[p].x, a.x); a.y = __fmaf_rn(c, s[p].y, a.y);
+                b.x = __fmaf_rn(w, d[p].x, b.x); b.y = __fmaf_rn(w, d[p].y, b.y);
+            }
+            const float2 ib = cimul<SIGN>(b);
+            V[q] = cadd(a, ib);
+            V[R - q] = csub(a, ib);
+        }
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = V[q];
+    }
+};
+
+// One Stockham pass of radix R over `batch` sequences (stride rs), l the product
+// of the radices before: element i + q n/R -> (i - i mod l) R + i mod l + q l.
+template <int R, int SIGN>
+__device__ __forceinline__ void fft_pass(const float2* __restrict__ in, float2* __restrict__ out, int batch, int rs,
+                                         int n, int l, float rnb, float rl, const float2* __restrict__ tw) {
+    const int nb = n / R, step = nb / l;            // twiddle of (q, k): tw[q k n / (l R)]
+    for (int t = threadIdx.x; t < batch * nb; t += blockDim.x) {
+        const int b = row_of(t, rnb), i = t - b * nb;
+        const int k = i - row_of(i, rl) * l;
+        float2 v[R];
+        const float2* x = in + b * rs;
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = x[fpad(i + q * nb)];
+        if (l > 1) {
+#pragma unroll
+            for (int q = 1; q < R; ++q) {
+                float2 w = tw[q * k * step];
+                if (SIGN > 0) w.y = -w.y;
+                v[q] = cmul(v[q], w);
+            }
+        }
+        Dft<R, SIGN>::run(v);
+        float2* y = out + b * rs;
+        const int o = (i - k) * R + k;
+#pragma unroll
+        for (int q = 0; q < R; ++q) y[fpad(o + q * l)] = v[q];
+    }
+}
+// The whole transform; the sequences are in `a` (written by this block, not yet
+// synced) and come back in the buffer returned (synced).
+template <int SIGN>
+__device__ __forceinline__ float2* fft_run(float2* a, float2* b, int batch, int rs, const FftPlan& p,
+                                           const float2* __restrict__ tw) {
+    int l = 1;
+    __syncthreads();
+    for (int s = 0; s < p.np; ++s) {
+        const int r = p.r[s];
+        const float rnb = p.rnb[s], rl = p.rl[s];
+        if (r == 8) fft_pass<8, SIGN>(a, b, batch, rs, p.n, l, rnb, rl, tw);
+        else if (r == 4) fft_pass<4, SIGN>(a, b, batch, rs, p.n, l, rnb, rl, tw);
+        else if (r == 2) fft_pass<2, SIGN>(a, b, batch, rs, p.n, l, rnb, rl, tw);
+        else if (r == 3) fft_pass<3, SIGN>(a, b, batch, rs, p.n, l, rnb, rl, tw);
+        else if (r == 5) fft_pass<5, SIGN>(a, b, batch, rs, p.n, l, rnb, rl, tw);
+        else fft_pass<7, SIGN>(a, b, batch, rs, p.n, l, rnb, rl, tw);
+        __syncthreads();
+        l *= r;
+        float2* t = a; a = b; b = t;
+    }
+    return a;
+}
+// The twiddle table into shared memory (published by fft_run's first barrier).
+__device__ __forceinline__ void load_twiddles(float2* __restrict__ dst, const float2* __restrict__ tw, int n) {
+    for (int t = threadIdx.x; t < n; t += kThreads) dst[t] = __ldg(tw + t);
+}
+// Stride of a sequence of n elements in shared memory: padded, and congruent to 4
+// modulo 16 elements so that neighbouring sequences start on different banks.
+__host__ __device__ inline int fft_stride(int n) {
+    const int p = n + (n >> 4) + 1;
+    return p + ((4 - p) & 15);
+}
+
+// What every kernel of a solve knows of the grid.
+struct GridFftArgs {
+    FftPlan px, py;
+    const float2 *twx, *twy;
+    int nx, ny, nkx, ncell, nk;
+    int pr;                            // row pairs per block
+    int rsx, rsy;                      // sequence strides
+};
+
+// ---- rows, forward ----------------------------------------------------------------
+struct RowsFwd {
+    GridFftArgs g;
+    const float* src[8];               // real planes (ACC = false)
+    unsigned long long* acc;           // ACC: the accumulators, field `first` + blockIdx.y
+    int first;
+    const float* S;
+    FinOut api;
+    double* part;                      // charge partials, or null
+    DevState* st;
+    int step_begin, darwin, sub_ref;
+    double dt;
+    float cref;
+    AdjDev* rec;
+    float2* out;                       // [field][nkx][ny]
+};
+template <bool ACC>
+__global__ void __launch_bounds__(kThreads) k_rows_fwd(RowsFwd A) {
+    extern __shared__ __align__(16) float2 fsm[];
+    const GridFftArgs& g = A.g;
+    const int f = blockIdx.y, p0 = blockIdx.x * g.pr;
+    float2* const tw = fsm;
+    float2* const b0 = tw + ((g.nx + 1) & ~1);
+    float2* const b1 = b0 + g.pr * g.rsx;
+    load_twiddles(tw, g.twx, g.nx);
+    double qsum = 0.0;
+    const double invS = ACC ? __drcp_rn(static_cast<double>(A.S[A.first + f])) : 0.0;
+    const double ref0 = (ACC && A.sub_ref && A.first + f == 0) ? A.st->rho_ref : 0.0;
+    const float rnx = 1.0f / static_cast<float>(g.nx);
+    unsigned long long* const acc = ACC ? A.acc + static_cast<size_t>(A.first + f) * g.ncell : nullptr;
+    const float* const src = ACC ? nullptr : A.src[f];
+    float* const api = ACC ? A.api.p[f] : nullptr;
+    auto value = [&](long long q, int c) {       // one cell's finalised value -> the caller's array, the transform's input
+        const double d = static_cast<double>(q) * invS;
+        const float a = __double2float_rn(d);
+        if (api) api[c] = a;
+        if (A.first + f != 0) return a;
+        qsum += static_cast<double>(a);
+        return __double2float_rn(d - ref0);
+    };
+    if (ACC && (g.nx & 1) == 0) {
+        // two cells of both rows per turn, U turns' loads before the first store
+        constexpr int U = 4;
+        const int hx = g.nx >> 1, m = g.pr * hx;
+        const float rhx = 1.0f / static_cast<float>(hx);
+        const longlong2* const q = reinterpret_cast<const longlong2*>(acc);
+        for (int t0 = threadIdx.x; t0 < m; t0 += U * kThreads) {
+            longlong2 v[U][2];
+            int c[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int t = t0 + u * kThreads;
+                const int pr = row_of(t, rhx), ja = 2 * (p0 + pr);
+                c[u] = ja * hx + t - pr * hx;                       // in pairs of cells
+                v[u][0] = v[u][1] = make_longlong2(0, 0);
+                if (t < m && ja < g.ny) v[u][0] = q[c[u]];
+                if (t < m && ja + 1 < g.ny) v[u][1] = q[c[u] + hx];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int t = t0 + u * kThreads;
+                if (t >= m) continue;
+                const int pr = row_of(t, rhx), x = 2 * (t - pr * hx), ja = 2 * (p0 + pr);
+                float a0 = 0.f, a1 = 0.f, b0v = 0.f, b1v = 0.f;
+                if (ja < g.ny) {
+                    reinterpret_cast<longlong2*>(acc)[c[u]] = make_longlong2(0, 0);
+                    a0 = value(v[u][0].x, 2 * c[u]); a1 = value(v[u][0].y, 2 * c[u] + 1);
+                }
+                if (ja + 1 < g.ny) {
+                    reinterpret_cast<longlong2*>(acc)[c[u] + hx] = make_longlong2(0, 0);
+                    b0v = value(v[u][1].x, 2 * c[u] + g.nx); b1v = value(v[u][1].y, 2 * c[u] + g.nx + 1);
+                }
+                float2* o = b0 + pr * g.rsx;
+                o[fpad(x)] = make_float2(a0, b0v);
+                o[fpad(x + 1)] = make_float2(a1, b1v);
+            }
+        }
+    } else {
+        for (int t = threadIdx.x; t < g.pr * g.nx; t += kThreads) {
+            const int pr = row_of(t, rnx), x = t - pr * g.nx;
+            const int ja = 2 * (p0 + pr);
+            float v[2] = {0.f, 0.f};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (ja + h >= g.ny) continue;
+                const int c = (ja + h) * g.nx + x;
+                if (ACC) {
+                    const long long q = static_cast<long long>(acc[c]);
+                    acc[c] = 0ull;
+                    v[h] = value(q, c);
+                } else {
+                    v[h] = src[c];
+                }
+            }
+            b0[pr * g.rsx + fpad(x)] = make_float2(v[0], v[1]);
+        }
+    }
+    const float2* z = fft_run<-1>(b0, b1, g.pr, g.rsx, g.px, tw);
+    // row a: (Z_k + conj Z_-k) / 2, row b: (Z_k - conj Z_-k) / (2 i)
+    float2* const out = A.out + static_cast<size_t>(f) * g.nk;
+    const float rpr = 1.0f / static_cast<float>(g.pr);
+    for (int t = threadIdx.x; t < g.pr * g.nkx; t += kThreads) {
+        const int k = row_of(t, rpr), pr = t - k * g.pr;
+        const int ja = 2 * (p0 + pr);
+        if (ja >= g.ny) continue;
+        const float2* s = z + pr * g.rsx;
+        const float2 zk = s[fpad(k)], zm = s[fpad(k == 0 ? 0 : g.nx - k)];
+        const float2 a = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+        const float2 b = make_float2(0.5f * (zk.y + zm.y), 0.5f * (zm.x - zk.x));
+        float2* o = out + static_cast<size_t>(k) * g.ny + ja;
+        if ((g.ny & 1) == 0) *reinterpret_cast<float4*>(o) = make_float4(a.x, a.y, b.x, b.y);
+        else { o[0] = a; if (ja + 1 < g.ny) o[1] = b; }
+    }
+    if (ACC && A.part && A.first + f == 0) {
+        __shared__ double sh[kThreads / 32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) qsum += __shfl_down_sync(0xffffffffu, qsum, o);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = qsum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double s = 0;
+            for (int w = 0; w < kThreads / 32; ++w) s += sh[w];
+            A.part[blockIdx.x * 5 + 2] = s;
+        }
+        // the partial rows no block of this launch owns
+        for (int b = gridDim.x + blockIdx.x * kThreads + threadIdx.x; b < kGridBlocks; b += gridDim.x * kThreads)
+            A.part[b * 5 + 2] = 0.0;
+    }
+    if (ACC && A.step_begin && blockIdx.x == 0 && f == 0 && threadIdx.x == 0) {
+        if (A.rec) A.rec->rec_slot += 1;     // the recorded step's trajectory slot
+        open_step(A.st, A.dt, A.cref, A.darwin != 0);
+    }
+}
+
+// ---- columns -----------------------------------------------------------------------
+// Op: NI planes in, NO planes out (at most NI or NO held at once), one mode at a time.
+template <class Op>
+struct ColsArgs {
+    GridFftArgs g;
+    const float2* in[Op::NI];          // [nkx][ny] each
+    float2* out;                       // [NO][nkx][ny]
+    int cols;                          // columns per block
+    Op op;
+};
+template <class Op>
+__global__ void __launch_bounds__(kThreads) k_cols(ColsArgs<Op> A) {
+    constexpr int NI = Op::NI, NO = Op::NO, NB = NI > NO ? NI : NO;
+    extern __shared__ __align__(16) float2 fsm[];
+    const GridFftArgs& g = A.g;
+    const int k0 = blockIdx.x * A.cols, C = min(A.cols, g.nkx - k0);
+    float2* const tw = fsm;
+    float2* const b0 = tw + ((g.ny + 1) & ~1);
+    float2* const b1 = b0 + NB * A.cols * g.rsy;
+    load_twiddles(tw, g.twy, g.ny);
+    const float rny = 1.0f / static_cast<float>(g.ny);
+    const int m = C * g.ny;
+#pragma unroll
+    for (int f = 0; f < NI; ++f)
+        for (int t = threadIdx.x; t < m; t += kThreads) {
+            const int c = row_of(t, rny), j = t - c * g.ny;
+            b0[(f * C + c) * g.rsy + fpad(j)] = __ldg(A.in[f] + static_cast<size_t>(k0) * g.ny + t);
+        }
+    float2* z = fft_run<-1>(b0, b1, NI * C, g.rsy, g.py, tw);
+    for (int t = threadIdx.x; t < m; t += kThreads) {
+        const int c = row_of(t, rny), j = t - c * g.ny;
+        float2 in[NI], out[NO];
+#pragma unroll
+        for (int f = 0; f < NI; ++f) in[f] = z[(f * C + c) * g.rsy + fpad(j)];
+        A.op(k0 + c, j, in, out);
+#pragma unroll
+        for (int f = 0; f < NO; ++f) z[(f * C + c) * g.rsy + fpad(j)] = out[f];
+    }
+    float2* const other = z == b0 ? b1 : b0;
+    const float2* y = fft_run<1>(z, other, NO * C, g.rsy, g.py, tw);
+#pragma unroll
+    for (int f = 0; f < NO; ++f)
+        for (int t = threadIdx.x; t < m; t += kThreads) {
+            const int c = row_of(t, rny), j = t - c * g.ny;
+            A.out[static_cast<size_t>(f) * g.nk + static_cast<size_t>(k0) * g.ny + t] = y[(f * C + c) * g.rsy + fpad(j)];
+        }
+}
+
+// ---- rows, inverse ------------------------------------------------------------------
+// Fin: what happens to a cell's NF field values; begin() and end() around a block's
+// cells (end may sync).
+template <class Fin>
+struct RowsInv {
+    GridFftArgs g;
+    const float2* in;                  // [NF][nkx][ny]
+    Fin fin;
+};
+template <class Fin>
+__global__ void __launch_bounds__(kThreads) k_rows_inv(RowsInv<Fin> A) {
+    constexpr int NF = Fin::NF;
+    extern __shared__ __align__(16) float2 fsm[];
+    const GridFftArgs& g = A.g;
+    const int p0 = blockIdx.x * g.pr;
+    float2* const tw = fsm;
+    float2* const b0 = tw + ((g.nx + 1) & ~1);
+    float2* const b1 = b0 + NF * g.pr * g.rsx;
+    load_twiddles(tw, g.twx, g.nx);
+    const float rpr = 1.0f / static_cast<float>(g.pr);
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+        for (int t = threadIdx.x; t < g.pr * g.nkx; t += kThreads) {
+            const int k = row_of(t, rpr), pr = t - k * g.pr;
+            const int ja = 2 * (p0 + pr);
+            float2 a = make_float2(0.f, 0.f), b = a;
+            if (ja < g.ny) {
+                const float2* o = A.in + static_cast<size_t>(f) * g.nk + static_cast<size_t>(k) * g.ny + ja;
+                if ((g.ny & 1) == 0) {
+                    const float4 q = __ldg(reinterpret_cast<const float4*>(o));
+                    a = make_float2(q.x, q.y); b = make_float2(q.z, q.w);
+                } else {
+                    a = __ldg(o);
+                    if (ja + 1 < g.ny) b = __ldg(o + 1);
+                }
+            }
+            // Z = A + i B with A, B Hermitian: the k = 0 and Nyquist modes of a real row are real
+            float2* s = b0 + (f * g.pr + pr) * g.rsx;
+            if (k == 0 || 2 * k == g.nx) {
+                s[fpad(k)] = make_float2(a.x, b.x);
+            } else {
+                s[fpad(k)] = make_float2(a.x - b.y, a.y + b.x);
+                s[fpad(g.nx - k)] = make_float2(a.x + b.y, b.x - a.y);
+            }
+        }
+    const float2* z = fft_run<1>(b0, b1, NF * g.pr, g.rsx, g.px, tw);
+    const float rnx = 1.0f / static_cast<float>(g.nx);
+    Fin fin = A.fin;
+    fin.begin();
+    for (int t = threadIdx.x; t < g.pr * g.nx; t += kThreads) {
+        const int pr = row_of(t, rnx), x = t - pr * g.nx;
+        const int ja = 2 * (p0 + pr);
+        if (ja >= g.ny) continue;
+        float va[NF], vb[NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const float2 v = z[(f * g.pr + pr) * g.rsx + fpad(x)];
+            va[f] = v.x; vb[f] = v.y;
+        }
+        fin.cell(ja * g.nx + x, x, va);
+        if (ja + 1 < g.ny) fin.cell((ja + 1) * g.nx + x, x, vb);
+    }
+    fin.end();
+}
+// Partial rows [blockIdx.x] of a grid of fewer than kGridBlocks blocks: the rows
+// that no block owns are zeroed.
+__device__ __forceinline__ void zero_spare_partials(double* __restrict__ part) {
+    for (int b = gridDim.x + blockIdx.x * kThreads + threadIdx.x; b < kGridBlocks; b += gridDim.x * kThreads) {
+        part[b * 5 + 0] = 0.0; part[b * 5 + 1] = 0.0; part[b * 5 + 3] = 0.0;
+    }
+}
+// ES fields: gather buffer, planes, caller's arrays, trajectory, energy partials.
+struct FinEs {
+    static constexpr int NF = 2;
+    float *gb, *ex, *ey, *r;
+    double* part;
+    float2* traj; const AdjDev* rec;
+    int ncell;
+    double se2, me2;
+    float2* te;
+    __device__ void begin() {
+        se2 = 0.0; me2 = 0.0;
+        te = traj ? traj + static_cast<size_t>(rec->rec_slot) * ncell : nullptr;
+    }
+    __device__ void cell(int c, int, const float (&v)[2]) {
+        reinterpret_cast<float2*>(gb)[c] = make_float2(v[0], v[1]);
+        if (r) { r[c] = v[0]; r[ncell + c] = v[1]; }
+        if (te) te[c] = make_float2(v[0], v[1]);
+        if (ex) ex[c] = v[0];
+        if (ey) ey[c] = v[1];
+        const double e2 = double(v[0]) * v[0] + double(v[1]) * v[1];
+        se2 += e2;
+        me2 = fmax(me2, e2);
+    }
+    __device__ void end() { zero_spare_partials(part); grid_partials(se2, me2, 0.0, part); }
+};
+// Darwin, after the E_L, B solve (k_fields_dcu): planes E_L for the second solve.
+struct FinDcu {
+    static constexpr int NF = 5;
+    float *gb, *r;
+    FieldAPI api;
+    float b0x, b0y, b0z;
+    PumpArgs pa;
+    DevState* st;
+    int ncell;
+    double t;
+    float emax, bmax;
+    __device__ void begin() { t = st->t; emax = 0.f; bmax = 0.f; }
+    __device__ void cell(int c, int i, const float (&v)[5]) {
+        const float elx = v[0], ely = v[1], bx = v[2] + b0x, by = v[3] + b0y, bz = v[4] + b0z;
+        float ex = elx, ey = ely, ez = 0.0f;
+        pump_add(pa, i, t, ex, ey, ez);
+        float4* q = reinterpret_cast<float4*>(gb) + 2 * static_cast<size_t>(c);
+        q[0] = make_float4(ex, ey, ez, bx);
+        q[1] = make_float4(by, bz, 0.f, 0.f);
+        r[c] = elx; r[ncell + c] = ely;
+        if (api.ELx) api.ELx[c] = elx;
+        if (api.ELy) api.ELy[c] = ely;
+        if (api.Bx) api.Bx[c] = bx;
+        if (api.By) api.By[c] = by;
+        if (api.Bz) api.Bz[c] = bz;
+        emax = fmaxf(emax, fmaxf(fabsf(ex), fmaxf(fabsf(ey), fabsf(ez))));
+        bmax = fmaxf(bmax, fmaxf(fabsf(bx), fmaxf(fabsf(by), fabsf(bz))));
+    }
+    __device__ void end() { block_max_eb(emax, bmax, st); }
+};
+// Darwin, after the E_T solve (k_fields_push).
+struct FinPush {
+    static constexpr int NF = 3;
+    const float* rel;
+    const float* gbd;
+    float* gb;
+    FieldAPI api;
+    PumpArgs pa;
+    const DevState* st;
+    double* part;
+    int ncell;
+    double t, se2, me2, sb2;
+    __device__ void begin() { t = st->t; se2 = 0.0; me2 = 0.0; sb2 = 0.0; }
+    __device__ void cell(int c, int i, const float (&v)[3]) {
+        const float4* qd = reinterpret_cast<const float4*>(gbd) + 2 * static_cast<size_t>(c);
+        const float4 b1 = qd[0], b2 = qd[1];
+        float ex = rel[c] + 1.0f * v[0], ey = rel[ncell + c] + 1.0f * v[1], ez = 1.0f * v[2];
+        pump_add(pa, i, t, ex, ey, ez);
+        float4* q = reinterpret_cast<float4*>(gb) + 2 * static_cast<size_t>(c);
+        q[0] = make_float4(ex, ey, ez, b1.w);
+        q[1] = make_float4(b2.x, b2.y, 0.f, 0.f);
+        if (api.Ex) api.Ex[c] = ex;
+        if (api.Ey) api.Ey[c] = ey;
+        if (api.Ez) api.Ez[c] = ez;
+        if (api.ETx) api.ETx[c] = v[0];
+        if (api.ETy) api.ETy[c] = v[1];
+        if (api.ETz) api.ETz[c] = v[2];
+        const double e2 = double(ex) * ex + double(ey) * ey;
+        se2 += e2;
+        me2 = fmax(me2, e2);
+        sb2 += double(b1.w) * b1.w + double(b2.x) * b2.x + double(b2.y) * b2.y;
+    }
+    __device__ void end() { zero_spare_partials(part); grid_partials(se2, me2, sb2, part); }
+};
+// Plain planes (the unfused solves).
+template <int N>
+struct FinPlanes {
+    static constexpr int NF = N;
+    float* out[N];
+    __device__ void begin() {}
+    __device__ void cell(int c, int, const float (&v)[N]) {
+#pragma unroll
+        for (int f = 0; f < N; ++f) out[f][c] = v[f];
+    }
+    __device__ void end() {}
+};
+
+// ---- the solves' multipliers -----------------------------------------------------------
+struct OpEs {
+    static constexpr int NI = 1, NO = 2;
+    SpecGeo g; double eps0;
+    __device__ void operator()(int i, int j, const float2 (&in)[1], float2 (&out)[2]) const {
+        es_k(in[0], i, j, g, eps0, out[0], out[1]);
+    }
+};
+struct OpElb {
+    static constexpr int NI = 4, NO = 5;
+    SpecGeo g; double eps0, c;
+    __device__ void operator()(int i, int j, const float2 (&in)[4], float2 (&out)[5]) const { elb_k(i, j, g, eps0, c, in, out); }
+};
+struct OpEt {
+    static constexpr int NI = 7, NO = 3;      // dcu x y z, amu 0..3
+    SpecGeo g; double eps0, c, n0;
+    __device__ void operator()(int i, int j, const float2 (&in)[7], float2 (&out)[3]) const { et_k(i, j, g, eps0, c, n0, in, out); }
+};

@@ -166,6 +166,9 @@ struct Ctx {
     cufftHandle p_r2c3 = 0, p_c2r3 = 0;     // dcu / E_T batch 3
     cufftHandle p_r2c4 = 0;                 // rho+J batch 4 (unfused solve)
     void* fft_work = nullptr;
+    // the three-kernel grid solves (aw_gridfft.cuh), or null: a grid they do not
+    // cover, solved through the plans above
+    struct GridFft* gf = nullptr;
     bool plans_made = false;
 
     // graph
@@ -316,6 +319,23 @@ void launch_finalize(Ctx& c, unsigned long long* acc, int first, int nf, const f
                      bool sub_ref = false);
 // st->rho_ref from the pending charge deposit (acc_src field 0, scale S_pend[0]).
 void launch_charge_ref(Ctx& c);
+// The grid solves in three kernels (aw_gridfft.cuh): rows forward, columns with the
+// solve's multiplier, rows inverse. gridfft_make sets c.gf where both sides are
+// products of 2, 3, 5, 7 of at most 1024; the buffers hold planes [nkx][ny].
+void gridfft_make(Ctx& c);
+void gridfft_free(Ctx& c);
+// acc fields [first, first + nf) finalised (as launch_finalize, not accumulating) and
+// transformed along x into out.
+void gridfft_rows_acc(Ctx& c, unsigned long long* acc, int first, int nf, const float* S, float* const* api,
+                      bool charge_partials, bool step_begin, bool sub_ref, cufftComplex* out);
+void gridfft_rows_real(Ctx& c, const float* const* src, int nf, cufftComplex* out);
+void gridfft_cols_es(Ctx& c, const cufftComplex* rho, cufftComplex* out);           // -> Ex, Ey
+void gridfft_cols_elb(Ctx& c, const cufftComplex* rho_j, cufftComplex* out);         // -> ELx, ELy, Bx, By, Bz
+void gridfft_cols_et(Ctx& c, const cufftComplex* dcu, const cufftComplex* amu, cufftComplex* out);   // -> ETx, ETy, ETz
+void gridfft_fields_es(Ctx& c, const cufftComplex* in, bool planes);   // planes: r_out too
+void gridfft_fields_dcu(Ctx& c, const cufftComplex* in);
+void gridfft_fields_push(Ctx& c, const cufftComplex* in);
+void gridfft_rows_planes(Ctx& c, const cufftComplex* in, float* const* out, int nf);   // 2, 3 or 5 planes
 void launch_kspace_es(Ctx& c, const cufftComplex* rho_k, cufftComplex* e_k);
 void launch_es_solve_k(Ctx& c, const cufftComplex* rho_k, cufftComplex* ex_k, cufftComplex* ey_k);
 void launch_kspace_elb(Ctx& c, const cufftComplex* src_k, cufftComplex* out_k);

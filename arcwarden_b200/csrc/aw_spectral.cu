@@ -22,6 +22,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <memory>
+#include <vector>
 
 namespace aw {
 namespace {
@@ -73,6 +75,22 @@ __device__ void make_src_scales(const DevState* st, float cref, float (&S)[8], b
 #pragma unroll
         for (int f = 1; f < 8; ++f)
             if (st->rms_src[f] > 0.0f) S[f] = scale_for_bound(fminf(b[f], __fmul_rn(8.0f, st->rms_src[f])));
+    }
+}
+
+// Opens a step (one thread): its time, the |u| maxima of the state the last push
+// wrote, fresh field maxima, the scales of the step's source deposit.
+__device__ void open_step(DevState* st, double dt, float cref, bool darwin) {
+    st->t = static_cast<double>(st->step) * dt;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) { st->ucur_bits[d] = st->umax_bits[d]; st->umax_bits[d] = 0u; }
+    st->emax_bits = 0u; st->bmax_bits = 0u;
+    st->red_ticket = 0u;
+    if (darwin) {
+        float S[8];
+        make_src_scales(st, cref, S, true);
+#pragma unroll
+        for (int f = 0; f < 8; ++f) st->S_next[f] = S[f];
     }
 }
 
@@ -170,18 +188,7 @@ k_finalize(unsigned long long* __restrict__ acc, int first, int ncell,
     }
     if (step_begin && blockIdx.x == 0 && threadIdx.x == 0) {
         if (rec) rec->rec_slot += 1;     // the recorded step's trajectory slot
-        st->t = static_cast<double>(st->step) * dt;
-        // the particle state is the last push's output: its |u| maxima
-#pragma unroll
-        for (int d = 0; d < 3; ++d) { st->ucur_bits[d] = st->umax_bits[d]; st->umax_bits[d] = 0u; }
-        st->emax_bits = 0u; st->bmax_bits = 0u;
-        st->red_ticket = 0u;
-        if (darwin) {
-            float S[8];
-            make_src_scales(st, cref, S, true);
-#pragma unroll
-            for (int f = 0; f < 8; ++f) st->S_next[f] = S[f];
-        }
+        open_step(st, dt, cref, darwin != 0);
     }
 }
 
@@ -221,27 +228,20 @@ __global__ void k_kspace_es(const cufftComplex* __restrict__ rho_k, cufftComplex
     ey_k[t] = ey;
 }
 
-// src_k = [rho, Jx, Jy, Jz, ...] (stride nk); out_k = [ELx, ELy, Bx, By, Bz].
-__global__ void k_kspace_elb(const cufftComplex* __restrict__ src_k, cufftComplex* __restrict__ out_k,
-                             SpecGeo g, double eps0, double c) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.nk) return;
-    const int i = t % g.nkx, j = t / g.nkx;
-    const size_t nk = g.nk;
-    cufftComplex ex, ey;
-    es_k(src_k[t], i, j, g, eps0, ex, ey);
-    out_k[t] = ex;
-    out_k[nk + t] = ey;
+// in = [rho, Jx, Jy, Jz], out = [ELx, ELy, Bx, By, Bz] of mode (i, j).
+__device__ __forceinline__ void elb_k(int i, int j, const SpecGeo& g, double eps0, double c, const cufftComplex (&in)[4],
+                                      cufftComplex (&out)[5]) {
+    es_k(in[0], i, j, g, eps0, out[0], out[1]);
 
     const double kxi = kx_of(i, g.dkx), kyj = ky_of(j, g.ny, g.dky);
     const double k2 = kxi * kxi + kyj * kyj;
-    const double G = (k2 > 0.0 ? 1.0 / (eps0 * c * c * k2) : 0.0) * ffac_of(g, t);
+    const double G = (k2 > 0.0 ? 1.0 / (eps0 * c * c * k2) : 0.0) * ffac_of(g, j * g.nkx + i);
     cufftComplex bx, by, bz;
     if (nyquist(i, j, g.nx, g.ny) || k2 == 0.0) {
         bx.x = bx.y = by.x = by.y = bz.x = bz.y = 0.0f;
     } else {
         const double kx = kx_of(i, g.dkx), ky = ky_of(j, g.ny, g.dky);
-        const cufftComplex Jx = src_k[nk + t], Jy = src_k[2 * nk + t], Jz = src_k[3 * nk + t];
+        const cufftComplex Jx = in[1], Jy = in[2], Jz = in[3];
         bx.x = static_cast<float>(-G * ky * Jz.y) * g.invN;
         bx.y = static_cast<float>( G * ky * Jz.x) * g.invN;
         by.x = static_cast<float>( G * kx * Jz.y) * g.invN;
@@ -251,31 +251,39 @@ __global__ void k_kspace_elb(const cufftComplex* __restrict__ src_k, cufftComple
         bz.x = static_cast<float>(-G * Cy) * g.invN;
         bz.y = static_cast<float>( G * Cx) * g.invN;
     }
-    out_k[2 * nk + t] = bx;
-    out_k[3 * nk + t] = by;
-    out_k[4 * nk + t] = bz;
+    out[2] = bx;
+    out[3] = by;
+    out[4] = bz;
 }
-
-// dcu_k = [dcux, dcuy, dcuz], amu_k = [amu0..amu3] (stride nk); et_k = [ETx, ETy, ETz].
-__global__ void k_kspace_et(const cufftComplex* __restrict__ dcu_k, const cufftComplex* __restrict__ amu_k,
-                            cufftComplex* __restrict__ et_k, SpecGeo g, double eps0, double c, double n0) {
+// src_k = [rho, Jx, Jy, Jz, ...] (stride nk); out_k = [ELx, ELy, Bx, By, Bz].
+__global__ void k_kspace_elb(const cufftComplex* __restrict__ src_k, cufftComplex* __restrict__ out_k,
+                             SpecGeo g, double eps0, double c) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.nk) return;
-    const int i = t % g.nkx, j = t / g.nkx;
     const size_t nk = g.nk;
+    const cufftComplex in[4] = {src_k[t], src_k[nk + t], src_k[2 * nk + t], src_k[3 * nk + t]};
+    cufftComplex out[5];
+    elb_k(t % g.nkx, t / g.nkx, g, eps0, c, in, out);
+#pragma unroll
+    for (int f = 0; f < 5; ++f) out_k[f * nk + t] = out[f];
+}
+
+// in = [dcux, dcuy, dcuz, amu0..amu3], out = [ETx, ETy, ETz] of mode (i, j).
+__device__ __forceinline__ void et_k(int i, int j, const SpecGeo& g, double eps0, double c, double n0,
+                                     const cufftComplex (&in)[7], cufftComplex (&out)[3]) {
     const double kxi = kx_of(i, g.dkx), kyj = ky_of(j, g.ny, g.dky);
     const double k2 = kxi * kxi + kyj * kyj;
-    const double G = (k2 > 0.0 ? 1.0 / (eps0 * c * c * k2 + n0) : 0.0) * ffac_of(g, t);
+    const double G = (k2 > 0.0 ? 1.0 / (eps0 * c * c * k2 + n0) : 0.0) * ffac_of(g, j * g.nkx + i);
     cufftComplex ex, ey, ez;
     if (nyquist(i, j, g.nx, g.ny) || k2 == 0.0) {
         ex.x = ex.y = ey.x = ey.y = ez.x = ez.y = 0.0f;
     } else {
         const double kx = kx_of(i, g.dkx), ky = ky_of(j, g.ny, g.dky);
-        const cufftComplex a0 = amu_k[t], a1 = amu_k[nk + t], a2 = amu_k[2 * nk + t], a3 = amu_k[3 * nk + t];
+        const cufftComplex a0 = in[3], a1 = in[4], a2 = in[5], a3 = in[6];
         const double Sx_r = kx*a0.x + ky*a1.x, Sx_i = kx*a0.y + ky*a1.y;
         const double Sy_r = kx*a1.x - ky*a0.x, Sy_i = kx*a1.y - ky*a0.y;
         const double Sz_r = kx*a2.x + ky*a3.x, Sz_i = kx*a2.y + ky*a3.y;
-        const cufftComplex dcx = dcu_k[t], dcy = dcu_k[nk + t], dcz = dcu_k[2 * nk + t];
+        const cufftComplex dcx = in[0], dcy = in[1], dcz = in[2];
         double Jx_r = dcx.x + Sx_i, Jx_i = dcx.y - Sx_r;
         double Jy_r = dcy.x + Sy_i, Jy_i = dcy.y - Sy_r;
         double Jz_r = dcz.x + Sz_i, Jz_i = dcz.y - Sz_r;
@@ -288,9 +296,22 @@ __global__ void k_kspace_et(const cufftComplex* __restrict__ dcu_k, const cufftC
         ey.x = static_cast<float>(-G*Jy_r) * g.invN; ey.y = static_cast<float>(-G*Jy_i) * g.invN;
         ez.x = static_cast<float>(-G*Jz_r) * g.invN; ez.y = static_cast<float>(-G*Jz_i) * g.invN;
     }
-    et_k[t] = ex;
-    et_k[nk + t] = ey;
-    et_k[2 * nk + t] = ez;
+    out[0] = ex;
+    out[1] = ey;
+    out[2] = ez;
+}
+// dcu_k = [dcux, dcuy, dcuz], amu_k = [amu0..amu3] (stride nk); et_k = [ETx, ETy, ETz].
+__global__ void k_kspace_et(const cufftComplex* __restrict__ dcu_k, const cufftComplex* __restrict__ amu_k,
+                            cufftComplex* __restrict__ out_k, SpecGeo g, double eps0, double c, double n0) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= g.nk) return;
+    const size_t nk = g.nk;
+    const cufftComplex in[7] = {dcu_k[t], dcu_k[nk + t], dcu_k[2 * nk + t], amu_k[t], amu_k[nk + t], amu_k[2 * nk + t],
+                                amu_k[3 * nk + t]};
+    cufftComplex out[3];
+    et_k(t % g.nkx, t / g.nkx, g, eps0, c, n0, in, out);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) out_k[f * nk + t] = out[f];
 }
 
 // ---- real-space finalisers ----------------------------------------------------
@@ -702,6 +723,8 @@ k_step_reduce(const double* __restrict__ pp, const float* __restrict__ pc, const
     }
 }
 
+#include "aw_gridfft.cuh"
+
 __global__ void k_set_step(DevState* st, long long n) { st->step = n; }
 // The scales a step-begin finalise chose become the pending deposit's scales.
 __global__ void k_promote_scales(DevState* st) {
@@ -890,6 +913,176 @@ void launch_charge_ref(Ctx& c) {
     k_charge_ref<<<blocks, 256, 0, c.stream>>>(c.acc_src, c.geo.ncell, c.st->S_pend,
                                                reinterpret_cast<long long*>(c.red_rows), c.st);
     AW_LAUNCH();
+}
+
+// ---- the three-kernel grid solves -------------------------------------------------
+struct GridFft {
+    FftPlan px, py;
+    float2* tw = nullptr;              // [nx] then [ny]
+};
+namespace {
+// Radices of n, or false when it has a factor the passes do not take.
+bool make_fft_plan(FftPlan& p, int n) {
+    p = FftPlan{};
+    p.n = n;
+    if (n > kFftMax) return false;
+    int m = n, l = 1;
+    while (m > 1) {
+        const int r = m % 8 == 0 ? 8 : m % 4 == 0 ? 4 : m % 2 == 0 ? 2 : m % 3 == 0 ? 3 : m % 5 == 0 ? 5 : m % 7 == 0 ? 7 : 0;
+        if (r == 0) return false;
+        p.r[p.np] = r;
+        p.rnb[p.np] = 1.0f / static_cast<float>(n / r);
+        p.rl[p.np] = 1.0f / static_cast<float>(l);
+        ++p.np;
+        m /= r;
+        l *= r;
+    }
+    return true;
+}
+GridFftArgs gf_args(const Ctx& c) {
+    GridFftArgs g{};
+    g.px = c.gf->px; g.py = c.gf->py;
+    g.twx = c.gf->tw; g.twy = c.gf->tw + c.geo.nx;
+    g.nx = c.geo.nx; g.ny = c.geo.ny; g.nkx = c.sg.nkx; g.ncell = c.geo.ncell; g.nk = c.sg.nk;
+    g.rsx = fft_stride(g.nx); g.rsy = fft_stride(g.ny);
+    return g;
+}
+int pairs_of(const Ctx& c) { return (c.geo.ny + 1) / 2; }
+constexpr size_t kGfSmem = 96 * 1024;         // two blocks per SM, beside their twiddles
+size_t tw_bytes(int n) { return static_cast<size_t>((n + 1) & ~1) * sizeof(float2); }
+// The most items (row pairs or columns) per block, up to `most`, that fit kGfSmem and
+// still give every SM a block: wider blocks read and write longer runs.
+int gf_batch(const Ctx& c, int total, int other_blocks, size_t bytes_each, int most) {
+    int b = most;
+    while (b > 1 && (b * bytes_each > kGfSmem || (total + b - 1) / b * other_blocks < c.sms)) b >>= 1;
+    return b;
+}
+template <class Fin>
+void launch_rows_inv(Ctx& c, const cufftComplex* in, const Fin& fin) {
+    RowsInv<Fin> a{gf_args(c), in, fin};
+    const size_t each = static_cast<size_t>(2) * Fin::NF * a.g.rsx * sizeof(float2);
+    a.g.pr = gf_batch(c, pairs_of(c), 1, each, 4);
+    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
+    opt_in_smem(reinterpret_cast<const void*>(k_rows_inv<Fin>), sh);
+    k_rows_inv<Fin><<<(pairs_of(c) + a.g.pr - 1) / a.g.pr, kThreads, sh, c.stream>>>(a);
+    AW_LAUNCH();
+}
+template <class Op>
+void launch_cols(Ctx& c, const cufftComplex* const* in, cufftComplex* out, const Op& op) {
+    ColsArgs<Op> a{};
+    a.g = gf_args(c);
+    for (int f = 0; f < Op::NI; ++f) a.in[f] = in[f];
+    a.out = out;
+    a.op = op;
+    const size_t each = static_cast<size_t>(2) * std::max(Op::NI, Op::NO) * a.g.rsy * sizeof(float2);
+    a.cols = gf_batch(c, c.sg.nkx, 1, each, 8);
+    const size_t sh = each * a.cols + tw_bytes(a.g.ny);
+    opt_in_smem(reinterpret_cast<const void*>(k_cols<Op>), sh);
+    k_cols<Op><<<(c.sg.nkx + a.cols - 1) / a.cols, kThreads, sh, c.stream>>>(a);
+    AW_LAUNCH();
+}
+template <bool ACC>
+void launch_rows_fwd(Ctx& c, RowsFwd& a, int nf) {
+    const size_t each = static_cast<size_t>(2) * a.g.rsx * sizeof(float2);
+    a.g.pr = gf_batch(c, pairs_of(c), nf, each, 4);
+    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
+    opt_in_smem(reinterpret_cast<const void*>(k_rows_fwd<ACC>), sh);
+    k_rows_fwd<ACC><<<dim3((pairs_of(c) + a.g.pr - 1) / a.g.pr, nf), kThreads, sh, c.stream>>>(a);
+    AW_LAUNCH();
+}
+}  // namespace
+
+void gridfft_make(Ctx& c) {
+    // A row pair is one block's work: below 24 of them too few SMs take part, and the
+    // library transforms are faster (512 x 1: 58 us a step against 71; 64 x 64, 32
+    // pairs: 27.6 us either way; 256 x 256: 76.8 against 80.6).
+    if (c.geo.ny < 48) return;
+    FftPlan px, py;
+    if (c.geo.nx < 2 || !make_fft_plan(px, c.geo.nx) || !make_fft_plan(py, c.geo.ny)) return;
+    std::vector<float2> tw;
+    for (int n : {c.geo.nx, c.geo.ny})
+        for (int k = 0; k < n; ++k) {
+            const double a = -6.28318530717958647692 * k / n;
+            tw.push_back(make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a))));
+        }
+    std::unique_ptr<GridFft> f(new GridFft());
+    f->px = px; f->py = py;
+    AW_CUDA(cudaMalloc(reinterpret_cast<void**>(&f->tw), tw.size() * sizeof(float2)));
+    c.gf = f.release();
+    AW_CUDA(cudaMemcpy(c.gf->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice));
+}
+void gridfft_free(Ctx& c) {
+    if (!c.gf) return;
+    if (c.gf->tw) cudaFree(c.gf->tw);
+    delete c.gf;
+    c.gf = nullptr;
+}
+void gridfft_rows_acc(Ctx& c, unsigned long long* acc, int first, int nf, const float* S, float* const* api,
+                      bool charge_partials, bool step_begin, bool sub_ref, cufftComplex* out) {
+    RowsFwd a{};
+    a.g = gf_args(c);
+    a.acc = acc; a.first = first; a.S = S;
+    for (int f = 0; f < nf; ++f) a.api.p[f] = api ? api[f] : nullptr;
+    a.part = charge_partials ? c.part_g : nullptr;
+    a.st = c.st;
+    a.step_begin = step_begin ? 1 : 0; a.darwin = c.model == AW_MODEL_DARWIN ? 1 : 0; a.sub_ref = sub_ref ? 1 : 0;
+    a.dt = c.prm.dt; a.cref = cref_of(c);
+    a.rec = step_begin ? c.rec_ad : nullptr;
+    a.out = out;
+    launch_rows_fwd<true>(c, a, nf);
+}
+void gridfft_rows_real(Ctx& c, const float* const* src, int nf, cufftComplex* out) {
+    RowsFwd a{};
+    a.g = gf_args(c);
+    for (int f = 0; f < nf; ++f) a.src[f] = src[f];
+    a.out = out;
+    launch_rows_fwd<false>(c, a, nf);
+}
+void gridfft_cols_es(Ctx& c, const cufftComplex* rho, cufftComplex* out) {
+    launch_cols(c, &rho, out, OpEs{c.sg, c.prm.eps0});
+}
+void gridfft_cols_elb(Ctx& c, const cufftComplex* rho_j, cufftComplex* out) {
+    const cufftComplex* in[4];
+    for (int f = 0; f < 4; ++f) in[f] = rho_j + static_cast<size_t>(f) * c.sg.nk;
+    launch_cols(c, in, out, OpElb{c.sg, c.prm.eps0, c.prm.c});
+}
+void gridfft_cols_et(Ctx& c, const cufftComplex* dcu, const cufftComplex* amu, cufftComplex* out) {
+    const cufftComplex* in[7];
+    for (int f = 0; f < 7; ++f) in[f] = (f < 3 ? dcu + static_cast<size_t>(f) * c.sg.nk : amu + static_cast<size_t>(f - 3) * c.sg.nk);
+    launch_cols(c, in, out, OpEt{c.sg, c.prm.eps0, c.prm.c, c.prm.n0});
+}
+void gridfft_fields_es(Ctx& c, const cufftComplex* in, bool planes) {
+    FinEs f{};
+    f.gb = c.gb_es; f.ex = c.fld.Ex; f.ey = c.fld.Ey; f.r = planes ? c.r_out : nullptr;
+    f.part = c.part_g;
+    f.traj = reinterpret_cast<float2*>(c.rec_E); f.rec = c.rec_ad;
+    f.ncell = c.geo.ncell;
+    launch_rows_inv(c, in, f);
+}
+void gridfft_fields_dcu(Ctx& c, const cufftComplex* in) {
+    FinDcu f{};
+    f.gb = c.gb_dcu; f.r = c.r_out; f.api = api_of(c.fld);
+    f.b0x = c.prm.B0[0]; f.b0y = c.prm.B0[1]; f.b0z = c.prm.B0[2];
+    f.pa = pump_of(c); f.st = c.st; f.ncell = c.geo.ncell;
+    launch_rows_inv(c, in, f);
+}
+void gridfft_fields_push(Ctx& c, const cufftComplex* in) {
+    FinPush f{};
+    f.rel = c.r_out; f.gbd = c.gb_dcu; f.gb = c.gb_push; f.api = api_of(c.fld);
+    f.pa = pump_of(c); f.st = c.st; f.part = c.part_g; f.ncell = c.geo.ncell;
+    launch_rows_inv(c, in, f);
+}
+void gridfft_rows_planes(Ctx& c, const cufftComplex* in, float* const* out, int nf) {
+    auto go = [&](auto fin) {
+        for (int f = 0; f < nf; ++f) fin.out[f] = out[f];
+        launch_rows_inv(c, in, fin);
+    };
+    switch (nf) {
+        case 2: go(FinPlanes<2>{}); break;
+        case 3: go(FinPlanes<3>{}); break;
+        case 5: go(FinPlanes<5>{}); break;
+        default: throw Error(AW_ERR_ARG, "gridfft_rows_planes: 2, 3 or 5 planes");
+    }
 }
 
 void launch_make_scales(Ctx& c) {
