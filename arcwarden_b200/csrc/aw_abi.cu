@@ -88,11 +88,10 @@ void free_all(Ctx& c) {
     free_dadj(c);
     gridfft_free(c);
     if (c.gexec) cudaGraphExecDestroy(c.gexec);
-    if (c.graph) cudaGraphDestroy(c.graph);
     cufftHandle* plans[] = {&c.p_r2c1, &c.p_c2r1, &c.p_r2cS, &c.p_c2rO, &c.p_r2c3, &c.p_c2r3, &c.p_r2c4};
     for (cufftHandle* h : plans) if (*h) cufftDestroy(*h);
     void* bufs[] = {c.st, c.acc_src, c.acc_dcu, c.r_src, c.r_out, c.r_dcu, c.r_et, c.k_src, c.k_out,
-                    c.k_dcu, c.k_et, c.gb_es, c.gb_dcu, c.gb_push, c.part_p, c.part_c, c.part_d, c.part_g, c.diag, c.red_rows,
+                    c.k_dcu, c.k_et, c.gb_es, c.gb_dcu, c.gb_push, c.part_p, c.part_c, c.part_d, c.part_g, c.diag, c.ring, c.red_rows,
                     c.bin_count, c.bin_off, c.bin_cursor, c.bin_idx, c.sort_tmp, c.fft_work, c.rs_buf,
                     c.rs_temp, c.ffac, c.acc_tmp};
     for (void* b : bufs) if (b) cudaFree(b);
@@ -101,8 +100,8 @@ void free_all(Ctx& c) {
 
 void drop_graph(Ctx& c) {
     if (c.gexec) { cudaGraphExecDestroy(c.gexec); c.gexec = nullptr; }
-    if (c.graph) { cudaGraphDestroy(c.graph); c.graph = nullptr; }
     adj_drop_graphs(c);
+    dadj_drop_graph(c);
 }
 
 void set_fft_stream(Ctx& c) {
@@ -249,8 +248,9 @@ namespace aw {
 namespace {
 // Simulation<Cfg>::init: the t = 0 field solve, the ES half-step rollback and
 // the pending deposit of step 0. Synchronises.
+// The captured graphs stay: whatever they hold (bindings, parameters, plan, form
+// factor, filter) drops them when it changes. (Re-capturing took 0.4 ms of an init.)
 void init_impl(Ctx& c) {
-    aw::drop_graph(c);
     if (c.resort_every > 0) resort_reserve(c);
     aw::launch_set_step(c, 0);
     AW_CUDA(cudaMemsetAsync(&c.st->have_rms, 0, sizeof(int), c.stream));
@@ -345,7 +345,7 @@ double grad_es_impl(Ctx& c, long long nsteps, int every, float* dux, float* duy,
     const long long n = c.parts.n;
     const size_t nc = static_cast<size_t>(c.geo.ncell);
     copy_parts_to(c, w.init_parts);
-    init_impl(c);                                   // drops the step graphs, re-created below
+    init_impl(c);
     prep_adj_scatter();
     if (!c.gexec) c.gexec = capture_exec(c, [&] { step_body(c); });
     const AdjK kf = adj_constants(c, 1.0f);
@@ -525,6 +525,8 @@ int aw_ctx_create(const aw_grid* g, const aw_params* p, int32_t model, void* str
             aw::dalloc(c.diag, 1);
             aw::dalloc(c.red_rows, static_cast<size_t>(aw::kRedBlocks) * aw::kRedVals);
             AW_CUDA(cudaMemset(c.diag, 0, sizeof(aw_diag)));
+            aw::dalloc(c.ring, 1);
+            AW_CUDA(cudaMemset(c.ring, 0, 2 * sizeof(long long)));
             c.npart_g = aw::grid_partial_blocks();
             aw::dalloc(c.part_g, static_cast<size_t>(c.npart_g) * 5);
             AW_CUDA(cudaMemset(c.part_g, 0, sizeof(double) * c.npart_g * 5));
@@ -957,40 +959,38 @@ int aw_step(aw_ctx* ctx, int64_t n) {
     });
 }
 
+}  // extern "C"
+namespace aw {
+namespace {
+// The steps n0 .. n0 + nsteps - 1 (aw_run).
+void run_impl(Ctx& c, int64_t n0, int64_t nsteps, bool use_graph) {
+    need(nsteps >= 0, AW_ERR_ARG, "run: negative nsteps");
+    require_parts(c);
+    ensure_pending(c);
+    launch_set_step(c, n0);
+    // periodic re-sort (between steps, never inside the captured step)
+    auto resort_before = [&](int64_t i) {
+        const int64_t s = n0 + i;
+        if (c.resort_every > 0 && s > 0 && s % c.resort_every == 0) launch_resort(c);
+    };
+    if (!use_graph) {
+        for (int64_t i = 0; i < nsteps; ++i) { resort_before(i); step_body(c); }
+        return;
+    }
+    if (!c.gexec) c.gexec = capture_exec(c, [&] { step_body(c); });
+    for (int64_t i = 0; i < nsteps; ++i) {
+        resort_before(i);
+        AW_CUDA(cudaGraphLaunch(c.gexec, c.stream));
+    }
+}
+}  // namespace
+}  // namespace aw
+extern "C" {
+
 int aw_run(aw_ctx* ctx, int64_t n0, int64_t nsteps, int32_t use_graph) {
     return guarded([&] {
         aw::need(ctx != nullptr, AW_ERR_ARG, "null ctx");
-        aw::need(nsteps >= 0, AW_ERR_ARG, "run: negative nsteps");
-        Ctx& c = ctx->c;
-        aw::require_parts(c);
-        aw::ensure_pending(c);
-        aw::launch_set_step(c, n0);
-        // periodic re-sort (between steps, never inside the captured step)
-        auto resort_before = [&](int64_t i) {
-            const int64_t s = n0 + i;
-            if (c.resort_every > 0 && s > 0 && s % c.resort_every == 0) aw::launch_resort(c);
-        };
-        if (!use_graph) {
-            for (int64_t i = 0; i < nsteps; ++i) { resort_before(i); aw::step_body(c); }
-            return;
-        }
-        if (!c.gexec) {
-            AW_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-            try {
-                aw::step_body(c);
-            } catch (...) {
-                cudaGraph_t g = nullptr;
-                cudaStreamEndCapture(c.stream, &g);
-                if (g) cudaGraphDestroy(g);
-                throw;
-            }
-            AW_CUDA(cudaStreamEndCapture(c.stream, &c.graph));
-            AW_CUDA(cudaGraphInstantiate(&c.gexec, c.graph, 0));
-        }
-        for (int64_t i = 0; i < nsteps; ++i) {
-            resort_before(i);
-            AW_CUDA(cudaGraphLaunch(c.gexec, c.stream));
-        }
+        aw::run_impl(ctx->c, n0, nsteps, use_graph != 0);
     });
 }
 
@@ -1188,7 +1188,8 @@ int aw_tune_kernels(aw_ctx* ctx, int32_t trial_steps, aw_kernel_plan* chosen) {
                         const size_t i = round == 0 ? q : cands.size() - 1 - q;
                         copy(false);
                         c.plan = cands[i];
-                        aw::init_impl(c);                    // drops the graph; synchronises
+                        aw::drop_graph(c);                   // the captured step holds the old plan
+                        aw::init_impl(c);                    // synchronises
                         check_status(aw_run(ctx, 0, 2, 1));    // capture + warm-up
                         AW_CUDA(cudaEventRecord(e0, c.stream));
                         check_status(aw_run(ctx, 2, trial_steps, 1));
@@ -1217,6 +1218,7 @@ int aw_tune_kernels(aw_ctx* ctx, int32_t trial_steps, aw_kernel_plan* chosen) {
             g_tuned.push_back({key, best});
         }
         c.plan = best;
+        aw::drop_graph(c);
         aw::init_impl(c);      // the caller's initial state, initialised as by aw_init
         if (chosen) *chosen = best;
     });
@@ -1234,10 +1236,23 @@ int aw_run_diag(aw_ctx* ctx, int64_t n0, int64_t nsteps, int32_t use_graph, aw_d
     return guarded([&] {
         aw::need(ctx && host_out, AW_ERR_ARG, "null argument");
         Ctx& c = ctx->c;
-        for (int64_t i = 0; i < nsteps; ++i) {
-            const int rc = aw_run(ctx, n0 + i, 1, use_graph);
-            if (rc != AW_OK) throw Error(rc, aw::g_last_error);
-            AW_CUDA(cudaMemcpyAsync(host_out + i, c.diag, sizeof(aw_diag), cudaMemcpyDeviceToHost, c.stream));
+        // the step reductions write their records to the device ring, which is copied
+        // out once per batch: a copy between two steps would sit in their chain
+        for (int64_t i = 0; i < nsteps; i += aw::kDiagRing) {
+            const int64_t m = std::min<int64_t>(nsteps - i, aw::kDiagRing);
+            if (c.parts.n == 0) {          // a Yee vacuum run: no push counts its steps
+                for (int64_t k = i; k < i + m; ++k) {
+                    aw::run_impl(c, n0 + k, 1, use_graph != 0);
+                    AW_CUDA(cudaMemcpyAsync(host_out + k, c.diag, sizeof(aw_diag), cudaMemcpyDeviceToHost, c.stream));
+                }
+                continue;
+            }
+            AW_CUDA(cudaMemsetAsync(c.ring->rec, 0, sizeof(aw_diag) * static_cast<size_t>(m), c.stream));
+            aw::launch_set_ring(c, n0 + i, m);
+            aw::run_impl(c, n0 + i, m, use_graph != 0);
+            AW_CUDA(cudaMemcpyAsync(host_out + i, c.ring->rec, sizeof(aw_diag) * static_cast<size_t>(m),
+                                    cudaMemcpyDeviceToHost, c.stream));
+            aw::launch_set_ring(c, 0, 0);
         }
     });
 }

@@ -71,7 +71,8 @@ struct DAdjWS {
     float* X = nullptr;                  // [5][n] the backward step's saved state
     float* gbs = nullptr;                // [2][ncell][8] its gather buffers
     cufftHandle r2c3 = 0, c2r7 = 0, r2c5 = 0, c2r4 = 0;
-    cudaGraphExec_t back = nullptr;      // one backward step
+    cudaGraphExec_t back = nullptr;      // one backward step of a gradient over back_steps steps
+    long long back_steps = 0;
     double* part = nullptr;              // [148] pump-term block partials
     ~DAdjWS() {
         if (back) cudaGraphExecDestroy(back);
@@ -82,6 +83,12 @@ struct DAdjWS {
         for (cufftHandle x : h) if (x) cufftDestroy(x);
     }
 };
+
+void dadj_drop_graph(Ctx& c) {
+    if (!c.dadj || !c.dadj->back) return;
+    cudaGraphExecDestroy(c.dadj->back);
+    c.dadj->back = nullptr;
+}
 
 void free_dadj(Ctx& c) {
     delete c.dadj;
@@ -589,10 +596,7 @@ double grad_darwin_impl(Ctx& c, long long nsteps, int every, float* dux, float* 
     }
     DAdjWS& w = *c.dadj;
     double* const part = w.part;
-    if (w.back) {                      // captured with the previous call's parameters
-        cudaGraphExecDestroy(w.back);
-        w.back = nullptr;
-    }
+    if (w.back_steps != nsteps) dadj_drop_graph(c);     // it knows the last step
     cufftHandle hs[] = {w.r2c3, w.c2r7, w.r2c5, w.c2r4};
     for (cufftHandle h : hs) AW_CUFFT(cufftSetStream(h, c.stream));
     AW_CUDA(cudaMemsetAsync(w.acc, 0, sizeof(unsigned long long) * 6 * nc, c.stream));
@@ -673,7 +677,8 @@ double grad_darwin_impl(Ctx& c, long long nsteps, int every, float* dux, float* 
     // the fixed buffers w.X, w.gbs, reads its step from w.slot[1] and moves the
     // slot one step back, so the same graph replays every step.
     prepare_scatter6();
-    {
+    if (!w.back) {
+        w.back_steps = nsteps;
         const float* X = w.X;
         const float* gbd = w.gbs;
         const float* gbp = w.gbs + 8 * static_cast<size_t>(nc);

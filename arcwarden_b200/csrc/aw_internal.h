@@ -141,6 +141,8 @@ struct Ctx {
     int     npart_p = 0, npart_g = 0;
     bool    parts_bound = false; // aw_particles_bind has run (n may be 0)
     aw_diag* diag = nullptr;    // device aw_diag
+    struct DiagRing* ring = nullptr;   // aw_run_diag's records: the step reduction writes step s's
+                                // to rec[s - base] while 0 <= s - base < n
     double* red_rows = nullptr; // k_step_reduce block rows [kRedBlocks][kRedVals]
     // tile binning scratch
     int* bin_count = nullptr; int* bin_off = nullptr; int* bin_cursor = nullptr;
@@ -172,7 +174,6 @@ struct Ctx {
     bool plans_made = false;
 
     // graph
-    cudaGraph_t     graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     bool inited = false;
     bool pending_valid = false;       // acc_src holds the deposit of the current state
@@ -205,6 +206,13 @@ struct Ctx {
 
     int nsrc() const { return model == AW_MODEL_DARWIN ? 8 : model == AW_MODEL_YEE ? 3 : 1; }
     int nout() const { return model == AW_MODEL_DARWIN ? 5 : 2; }
+};
+
+// The records of a batch of steps on the device (aw_run_diag copies them out together).
+constexpr int kDiagRing = 1024;
+struct DiagRing {
+    long long base, n;
+    aw_diag rec[kDiagRing];
 };
 
 // Device constants of one ES adjoint step: the push's half-step factor, the
@@ -351,6 +359,7 @@ void launch_add_pump(Ctx& c, double t);
 void launch_pack_em(Ctx& c);
 void launch_grid_diag(Ctx& c);
 void launch_set_step(Ctx& c, long long n);
+void launch_set_ring(Ctx& c, long long base, long long n);
 void launch_copy_umax(Ctx& c);
 void launch_promote_scales(Ctx& c);                // S_pend = S_next
 void launch_rms_reduce(Ctx& c, bool src, bool dcu);
@@ -384,6 +393,7 @@ AdjK adj_constants(const Ctx& c, float dt_scale);
 void adj_prepare(Ctx& c, long long nsteps, int every);   // (re)allocates c.adj
 void free_adjoint(Ctx& c);
 void free_dadj(Ctx& c);      // aw_adjoint_darwin.cu: releases c.dadj
+void dadj_drop_graph(Ctx& c);
 // lE = acc / S + ad->ext_scale * E_slot (E of the slot's step, interleaved
 // [ncell][2]); acc is zeroed.
 void launch_adj_finalize(Ctx& c);

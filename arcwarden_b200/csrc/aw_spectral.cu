@@ -649,7 +649,7 @@ template <bool RMS>
 __global__ void __launch_bounds__(kThreads)
 k_step_reduce(const double* __restrict__ pp, const float* __restrict__ pc, const float* __restrict__ pd,
               int np, const double* __restrict__ pg, int ng, double* __restrict__ rows,
-              double eps0, double dxdy, aw_diag* out, DevState* st) {
+              double eps0, double dxdy, aw_diag* out, DevState* st, DiagRing* ring) {
     constexpr int NV = kRedVals;
     constexpr int NW = kThreads / 32;
     __shared__ double sh[NV][NW];
@@ -712,6 +712,8 @@ k_step_reduce(const double* __restrict__ pp, const float* __restrict__ pc, const
         out->max_e = sqrt(sh[5][0]);
         out->charge = sh[6][0] * dxdy;
         out->eb = 0.5 * sh[7][0] * dxdy;
+        const long long k = st->step - 1 - ring->base;         // the push has counted the step
+        if (k >= 0 && k < ring->n) ring->rec[k] = *out;
         if (RMS) {
             if (sh[16][0] > 0.0)
                 for (int f = 0; f < 8; ++f) st->rms_src[f] = static_cast<float>(sqrt(sh[8 + f][0] / sh[16][0]));
@@ -726,6 +728,7 @@ k_step_reduce(const double* __restrict__ pp, const float* __restrict__ pc, const
 #include "aw_gridfft.cuh"
 
 __global__ void k_set_step(DevState* st, long long n) { st->step = n; }
+__global__ void k_set_ring(DiagRing* r, long long base, long long n) { r->base = base; r->n = n; }
 // The scales a step-begin finalise chose become the pending deposit's scales.
 __global__ void k_promote_scales(DevState* st) {
     for (int f = 0; f < 8; ++f) st->S_pend[f] = st->S_next[f];
@@ -1231,6 +1234,10 @@ void launch_set_step(Ctx& c, long long n) {
     k_set_step<<<1, 1, 0, c.stream>>>(c.st, n);
     AW_LAUNCH();
 }
+void launch_set_ring(Ctx& c, long long base, long long n) {
+    k_set_ring<<<1, 1, 0, c.stream>>>(c.ring, base, n);
+    AW_LAUNCH();
+}
 void launch_rms_reduce(Ctx& c, bool src, bool dcu) {
     k_rms_reduce<<<1, kRmsThreads, 0, c.stream>>>(src ? c.part_c : nullptr, c.npart_p,
                                                   dcu ? c.part_d : nullptr, c.npart_p, c.st);
@@ -1241,11 +1248,11 @@ void launch_step_reduce(Ctx& c) {
     if (c.model == AW_MODEL_DARWIN)
         k_step_reduce<true><<<kRedBlocks, kThreads, 0, c.stream>>>(c.part_p, c.part_c, c.part_d, c.npart_p, c.part_g,
                                                                     kGridBlocks, c.red_rows, c.prm.eps0, dxdy,
-                                                                    c.diag, c.st);
+                                                                    c.diag, c.st, c.ring);
     else
         k_step_reduce<false><<<kRedBlocks, kThreads, 0, c.stream>>>(c.part_p, nullptr, nullptr, c.npart_p, c.part_g,
                                                                      kGridBlocks, c.red_rows, c.prm.eps0, dxdy,
-                                                                     c.diag, c.st);
+                                                                     c.diag, c.st, c.ring);
     AW_LAUNCH();
 }
 void launch_promote_scales(Ctx& c) {
