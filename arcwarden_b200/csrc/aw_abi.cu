@@ -145,12 +145,6 @@ struct NoMark { void operator()(int) const {} };
 template <class Mark>
 void es_fields_from_pending(Ctx& c, bool step_begin, Mark mark) {
     float* api[1] = {c.src.rho};
-    if (c.gf) {
-        gridfft_rows_acc(c, c.acc_src, 0, 1, c.st->S_pend, api, true, step_begin, true, c.k_src); mark(0); mark(1);
-        gridfft_cols_es(c, c.k_src, c.k_out); mark(2); mark(3);
-        gridfft_fields_es(c, c.k_out, !step_begin); mark(4);        // aw_init's rollback reads the planes
-        return;
-    }
     launch_finalize(c, c.acc_src, 0, 1, c.st->S_pend, c.r_src, api, false, true, step_begin, true); mark(0);
     AW_CUFFT(cufftExecR2C(c.p_r2cS, c.r_src, c.k_src)); mark(1);
     launch_kspace_es(c, c.k_src, c.k_out); mark(2);
@@ -164,12 +158,6 @@ void es_fields_from_pending(Ctx& c, bool step_begin) { es_fields_from_pending(c,
 template <class Mark>
 void darwin_fields_a(Ctx& c, bool step_begin, Mark mark) {
     float* api[8] = {c.src.rho, c.src.Jx, c.src.Jy, c.src.Jz, c.src.amu0, c.src.amu1, c.src.amu2, c.src.amu3};
-    if (c.gf) {
-        gridfft_rows_acc(c, c.acc_src, 0, 8, c.st->S_pend, api, true, step_begin, true, c.k_src); mark(0); mark(1);
-        gridfft_cols_elb(c, c.k_src, c.k_out); mark(2); mark(3);
-        gridfft_fields_dcu(c, c.k_out); mark(4);
-        return;
-    }
     launch_finalize(c, c.acc_src, 0, 8, c.st->S_pend, c.r_src, api, false, true, step_begin, true); mark(0);
     AW_CUFFT(cufftExecR2C(c.p_r2cS, c.r_src, c.k_src)); mark(1);
     launch_kspace_elb(c, c.k_src, c.k_out); mark(2);
@@ -179,12 +167,6 @@ void darwin_fields_a(Ctx& c, bool step_begin, Mark mark) {
 template <class Mark>
 void darwin_fields_b(Ctx& c, Mark mark) {
     float* apid[3] = {c.src.dcux, c.src.dcuy, c.src.dcuz};
-    if (c.gf) {      // amu waits in k_src, transformed along x
-        gridfft_rows_acc(c, c.acc_dcu, 0, 3, c.st->S_dcu, apid, false, false, false, c.k_dcu); mark(6); mark(7);
-        gridfft_cols_et(c, c.k_dcu, c.k_src + static_cast<size_t>(4) * c.sg.nk, c.k_et); mark(8); mark(9);
-        gridfft_fields_push(c, c.k_et); mark(10);
-        return;
-    }
     launch_finalize(c, c.acc_dcu, 0, 3, c.st->S_dcu, c.r_dcu, apid, false, false, false); mark(6);
     AW_CUFFT(cufftExecR2C(c.p_r2c3, c.r_dcu, c.k_dcu)); mark(7);
     launch_kspace_et(c, c.k_dcu, c.k_src + static_cast<size_t>(4) * c.sg.nk, c.k_et); mark(8);
@@ -371,6 +353,7 @@ double grad_es_impl(Ctx& c, long long nsteps, int every, float* dux, float* duy,
             Recording r(c, w);
             step_body(c);
         });
+    if (!w.g_bwd) adj_transpose_solve(c);      // its kernels' shared-memory opt-ins, before the capture
     if (!w.g_bwd)
         w.g_bwd = capture_exec(c, [&] {
             launch_adj_scatter(c, a, kf, w.traj_E, w.ad, w.acc, w.st);

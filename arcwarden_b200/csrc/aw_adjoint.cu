@@ -23,13 +23,18 @@
 namespace aw {
 namespace {
 
+#include "aw_transpose.cuh"
+
 constexpr int kT = 256;
 
-__global__ void k_adj_finalize(unsigned long long* __restrict__ acc, const AdjDev* ad, const float2* trajE,
+// The scatter's sums back to float. Between the scatter (which read the bound
+// max |lu3|) and the gather (which takes it anew) it resets that bound.
+__global__ void k_adj_finalize(unsigned long long* __restrict__ acc, AdjDev* ad, const float2* trajE,
                                float* __restrict__ lE, int ncell) {
     const double i0 = 1.0 / static_cast<double>(ad->S[0]);
     const double i1 = 1.0 / static_cast<double>(ad->S[1]);
     const float ext = ad->ext_scale;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ad->lmax_bits = 0u;
     const float2* __restrict__ E = trajE + static_cast<size_t>(ad->slot) * ncell;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
         const long long a0 = static_cast<long long>(acc[c]);
@@ -48,31 +53,13 @@ __global__ void k_adj_finalize(unsigned long long* __restrict__ acc, const AdjDe
     }
 }
 
-// lrho_k = sum_d conj(K_d) lE_d,k with K_d = -i k_d / (eps0 k^2) (times 1/N for
-// the unnormalised C2R), zero at k = 0 and on the Nyquist lines like the
-// forward solve (es_k in aw_spectral.cu). Between the scatter (which read the
-// bound max |lu3|) and the gather (which takes it anew) it resets that bound.
+// The transposed solve on [ny][nkx] planes, for the library transforms.
 __global__ void k_adj_kspace(const cufftComplex* __restrict__ lEk, cufftComplex* __restrict__ lrk, SpecGeo g,
-                             double eps0, AdjDev* ad) {
+                             double eps0) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) ad->lmax_bits = 0u;
     if (t >= g.nk) return;
-    const int i = t % g.nkx, j = t / g.nkx;
-    const double kx = i * g.dkx;
-    const int m = (j <= g.ny / 2) ? j : j - g.ny;
-    const double ky = m * g.dky;
-    const double k2 = kx * kx + ky * ky;
-    const bool nyq = ((g.nx % 2 == 0) && i == g.nx / 2) || ((g.ny % 2 == 0) && j == g.ny / 2);
-    cufftComplex r;
-    r.x = r.y = 0.0f;
-    if (k2 > 0.0 && !nyq) {
-        const cufftComplex ax = lEk[t], ay = lEk[g.nk + t];
-        const double gr = 1.0 / (eps0 * k2) * static_cast<double>(g.invN) * (g.ff ? g.ff[t] : 1.0);
-        const double zx = kx * ax.x + ky * ay.x, zy = kx * ax.y + ky * ay.y;   // k . lE
-        r.x = static_cast<float>(-zy * gr);                                      // i z
-        r.y = static_cast<float>(zx * gr);
-    }
-    lrk[t] = r;
+    const cufftComplex in[2] = {lEk[t], lEk[g.nk + t]};
+    es_T_k(t % g.nkx, t / g.nkx, g, eps0, in, lrk[t]);
 }
 
 // Slot counters: which = 0 the backward's, 1 the recording's.
@@ -270,9 +257,17 @@ void launch_merge_err(Ctx& c) {
 
 void adj_transpose_solve(Ctx& c) {
     AdjWS& w = *c.adj;
+    if (c.gf) {
+        const float* in[2] = {w.lE, w.lE + c.geo.ncell};
+        float* out[1] = {w.lrho};
+        gridfft_rows_real(c, in, 2, w.lEk);
+        gridfft_cols_es_T(c, w.lEk, w.lrk);
+        gridfft_rows_planes(c, w.lrk, out, 1);
+        return;
+    }
     AW_CUFFT(cufftSetStream(w.p_r2c2, c.stream));
     AW_CUFFT(cufftExecR2C(w.p_r2c2, w.lE, w.lEk));
-    k_adj_kspace<<<blocks_n(c.sg.nk), kT, 0, c.stream>>>(w.lEk, w.lrk, c.sg, c.prm.eps0, w.ad);
+    k_adj_kspace<<<blocks_n(c.sg.nk), kT, 0, c.stream>>>(w.lEk, w.lrk, c.sg, c.prm.eps0);
     AW_LAUNCH();
     AW_CUFFT(cufftSetStream(w.p_c2r1, c.stream));
     AW_CUFFT(cufftExecC2R(w.p_c2r1, w.lrk, w.lrho));

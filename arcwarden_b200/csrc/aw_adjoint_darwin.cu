@@ -68,8 +68,6 @@ struct DAdjWS {
     DevState* st = nullptr;              // error word and counters of the sweep
     long long* slot = nullptr;           // [2] the current trajectory slot and step
     unsigned* ticket = nullptr;          // [1] last-block counter of k_dadj_save_gb
-    float* X = nullptr;                  // [5][n] the backward step's saved state
-    float* gbs = nullptr;                // [2][ncell][8] its gather buffers
     cufftHandle r2c3 = 0, c2r7 = 0, r2c5 = 0, c2r4 = 0;
     cudaGraphExec_t back = nullptr;      // one backward step of a gradient over back_steps steps
     long long back_steps = 0;
@@ -77,7 +75,7 @@ struct DAdjWS {
     ~DAdjWS() {
         if (back) cudaGraphExecDestroy(back);
         void* b[] = {init, ck, ck_acc, ck_st, traj, traj_gb, lam, vals, vmax, S, acc, lEB, l5, l7, l4, lsrc, k3, k7,
-                     dpump, st, slot, ticket, X, gbs, part};
+                     dpump, st, slot, ticket, part};
         for (void* p : b) if (p) cudaFree(p);
         cufftHandle h[] = {r2c3, c2r7, r2c5, c2r4};
         for (cufftHandle x : h) if (x) cufftDestroy(x);
@@ -114,12 +112,7 @@ void plan(cufftHandle& h, int ny, int nx, cufftType type, int batch) {
 __device__ __forceinline__ bool in_grid(float x, float y, const Geo& g) {
     return x >= 0.0f && x < g.nxf && y >= 0.0f && y < g.nyf;
 }
-// wavenumbers of R2C mode (i, j) and the Nyquist test, as the forward solves take them
-__device__ __forceinline__ double kx_of(int i, double dkx) { return i * dkx; }
-__device__ __forceinline__ double ky_of(int j, int ny, double dky) { return ((j <= ny / 2) ? j : j - ny) * dky; }
-__device__ __forceinline__ bool nyquist(int i, int j, int nx, int ny) {
-    return ((nx % 2 == 0) && i == nx / 2) || ((ny % 2 == 0) && j == ny / 2);
-}
+#include "aw_transpose.cuh"
 // CIC corners of a position (in the grid), and a field's value and its
 // derivatives in x and y (cell units) there.
 struct Corners {
@@ -189,26 +182,51 @@ __device__ __forceinline__ void vmax_flush(const float (&m)[6], unsigned* vmax) 
     }
 }
 
-struct PArgs { const float* X; const float* w; float* lam; float* vals; unsigned* vmax; long long n; Geo g; };
+// The particle passes read the state and gather buffers of the trajectory slot *slot.
+struct PArgs {
+    const float* traj; const float* traj_gb; const long long* slot;
+    const float* w; float* lam; float* vals; unsigned* vmax; long long n; Geo g;
+    __device__ __forceinline__ const float* state() const { return traj + *slot * 5 * n; }
+    __device__ __forceinline__ const float* gb_dcu() const { return traj_gb + *slot * 16 * g.ncell; }
+    __device__ __forceinline__ const float* gb_push() const { return gb_dcu() + 8 * static_cast<size_t>(g.ncell); }
+};
+// A particle's saved state, cotangents and weight, all loads in flight together (the
+// passes are bound by the latency of their two dependent rounds of loads: the
+// particle, then the cells around it).
+struct PLoad {
+    float x, y, u[3], l[5], w;
+    __device__ __forceinline__ PLoad(const PArgs& a, const float* __restrict__ X, long long p, bool weight) {
+        const long long n = a.n;
+        x = -1.0f;                           // (no particle)
+        if (p >= n) return;
+        x = X[p]; y = X[n + p];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) u[d] = X[(2 + d) * n + p];
+#pragma unroll
+        for (int d = 0; d < 5; ++d) l[d] = a.lam[d * n + p];
+        if (weight) w = a.w[p];
+    }
+};
 
 // Backward push: Boris transpose with the particle's own B (u1 = u + h e,
 // up = u1 + u1 x t, u2 = u1 + up x s, u3 = u2 + h e; t = h b, s = 2t / (1 + t^2)).
-__global__ void __launch_bounds__(256) k_dadj_push(PArgs a, const float* __restrict__ gbp, float h, float dtx,
-                                                   float dty) {
+__global__ void __launch_bounds__(256) k_dadj_push(PArgs a, float h, float dtx, float dty) {
     const long long n = a.n;
+    const float* __restrict__ X = a.state();
+    const float* __restrict__ gbp = a.gb_push();
     float vm[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (long long p0 = blockIdx.x * static_cast<long long>(blockDim.x); p0 < n;
          p0 += static_cast<long long>(gridDim.x) * blockDim.x) {
         const long long p = p0 + threadIdx.x;
         float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        const float x = p < n ? a.X[p] : -1.0f, y = p < n ? a.X[n + p] : -1.0f;
-        if (p < n && in_grid(x, y, a.g)) {
-            const Corners k = corners(x, y, a.g);
+        const PLoad q(a, X, p, false);
+        if (p < n && in_grid(q.x, q.y, a.g)) {
+            const Corners k = corners(q.x, q.y, a.g);
             VG f[6];
             gather6(gbp, k, f);
-            const float u[3] = {a.X[2 * n + p], a.X[3 * n + p], a.X[4 * n + p]};
-            float lx = a.lam[p], ly = a.lam[n + p];
-            const float l3[3] = {a.lam[2 * n + p] + dtx * lx, a.lam[3 * n + p] + dty * ly, a.lam[4 * n + p]};
+            const float (&u)[3] = q.u;
+            float lx = q.l[0], ly = q.l[1];
+            const float l3[3] = {q.l[2] + dtx * lx, q.l[3] + dty * ly, q.l[4]};
             const float e[3] = {f[0].v, f[1].v, f[2].v}, b[3] = {f[3].v, f[4].v, f[5].v};
             float u1[3], t[3];
             for (int d = 0; d < 3; ++d) { u1[d] = u[d] + h * e[d]; t[d] = h * b[d]; }
@@ -243,33 +261,34 @@ __global__ void __launch_bounds__(256) k_dadj_push(PArgs a, const float* __restr
 
 // Backward dcu deposit: g = G(ldcu); the scatter values (c g, c (g x u));
 // lu += c G(Bt) x g; lx += the deposit's and the gathers' position derivatives.
-__global__ void __launch_bounds__(256) k_dadj_dcu(PArgs a, const float* __restrict__ gbd, const float* __restrict__ ldcu,
-                                                  double qm2oa) {
+__global__ void __launch_bounds__(256) k_dadj_dcu(PArgs a, const float* __restrict__ ldcu, double qm2oa) {
     const long long n = a.n;
+    const float* __restrict__ X = a.state();
+    const float* __restrict__ gbd = a.gb_dcu();
     const int nc = a.g.ncell;
     float vm[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (long long p0 = blockIdx.x * static_cast<long long>(blockDim.x); p0 < n;
          p0 += static_cast<long long>(gridDim.x) * blockDim.x) {
         const long long p = p0 + threadIdx.x;
         float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        const float x = p < n ? a.X[p] : -1.0f, y = p < n ? a.X[n + p] : -1.0f;
-        if (p < n && in_grid(x, y, a.g)) {
-            const Corners k = corners(x, y, a.g);
+        const PLoad q(a, X, p, true);
+        if (p < n && in_grid(q.x, q.y, a.g)) {
+            const Corners k = corners(q.x, q.y, a.g);
             VG f[6], gl[3];
             gather6(gbd, k, f);
             for (int d = 0; d < 3; ++d) {
                 const float* L = ldcu + static_cast<size_t>(d) * nc;
                 gl[d] = vg(k, __ldg(L + k.c00), __ldg(L + k.c10), __ldg(L + k.c01), __ldg(L + k.c11));
             }
-            const float u[3] = {a.X[2 * n + p], a.X[3 * n + p], a.X[4 * n + p]};
-            const float c = static_cast<float>(qm2oa * static_cast<double>(a.w[p]));
+            const float (&u)[3] = q.u;
+            const float c = static_cast<float>(qm2oa * static_cast<double>(q.w));
             const float g[3] = {gl[0].v, gl[1].v, gl[2].v};
             const float fd[3] = {f[0].v, f[1].v, f[2].v}, bt[3] = {f[3].v, f[4].v, f[5].v};
             float uxb[3], gxu[3], bxg[3];
             cross(u, bt, uxb);
             cross(g, u, gxu);
             cross(bt, g, bxg);
-            float lx = a.lam[p], ly = a.lam[n + p];
+            float lx = q.l[0], ly = q.l[1];
             for (int d = 0; d < 3; ++d) {
                 const float dcu = c * (fd[d] + uxb[d]);
                 lx += dcu * gl[d].dx; ly += dcu * gl[d].dy;
@@ -278,7 +297,7 @@ __global__ void __launch_bounds__(256) k_dadj_dcu(PArgs a, const float* __restri
             }
             for (int d = 0; d < 6; ++d) { lx += v[d] * f[d].dx; ly += v[d] * f[d].dy; }
             a.lam[p] = lx; a.lam[n + p] = ly;
-            for (int d = 0; d < 3; ++d) a.lam[(2 + d) * n + p] += c * bxg[d];
+            for (int d = 0; d < 3; ++d) a.lam[(2 + d) * n + p] = q.l[2 + d] + c * bxg[d];
         }
         if (p < n)
             for (int d = 0; d < 6; ++d) a.vals[d * n + p] = v[d];
@@ -290,11 +309,12 @@ __global__ void __launch_bounds__(256) k_dadj_dcu(PArgs a, const float* __restri
 // Backward source deposit: from lsrc [ncell][8] = (lrho, lJ, lamu).
 __global__ void __launch_bounds__(256) k_dadj_src(PArgs a, const float* __restrict__ lsrc, double qoa) {
     const long long n = a.n;
+    const float* __restrict__ X = a.state();
     for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < n;
          p += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const float x = a.X[p], y = a.X[n + p];
-        if (!in_grid(x, y, a.g)) continue;
-        const Corners k = corners(x, y, a.g);
+        const PLoad s(a, X, p, true);
+        if (!in_grid(s.x, s.y, a.g)) continue;
+        const Corners k = corners(s.x, s.y, a.g);
         const float4* q4 = reinterpret_cast<const float4*>(lsrc);
         const float4 a0 = __ldg(q4 + 2 * k.c00), a1 = __ldg(q4 + 2 * k.c10), a2 = __ldg(q4 + 2 * k.c01),
                      a3 = __ldg(q4 + 2 * k.c11);
@@ -304,17 +324,17 @@ __global__ void __launch_bounds__(256) k_dadj_src(PArgs a, const float* __restri
         const VG j[3] = {vg(k, a0.y, a1.y, a2.y, a3.y), vg(k, a0.z, a1.z, a2.z, a3.z), vg(k, a0.w, a1.w, a2.w, a3.w)};
         const VG m[4] = {vg(k, b0.x, b1.x, b2.x, b3.x), vg(k, b0.y, b1.y, b2.y, b3.y), vg(k, b0.z, b1.z, b2.z, b3.z),
                          vg(k, b0.w, b1.w, b2.w, b3.w)};
-        const float ux = a.X[2 * n + p], uy = a.X[3 * n + p], uz = a.X[4 * n + p];
-        const float q = static_cast<float>(qoa * static_cast<double>(a.w[p]));
+        const float ux = s.u[0], uy = s.u[1], uz = s.u[2];
+        const float q = static_cast<float>(qoa * static_cast<double>(s.w));
         const float am[4] = {0.5f * (ux * ux - uy * uy), ux * uy, uz * ux, uz * uy};
-        a.lam[2 * n + p] += q * (j[0].v + m[0].v * ux + m[1].v * uy + m[2].v * uz);
-        a.lam[3 * n + p] += q * (j[1].v - m[0].v * uy + m[1].v * ux + m[3].v * uz);
-        a.lam[4 * n + p] += q * (j[2].v + m[2].v * ux + m[3].v * uy);
+        a.lam[2 * n + p] = s.l[2] + q * (j[0].v + m[0].v * ux + m[1].v * uy + m[2].v * uz);
+        a.lam[3 * n + p] = s.l[3] + q * (j[1].v - m[0].v * uy + m[1].v * ux + m[3].v * uz);
+        a.lam[4 * n + p] = s.l[4] + q * (j[2].v + m[2].v * ux + m[3].v * uy);
         float dx = r.dx + ux * j[0].dx + uy * j[1].dx + uz * j[2].dx;
         float dy = r.dy + ux * j[0].dy + uy * j[1].dy + uz * j[2].dy;
         for (int t = 0; t < 4; ++t) { dx += am[t] * m[t].dx; dy += am[t] * m[t].dy; }
-        a.lam[p] += q * dx;
-        a.lam[n + p] += q * dy;
+        a.lam[p] = s.l[0] + q * dx;
+        a.lam[n + p] = s.l[1] + q * dy;
     }
 }
 
@@ -340,7 +360,7 @@ __device__ __forceinline__ void pump_at(const PumpD& pd, int i, double t, double
 // t = step dt.
 __global__ void __launch_bounds__(256) k_dadj_fin(unsigned long long* __restrict__ acc, const float* __restrict__ S,
                                                   int ncell, int nx, int mode, float* __restrict__ out,
-                                                  const float* __restrict__ lEB, const float* __restrict__ gbp,
+                                                  const float* __restrict__ lEB, const float* __restrict__ traj_gb,
                                                   float seedv, long long last, const long long* __restrict__ slot,
                                                   PumpD pd, double dt, double* __restrict__ part) {
     const long long step = slot[1];
@@ -356,6 +376,7 @@ __global__ void __launch_bounds__(256) k_dadj_fin(unsigned long long* __restrict
         }
         if (mode == 0) {
             if (seed != 0.0f) {
+                const float* gbp = traj_gb + (slot[0] * 16 + 8) * static_cast<long long>(ncell);
                 const float4 e = reinterpret_cast<const float4*>(gbp)[2 * static_cast<size_t>(c)];
                 v[0] += seed * e.x;
                 v[1] += seed * e.y;
@@ -392,74 +413,26 @@ __global__ void k_dadj_pump(const double* __restrict__ part, int nb, double* __r
     }
 }
 
-// k-space transposes: the conjugates of the forward multipliers, with the 1/N scale.
-// lE (3) -> ldcu (3), lamu (4): E_T = -gT P (dcu - i S(amu)).
+// The same on [ny][nkx] planes, for the library transforms.
 __global__ void k_dadj_et_T(const cufftComplex* __restrict__ L, cufftComplex* __restrict__ out, SpecGeo g,
                             double eps0, double c, double n0) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.nk) return;
-    const int i = t % g.nkx, j = t / g.nkx;
     const size_t nk = g.nk;
-    const double kx = kx_of(i, g.dkx), ky = ky_of(j, g.ny, g.dky);
-    const double k2 = kx * kx + ky * ky;
-    cufftComplex z; z.x = z.y = 0.0f;
-    if (nyquist(i, j, g.nx, g.ny) || k2 == 0.0) {
-        for (int f = 0; f < 7; ++f) out[f * nk + t] = z;
-        return;
-    }
-    const double G = -1.0 / (eps0 * c * c * k2 + n0) * (g.ff ? g.ff[t] : 1.0);
-    double pr[3], pi[3];
-    for (int d = 0; d < 3; ++d) { pr[d] = G * L[d * nk + t].x; pi[d] = G * L[d * nk + t].y; }
-    const double kdr = (kx * pr[0] + ky * pr[1]) / k2, kdi = (kx * pi[0] + ky * pi[1]) / k2;
-    pr[0] -= kx * kdr; pi[0] -= kx * kdi;
-    pr[1] -= ky * kdr; pi[1] -= ky * kdi;
-    for (int d = 0; d < 3; ++d) {
-        cufftComplex o; o.x = static_cast<float>(pr[d]) * g.invN; o.y = static_cast<float>(pi[d]) * g.invN;
-        out[d * nk + t] = o;
-    }
-    // lamu = conj(-i) S^T PL = i S^T PL: i (re + i im) = -im + i re
-    const double w0r = -pi[0], w0i = pr[0], w1r = -pi[1], w1i = pr[1], w2r = -pi[2], w2i = pr[2];
-    const double ar[4] = {kx * w0r - ky * w1r, ky * w0r + kx * w1r, kx * w2r, ky * w2r};
-    const double ai[4] = {kx * w0i - ky * w1i, ky * w0i + kx * w1i, kx * w2i, ky * w2i};
-    for (int m = 0; m < 4; ++m) {
-        cufftComplex o; o.x = static_cast<float>(ar[m]) * g.invN; o.y = static_cast<float>(ai[m]) * g.invN;
-        out[(3 + m) * nk + t] = o;
-    }
+    const cufftComplex in[3] = {L[t], L[nk + t], L[2 * nk + t]};
+    cufftComplex o[7];
+    et_T_k(t % g.nkx, t / g.nkx, g, eps0, c, n0, in, o);
+    for (int f = 0; f < 7; ++f) out[f * nk + t] = o[f];
 }
-// (lE_L x y, lB x y z) -> (lrho, lJx, lJy, lJz): the transpose of k_kspace_elb.
 __global__ void k_dadj_elb_T(const cufftComplex* __restrict__ L, cufftComplex* __restrict__ out, SpecGeo g,
                              double eps0, double c) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.nk) return;
-    const int i = t % g.nkx, j = t / g.nkx;
     const size_t nk = g.nk;
-    const double kx = kx_of(i, g.dkx), ky = ky_of(j, g.ny, g.dky);
-    const double k2 = kx * kx + ky * ky;
-    cufftComplex z; z.x = z.y = 0.0f;
-    if (nyquist(i, j, g.nx, g.ny) || k2 == 0.0) {
-        for (int f = 0; f < 4; ++f) out[f * nk + t] = z;
-        return;
-    }
-    const double ff = g.ff ? g.ff[t] : 1.0;
-    const double gE = ff / (eps0 * k2), gB = ff / (eps0 * c * c * k2);
-    const cufftComplex lx = L[t], ly = L[nk + t], bx = L[2 * nk + t], by = L[3 * nk + t], bz = L[4 * nk + t];
-    // forward: ELx = -i kx gE rho, ELy = -i ky gE rho; Bx = i gB ky Jz, By = -i gB kx Jz,
-    // Bz = i gB (kx Jy - ky Jx). transpose: conj of each factor, i.e. i <-> -i.
-    // (re + i im) * i f = -f im + i f re; (re + i im) * (-i f) = f im - i f re
-    // lrho <- conj(-i kx gE) lEx + conj(-i ky gE) lEy = gE (i kx lEx + i ky lEy)
-    const double rr = -gE * (kx * lx.y + ky * ly.y), ri = gE * (kx * lx.x + ky * ly.x);
-    double Jxr, Jxi, Jyr, Jyi, Jzr, Jzi;
-    // Jx <- conj(-i gB ky) bz = (i gB ky) bz = gB ky (-bz.y + i bz.x)
-    Jxr = -gB * ky * bz.y; Jxi = gB * ky * bz.x;
-    // Jy <- conj(i gB kx) bz = (-i gB kx) bz = gB kx (bz.y - i bz.x)
-    Jyr = gB * kx * bz.y; Jyi = -gB * kx * bz.x;
-    // Jz <- conj(i gB ky) bx + conj(-i gB kx) by = gB ky (bx.y - i bx.x) + gB kx (-by.y + i by.x)
-    Jzr = gB * ky * bx.y - gB * kx * by.y; Jzi = -gB * ky * bx.x + gB * kx * by.x;
-    cufftComplex o;
-    o.x = static_cast<float>(rr) * g.invN; o.y = static_cast<float>(ri) * g.invN; out[t] = o;
-    o.x = static_cast<float>(Jxr) * g.invN; o.y = static_cast<float>(Jxi) * g.invN; out[nk + t] = o;
-    o.x = static_cast<float>(Jyr) * g.invN; o.y = static_cast<float>(Jyi) * g.invN; out[2 * nk + t] = o;
-    o.x = static_cast<float>(Jzr) * g.invN; o.y = static_cast<float>(Jzi) * g.invN; out[3 * nk + t] = o;
+    const cufftComplex in[5] = {L[t], L[nk + t], L[2 * nk + t], L[3 * nk + t], L[4 * nk + t]};
+    cufftComplex o[4];
+    elb_T_k(t % g.nkx, t / g.nkx, g, eps0, c, in, o);
+    for (int f = 0; f < 4; ++f) out[f * nk + t] = o[f];
 }
 // lsrc [ncell][8] = (lrho, lJx, lJy, lJz, lamu0..3) from the planes l4 [4][ncell], lamu [4][ncell].
 __global__ void k_dadj_pack(const float* __restrict__ l4, const float* __restrict__ lamu, int ncell,
@@ -528,19 +501,6 @@ __global__ void k_dadj_save_gb(const float4* __restrict__ gbd, const float4* __r
         }
     }
 }
-// Trajectory slot slot[0] (state and gather buffers) into the fixed buffers the
-// backward step reads.
-__global__ void k_dadj_load(const float* __restrict__ traj, const float4* __restrict__ traj_gb,
-                            const long long* __restrict__ slot, long long n, int nc, float* __restrict__ X,
-                            float4* __restrict__ gbs) {
-    const float* t = traj + slot[0] * 5 * n;
-    const float4* tg = traj_gb + slot[0] * 4 * nc;
-    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < 5 * n; i += stride)
-        X[i] = t[i];
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < 4LL * nc; i += stride)
-        gbs[i] = tg[i];
-}
 // The previous step: slot[0] -= 1, slot[1] -= 1 (the end of a backward step).
 __global__ void k_dadj_prev(long long* slot) {
     if (threadIdx.x == 0 && blockIdx.x == 0) { slot[0] -= 1; slot[1] -= 1; }
@@ -585,8 +545,6 @@ double grad_darwin_impl(Ctx& c, long long nsteps, int every, float* dux, float* 
         dmalloc(w.st, 1);
         dmalloc(w.slot, 2);
         dmalloc(w.ticket, 1);
-        dmalloc(w.X, 5 * static_cast<size_t>(n));
-        dmalloc(w.gbs, 16 * static_cast<size_t>(nc));
         dmalloc(w.part, fin_blocks);
         plan(w.r2c3, c.geo.ny, c.geo.nx, CUFFT_R2C, 3);
         plan(w.c2r7, c.geo.ny, c.geo.nx, CUFFT_C2R, 7);
@@ -673,51 +631,74 @@ double grad_darwin_impl(Ctx& c, long long nsteps, int every, float* dux, float* 
     const int pb_src = static_cast<int>(std::max<long long>(1, std::min<long long>(static_cast<long long>(sms) *
                                                                                     std::max(per_sm, 1),
                                                                                     (n + 255) / 256)));
-    // One backward step, captured once: it copies trajectory slot w.slot[0] into
-    // the fixed buffers w.X, w.gbs, reads its step from w.slot[1] and moves the
-    // slot one step back, so the same graph replays every step.
+    // One backward step, captured once: it reads trajectory slot w.slot[0] and its
+    // step from w.slot[1] and moves the slot one step back, so the same graph replays
+    // every step.
     prepare_scatter6();
     if (!w.back) {
         w.back_steps = nsteps;
-        const float* X = w.X;
-        const float* gbd = w.gbs;
-        const float* gbp = w.gbs + 8 * static_cast<size_t>(nc);
-        const PArgs a{X, c.parts.w, w.lam, w.vals, w.vmax, n, c.geo};
+        const float* X = w.traj;           // (of slot w.slot[0])
+        const PArgs a{w.traj, w.traj_gb, w.slot, c.parts.w, w.lam, w.vals, w.vmax, n, c.geo};
+        auto planes = [&](float* base, int nf, float* (&out)[7]) {
+            for (int f = 0; f < nf; ++f) out[f] = base + static_cast<size_t>(f) * nc;
+        };
+        auto et_T = [&] {                  // lEB (3 planes) -> l7 = ldcu, lamu
+            if (!c.gf) {
+                AW_CUFFT(cufftExecR2C(w.r2c3, w.lEB, w.k3));
+                k_dadj_et_T<<<(c.sg.nk + 255) / 256, 256, 0, c.stream>>>(w.k3, w.k7, c.sg, c.prm.eps0, c.prm.c,
+                                                                         c.prm.n0);
+                AW_LAUNCH();
+                AW_CUFFT(cufftExecC2R(w.c2r7, w.k7, w.l7));
+                return;
+            }
+            float *in[7], *out[7];
+            planes(w.lEB, 3, in);
+            planes(w.l7, 7, out);
+            gridfft_rows_real(c, in, 3, w.k3);
+            gridfft_cols_et_T(c, w.k3, w.k7);
+            gridfft_rows_planes(c, w.k7, out, 7);
+        };
+        auto elb_T = [&] {                 // l5 -> l4 = lrho, lJ
+            if (!c.gf) {
+                AW_CUFFT(cufftExecR2C(w.r2c5, w.l5, w.k7));
+                k_dadj_elb_T<<<(c.sg.nk + 255) / 256, 256, 0, c.stream>>>(w.k7, w.k7 + 5 * nk, c.sg, c.prm.eps0,
+                                                                          c.prm.c);
+                AW_LAUNCH();
+                AW_CUFFT(cufftExecC2R(w.c2r4, w.k7 + 5 * nk, w.l4));
+                return;
+            }
+            float *in[7], *out[7];
+            planes(w.l5, 5, in);
+            planes(w.l4, 4, out);
+            gridfft_rows_real(c, in, 5, w.k7);
+            gridfft_cols_elb_T(c, w.k7, w.k7 + 5 * nk);
+            gridfft_rows_planes(c, w.k7 + 5 * nk, out, 4);
+        };
+        if (c.gf) { et_T(); elb_T(); }     // the kernels' shared-memory opt-ins, before the capture
         const long long last = nsteps - 1;
         w.back = capture_graph(c.stream, [&] {
-            k_dadj_load<<<pb, 256, 0, c.stream>>>(w.traj, reinterpret_cast<const float4*>(w.traj_gb), w.slot, n, nc,
-                                                  w.X, reinterpret_cast<float4*>(w.gbs));
-            AW_LAUNCH();
             // push transpose -> lE, lBt
             AW_CUDA(cudaMemsetAsync(w.vmax, 0, 6 * sizeof(unsigned), c.stream));
-            k_dadj_push<<<pb, 256, 0, c.stream>>>(a, gbp, h, dtx, dty);
+            k_dadj_push<<<pb, 256, 0, c.stream>>>(a, h, dtx, dty);
             AW_LAUNCH();
-            launch_scatter6(c, c.stream, X, X + n, w.vals, n, w.vmax, w.S, w.acc, w.st);
-            k_dadj_fin<<<gbk, 256, 0, c.stream>>>(w.acc, w.S, nc, c.geo.nx, 0, w.lEB, nullptr, gbp, seed, last, w.slot,
+            launch_scatter6(c, c.stream, X, X + n, w.vals, n, w.vmax, w.S, w.acc, w.st, w.slot);
+            k_dadj_fin<<<gbk, 256, 0, c.stream>>>(w.acc, w.S, nc, c.geo.nx, 0, w.lEB, nullptr, w.traj_gb, seed, last, w.slot,
                                                   pd, c.prm.dt, nullptr);
             AW_LAUNCH();
             // E_T transpose -> ldcu, lamu
-            AW_CUFFT(cufftExecR2C(w.r2c3, w.lEB, w.k3));
-            k_dadj_et_T<<<(c.sg.nk + 255) / 256, 256, 0, c.stream>>>(w.k3, w.k7, c.sg, c.prm.eps0, c.prm.c,
-                                                                     c.prm.n0);
-            AW_LAUNCH();
-            AW_CUFFT(cufftExecC2R(w.c2r7, w.k7, w.l7));
+            et_T();
             // dcu transpose -> lFd, lBt'; combined with lE, lBt into (lE_L, lB); the pump term
             AW_CUDA(cudaMemsetAsync(w.vmax, 0, 6 * sizeof(unsigned), c.stream));
-            k_dadj_dcu<<<pb, 256, 0, c.stream>>>(a, gbd, w.l7, qm2oa);
+            k_dadj_dcu<<<pb, 256, 0, c.stream>>>(a, w.l7, qm2oa);
             AW_LAUNCH();
-            launch_scatter6(c, c.stream, X, X + n, w.vals, n, w.vmax, w.S, w.acc, w.st);
+            launch_scatter6(c, c.stream, X, X + n, w.vals, n, w.vmax, w.S, w.acc, w.st, w.slot);
             k_dadj_fin<<<gbk, 256, 0, c.stream>>>(w.acc, w.S, nc, c.geo.nx, 1, w.l5, w.lEB, nullptr, 0.0f, last,
                                                   w.slot, pd, c.prm.dt, part);
             AW_LAUNCH();
             k_dadj_pump<<<1, 32, 0, c.stream>>>(part, gbk, w.dpump);
             AW_LAUNCH();
             // E_L, B transpose -> lrho, lJ; with lamu into the source gather buffer
-            AW_CUFFT(cufftExecR2C(w.r2c5, w.l5, w.k7));
-            k_dadj_elb_T<<<(c.sg.nk + 255) / 256, 256, 0, c.stream>>>(w.k7, w.k7 + 5 * nk, c.sg, c.prm.eps0,
-                                                                      c.prm.c);
-            AW_LAUNCH();
-            AW_CUFFT(cufftExecC2R(w.c2r4, w.k7 + 5 * nk, w.l4));
+            elb_T();
             k_dadj_pack<<<gbk, 256, 0, c.stream>>>(w.l4, w.l7 + 3 * static_cast<size_t>(nc), nc, w.lsrc);
             AW_LAUNCH();
             k_dadj_src<<<pb_src, 256, 0, c.stream>>>(a, w.lsrc, qoa);

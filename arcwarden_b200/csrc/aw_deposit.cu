@@ -1954,9 +1954,10 @@ bool pow2_geo(const Ctx& c) { return is_pow2(c.geo.dx) && is_pow2(c.geo.dy); }
 // (block 0) for the finaliser. Stage: x, y, then the six scaled values.
 constexpr int kScatterNF = 6;
 __global__ void __launch_bounds__(kThreads, 2)
-k_scatter6(const float* __restrict__ xs, const float* __restrict__ ys, const float* __restrict__ vals, long long n,
+k_scatter6(const float* xs, const float* ys, const float* __restrict__ vals, long long n,
            Geo g, const unsigned* __restrict__ vmax, float* __restrict__ Sout,
-           unsigned long long* __restrict__ acc, DevState* st, int vec_ok, int cs_) {
+           unsigned long long* __restrict__ acc, DevState* st, int vec_ok, int cs_, const long long* __restrict__ slot) {
+    if (slot) { const long long o = *slot * 5 * n; xs += o; ys += o; }
     constexpr int NF = kScatterNF, NS = 2 + NF;
     constexpr bool T0 = false;
     constexpr int PC = wmax_cells(NF);
@@ -2033,14 +2034,14 @@ void prep_adj_scatter() { prep_smem(k_adj_scatter, smem_bytes(2, 4)); }
 
 void prepare_scatter6() { prep_smem(k_scatter6, smem_bytes(kScatterNF, 2 + kScatterNF)); }
 void launch_scatter6(Ctx& c, cudaStream_t s, const float* xs, const float* ys, const float* vals, long long n,
-                     const unsigned* vmax, float* Sout, unsigned long long* acc, DevState* st) {
+                     const unsigned* vmax, float* Sout, unsigned long long* acc, DevState* st, const long long* slot) {
     if (n == 0) return;
     const size_t sh = smem_bytes(kScatterNF, 2 + kScatterNF);
     prep_smem(k_scatter6, sh);
     const int vec = (n % 4 == 0 && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(ys) & 15) == 0 && (reinterpret_cast<uintptr_t>(vals) & 15) == 0) ? 1 : 0;
     const int cs = chunk_size(n, 2 * c.sms);        // two CTAs per SM
-    k_scatter6<<<nchunks(n, cs), kThreads, sh, s>>>(xs, ys, vals, n, c.geo, vmax, Sout, acc, st, vec, cs);
+    k_scatter6<<<nchunks(n, cs), kThreads, sh, s>>>(xs, ys, vals, n, c.geo, vmax, Sout, acc, st, vec, cs, slot);
     AW_LAUNCH();
 }
 

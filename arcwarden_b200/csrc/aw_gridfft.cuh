@@ -1,18 +1,18 @@
-// aw_gridfft.cuh — the grid solves as three kernels each (included by
-// aw_spectral.cu inside its anonymous namespace).
+// aw_gridfft.cuh — grid solves as three kernels (included by aw_spectral.cu inside
+// its anonymous namespace): the unfused solves on the caller's arrays and the
+// adjoints' transposed solves.
 //
-//   k_rows_fwd   rows in, real -> complex along x. The rows come from the int64
-//                accumulators (the finalisation: scale, reset, caller's arrays,
-//                charge partial, the step's opening) or from real planes.
-//   k_cols       complex along y, the solve's multiplier in k-space, and back.
-//   k_rows_inv   complex -> real along x, and what the fields are for: gather
-//                buffers, caller's arrays, maxima and energy partials.
+//   k_rows_fwd   rows of real planes -> complex along x
+//   k_cols       complex along y, the solve's multiplier in k-space, and back
+//   k_rows_inv   complex -> real along x, into planes
 //
-// A solve through the library transforms takes seven launches and writes every
-// plane to memory between them; on grids of this path (up to 1024 on a side, a few
-// MB) the launches and the latency of seven dependent kernels are its time, not the
-// bytes or the arithmetic. Here a row or column lives in shared memory from its
-// load to its last use.
+// One library transform per caller array and direction took 20 launches a solve; on
+// grids of this path (up to 1024 on a side, a few MB) the latency of dependent launches
+// is the time, not the bytes or the arithmetic. Here a row or column lives in shared
+// memory from its load to its last use (the unfused Darwin step at 256 x 256: 604 ->
+// 474 us). The fused steps, whose planes are contiguous and batched, keep the library
+// transforms: the gain there is 1 to 4%, and the FP32 rounding of E decides in which
+// step a particle crosses a cell edge, which a gradient shows.
 //
 // Two rows share one complex transform (z = a + i b, a and b of one field, so their
 // magnitudes are alike). Between the kernels a field is stored transposed,
@@ -194,20 +194,9 @@ struct GridFftArgs {
 // ---- rows, forward ----------------------------------------------------------------
 struct RowsFwd {
     GridFftArgs g;
-    const float* src[8];               // real planes (ACC = false)
-    unsigned long long* acc;           // ACC: the accumulators, field `first` + blockIdx.y
-    int first;
-    const float* S;
-    FinOut api;
-    double* part;                      // charge partials, or null
-    DevState* st;
-    int step_begin, darwin, sub_ref;
-    double dt;
-    float cref;
-    AdjDev* rec;
+    const float* src[8];               // real planes [ny][nx]
     float2* out;                       // [field][nkx][ny]
 };
-template <bool ACC>
 __global__ void __launch_bounds__(kThreads) k_rows_fwd(RowsFwd A) {
     extern __shared__ __align__(16) float2 fsm[];
     const GridFftArgs& g = A.g;
@@ -216,77 +205,15 @@ __global__ void __launch_bounds__(kThreads) k_rows_fwd(RowsFwd A) {
     float2* const b0 = tw + ((g.nx + 1) & ~1);
     float2* const b1 = b0 + g.pr * g.rsx;
     load_twiddles(tw, g.twx, g.nx);
-    double qsum = 0.0;
-    const double invS = ACC ? __drcp_rn(static_cast<double>(A.S[A.first + f])) : 0.0;
-    const double ref0 = (ACC && A.sub_ref && A.first + f == 0) ? A.st->rho_ref : 0.0;
     const float rnx = 1.0f / static_cast<float>(g.nx);
-    unsigned long long* const acc = ACC ? A.acc + static_cast<size_t>(A.first + f) * g.ncell : nullptr;
-    const float* const src = ACC ? nullptr : A.src[f];
-    float* const api = ACC ? A.api.p[f] : nullptr;
-    auto value = [&](long long q, int c) {       // one cell's finalised value -> the caller's array, the transform's input
-        const double d = static_cast<double>(q) * invS;
-        const float a = __double2float_rn(d);
-        if (api) api[c] = a;
-        if (A.first + f != 0) return a;
-        qsum += static_cast<double>(a);
-        return __double2float_rn(d - ref0);
-    };
-    if (ACC && (g.nx & 1) == 0) {
-        // two cells of both rows per turn, U turns' loads before the first store
-        constexpr int U = 4;
-        const int hx = g.nx >> 1, m = g.pr * hx;
-        const float rhx = 1.0f / static_cast<float>(hx);
-        const longlong2* const q = reinterpret_cast<const longlong2*>(acc);
-        for (int t0 = threadIdx.x; t0 < m; t0 += U * kThreads) {
-            longlong2 v[U][2];
-            int c[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int t = t0 + u * kThreads;
-                const int pr = row_of(t, rhx), ja = 2 * (p0 + pr);
-                c[u] = ja * hx + t - pr * hx;                       // in pairs of cells
-                v[u][0] = v[u][1] = make_longlong2(0, 0);
-                if (t < m && ja < g.ny) v[u][0] = q[c[u]];
-                if (t < m && ja + 1 < g.ny) v[u][1] = q[c[u] + hx];
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int t = t0 + u * kThreads;
-                if (t >= m) continue;
-                const int pr = row_of(t, rhx), x = 2 * (t - pr * hx), ja = 2 * (p0 + pr);
-                float a0 = 0.f, a1 = 0.f, b0v = 0.f, b1v = 0.f;
-                if (ja < g.ny) {
-                    reinterpret_cast<longlong2*>(acc)[c[u]] = make_longlong2(0, 0);
-                    a0 = value(v[u][0].x, 2 * c[u]); a1 = value(v[u][0].y, 2 * c[u] + 1);
-                }
-                if (ja + 1 < g.ny) {
-                    reinterpret_cast<longlong2*>(acc)[c[u] + hx] = make_longlong2(0, 0);
-                    b0v = value(v[u][1].x, 2 * c[u] + g.nx); b1v = value(v[u][1].y, 2 * c[u] + g.nx + 1);
-                }
-                float2* o = b0 + pr * g.rsx;
-                o[fpad(x)] = make_float2(a0, b0v);
-                o[fpad(x + 1)] = make_float2(a1, b1v);
-            }
-        }
-    } else {
-        for (int t = threadIdx.x; t < g.pr * g.nx; t += kThreads) {
-            const int pr = row_of(t, rnx), x = t - pr * g.nx;
-            const int ja = 2 * (p0 + pr);
-            float v[2] = {0.f, 0.f};
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (ja + h >= g.ny) continue;
-                const int c = (ja + h) * g.nx + x;
-                if (ACC) {
-                    const long long q = static_cast<long long>(acc[c]);
-                    acc[c] = 0ull;
-                    v[h] = value(q, c);
-                } else {
-                    v[h] = src[c];
-                }
-            }
-            b0[pr * g.rsx + fpad(x)] = make_float2(v[0], v[1]);
-        }
+    const float* __restrict__ src = A.src[f];
+#pragma unroll 4
+    for (int t = threadIdx.x; t < g.pr * g.nx; t += kThreads) {
+        const int pr = row_of(t, rnx), x = t - pr * g.nx;
+        const int ja = 2 * (p0 + pr);
+        const float a = ja < g.ny ? __ldg(src + ja * g.nx + x) : 0.f;
+        const float b = ja + 1 < g.ny ? __ldg(src + (ja + 1) * g.nx + x) : 0.f;
+        b0[pr * g.rsx + fpad(x)] = make_float2(a, b);
     }
     const float2* z = fft_run<-1>(b0, b1, g.pr, g.rsx, g.px, tw);
     // row a: (Z_k + conj Z_-k) / 2, row b: (Z_k - conj Z_-k) / (2 i)
@@ -303,25 +230,6 @@ __global__ void __launch_bounds__(kThreads) k_rows_fwd(RowsFwd A) {
         float2* o = out + static_cast<size_t>(k) * g.ny + ja;
         if ((g.ny & 1) == 0) *reinterpret_cast<float4*>(o) = make_float4(a.x, a.y, b.x, b.y);
         else { o[0] = a; if (ja + 1 < g.ny) o[1] = b; }
-    }
-    if (ACC && A.part && A.first + f == 0) {
-        __shared__ double sh[kThreads / 32];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) qsum += __shfl_down_sync(0xffffffffu, qsum, o);
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = qsum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0;
-            for (int w = 0; w < kThreads / 32; ++w) s += sh[w];
-            A.part[blockIdx.x * 5 + 2] = s;
-        }
-        // the partial rows no block of this launch owns
-        for (int b = gridDim.x + blockIdx.x * kThreads + threadIdx.x; b < kGridBlocks; b += gridDim.x * kThreads)
-            A.part[b * 5 + 2] = 0.0;
-    }
-    if (ACC && A.step_begin && blockIdx.x == 0 && f == 0 && threadIdx.x == 0) {
-        if (A.rec) A.rec->rec_slot += 1;     // the recorded step's trajectory slot
-        open_step(A.st, A.dt, A.cref, A.darwin != 0);
     }
 }
 
@@ -374,177 +282,57 @@ __global__ void __launch_bounds__(kThreads) k_cols(ColsArgs<Op> A) {
 }
 
 // ---- rows, inverse ------------------------------------------------------------------
-// Fin: what happens to a cell's NF field values; begin() and end() around a block's
-// cells (end may sync).
-template <class Fin>
 struct RowsInv {
     GridFftArgs g;
     const float2* in;                  // [NF][nkx][ny]
-    Fin fin;
+    float* out[8];                     // real planes [ny][nx]
 };
-template <class Fin>
-__global__ void __launch_bounds__(kThreads) k_rows_inv(RowsInv<Fin> A) {
-    constexpr int NF = Fin::NF;
+// One field per blockIdx.y.
+__global__ void __launch_bounds__(kThreads) k_rows_inv(RowsInv A) {
     extern __shared__ __align__(16) float2 fsm[];
     const GridFftArgs& g = A.g;
     const int p0 = blockIdx.x * g.pr;
     float2* const tw = fsm;
     float2* const b0 = tw + ((g.nx + 1) & ~1);
-    float2* const b1 = b0 + NF * g.pr * g.rsx;
+    float2* const b1 = b0 + g.pr * g.rsx;
     load_twiddles(tw, g.twx, g.nx);
     const float rpr = 1.0f / static_cast<float>(g.pr);
-#pragma unroll
-    for (int f = 0; f < NF; ++f)
-        for (int t = threadIdx.x; t < g.pr * g.nkx; t += kThreads) {
-            const int k = row_of(t, rpr), pr = t - k * g.pr;
-            const int ja = 2 * (p0 + pr);
-            float2 a = make_float2(0.f, 0.f), b = a;
-            if (ja < g.ny) {
-                const float2* o = A.in + static_cast<size_t>(f) * g.nk + static_cast<size_t>(k) * g.ny + ja;
-                if ((g.ny & 1) == 0) {
-                    const float4 q = __ldg(reinterpret_cast<const float4*>(o));
-                    a = make_float2(q.x, q.y); b = make_float2(q.z, q.w);
-                } else {
-                    a = __ldg(o);
-                    if (ja + 1 < g.ny) b = __ldg(o + 1);
-                }
-            }
-            // Z = A + i B with A, B Hermitian: the k = 0 and Nyquist modes of a real row are real
-            float2* s = b0 + (f * g.pr + pr) * g.rsx;
-            if (k == 0 || 2 * k == g.nx) {
-                s[fpad(k)] = make_float2(a.x, b.x);
+    const int f = blockIdx.y;
+    for (int t = threadIdx.x; t < g.pr * g.nkx; t += kThreads) {
+        const int k = row_of(t, rpr), pr = t - k * g.pr;
+        const int ja = 2 * (p0 + pr);
+        float2 a = make_float2(0.f, 0.f), b = a;
+        if (ja < g.ny) {
+            const float2* o = A.in + static_cast<size_t>(f) * g.nk + static_cast<size_t>(k) * g.ny + ja;
+            if ((g.ny & 1) == 0) {
+                const float4 q = __ldg(reinterpret_cast<const float4*>(o));
+                a = make_float2(q.x, q.y); b = make_float2(q.z, q.w);
             } else {
-                s[fpad(k)] = make_float2(a.x - b.y, a.y + b.x);
-                s[fpad(g.nx - k)] = make_float2(a.x + b.y, b.x - a.y);
+                a = __ldg(o);
+                if (ja + 1 < g.ny) b = __ldg(o + 1);
             }
         }
-    const float2* z = fft_run<1>(b0, b1, NF * g.pr, g.rsx, g.px, tw);
+        // Z = A + i B with A, B Hermitian: the k = 0 and Nyquist modes of a real row are real
+        float2* s = b0 + pr * g.rsx;
+        if (k == 0 || 2 * k == g.nx) {
+            s[fpad(k)] = make_float2(a.x, b.x);
+        } else {
+            s[fpad(k)] = make_float2(a.x - b.y, a.y + b.x);
+            s[fpad(g.nx - k)] = make_float2(a.x + b.y, b.x - a.y);
+        }
+    }
+    const float2* z = fft_run<1>(b0, b1, g.pr, g.rsx, g.px, tw);
     const float rnx = 1.0f / static_cast<float>(g.nx);
-    Fin fin = A.fin;
-    fin.begin();
+    float* __restrict__ out = A.out[f];
     for (int t = threadIdx.x; t < g.pr * g.nx; t += kThreads) {
         const int pr = row_of(t, rnx), x = t - pr * g.nx;
         const int ja = 2 * (p0 + pr);
         if (ja >= g.ny) continue;
-        float va[NF], vb[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const float2 v = z[(f * g.pr + pr) * g.rsx + fpad(x)];
-            va[f] = v.x; vb[f] = v.y;
-        }
-        fin.cell(ja * g.nx + x, x, va);
-        if (ja + 1 < g.ny) fin.cell((ja + 1) * g.nx + x, x, vb);
-    }
-    fin.end();
-}
-// Partial rows [blockIdx.x] of a grid of fewer than kGridBlocks blocks: the rows
-// that no block owns are zeroed.
-__device__ __forceinline__ void zero_spare_partials(double* __restrict__ part) {
-    for (int b = gridDim.x + blockIdx.x * kThreads + threadIdx.x; b < kGridBlocks; b += gridDim.x * kThreads) {
-        part[b * 5 + 0] = 0.0; part[b * 5 + 1] = 0.0; part[b * 5 + 3] = 0.0;
+        const float2 v = z[pr * g.rsx + fpad(x)];
+        out[ja * g.nx + x] = v.x;
+        if (ja + 1 < g.ny) out[(ja + 1) * g.nx + x] = v.y;
     }
 }
-// ES fields: gather buffer, planes, caller's arrays, trajectory, energy partials.
-struct FinEs {
-    static constexpr int NF = 2;
-    float *gb, *ex, *ey, *r;
-    double* part;
-    float2* traj; const AdjDev* rec;
-    int ncell;
-    double se2, me2;
-    float2* te;
-    __device__ void begin() {
-        se2 = 0.0; me2 = 0.0;
-        te = traj ? traj + static_cast<size_t>(rec->rec_slot) * ncell : nullptr;
-    }
-    __device__ void cell(int c, int, const float (&v)[2]) {
-        reinterpret_cast<float2*>(gb)[c] = make_float2(v[0], v[1]);
-        if (r) { r[c] = v[0]; r[ncell + c] = v[1]; }
-        if (te) te[c] = make_float2(v[0], v[1]);
-        if (ex) ex[c] = v[0];
-        if (ey) ey[c] = v[1];
-        const double e2 = double(v[0]) * v[0] + double(v[1]) * v[1];
-        se2 += e2;
-        me2 = fmax(me2, e2);
-    }
-    __device__ void end() { zero_spare_partials(part); grid_partials(se2, me2, 0.0, part); }
-};
-// Darwin, after the E_L, B solve (k_fields_dcu): planes E_L for the second solve.
-struct FinDcu {
-    static constexpr int NF = 5;
-    float *gb, *r;
-    FieldAPI api;
-    float b0x, b0y, b0z;
-    PumpArgs pa;
-    DevState* st;
-    int ncell;
-    double t;
-    float emax, bmax;
-    __device__ void begin() { t = st->t; emax = 0.f; bmax = 0.f; }
-    __device__ void cell(int c, int i, const float (&v)[5]) {
-        const float elx = v[0], ely = v[1], bx = v[2] + b0x, by = v[3] + b0y, bz = v[4] + b0z;
-        float ex = elx, ey = ely, ez = 0.0f;
-        pump_add(pa, i, t, ex, ey, ez);
-        float4* q = reinterpret_cast<float4*>(gb) + 2 * static_cast<size_t>(c);
-        q[0] = make_float4(ex, ey, ez, bx);
-        q[1] = make_float4(by, bz, 0.f, 0.f);
-        r[c] = elx; r[ncell + c] = ely;
-        if (api.ELx) api.ELx[c] = elx;
-        if (api.ELy) api.ELy[c] = ely;
-        if (api.Bx) api.Bx[c] = bx;
-        if (api.By) api.By[c] = by;
-        if (api.Bz) api.Bz[c] = bz;
-        emax = fmaxf(emax, fmaxf(fabsf(ex), fmaxf(fabsf(ey), fabsf(ez))));
-        bmax = fmaxf(bmax, fmaxf(fabsf(bx), fmaxf(fabsf(by), fabsf(bz))));
-    }
-    __device__ void end() { block_max_eb(emax, bmax, st); }
-};
-// Darwin, after the E_T solve (k_fields_push).
-struct FinPush {
-    static constexpr int NF = 3;
-    const float* rel;
-    const float* gbd;
-    float* gb;
-    FieldAPI api;
-    PumpArgs pa;
-    const DevState* st;
-    double* part;
-    int ncell;
-    double t, se2, me2, sb2;
-    __device__ void begin() { t = st->t; se2 = 0.0; me2 = 0.0; sb2 = 0.0; }
-    __device__ void cell(int c, int i, const float (&v)[3]) {
-        const float4* qd = reinterpret_cast<const float4*>(gbd) + 2 * static_cast<size_t>(c);
-        const float4 b1 = qd[0], b2 = qd[1];
-        float ex = rel[c] + 1.0f * v[0], ey = rel[ncell + c] + 1.0f * v[1], ez = 1.0f * v[2];
-        pump_add(pa, i, t, ex, ey, ez);
-        float4* q = reinterpret_cast<float4*>(gb) + 2 * static_cast<size_t>(c);
-        q[0] = make_float4(ex, ey, ez, b1.w);
-        q[1] = make_float4(b2.x, b2.y, 0.f, 0.f);
-        if (api.Ex) api.Ex[c] = ex;
-        if (api.Ey) api.Ey[c] = ey;
-        if (api.Ez) api.Ez[c] = ez;
-        if (api.ETx) api.ETx[c] = v[0];
-        if (api.ETy) api.ETy[c] = v[1];
-        if (api.ETz) api.ETz[c] = v[2];
-        const double e2 = double(ex) * ex + double(ey) * ey;
-        se2 += e2;
-        me2 = fmax(me2, e2);
-        sb2 += double(b1.w) * b1.w + double(b2.x) * b2.x + double(b2.y) * b2.y;
-    }
-    __device__ void end() { zero_spare_partials(part); grid_partials(se2, me2, sb2, part); }
-};
-// Plain planes (the unfused solves).
-template <int N>
-struct FinPlanes {
-    static constexpr int NF = N;
-    float* out[N];
-    __device__ void begin() {}
-    __device__ void cell(int c, int, const float (&v)[N]) {
-#pragma unroll
-        for (int f = 0; f < N; ++f) out[f][c] = v[f];
-    }
-    __device__ void end() {}
-};
 
 // ---- the solves' multipliers -----------------------------------------------------------
 struct OpEs {
@@ -563,4 +351,20 @@ struct OpEt {
     static constexpr int NI = 7, NO = 3;      // dcu x y z, amu 0..3
     SpecGeo g; double eps0, c, n0;
     __device__ void operator()(int i, int j, const float2 (&in)[7], float2 (&out)[3]) const { et_k(i, j, g, eps0, c, n0, in, out); }
+};
+// The adjoints' transposes: the conjugate multipliers.
+struct OpEsT {       // lrho_k = sum_d conj(K_d) lE_d,k, K_d = -i k_d / (eps0 k^2)
+    static constexpr int NI = 2, NO = 1;
+    SpecGeo g; double eps0;
+    __device__ void operator()(int i, int j, const float2 (&in)[2], float2 (&out)[1]) const { es_T_k(i, j, g, eps0, in, out[0]); }
+};
+struct OpEtT {
+    static constexpr int NI = 3, NO = 7;
+    SpecGeo g; double eps0, c, n0;
+    __device__ void operator()(int i, int j, const float2 (&in)[3], float2 (&out)[7]) const { et_T_k(i, j, g, eps0, c, n0, in, out); }
+};
+struct OpElbT {
+    static constexpr int NI = 5, NO = 4;
+    SpecGeo g; double eps0, c;
+    __device__ void operator()(int i, int j, const float2 (&in)[5], float2 (&out)[4]) const { elb_T_k(i, j, g, eps0, c, in, out); }
 };

@@ -168,8 +168,8 @@ struct Ctx {
     cufftHandle p_r2c3 = 0, p_c2r3 = 0;     // dcu / E_T batch 3
     cufftHandle p_r2c4 = 0;                 // rho+J batch 4 (unfused solve)
     void* fft_work = nullptr;
-    // the three-kernel grid solves (aw_gridfft.cuh), or null: a grid they do not
-    // cover, solved through the plans above
+    // the three-kernel grid solves (aw_gridfft.cuh) of the unfused operators and the
+    // adjoints, or null: a grid they do not cover, solved through the plans above
     struct GridFft* gf = nullptr;
     bool plans_made = false;
 
@@ -304,8 +304,10 @@ void launch_adj_scatter(Ctx& c, const AdjP& a, const AdjK& k, const float* trajE
 void prep_adj_scatter();   // its shared-memory opt-in (before any capture)
 // acc[6][ncell] += the exact CIC scatter of the six value planes vals[f * n + p] at
 // the positions (xs, ys); scales from the maxima vmax[6] (float bits), stored to Sout.
+// With `slot`, the positions are those of slot *slot of a trajectory: xs + *slot * 5 n.
 void launch_scatter6(Ctx& c, cudaStream_t s, const float* xs, const float* ys, const float* vals, long long n,
-                     const unsigned* vmax, float* Sout, unsigned long long* acc, DevState* st);
+                     const unsigned* vmax, float* Sout, unsigned long long* acc, DevState* st,
+                     const long long* slot = nullptr);
 // The shared-memory opt-in of k_scatter6 on the current device (before a
 // stream capture that launches it).
 void prepare_scatter6();
@@ -332,18 +334,15 @@ void launch_charge_ref(Ctx& c);
 // products of 2, 3, 5, 7 of at most 1024; the buffers hold planes [nkx][ny].
 void gridfft_make(Ctx& c);
 void gridfft_free(Ctx& c);
-// acc fields [first, first + nf) finalised (as launch_finalize, not accumulating) and
-// transformed along x into out.
-void gridfft_rows_acc(Ctx& c, unsigned long long* acc, int first, int nf, const float* S, float* const* api,
-                      bool charge_partials, bool step_begin, bool sub_ref, cufftComplex* out);
 void gridfft_rows_real(Ctx& c, const float* const* src, int nf, cufftComplex* out);
 void gridfft_cols_es(Ctx& c, const cufftComplex* rho, cufftComplex* out);           // -> Ex, Ey
 void gridfft_cols_elb(Ctx& c, const cufftComplex* rho_j, cufftComplex* out);         // -> ELx, ELy, Bx, By, Bz
 void gridfft_cols_et(Ctx& c, const cufftComplex* dcu, const cufftComplex* amu, cufftComplex* out);   // -> ETx, ETy, ETz
-void gridfft_fields_es(Ctx& c, const cufftComplex* in, bool planes);   // planes: r_out too
-void gridfft_fields_dcu(Ctx& c, const cufftComplex* in);
-void gridfft_fields_push(Ctx& c, const cufftComplex* in);
-void gridfft_rows_planes(Ctx& c, const cufftComplex* in, float* const* out, int nf);   // 2, 3 or 5 planes
+// the transposes of the adjoints
+void gridfft_cols_es_T(Ctx& c, const cufftComplex* le, cufftComplex* out);           // lEx, lEy -> lrho
+void gridfft_cols_et_T(Ctx& c, const cufftComplex* let, cufftComplex* out);          // lE (3) -> ldcu (3), lamu (4)
+void gridfft_cols_elb_T(Ctx& c, const cufftComplex* l5, cufftComplex* out);          // lE_L, lB -> lrho, lJ (3)
+void gridfft_rows_planes(Ctx& c, const cufftComplex* in, float* const* out, int nf);   // 1 to 7 planes
 void launch_kspace_es(Ctx& c, const cufftComplex* rho_k, cufftComplex* e_k);
 void launch_es_solve_k(Ctx& c, const cufftComplex* rho_k, cufftComplex* ex_k, cufftComplex* ey_k);
 void launch_kspace_elb(Ctx& c, const cufftComplex* src_k, cufftComplex* out_k);

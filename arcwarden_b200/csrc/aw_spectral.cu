@@ -28,16 +28,9 @@
 namespace aw {
 namespace {
 
-constexpr int kGridBlocks = 592;   // 4 x 148 SMs; fixed so partials reduce in a fixed order
+#include "aw_transpose.cuh"
 
-__device__ __forceinline__ double kx_of(int i, double dkx) { return i * dkx; }
-__device__ __forceinline__ double ky_of(int j, int ny, double dky) {
-    const int m = (j <= ny / 2) ? j : j - ny;
-    return m * dky;
-}
-__device__ __forceinline__ bool nyquist(int i, int j, int nx, int ny) {
-    return ((nx % 2 == 0) && i == nx / 2) || ((ny % 2 == 0) && j == ny / 2);
-}
+constexpr int kGridBlocks = 592;   // 4 x 148 SMs; fixed so partials reduce in a fixed order
 
 // Trapezoidal pump ramp — include/pic/pump.hpp:27-32.
 __device__ __forceinline__ double pump_ramp(double t, double trmp, double toff) {
@@ -960,16 +953,6 @@ int gf_batch(const Ctx& c, int total, int other_blocks, size_t bytes_each, int m
     while (b > 1 && (b * bytes_each > kGfSmem || (total + b - 1) / b * other_blocks < c.sms)) b >>= 1;
     return b;
 }
-template <class Fin>
-void launch_rows_inv(Ctx& c, const cufftComplex* in, const Fin& fin) {
-    RowsInv<Fin> a{gf_args(c), in, fin};
-    const size_t each = static_cast<size_t>(2) * Fin::NF * a.g.rsx * sizeof(float2);
-    a.g.pr = gf_batch(c, pairs_of(c), 1, each, 4);
-    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
-    opt_in_smem(reinterpret_cast<const void*>(k_rows_inv<Fin>), sh);
-    k_rows_inv<Fin><<<(pairs_of(c) + a.g.pr - 1) / a.g.pr, kThreads, sh, c.stream>>>(a);
-    AW_LAUNCH();
-}
 template <class Op>
 void launch_cols(Ctx& c, const cufftComplex* const* in, cufftComplex* out, const Op& op) {
     ColsArgs<Op> a{};
@@ -984,21 +967,11 @@ void launch_cols(Ctx& c, const cufftComplex* const* in, cufftComplex* out, const
     k_cols<Op><<<(c.sg.nkx + a.cols - 1) / a.cols, kThreads, sh, c.stream>>>(a);
     AW_LAUNCH();
 }
-template <bool ACC>
-void launch_rows_fwd(Ctx& c, RowsFwd& a, int nf) {
-    const size_t each = static_cast<size_t>(2) * a.g.rsx * sizeof(float2);
-    a.g.pr = gf_batch(c, pairs_of(c), nf, each, 4);
-    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
-    opt_in_smem(reinterpret_cast<const void*>(k_rows_fwd<ACC>), sh);
-    k_rows_fwd<ACC><<<dim3((pairs_of(c) + a.g.pr - 1) / a.g.pr, nf), kThreads, sh, c.stream>>>(a);
-    AW_LAUNCH();
-}
 }  // namespace
 
 void gridfft_make(Ctx& c) {
-    // A row pair is one block's work: below 24 of them too few SMs take part, and the
-    // library transforms are faster (512 x 1: 58 us a step against 71; 64 x 64, 32
-    // pairs: 27.6 us either way; 256 x 256: 76.8 against 80.6).
+    // A row pair is one block's work: with few of them few SMs take part, and the
+    // library transforms are as fast (512 x 1: slower here by a fifth).
     if (c.geo.ny < 48) return;
     FftPlan px, py;
     if (c.geo.nx < 2 || !make_fft_plan(px, c.geo.nx) || !make_fft_plan(py, c.geo.ny)) return;
@@ -1020,26 +993,29 @@ void gridfft_free(Ctx& c) {
     delete c.gf;
     c.gf = nullptr;
 }
-void gridfft_rows_acc(Ctx& c, unsigned long long* acc, int first, int nf, const float* S, float* const* api,
-                      bool charge_partials, bool step_begin, bool sub_ref, cufftComplex* out) {
-    RowsFwd a{};
-    a.g = gf_args(c);
-    a.acc = acc; a.first = first; a.S = S;
-    for (int f = 0; f < nf; ++f) a.api.p[f] = api ? api[f] : nullptr;
-    a.part = charge_partials ? c.part_g : nullptr;
-    a.st = c.st;
-    a.step_begin = step_begin ? 1 : 0; a.darwin = c.model == AW_MODEL_DARWIN ? 1 : 0; a.sub_ref = sub_ref ? 1 : 0;
-    a.dt = c.prm.dt; a.cref = cref_of(c);
-    a.rec = step_begin ? c.rec_ad : nullptr;
-    a.out = out;
-    launch_rows_fwd<true>(c, a, nf);
-}
 void gridfft_rows_real(Ctx& c, const float* const* src, int nf, cufftComplex* out) {
     RowsFwd a{};
     a.g = gf_args(c);
     for (int f = 0; f < nf; ++f) a.src[f] = src[f];
     a.out = out;
-    launch_rows_fwd<false>(c, a, nf);
+    const size_t each = static_cast<size_t>(2) * a.g.rsx * sizeof(float2);
+    a.g.pr = gf_batch(c, pairs_of(c), nf, each, 4);
+    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
+    opt_in_smem(reinterpret_cast<const void*>(k_rows_fwd), sh);
+    k_rows_fwd<<<dim3((pairs_of(c) + a.g.pr - 1) / a.g.pr, nf), kThreads, sh, c.stream>>>(a);
+    AW_LAUNCH();
+}
+void gridfft_rows_planes(Ctx& c, const cufftComplex* in, float* const* out, int nf) {
+    RowsInv a{};
+    a.g = gf_args(c);
+    a.in = in;
+    for (int f = 0; f < nf; ++f) a.out[f] = out[f];
+    const size_t each = static_cast<size_t>(2) * a.g.rsx * sizeof(float2);
+    a.g.pr = gf_batch(c, pairs_of(c), nf, each, 4);
+    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
+    opt_in_smem(reinterpret_cast<const void*>(k_rows_inv), sh);
+    k_rows_inv<<<dim3((pairs_of(c) + a.g.pr - 1) / a.g.pr, nf), kThreads, sh, c.stream>>>(a);
+    AW_LAUNCH();
 }
 void gridfft_cols_es(Ctx& c, const cufftComplex* rho, cufftComplex* out) {
     launch_cols(c, &rho, out, OpEs{c.sg, c.prm.eps0});
@@ -1054,38 +1030,18 @@ void gridfft_cols_et(Ctx& c, const cufftComplex* dcu, const cufftComplex* amu, c
     for (int f = 0; f < 7; ++f) in[f] = (f < 3 ? dcu + static_cast<size_t>(f) * c.sg.nk : amu + static_cast<size_t>(f - 3) * c.sg.nk);
     launch_cols(c, in, out, OpEt{c.sg, c.prm.eps0, c.prm.c, c.prm.n0});
 }
-void gridfft_fields_es(Ctx& c, const cufftComplex* in, bool planes) {
-    FinEs f{};
-    f.gb = c.gb_es; f.ex = c.fld.Ex; f.ey = c.fld.Ey; f.r = planes ? c.r_out : nullptr;
-    f.part = c.part_g;
-    f.traj = reinterpret_cast<float2*>(c.rec_E); f.rec = c.rec_ad;
-    f.ncell = c.geo.ncell;
-    launch_rows_inv(c, in, f);
+void gridfft_cols_es_T(Ctx& c, const cufftComplex* le, cufftComplex* out) {
+    const cufftComplex* in[2] = {le, le + c.sg.nk};
+    launch_cols(c, in, out, OpEsT{c.sg, c.prm.eps0});
 }
-void gridfft_fields_dcu(Ctx& c, const cufftComplex* in) {
-    FinDcu f{};
-    f.gb = c.gb_dcu; f.r = c.r_out; f.api = api_of(c.fld);
-    f.b0x = c.prm.B0[0]; f.b0y = c.prm.B0[1]; f.b0z = c.prm.B0[2];
-    f.pa = pump_of(c); f.st = c.st; f.ncell = c.geo.ncell;
-    launch_rows_inv(c, in, f);
+void gridfft_cols_et_T(Ctx& c, const cufftComplex* let, cufftComplex* out) {
+    const cufftComplex* in[3] = {let, let + c.sg.nk, let + 2 * static_cast<size_t>(c.sg.nk)};
+    launch_cols(c, in, out, OpEtT{c.sg, c.prm.eps0, c.prm.c, c.prm.n0});
 }
-void gridfft_fields_push(Ctx& c, const cufftComplex* in) {
-    FinPush f{};
-    f.rel = c.r_out; f.gbd = c.gb_dcu; f.gb = c.gb_push; f.api = api_of(c.fld);
-    f.pa = pump_of(c); f.st = c.st; f.part = c.part_g; f.ncell = c.geo.ncell;
-    launch_rows_inv(c, in, f);
-}
-void gridfft_rows_planes(Ctx& c, const cufftComplex* in, float* const* out, int nf) {
-    auto go = [&](auto fin) {
-        for (int f = 0; f < nf; ++f) fin.out[f] = out[f];
-        launch_rows_inv(c, in, fin);
-    };
-    switch (nf) {
-        case 2: go(FinPlanes<2>{}); break;
-        case 3: go(FinPlanes<3>{}); break;
-        case 5: go(FinPlanes<5>{}); break;
-        default: throw Error(AW_ERR_ARG, "gridfft_rows_planes: 2, 3 or 5 planes");
-    }
+void gridfft_cols_elb_T(Ctx& c, const cufftComplex* l5, cufftComplex* out) {
+    const cufftComplex* in[5];
+    for (int f = 0; f < 5; ++f) in[f] = l5 + static_cast<size_t>(f) * c.sg.nk;
+    launch_cols(c, in, out, OpElbT{c.sg, c.prm.eps0, c.prm.c});
 }
 
 void launch_make_scales(Ctx& c) {
