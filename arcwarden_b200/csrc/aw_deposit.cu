@@ -2073,12 +2073,21 @@ void launch_adj_scatter(Ctx& c, const AdjP& a, const AdjK& k, const float* trajE
 // as the Darwin J deposit, S_x = scale for cm U_x (S_next[1..3], set at the step
 // begin from the |u| maxima). A particle whose bound exceeds the fast range
 // (it sped up past 1.25 x the previous maximum) takes the exact slow path.
+//
+// Bound by instruction issue (76 % of the issue slots, 790 instructions a particle;
+// the particle traffic alone would take 0.26 ms where the kernel takes 1.10). Measured at 625 x 625, 39 M
+// particles, cell order, ms:
+//   1.48  each component with its own floors, wraps and weights, divisions in the
+//         moves, a branch per Esirkepov weight
+//   1.31  the two axes per dimension shared by the six gathers, the moves by
+//         reciprocal, the coefficients kept while the weight stays, predicates
+//   1.10  moves inside one cell with their 8 weights, the rest listed (yee_window_pass)
 constexpr int kYeePlanes = 7, kYeeWindow = 576;
 struct YeeArgs {
     Parts p; Geo g;
     const float *ex, *ey, *ez, *bx, *by, *bz;   // Yee lattices [ny][nx]
     float qmh, qm, invdt, dxp, dyp, b0x, b0y, b0z;
-    double dt, dxd, dyd;                      // dxd, dyd: the float cell sizes, widened
+    double dt, dxd, dyd, rdx, rdy;            // dxd, dyd: the float cell sizes, widened; their reciprocals
     PumpP pump;
     unsigned long long* acc; int wmaxc; double* part; DevState* st; int write_cell;
 };
@@ -2086,35 +2095,45 @@ struct YeeArgs {
 // node shape over {b - 1, .., b + 2}: S = max(0, 1 - |x - p|) (yee2d.hpp:124-130).
 // With b = floor(min(x0, x1)) the first node is always 0: x - (b - 1) >= 1,
 // and the float difference rounds monotonically from the exact 1 of x = b. So
-// only nodes 1..3 are computed and S[0] is the constant 0.
+// only nodes 1..3 are computed.
 __device__ __forceinline__ void yee_shape4(float x, int b, float (&S)[4]) {
     S[0] = 0.f;
 #pragma unroll
-    for (int n = 1; n < 4; ++n) {
-        const float d = fabsf(x - (float)(b - 1 + n));
-        S[n] = d < 1.f ? 1.f - d : 0.f;
-    }
+    for (int n = 1; n < 4; ++n) S[n] = fmaxf(1.f - fabsf(x - (float)(b - 1 + n)), 0.f);
 }
 
-// Staggered CIC gather (yee2d.hpp:103-112): component lattice offset (ox, oy).
-__device__ __forceinline__ float yee_gather(const float* __restrict__ a, const Geo& g, float x, float y,
-                                            float ox, float oy) {
-    const float xs = x - ox, ys = y - oy;
-    const int i0 = (int)floorf(xs), j0 = (int)floorf(ys);
-    const float fx = xs - i0, fy = ys - j0;
-    const int ia = wrap_once(i0, g.nx), ib = wrap_once(i0 + 1, g.nx);
-    const int ja = wrap_once(j0, g.ny) * g.nx, jb = wrap_once(j0 + 1, g.ny) * g.nx;
-    return (1.f - fx) * (1.f - fy) * __ldg(a + ja + ia)
-         +        fx  * (1.f - fy) * __ldg(a + ja + ib)
-         + (1.f - fx) *        fy  * __ldg(a + jb + ia)
-         +        fx  *        fy  * __ldg(a + jb + ib);
+// One axis of the staggered CIC gathers: the position against the nodes (offset 0)
+// or the half nodes (0.5): the two wrapped nodes and the weights (yee2d.hpp:103-112).
+// The six components share two such axes in x and two in y.
+struct YeeAxis { int a, b; float f, g; };
+__device__ __forceinline__ YeeAxis yee_axis(float x, float off, int n) {
+    const float xs = x - off;
+    const float fl = floorf(xs);
+    const int i = (int)fl;
+    YeeAxis r;
+    r.f = xs - fl;
+    r.g = 1.f - r.f;
+    r.a = wrap_once(i, n);
+    r.b = wrap_once(i + 1, n);
+    return r;
+}
+// sum of the four corners in the reference's order, w0 a and the later terms fused,
+// w1 b rounded (its compiled form).
+__device__ __forceinline__ float yee_gather(const float* __restrict__ a, const YeeAxis& X, const YeeAxis& Y) {
+    const float r = __fmaf_rn(__fmul_rn(X.g, Y.g), __ldg(a + Y.a + X.a), __fmul_rn(__fmul_rn(X.f, Y.g), __ldg(a + Y.a + X.b)));
+    return __fmaf_rn(__fmul_rn(X.f, Y.f), __ldg(a + Y.b + X.b), __fmaf_rn(__fmul_rn(X.g, Y.f), __ldg(a + Y.b + X.a), r));
+}
+
+__device__ __forceinline__ float yee_wz(float sx0, float sy0, float dsx, float dsy) {
+    return sx0 * sy0 + 0.5f * (dsx * sy0 + sx0 * dsy) + (1.f / 3.f) * dsx * dsy;
 }
 
 // The Esirkepov node weights of one move (yee2d.hpp:307-355, its operation
-// order): emit(f, ni, nj, w) for every nonzero weight of field f (0: the Jx
-// prefix sums, 1: the Jy prefix sums, 2: Jz) at node (ib - 1 + ni, jb - 1 + nj).
+// order): emit(f, ni, nj, w) for every weight of field f (0: the Jx prefix sums,
+// 1: the Jy prefix sums, 2: Jz) at node (ib - 1 + ni, jb - 1 + nj), zero or not:
+// the emitter drops what rounds to nothing with a predicate.
 // The reference's 4 x 4 loops start at node 0, whose shapes are 0: its Jx and
-// Jy prefix sums stay exactly +0 there and its Jz weights are 0, all skipped.
+// Jy prefix sums stay exactly +0 there and its Jz weights are 0.
 // Starting at node 1 emits the same float values.
 template <class Emit>
 __device__ __forceinline__ void esirkepov_weights(float x0, float y0, float x1, float y1, int ib, int jb,
@@ -2132,7 +2151,7 @@ __device__ __forceinline__ void esirkepov_weights(float x0, float y0, float x1, 
 #pragma unroll
         for (int ni = 1; ni < 4; ++ni) {
             a += DSx[ni] * sy;
-            if (a != 0.f) emit(0, ni, nj, a);
+            emit(0, ni, nj, a);
         }
     }
 #pragma unroll
@@ -2142,16 +2161,15 @@ __device__ __forceinline__ void esirkepov_weights(float x0, float y0, float x1, 
 #pragma unroll
         for (int nj = 1; nj < 4; ++nj) {
             a += DSy[nj] * sx;
-            if (a != 0.f) emit(1, ni, nj, a);
+            emit(1, ni, nj, a);
         }
     }
 #pragma unroll
     for (int nj = 1; nj < 4; ++nj)
 #pragma unroll
         for (int ni = 1; ni < 4; ++ni) {
-            const float wz = Sx0[ni] * Sy0[nj] + 0.5f * (DSx[ni] * Sy0[nj] + Sx0[ni] * DSy[nj])
-                           + (1.f / 3.f) * DSx[ni] * DSy[nj];
-            if (wz != 0.f) emit(2, ni, nj, wz);
+            const float wz = yee_wz(Sx0[ni], Sy0[nj], DSx[ni], DSy[nj]);
+            emit(2, ni, nj, wz);
         }
 }
 
@@ -2160,29 +2178,99 @@ __device__ __forceinline__ int wrap_node(int i, int n) {
     return i < 0 ? i + n : i;
 }
 
+// The weights of a move that stays inside cell (ib, jb), 8 of the 27: only nodes 1
+// and 2 have shapes, and a prefix sum is one value at node 1 (of rows or columns 1
+// and 2) and a remainder from node 2 on. False if the general weights are due: a move
+// that changes its cell, or shape differences that don't cancel exactly (positions
+// below 1, where 1 - x rounds). When they do, the remainder is the rounding error of
+// one product of at most 2^22 once scaled (the caller's bound), at most 0.25: it
+// rounds to no integer, so these 8 are all that the general weights would add.
+struct YeeIn { float x[2], y[2], z[2][2]; };      // x: Jx rows 1, 2; y: Jy columns 1, 2; z[nj][ni]
+__device__ __forceinline__ bool yee_in_cell(float x0, float y0, float x1, float y1, float fi, float fj, YeeIn& w) {
+    const float xb = fi + 1.f, yb = fj + 1.f;
+    const float sx0[2] = {1.f - (x0 - fi), 1.f - (xb - x0)}, sx1[2] = {1.f - (x1 - fi), 1.f - (xb - x1)};
+    const float sy0[2] = {1.f - (y0 - fj), 1.f - (yb - y0)}, sy1[2] = {1.f - (y1 - fj), 1.f - (yb - y1)};
+    const float dx[2] = {sx1[0] - sx0[0], sx1[1] - sx0[1]}, dy[2] = {sy1[0] - sy0[0], sy1[1] - sy0[1]};
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        w.x[n] = dx[0] * (sy0[n] + 0.5f * dy[n]);
+        w.y[n] = dy[0] * (sx0[n] + 0.5f * dx[n]);
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) w.z[n][ni] = yee_wz(sx0[ni], sy0[n], dx[ni], dy[n]);
+    }
+    return fmaxf(x0, x1) < xb && fmaxf(y0, y1) < yb && dx[1] == -dx[0] && dy[1] == -dy[0];
+}
+
 // Stage planes: 0 x0 (sign set: skipped, listed for the slow pass), 1 y0, 2 x1,
-// 3 y1 (unwrapped), 4..6 the scaled coefficients ax ay az.
+// 3 y1 (unwrapped), 4..6 the scaled coefficients ax ay az. Two rounds: the moves
+// inside one cell, by far the most (a step moves a particle a few hundredths of a
+// cell), with their 8 weights; the others, listed from the end of `list` down (the
+// slow pass's entries grow from its start; no slot is in both), then have all 27 at
+// full warps. One round with every weight behind a predicate took 27 weights for
+// each warp that had a single such move: see k_push_esirkepov.
+struct YeeCell { float x0, y0, x1, y1, a0, a1, a2, fi, fj; int ib, jb, o; };
+__device__ __forceinline__ bool yee_load(const float* __restrict__ stage, const Win& wn, const Geo& g, int d,
+                                         YeeCell& q) {
+    q.x0 = stage[d];
+    if (__float_as_int(q.x0) < 0) return false;
+    q.y0 = stage[kChunk + d]; q.x1 = stage[2 * kChunk + d]; q.y1 = stage[3 * kChunk + d];
+    q.a0 = stage[4 * kChunk + d]; q.a1 = stage[5 * kChunk + d]; q.a2 = stage[6 * kChunk + d];
+    q.fi = floorf(fminf(q.x0, q.x1)); q.fj = floorf(fminf(q.y0, q.y1));
+    q.ib = (int)q.fi; q.jb = (int)q.fj;
+    // window cell of node 1 (ib, jb): the stencil's first nonzero node
+    q.o = (win_off(q.jb, wn.jr, g.ny) - wn.mj) * wn.W + win_off(q.ib, wn.ir, g.nx) - wn.mi;
+    return true;
+}
+template <bool TRACK>
+__device__ __forceinline__ void yee_add(int* e, int v) {
+    if (TRACK) {
+        if (v != 0) add_tracked(e, 3 * kYeeWindow, v);
+    } else {
+        atomicAdd(e, v);
+    }
+}
+template <bool TRACK>
 __device__ __forceinline__ void yee_window_pass(const float* __restrict__ stage, int* __restrict__ win,
-                                                const Win& wn, int csz, const Geo& g) {
-    if (!wn.use) return;
-    const Spread sp(csz);
-    const int ppt = csz / kThreads;
+                                                const Win& wn, int csz, const Geo& g,
+                                                unsigned short* __restrict__ list, int* ncross) {
+    const int W = wn.W;
+    if (wn.use) {
+        const Spread sp(csz);
+        const int ppt = csz / kThreads;
 #pragma unroll 1
-    for (int k = 0; k < ppt; ++k) {
-        const int d = sp.slot(k);
-        const float x0 = stage[d];
-        if (__float_as_int(x0) < 0) continue;
-        const float y0 = stage[kChunk + d], x1 = stage[2 * kChunk + d], y1 = stage[3 * kChunk + d];
-        const float a0 = stage[4 * kChunk + d], a1 = stage[5 * kChunk + d], a2 = stage[6 * kChunk + d];
-        const int ib = (int)floorf(fminf(x0, x1)), jb = (int)floorf(fminf(y0, y1));
-        // window column / row of node 1 (ib, jb): the stencil's first nonzero node
-        const int ci = win_off(ib, wn.ir, g.nx) - wn.mi - 1, cj = win_off(jb, wn.jr, g.ny) - wn.mj - 1;
-        esirkepov_weights(x0, y0, x1, y1, ib, jb, [&](int f, int ni, int nj, float w) {
-            const int v = quant(f == 0 ? a0 : f == 1 ? a1 : a2, w);
-            if (v == 0) return;                    // prefix-sum residues that round to nothing
-            int* e = win + f * wn.P + (cj + nj) * wn.W + (ci + ni);
-            if (wn.track_all) add_tracked(e, 3 * wn.P, v);
-            else atomicAdd(e, v);
+        for (int k = 0; k < ppt; ++k) {
+            const int d = sp.slot(k);
+            YeeCell q;
+            if (!yee_load(stage, wn, g, d, q)) continue;
+            YeeIn w;
+            if (!yee_in_cell(q.x0, q.y0, q.x1, q.y1, q.fi, q.fj, w)) {
+                list[csz - 1 - atomicAdd(ncross, 1)] = static_cast<unsigned short>(d);
+                continue;
+            }
+            int* const e0 = win + q.o;
+            int* const e1 = e0 + W;
+            yee_add<TRACK>(e0, quant(q.a0, w.x[0]));
+            yee_add<TRACK>(e1, quant(q.a0, w.x[1]));
+            yee_add<TRACK>(e0 + kYeeWindow, quant(q.a1, w.y[0]));
+            yee_add<TRACK>(e0 + kYeeWindow + 1, quant(q.a1, w.y[1]));
+            yee_add<TRACK>(e0 + 2 * kYeeWindow, quant(q.a2, w.z[0][0]));
+            yee_add<TRACK>(e0 + 2 * kYeeWindow + 1, quant(q.a2, w.z[0][1]));
+            yee_add<TRACK>(e1 + 2 * kYeeWindow, quant(q.a2, w.z[1][0]));
+            yee_add<TRACK>(e1 + 2 * kYeeWindow + 1, quant(q.a2, w.z[1][1]));
+        }
+    }
+    __syncthreads();
+    const int nc = *ncross;
+    for (int k = threadIdx.x; k < nc; k += kThreads) {
+        YeeCell q;
+        yee_load(stage, wn, g, list[csz - 1 - k], q);
+        int* const e0 = win + q.o;
+        int* const e1 = e0 + W;
+        int* const e2 = e1 + W;
+        esirkepov_weights(q.x0, q.y0, q.x1, q.y1, q.ib, q.jb, [&](int f, int ni, int nj, float w) {
+            const int v = quant(f == 0 ? q.a0 : f == 1 ? q.a1 : q.a2, w);
+            if (v == 0) return;                    // no weight, or a remainder that rounds to nothing
+            yee_add<TRACK>((nj == 1 ? e0 : nj == 2 ? e1 : e2) + f * kYeeWindow + (ni - 1), v);
         });
     }
 }
@@ -2236,7 +2324,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const Smem m = carve(smem, kYeePlanes, 2 * NF, A.wmaxc);   // sums and carries: no count plane
     __shared__ unsigned long long bar;
-    __shared__ int nlist;
+    __shared__ int nlist, ncross;
     __shared__ double dsh[4 * (kThreads / 32)];
     __shared__ unsigned umx[3][kThreads / 32];
 
@@ -2249,7 +2337,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
     const double tnow = st->t;
     const bool pump = A.pump.on && tnow < A.pump.toff;
     const double ramp = pump ? yee_ramp(tnow, A.pump.trmp, A.pump.toff) : 0.0;
-    if (threadIdx.x == 0) nlist = 0;
+    if (threadIdx.x == 0) { nlist = 0; ncross = 0; }
     const ChunkSrc src{{p.x, p.y, p.ux, p.uy, p.uz, nullptr}};
     float xr, yr;
     if (!load_chunk(m.stage, src, NIN, c0, cnt, p.vec_ok != 0, &bar, st, &xr, &yr)) return;
@@ -2260,6 +2348,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
     float l1[NF] = {};
     double ke = 0, px = 0, py = 0, pz = 0;
     float m0 = 0.f, m1 = 0.f, m2 = 0.f;
+    float wlast = __int_as_float(0x7fffffff), qw = 0.f, cx = 0.f, cy = 0.f;     // NaN: no weight yet
 #pragma unroll 1
     for (int it = 0; it < ppt; ++it) {
         const int s = it * kThreads + threadIdx.x;
@@ -2270,22 +2359,26 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
         float xs = -1.0f, x1 = 0.f, y1 = 0.f, ax = 0.f, ay = 0.f, az = 0.f;
         if (s < cnt) {
             if (in_grid(x0, y0, g)) {
-                float ex = yee_gather(A.ex, g, x0, y0, 0.5f, 0.f);
-                float ey = yee_gather(A.ey, g, x0, y0, 0.f, 0.5f);
-                float ez = yee_gather(A.ez, g, x0, y0, 0.f, 0.f);
+                const YeeAxis xn = yee_axis(x0, 0.f, g.nx), xh = yee_axis(x0, 0.5f, g.nx);
+                YeeAxis yn = yee_axis(y0, 0.f, g.ny), yh = yee_axis(y0, 0.5f, g.ny);
+                yn.a *= g.nx; yn.b *= g.nx; yh.a *= g.nx; yh.b *= g.nx;
+                float ex = yee_gather(A.ex, xh, yn);
+                float ey = yee_gather(A.ey, xn, yh);
+                float ez = yee_gather(A.ez, xn, yn);
                 if (pump) {
                     const double th = A.pump.k0 * static_cast<double>(x0) * A.dxd - A.pump.w0 * tnow;
                     ex += (float)(A.pump.ex * cos(th) * ramp);
                     ey += (float)(-A.pump.ey * sin(th) * ramp);
                     ez += (float)(A.pump.ez * cos(th) * ramp);
                 }
-                const float bx = yee_gather(A.bx, g, x0, y0, 0.f, 0.5f) + A.b0x;
-                const float by = yee_gather(A.by, g, x0, y0, 0.5f, 0.f) + A.b0y;
-                const float bz = yee_gather(A.bz, g, x0, y0, 0.5f, 0.5f) + A.b0z;
+                const float bx = yee_gather(A.bx, xn, yh) + A.b0x;
+                const float by = yee_gather(A.by, xh, yn) + A.b0y;
+                const float bz = yee_gather(A.bz, xh, yh) + A.b0z;
                 boris_em(ux, uy, uz, ex, ey, ez, bx, by, bz, A.qmh);
-                x1 = move1(x0, ux, A.dt, A.dxd);
-                y1 = move1(y0, uy, A.dt, A.dyd);
-                const float xw = wrap_pos(x1, g.nxf), yw = wrap_pos(y1, g.nyf);
+                x1 = move1_by(x0, ux, A.dt, A.dxd, A.rdx);
+                y1 = move1_by(y0, uy, A.dt, A.dyd, A.rdy);
+                float xw = x1, yw = y1;
+                if (!in_grid(x1, y1, g)) { xw = wrap_pos(x1, g.nxf); yw = wrap_pos(y1, g.nyf); }
                 __stcs(p.x + i, xw); __stcs(p.y + i, yw); __stcs(p.ux + i, ux); __stcs(p.uy + i, uy);
                 __stcs(p.uz + i, uz);
                 if (A.write_cell && p.cell) {
@@ -2295,9 +2388,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
                 }
                 m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy)); m2 = fmaxf(m2, fabsf(uz));
                 // coefficients: cJx = -q w / (dt dy), cJy = -q w / (dt dx), cJz = q w vz / (dx dy)
-                const float qw = A.qm * w;
-                ax = __fmul_rn(-qw * A.invdt / A.dyp, S[0]);
-                ay = __fmul_rn(-qw * A.invdt / A.dxp, S[1]);
+                if (w != wlast) {        // (a species' weights are equal: its coefficients are taken once)
+                    wlast = w;
+                    qw = A.qm * w;
+                    cx = __fmul_rn(-qw * A.invdt / A.dyp, S[0]);
+                    cy = __fmul_rn(-qw * A.invdt / A.dxp, S[1]);
+                }
+                ax = cx; ay = cy;
                 az = __fmul_rn(qw * uz / (A.dxp * A.dyp), S[2]);
                 const int ib = (int)floorf(fminf(x0, x1)), jb = (int)floorf(fminf(y0, y1));
                 bb.add(ib, jb, ir, jr, g);                 // nodes ib..ib+2 (node ib-1 has no weight)
@@ -2352,7 +2449,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_esirkepov(YeeArgs A) {
         atomicMax(&st->umax_bits[threadIdx.x], mx);
     }
     __syncthreads();
-    yee_window_pass(m.stage, m.win, wn, cs_, g);
+    if (wn.track_all) yee_window_pass<true>(m.stage, m.win, wn, cs_, g, m.slow, &ncross);
+    else yee_window_pass<false>(m.stage, m.win, wn, cs_, g, m.slow, &ncross);
     __syncthreads();
     win_flush<NF, false>(m.win, wn, acc, g);
     yee_slow_pass(m.stage, m.slow, nlist, !wn.use, cs_, acc, g, st);
@@ -2483,6 +2581,7 @@ void launch_push_esirkepov(Ctx& c) {
     a.b0x = c.prm.B0[0]; a.b0y = c.prm.B0[1]; a.b0z = c.prm.B0[2];
     a.dt = c.prm.dt;
     a.dxd = static_cast<double>(a.dxp); a.dyd = static_cast<double>(a.dyp);
+    a.rdx = 1.0 / a.dxd; a.rdy = 1.0 / a.dyd;
     a.pump.on = c.prm.pump;
     a.pump.ex = c.prm.pump_ex; a.pump.ey = c.prm.pump_ey; a.pump.ez = c.prm.pump_ez;
     a.pump.k0 = c.prm.pump_k0; a.pump.w0 = c.prm.pump_w0; a.pump.trmp = c.prm.pump_trmp; a.pump.toff = c.prm.pump_toff;

@@ -769,13 +769,15 @@ __device__ __forceinline__ int yee_idx(int i, int j, int nx, int ny) {
 __global__ void k_yee_faraday(YeeF v, float dt2, DevState* st, int begin, double dt, float cref) {
     const int n = v.nx * v.ny;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        const int i = c % v.nx, j = c / v.nx;
-        const float ez_xp = v.ez[yee_idx(i + 1, j, v.nx, v.ny)], ez_yp = v.ez[yee_idx(i, j + 1, v.nx, v.ny)];
-        const float ex_yp = v.ex[yee_idx(i, j + 1, v.nx, v.ny)];
-        const float ey_xp = v.ey[yee_idx(i + 1, j, v.nx, v.ny)];
-        v.bx[c] -= dt2 * (ez_yp - v.ez[c]) / v.dyp;
-        v.by[c] += dt2 * (ez_xp - v.ez[c]) / v.dxp;
-        v.bz[c] -= dt2 * ((ey_xp - v.ey[c]) / v.dxp - (ex_yp - v.ex[c]) / v.dyp);
+        const int j = c / v.nx, i = c - j * v.nx;
+        const int cxp = i + 1 < v.nx ? c + 1 : c + 1 - v.nx, cyp = j + 1 < v.ny ? c + v.nx : c + v.nx - n;
+        const float ez0 = v.ez[c], ex0 = v.ex[c], ey0 = v.ey[c];
+        const float ez_xp = v.ez[cxp], ez_yp = v.ez[cyp], ex_yp = v.ex[cyp], ey_xp = v.ey[cxp];
+        float bx = v.bx[c], by = v.by[c], bz = v.bz[c];
+        bx -= dt2 * (ez_yp - ez0) / v.dyp;
+        by += dt2 * (ez_xp - ez0) / v.dxp;
+        bz -= dt2 * ((ey_xp - ey0) / v.dxp - (ex_yp - ex0) / v.dyp);
+        v.bx[c] = bx; v.by[c] = by; v.bz[c] = bz;
     }
     if (begin && blockIdx.x == 0 && threadIdx.x == 0) {
         st->t = static_cast<double>(st->step) * dt;
@@ -796,24 +798,32 @@ __global__ void k_yee_faraday(YeeF v, float dt2, DevState* st, int begin, double
 // J'(i, j) = sum_{a, b} C(2m, a) C(2m, b) J(i + a - m, j + b - m) / 16^m. On the
 // integer accumulator the sums are exact; the 16^m goes into the finalising
 // scale. One pass along x (in -> out) or y, three fields, periodic.
-__global__ void k_yee_binomial(const unsigned long long* __restrict__ in, unsigned long long* __restrict__ out,
-                               int nx, int ny, int m, int along_y) {
-    const int n = nx * ny;
-    long long cb[9];
-    cb[0] = 1;
-    for (int k = 1; k <= 2 * m; ++k) cb[k] = cb[k - 1] * (2 * m - k + 1) / k;   // C(2m, k)
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * n; t += gridDim.x * blockDim.x) {
-        const int f = t / n, c = t - f * n;
-        const int i = c % nx, j = c / nx;
-        const unsigned long long* a = in + static_cast<size_t>(f) * n;
-        long long s = 0;
-        for (int k = 0; k <= 2 * m; ++k) {
-            int ii = i, jj = j;
-            if (along_y) { jj = (j + k - m) % ny; if (jj < 0) jj += ny; }
-            else { ii = (i + k - m) % nx; if (ii < 0) ii += nx; }
-            s += cb[k] * static_cast<long long>(a[jj * nx + ii]);
+__global__ void __launch_bounds__(kThreads) k_yee_binomial(const unsigned long long* __restrict__ in,
+                                                           unsigned long long* __restrict__ out, int nx, int ny, int m,
+                                                           int along_y) {
+    const int n = nx * ny, len = along_y ? ny : nx, stride = along_y ? nx : 1;
+    long long cb[5];                               // C(2m, m - k), k = 0..m
+    cb[4] = 0;
+    {
+        long long c = 1;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) cb[k] = 0;
+        for (int k = 0; k <= m; ++k) { cb[m - k] = c; c = c * (2 * m - k) / (k + 1); }
+    }
+    const unsigned long long* a = in + static_cast<size_t>(blockIdx.y) * n;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+        const int j = c / nx, i = c - j * nx, at = along_y ? j : i;
+        const unsigned long long* row = a + (c - at * stride);
+        long long s = cb[0] * static_cast<long long>(a[c]);
+#pragma unroll
+        for (int k = 1; k <= 4; ++k) {
+            if (k > m) break;
+            int lo = at - k, hi = at + k;          // wrapped (a dimension may be shorter than the stencil)
+            while (lo < 0) lo += len;
+            while (hi >= len) hi -= len;
+            s += cb[k] * (static_cast<long long>(row[lo * stride]) + static_cast<long long>(row[hi * stride]));
         }
-        out[t] = static_cast<unsigned long long>(s);
+        out[static_cast<size_t>(blockIdx.y) * n + c] = static_cast<unsigned long long>(s);
     }
 }
 
@@ -829,9 +839,15 @@ __global__ void k_yee_ampere(YeeF v, unsigned long long* __restrict__ acc, const
     const double iz = fscale / static_cast<double>(st->S_next[3]);
     double se2 = 0.0, me2 = 0.0, sb2 = 0.0;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+        // every load before the first store: they are in flight together
         const long long ax = static_cast<long long>(acc[c]);
         const long long ay = static_cast<long long>(acc[n + c]);
         const long long az = static_cast<long long>(acc[2 * n + c]);
+        const int j = c / v.nx, i = c - j * v.nx;
+        const int cxm = i > 0 ? c - 1 : c + v.nx - 1, cym = j > 0 ? c - v.nx : c + n - v.nx;
+        const float bx0 = v.bx[c], by0 = v.by[c], bz0 = v.bz[c];
+        const float bz_ym = v.bz[cym], bz_xm = v.bz[cxm], bx_ym = v.bx[cym], by_xm = v.by[cxm];
+        float ex = v.ex[c], ey = v.ey[c], ez = v.ez[c];
         acc[c] = 0ull; acc[n + c] = 0ull; acc[2 * n + c] = 0ull;
         const float jx = __double2float_rn(static_cast<double>(ax) * ix);
         const float jy = __double2float_rn(static_cast<double>(ay) * iy);
@@ -839,21 +855,15 @@ __global__ void k_yee_ampere(YeeF v, unsigned long long* __restrict__ acc, const
         if (jx_api) jx_api[c] = jx;
         if (jy_api) jy_api[c] = jy;
         if (jz_api) jz_api[c] = jz;
-        const int i = c % v.nx, j = c / v.nx;
-        const float bz_ym = v.bz[yee_idx(i, j - 1, v.nx, v.ny)];
-        const float bz_xm = v.bz[yee_idx(i - 1, j, v.nx, v.ny)];
-        const float bx_ym = v.bx[yee_idx(i, j - 1, v.nx, v.ny)];
-        const float by_xm = v.by[yee_idx(i - 1, j, v.nx, v.ny)];
-        v.ex[c] += v.dt * ( v.c2 * (v.bz[c] - bz_ym) / v.dyp - jx);
-        v.ey[c] += v.dt * (-v.c2 * (v.bz[c] - bz_xm) / v.dxp - jy);
-        v.ez[c] += v.dt * ( v.c2 * ((v.by[c] - by_xm) / v.dxp
-                                  - (v.bx[c] - bx_ym) / v.dyp) - jz);
-        const double e2 = static_cast<double>(v.ex[c]) * v.ex[c] + static_cast<double>(v.ey[c]) * v.ey[c] +
-                          static_cast<double>(v.ez[c]) * v.ez[c];
+        ex += v.dt * ( v.c2 * (bz0 - bz_ym) / v.dyp - jx);
+        ey += v.dt * (-v.c2 * (bz0 - bz_xm) / v.dxp - jy);
+        ez += v.dt * ( v.c2 * ((by0 - by_xm) / v.dxp
+                             - (bx0 - bx_ym) / v.dyp) - jz);
+        v.ex[c] = ex; v.ey[c] = ey; v.ez[c] = ez;
+        const double e2 = static_cast<double>(ex) * ex + static_cast<double>(ey) * ey + static_cast<double>(ez) * ez;
         se2 += e2;
         me2 = fmax(me2, e2);
-        sb2 += static_cast<double>(v.bx[c]) * v.bx[c] + static_cast<double>(v.by[c]) * v.by[c] +
-               static_cast<double>(v.bz[c]) * v.bz[c];
+        sb2 += static_cast<double>(bx0) * bx0 + static_cast<double>(by0) * by0 + static_cast<double>(bz0) * bz0;
     }
     grid_partials(se2, me2, sb2, part);
 }
@@ -1128,7 +1138,7 @@ void launch_yee_ampere(Ctx& c) {
 void launch_yee_filter(Ctx& c) {
     if (c.yee_jfilter <= 0) return;
     const int n = c.geo.ncell;
-    const int blocks = std::min(4096, (3 * n + kThreads - 1) / kThreads);
+    const dim3 blocks(std::min(2048, (n + kThreads - 1) / kThreads), 3);
     k_yee_binomial<<<blocks, kThreads, 0, c.stream>>>(c.acc_src, c.acc_tmp, c.geo.nx, c.geo.ny, c.yee_jfilter, 0);
     AW_LAUNCH();
     k_yee_binomial<<<blocks, kThreads, 0, c.stream>>>(c.acc_tmp, c.acc_src, c.geo.nx, c.geo.ny, c.yee_jfilter, 1);

@@ -181,6 +181,81 @@ def test_yee_is_deterministic_and_order_free(torch_cuda, aw, ref):
         c.close()
 
 
+@pytest.mark.parametrize("nx,ny,move", [(64, 48, 0.9), (64, 48, 0.02), (63, 49, 1e-4), (300, 5, 1e-6),
+                                        (200, 33, 1.5)])
+def test_yee_moves_inside_a_cell_equal_the_general_weights(torch_cuda, aw, nx, ny, move):
+    """In cell order the chunks deposit in windows, where a move that stays in its cell
+    has 8 weights and the others all 27; shuffled over the whole grid they don't fit one
+    and every particle takes the exact path, which has the 27 for all. J, E and B agree
+    bit for bit, for moves of a millionth of a cell to several cells, positions on cell
+    edges, one ulp below them and within 1e-6 of zero, particles at rest, and weights
+    of both signs and of different sizes."""
+    n = nx * ny * 24 - 5
+    rng = np.random.default_rng(nx + ny)
+    cell = np.repeat(np.arange(nx * ny), 24)[:n]
+    fx, fy = rng.random(n), rng.random(n)
+    fx[::7] = 0.0
+    fy[::11] = 0.0
+    x, y = (cell % nx + fx).astype(np.float32), (cell // nx + fy).astype(np.float32)
+    x[::13] = np.nextafter(cell[::13] % nx + np.float32(1), np.float32(0), dtype=np.float32)
+    y[::17] = np.nextafter(cell[::17] // nx + np.float32(1), np.float32(0), dtype=np.float32)
+    x[:200] *= np.float32(1e-6)
+    x, y = np.minimum(x, np.nextafter(np.float32(nx), np.float32(0))), np.minimum(y, np.nextafter(np.float32(ny), np.float32(0)))
+    dx, dy, dt = 0.3, 0.7, 0.05
+    P = {"x": x, "y": y, "w": rng.choice([-0.7, 0.3, 1.0], n)}
+    for k, d in (("ux", dx), ("uy", dy), ("uz", 1.0)):
+        P[k] = rng.uniform(-1, 1, n) * move * d / dt
+        P[k][::19] = 0.0
+    P = {k: v.astype(np.float32) for k, v in P.items()}
+    out = []
+    for order in (np.arange(n), rng.permutation(n)):
+        s = Setup(torch_cuda, aw, nx, ny, nx * dx, ny * dy, n, aw.AW_MODEL_YEE, dt=dt, c=0.5, qm=-1.0, B0=(0.1, 0.0, 0.3))
+        try:
+            for k in PARTICLE_KEYS:
+                s.put(k, P[k][order])
+            s.ctx.init()
+            s.ctx.run(0, 1)
+            st = s.ctx.stats()
+            assert s.ctx.error_word() == 0
+            out.append(({k: s.grid(k) for k in FIELDS + CURRENTS}, st))
+        finally:
+            s.close()
+    (a, sa), (b, sb) = out
+    assert sa["window_overflow"] * 2 < sa["chunks"] and sb["window_overflow"] == sb["chunks"], (sa, sb)
+    for k in FIELDS + CURRENTS:
+        assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("nx,ny,passes", [(40, 3, 4), (5, 30, 3), (33, 1, 4), (64, 48, 1)])
+def test_yee_current_filter_wraps_short_dimensions(torch_cuda, aw, nx, ny, passes):
+    """The filtered J is the unfiltered one under `passes` periodic (1 2 1)/4 passes per
+    dimension, also where a dimension is shorter than the stencil. Both are one
+    rounding of exact sums, and the weights add up to 1: 2 x 2^-24 of the maxima."""
+    n = nx * ny * 16
+    rng = np.random.default_rng(nx + ny)
+    P = {"x": rng.random(n) * nx, "y": rng.random(n) * ny, "w": np.ones(n)}
+    P.update({k: rng.normal(0, 0.5, n) for k in ("ux", "uy", "uz")})
+    J = []
+    for m in (0, passes):
+        s = Setup(torch_cuda, aw, nx, ny, nx * 0.5, ny * 0.5, n, aw.AW_MODEL_YEE, dt=0.1, c=1.0, qm=-1.0)
+        try:
+            for k in PARTICLE_KEYS:
+                v = P[k].astype(np.float32)
+                s.put(k, np.minimum(v, np.nextafter(np.float32({"x": nx, "y": ny}[k]), np.float32(0))) if k in "xy" else v)
+            s.ctx.init()
+            s.ctx.set_current_filter(m)
+            s.ctx.run(0, 1)
+            J.append({k: s.grid(k).astype(np.float64) for k in CURRENTS})
+        finally:
+            s.close()
+    for k in CURRENTS:
+        f = J[0][k]
+        for _ in range(passes):
+            for ax in (0, 1):
+                f = (np.roll(f, 1, ax) + 2 * f + np.roll(f, -1, ax)) / 4
+        assert np.abs(J[1][k] - f).max() <= 2.0 ** -23 * np.abs(J[0][k]).max(), k
+
+
 def test_yee_vacuum_runs_without_particles(torch_cuda, aw):
     """No particles bound (n = 0): the Yee step is the field half alone, as in
     the reference's test_yee_vacuum.cu. A standing Ez mode (2, 3) on a 32 x 24
