@@ -405,10 +405,17 @@ __global__ void __launch_bounds__(256) k_dadj_fin(unsigned long long* __restrict
     }
 }
 // dpump += the block partials, in block order.
-__global__ void k_dadj_pump(const double* __restrict__ part, int nb, double* __restrict__ dpump) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < nb; ++b) s += part[b];
+__global__ void __launch_bounds__(256) k_dadj_pump(const double* __restrict__ part, int nb,
+                                                   double* __restrict__ dpump) {
+    __shared__ double sh[8];
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nb; b += 256) s += part[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) s += sh[w];
         *dpump += s;
     }
 }
@@ -695,7 +702,7 @@ double grad_darwin_impl(Ctx& c, long long nsteps, int every, float* dux, float* 
             k_dadj_fin<<<gbk, 256, 0, c.stream>>>(w.acc, w.S, nc, c.geo.nx, 1, w.l5, w.lEB, nullptr, 0.0f, last,
                                                   w.slot, pd, c.prm.dt, part);
             AW_LAUNCH();
-            k_dadj_pump<<<1, 32, 0, c.stream>>>(part, gbk, w.dpump);
+            k_dadj_pump<<<1, 256, 0, c.stream>>>(part, gbk, w.dpump);
             AW_LAUNCH();
             // E_L, B transpose -> lrho, lJ; with lamu into the source gather buffer
             elb_T();

@@ -50,7 +50,7 @@ constexpr int   kMagicBits = 0x4B400000;
 constexpr unsigned kMagicU  = 0x4B400000u;
 
 // End-of-step reduction (k_step_reduce): blocks and values per block row.
-constexpr int kRedBlocks = 32;
+constexpr int kRedBlocks = 8, kRedThreads = 512;   // k_step_reduce: one cluster
 constexpr int kRedVals   = 21;   // ke px py pz | se2 me2 q sb2 | 8 src sq + n | 3 dcu sq + n
 
 // Geometry passed by value into every kernel.
@@ -80,7 +80,7 @@ struct DevState {
     float     rms_src[8];      // rms of the source deposit coefficients (unscaled)
     float     rms_dcu[4];      // rms of the dcu coefficients (unscaled)
     unsigned long long chunks, overflow, slow;
-    unsigned  red_ticket;      // k_step_reduce blocks finished (reset by the last)
+    unsigned  red_ticket;      // k_charge_ref blocks finished (reset by the last)
     unsigned long long one_pass;   // chunks taken by the single-pass path
     unsigned  wait_polls;      // polls before a bounded device wait gives up (0: kWaitLimit)
     unsigned  dbg_extra_tx;    // bytes a chunk load's mbarrier expects beyond those issued

@@ -143,7 +143,7 @@ struct Ctx {
     aw_diag* diag = nullptr;    // device aw_diag
     struct DiagRing* ring = nullptr;   // aw_run_diag's records: the step reduction writes step s's
                                 // to rec[s - base] while 0 <= s - base < n
-    double* red_rows = nullptr; // k_step_reduce block rows [kRedBlocks][kRedVals]
+    double* red_rows = nullptr; // k_charge_ref block sums
     // tile binning scratch
     int* bin_count = nullptr; int* bin_off = nullptr; int* bin_cursor = nullptr;
     int* bin_idx = nullptr;   long long bin_idx_n = 0;

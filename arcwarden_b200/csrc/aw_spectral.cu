@@ -18,6 +18,7 @@
 //
 // Scale folding is exact: nx*ny is a power of two for every grid this path is
 // run on, and multiplying by 2^-k commutes with FP32 rounding.
+#include <cooperative_groups.h>
 #include "aw_internal.h"
 
 #include <algorithm>
@@ -46,52 +47,53 @@ __device__ __forceinline__ double pump_ramp(double t, double trmp, double toff) 
 // rms its coefficients had in the previous deposit; the few contributions
 // beyond that take the exact slow path. See aw_device.cuh for the fast-path
 // contract.
-__device__ void make_src_scales(const DevState* st, float cref, float (&S)[8], bool use_rms) {
-    float U[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-        U[d] = fmaxf(__fmul_rn(1.25f, __uint_as_float(st->ucur_bits[d])), __fmul_rn(0.01f, cref));
-    const float cm = st->coef_max;
-    S[0] = scale_for_bound(cm);
-    S[1] = scale_for_bound(__fmul_rn(cm, U[0]));
-    S[2] = scale_for_bound(__fmul_rn(cm, U[1]));
-    S[3] = scale_for_bound(__fmul_rn(cm, U[2]));
-    S[4] = scale_for_bound(__fmul_rn(__fmul_rn(cm, 0.5f), fmaxf(__fmul_rn(U[0], U[0]), __fmul_rn(U[1], U[1]))));
-    S[5] = scale_for_bound(__fmul_rn(__fmul_rn(cm, U[0]), U[1]));
-    S[6] = scale_for_bound(__fmul_rn(__fmul_rn(cm, U[2]), U[0]));
-    S[7] = scale_for_bound(__fmul_rn(__fmul_rn(cm, U[2]), U[1]));
-    if (use_rms && st->have_rms) {
-        float b[8] = {0.f, __fmul_rn(cm, U[0]), __fmul_rn(cm, U[1]), __fmul_rn(cm, U[2]),
-                      __fmul_rn(__fmul_rn(cm, 0.5f), fmaxf(__fmul_rn(U[0], U[0]), __fmul_rn(U[1], U[1]))),
-                      __fmul_rn(__fmul_rn(cm, U[0]), U[1]), __fmul_rn(__fmul_rn(cm, U[2]), U[0]),
-                      __fmul_rn(__fmul_rn(cm, U[2]), U[1])};
-#pragma unroll
-        for (int f = 1; f < 8; ++f)
-            if (st->rms_src[f] > 0.0f) S[f] = scale_for_bound(fminf(b[f], __fmul_rn(8.0f, st->rms_src[f])));
-    }
+__device__ __forceinline__ float src_scale(int f, float cm, const float (&U)[3], float rms) {
+    float b = cm;
+    if (f >= 1 && f <= 3) b = __fmul_rn(cm, f == 1 ? U[0] : f == 2 ? U[1] : U[2]);
+    if (f == 4) b = __fmul_rn(__fmul_rn(cm, 0.5f), fmaxf(__fmul_rn(U[0], U[0]), __fmul_rn(U[1], U[1])));
+    if (f == 5) b = __fmul_rn(__fmul_rn(cm, U[0]), U[1]);
+    if (f >= 6) b = __fmul_rn(__fmul_rn(cm, U[2]), f == 6 ? U[0] : U[1]);
+    if (f >= 1 && rms > 0.0f) b = fminf(b, __fmul_rn(8.0f, rms));
+    return scale_for_bound(b);
+}
+__device__ __forceinline__ float u_bound(unsigned bits, float cref) {
+    return fmaxf(__fmul_rn(1.25f, __uint_as_float(bits)), __fmul_rn(0.01f, cref));
 }
 
-// Opens a step (one thread): its time, the |u| maxima of the state the last push
-// wrote, fresh field maxima, the scales of the step's source deposit.
+// Opens a step (one whole warp): its time, the |u| maxima of the state the last push
+// wrote, fresh field maxima, the scales of the step's source deposit. It is a chain of
+// dependent accesses and some 600 instructions of scales that the step waits for, so
+// the loads go first, together, and lane f takes the scale of field f.
 __device__ void open_step(DevState* st, double dt, float cref, bool darwin) {
-    st->t = static_cast<double>(st->step) * dt;
+    const int lane = threadIdx.x & 31;
+    unsigned um[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) { st->ucur_bits[d] = st->umax_bits[d]; st->umax_bits[d] = 0u; }
-    st->emax_bits = 0u; st->bmax_bits = 0u;
-    st->red_ticket = 0u;
-    if (darwin) {
-        float S[8];
-        make_src_scales(st, cref, S, true);
+    for (int d = 0; d < 3; ++d) um[d] = st->umax_bits[d];
+    const float cm = st->coef_max;
+    const float rms = (darwin && lane >= 1 && lane < 8) ? st->rms_src[lane] : 0.0f;
+    const bool have = st->have_rms != 0;
+    const long long step = st->step;
+    __syncwarp();                                     // every lane has read
+    if (lane == 0) {
+        st->t = static_cast<double>(step) * dt;
 #pragma unroll
-        for (int f = 0; f < 8; ++f) st->S_next[f] = S[f];
+        for (int d = 0; d < 3; ++d) { st->ucur_bits[d] = um[d]; st->umax_bits[d] = 0u; }
+        st->emax_bits = 0u; st->bmax_bits = 0u;
+        st->red_ticket = 0u;
+    }
+    if (darwin && lane < 8) {
+        const float U[3] = {u_bound(um[0], cref), u_bound(um[1], cref), u_bound(um[2], cref)};
+        st->S_next[lane] = src_scale(lane, cm, U, have ? rms : 0.0f);
     }
 }
 
 __global__ void k_make_scales(DevState* st, float cref) {
-    float S[8];
-    make_src_scales(st, cref, S, false);
-#pragma unroll
-    for (int f = 0; f < 8; ++f) { st->S_next[f] = S[f]; st->S_pend[f] = S[f]; }
+    const float U[3] = {u_bound(st->ucur_bits[0], cref), u_bound(st->ucur_bits[1], cref),
+                        u_bound(st->ucur_bits[2], cref)};
+    const int f = threadIdx.x;
+    if (f >= 8) return;
+    const float S = src_scale(f, st->coef_max, U, 0.0f);
+    st->S_next[f] = S; st->S_pend[f] = S;
 }
 
 // Finalise NF fields of the accumulator block acc[f*ncell + c] (f = first..)
@@ -112,6 +114,13 @@ k_finalize(unsigned long long* __restrict__ acc, int first, int ncell,
            const float* __restrict__ Sdev, float* __restrict__ r, FinOut api, int accumulate,
            double* __restrict__ part, DevState* st, int step_begin, double dt, float cref, int darwin,
            AdjDev* rec, int sub_ref) {
+    // one warp opens the step before its share of the cells, beside the others. (Against
+    // one thread after its share: a step of the 512 x 1 Darwin run 54.1 -> 52.1 us, of
+    // the 512 x 512 one 586.5 -> 584.7; the electrostatic one, without scales, the same.)
+    if (step_begin && blockIdx.x == 0 && threadIdx.x >= kThreads - 32) {
+        if (rec && threadIdx.x == kThreads - 1) rec->rec_slot += 1;     // the recorded step's trajectory slot
+        open_step(st, dt, cref, darwin != 0);
+    }
     double qsum = 0.0;
     const double ref0 = (sub_ref && first == 0) ? st->rho_ref : 0.0;
     const int npair = (ncell + 1) >> 1;
@@ -178,10 +187,6 @@ k_finalize(unsigned long long* __restrict__ acc, int first, int ncell,
             for (int w = 0; w < kThreads / 32; ++w) s += sh[w];
             part[blockIdx.x * 5 + 2] = s;
         }
-    }
-    if (step_begin && blockIdx.x == 0 && threadIdx.x == 0) {
-        if (rec) rec->rec_slot += 1;     // the recorded step's trajectory slot
-        open_step(st, dt, cref, darwin != 0);
     }
 }
 
@@ -631,90 +636,123 @@ k_rms_reduce(const float* __restrict__ pc, int nbc, const float* __restrict__ pd
     }
 }
 
-// End-of-step reduction of the fused step, in one launch of kRedBlocks blocks:
-// the diagnostics of k_diag_reduce and, for Darwin, the coefficient rms of
-// k_rms_reduce. Block b owns a fixed contiguous range of the chunk partials
-// (part_p, part_c, part_d) and of the grid partials (part_g); thread t sums
-// entries t, t + 256, ... of its block's ranges, a fixed warp/shared tree makes
-// the block row, and the last block to finish (ticket) reduces the rows in row
-// order. Every sum is a pure function of the partials, whichever block is last.
-template <bool RMS>
-__global__ void __launch_bounds__(kThreads)
-k_step_reduce(const double* __restrict__ pp, const float* __restrict__ pc, const float* __restrict__ pd,
-              int np, const double* __restrict__ pg, int ng, double* __restrict__ rows,
-              double eps0, double dxdy, aw_diag* out, DevState* st, DiagRing* ring) {
-    constexpr int NV = kRedVals;
-    constexpr int NW = kThreads / 32;
-    __shared__ double sh[NV][NW];
-    __shared__ double rs[kRedBlocks][NV];
-    __shared__ int last;
-    const int t = threadIdx.x, b = blockIdx.x;
-    double a[NV];
+// Sums of M per-lane values over a warp: each step exchanges one half of the values
+// for the other, so lane l ends with the total of one value (idx; own false: none, or
+// a lane with the same bits but the low ones owns it). M + 4 exchanges instead of the
+// 5 M of a tree per value. The order of the additions is fixed.
+template <int M, int O>
+struct WarpSums {
+    __device__ static __forceinline__ double run(const double (&a)[M], int lane, int& idx, int& cnt, bool& own) {
+        if constexpr (O == 0) {
+            return a[0];
+        } else if constexpr (M == 1) {
+            const double r[1] = {a[0] + __shfl_xor_sync(0xffffffffu, a[0], O)};
+            if (lane & O) own = false;
+            return WarpSums<1, O / 2>::run(r, lane, idx, cnt, own);
+        } else {
+            constexpr int H = (M + 1) / 2;
+            const bool up = (lane & O) != 0;
+            double r[H];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) a[k] = 0.0;
-    const int plo = static_cast<int>(static_cast<long long>(b) * np / kRedBlocks);
-    const int phi = static_cast<int>(static_cast<long long>(b + 1) * np / kRedBlocks);
-    for (int i = plo + t; i < phi; i += kThreads) {
+            for (int k = 0; k < H; ++k) {
+                const double hi = k + H < M ? a[k + H < M ? k + H : 0] : 0.0;
+                r[k] = (up ? hi : a[k]) + __shfl_xor_sync(0xffffffffu, up ? a[k] : hi, O);
+            }
+            if (up) idx += H;
+            cnt = up ? max(cnt - H, 0) : min(cnt, H);
+            return WarpSums<H, O / 2>::run(r, lane, idx, cnt, own);
+        }
+    }
+};
+
+// End-of-step reduction of the fused step, in one launch of one cluster of
+// kRedBlocks blocks: the diagnostics of k_diag_reduce and, for Darwin, the
+// coefficient rms of k_rms_reduce. The partials (chunks: part_p, part_c, part_d;
+// grid: part_g) go to the threads in fixed strides, a fixed warp and shared tree
+// makes each block's row, written straight into block 0's shared memory, and
+// block 0 adds the rows in order. Every sum is a pure function of the partials.
+//
+// Bound by the latency of its serial chain, not by the partials it reads (0.1 to
+// 2 MB): it is on the critical path of every step. Against 32 blocks
+// that met at a ticket in global memory, with a shuffle tree per value: a step of the
+// 64 x 64 electrostatic run 29.6 -> 25.7 us, of the 512 x 1 Darwin run 58.2 -> 54.1.
+template <bool RMS>
+__global__ void __cluster_dims__(kRedBlocks, 1, 1) __launch_bounds__(kRedThreads)
+k_step_reduce(const double* __restrict__ pp, const float* __restrict__ pc, const float* __restrict__ pd,
+              int np, const double* __restrict__ pg, int ng, double eps0, double dxdy, aw_diag* out, DevState* st,
+              DiagRing* ring) {
+    namespace cg = cooperative_groups;
+    constexpr int NS = RMS ? kRedVals - 1 : 7;   // the sums; the one maximum (max E^2) is kept apart
+    constexpr int NW = kRedThreads / 32;
+    __shared__ double sh[NS + 1][NW];
+    __shared__ double rs[kRedBlocks][NS + 1];
+    __shared__ double tot[NS + 1];
+    cg::cluster_group cl = cg::this_cluster();
+    const auto token = cl.barrier_arrive();      // (block 0's shared memory is written below)
+    const int t = threadIdx.x, b = blockIdx.x, lane = t & 31;
+    long long slot = 0, nring = 0;
+    if (b == 0 && t == 0) { slot = st->step - 1 - ring->base; nring = ring->n; }   // the push has counted the step
+    double a[NS], mx = 0.0;                      // ke px py pz se2 q sb2 | 8 src sq + n | 3 dcu sq + n
+#pragma unroll
+    for (int k = 0; k < NS; ++k) a[k] = 0.0;
+#pragma unroll 2
+    for (int i = b * kRedThreads + t; i < np; i += kRedThreads * kRedBlocks) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) a[k] += pp[i * 5 + k];
-        if (RMS) {
+        if constexpr (RMS) {
 #pragma unroll
-            for (int k = 0; k < 9; ++k) a[8 + k] += pc[i * 9 + k];
+            for (int k = 0; k < 9; ++k) a[7 + k] += pc[i * 9 + k];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) a[17 + k] += pd[i * 4 + k];
+            for (int k = 0; k < 4; ++k) a[16 + k] += pd[i * 4 + k];
         }
     }
-    const int glo = b * ng / kRedBlocks, ghi = (b + 1) * ng / kRedBlocks;
-    for (int i = glo + t; i < ghi; i += kThreads) {
-        a[4] += pg[i * 5 + 0]; a[5] = fmax(a[5], pg[i * 5 + 1]); a[6] += pg[i * 5 + 2]; a[7] += pg[i * 5 + 3];
+    for (int i = b * kRedThreads + t; i < ng; i += kRedThreads * kRedBlocks) {
+        a[4] += pg[i * 5 + 0]; mx = fmax(mx, pg[i * 5 + 1]); a[5] += pg[i * 5 + 2]; a[6] += pg[i * 5 + 3];
     }
+    int idx = 0, cnt = NS;
+    bool own = true;
+    const double v = WarpSums<NS, 16>::run(a, lane, idx, cnt, own);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (own && cnt > 0) sh[idx][t >> 5] = v;
+    if (lane == 0) sh[NS][t >> 5] = mx;
+    __syncthreads();
+    cl.barrier_wait(cg::cluster_group::arrival_token(token));
+    if (t <= NS) {
+        double r[4];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            const double v = __shfl_down_sync(0xffffffffu, a[k], o);
-            a[k] = (k == 5) ? fmax(a[k], v) : a[k] + v;
+        for (int q = 0; q < 4; ++q) {
+            r[q] = sh[t][q];
+#pragma unroll
+            for (int w = q + 4; w < NW; w += 4) r[q] = t == NS ? fmax(r[q], sh[t][w]) : r[q] + sh[t][w];
         }
-    if ((t & 31) == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sh[k][t >> 5] = a[k];
-    __syncthreads();
-    if (t < NV) {
-        double v = sh[t][0];
-        for (int w = 1; w < NW; ++w) v = (t == 5) ? fmax(v, sh[t][w]) : v + sh[t][w];
-        rows[b * NV + t] = v;
-        __threadfence();
+        *cl.map_shared_rank(&rs[b][t], 0) = t == NS ? fmax(fmax(r[0], r[1]), fmax(r[2], r[3]))
+                                                    : (r[0] + r[1]) + (r[2] + r[3]);
     }
-    __syncthreads();
-    if (t == 0) last = (atomicAdd(&st->red_ticket, 1u) == kRedBlocks - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int i = t; i < kRedBlocks * NV; i += kThreads) rs[i / NV][i % NV] = __ldcg(rows + i);
-    __syncthreads();
-    if (t < NV) {
-        double v = rs[0][t];
-        for (int r = 1; r < kRedBlocks; ++r) v = (t == 5) ? fmax(v, rs[r][t]) : v + rs[r][t];
-        sh[t][0] = v;
+    cl.sync();
+    if (b != 0) return;
+    if (t <= NS) {
+        double r = rs[0][t];
+#pragma unroll
+        for (int k = 1; k < kRedBlocks; ++k) r = t == NS ? fmax(r, rs[k][t]) : r + rs[k][t];
+        tot[t] = r;
     }
     __syncthreads();
     if (t == 0) {
-        out->ke = 0.5 * sh[0][0];
-        out->px = sh[1][0]; out->py = sh[2][0]; out->pz = sh[3][0];
-        out->ee = 0.5 * eps0 * sh[4][0] * dxdy;
-        out->max_e = sqrt(sh[5][0]);
-        out->charge = sh[6][0] * dxdy;
-        out->eb = 0.5 * sh[7][0] * dxdy;
-        const long long k = st->step - 1 - ring->base;         // the push has counted the step
-        if (k >= 0 && k < ring->n) ring->rec[k] = *out;
-        if (RMS) {
-            if (sh[16][0] > 0.0)
-                for (int f = 0; f < 8; ++f) st->rms_src[f] = static_cast<float>(sqrt(sh[8 + f][0] / sh[16][0]));
-            if (sh[20][0] > 0.0)
-                for (int k = 0; k < 3; ++k) st->rms_dcu[k] = static_cast<float>(sqrt(sh[17 + k][0] / sh[20][0]));
-            st->have_rms = 1;
-        }
-        st->red_ticket = 0u;
+        aw_diag d;
+        d.ke = 0.5 * tot[0];
+        d.px = tot[1]; d.py = tot[2]; d.pz = tot[3];
+        d.ee = 0.5 * eps0 * tot[4] * dxdy;
+        d.max_e = sqrt(tot[NS]);
+        d.charge = tot[5] * dxdy;
+        d.eb = 0.5 * tot[6] * dxdy;
+        *out = d;
+        if (slot >= 0 && slot < nring) ring->rec[slot] = d;
+    }
+    if constexpr (RMS) {
+        if (t >= 32 && t < 40 && tot[15] > 0.0) st->rms_src[t - 32] = static_cast<float>(sqrt(tot[7 + t - 32] / tot[15]));
+        if (t >= 64 && t < 67 && tot[19] > 0.0) st->rms_dcu[t - 64] = static_cast<float>(sqrt(tot[16 + t - 64] / tot[19]));
+        if (t == 96) st->have_rms = 1;
     }
 }
 
@@ -1055,7 +1093,7 @@ void gridfft_cols_elb_T(Ctx& c, const cufftComplex* l5, cufftComplex* out) {
 }
 
 void launch_make_scales(Ctx& c) {
-    k_make_scales<<<1, 1, 0, c.stream>>>(c.st, cref_of(c));
+    k_make_scales<<<1, 32, 0, c.stream>>>(c.st, cref_of(c));
     AW_LAUNCH();
 }
 
@@ -1212,13 +1250,13 @@ void launch_rms_reduce(Ctx& c, bool src, bool dcu) {
 void launch_step_reduce(Ctx& c) {
     const double dxdy = c.geo.dx * c.geo.dy;
     if (c.model == AW_MODEL_DARWIN)
-        k_step_reduce<true><<<kRedBlocks, kThreads, 0, c.stream>>>(c.part_p, c.part_c, c.part_d, c.npart_p, c.part_g,
-                                                                    kGridBlocks, c.red_rows, c.prm.eps0, dxdy,
-                                                                    c.diag, c.st, c.ring);
+        k_step_reduce<true><<<kRedBlocks, kRedThreads, 0, c.stream>>>(c.part_p, c.part_c, c.part_d, c.npart_p, c.part_g,
+                                                                      kGridBlocks, c.prm.eps0, dxdy, c.diag, c.st,
+                                                                      c.ring);
     else
-        k_step_reduce<false><<<kRedBlocks, kThreads, 0, c.stream>>>(c.part_p, nullptr, nullptr, c.npart_p, c.part_g,
-                                                                     kGridBlocks, c.red_rows, c.prm.eps0, dxdy,
-                                                                     c.diag, c.st, c.ring);
+        k_step_reduce<false><<<kRedBlocks, kRedThreads, 0, c.stream>>>(c.part_p, nullptr, nullptr, c.npart_p, c.part_g,
+                                                                       kGridBlocks, c.prm.eps0, dxdy, c.diag, c.st,
+                                                                       c.ring);
     AW_LAUNCH();
 }
 void launch_promote_scales(Ctx& c) {
