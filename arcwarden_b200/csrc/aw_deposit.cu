@@ -14,9 +14,11 @@
 //                        (pusher.hpp:212-258 + particles.hpp:294-315 +
 //                        depositor.hpp:161-270), KE/momentum partials, |u| max.
 //
-// Structure of every kernel (one CTA = one chunk of kChunk consecutive
-// particles; no kernel sorts particles, so the ES path keeps the reference's
-// particle order):
+// Structure of every kernel (one CTA = one chunk of up to kChunk consecutive
+// particles, see chunk_size; no kernel sorts particles, so the ES path keeps the
+// reference's particle order). The fused kernels deposit in the pass that pushes
+// wherever the chunk's widened box fits their window (Win1, Tile1 below); the two
+// passes described here serve the rest, the unfused deposits and the adjoint scatter:
 //   load    one thread issues a bulk copy (cp.async.bulk, the TMA engine) per
 //           SoA array of the chunk into shared memory; the chunk's bytes are all
 //           in flight at once and every thread waits on one mbarrier.

@@ -472,11 +472,11 @@ def adj_bytes_per_particle_step(nsteps, every):
 
 def adj_launches(nsteps, every):
     """Kernels of this library one gradient launches: aw_init's 13; per forward
-    step 5; per recomputed step 4 (no reduction); per backward step 4; two slot
+    step 5; per recomputed step 4 (no reduction); per backward step 6; two slot
     settings per segment; the output and the error merge."""
     nseg = math.ceil(nsteps / every)
     last = nsteps - (nseg - 1) * every
-    return 13 + 5 * nsteps + 4 * (nsteps - last) + 4 * nsteps + 2 * nseg + 2
+    return 13 + 5 * nsteps + 4 * (nsteps - last) + 6 * nsteps + 2 * nseg + 2
 
 
 def adj_darwin_bytes_per_particle_step():
@@ -491,11 +491,11 @@ def adj_darwin_bytes_per_particle_step():
 def adj_darwin_launches(nsteps, every):
     """Kernels of this library one Darwin gradient launches: aw_init's 13; 9 per
     forward step; per segment a restored state and its recompute (9 per step);
-    11 per backward step (push transpose, two 6-field scatters and their
-    conversions, the E_T and E_L/B transposes, the pump sum, the source pack and
-    transpose); the output."""
+    16 per backward step (push and dcu transposes, two 6-field scatters and their
+    conversions, three each for the E_T and E_L/B transposes, the pump sum, the
+    source pack and transpose, the slot); the output."""
     nseg = math.ceil(nsteps / every)
-    return 13 + 9 * nsteps + 9 * nsteps + 11 * nsteps + nseg + 1
+    return 13 + 9 * nsteps + 9 * nsteps + 16 * nsteps + nseg + 1
 
 
 def run_adjoint(args, wl, rank, world, dist):

@@ -119,10 +119,10 @@ typedef struct aw_diag {
  * the same bits (the deposits are exact and order-free); they only change the
  * speed. -1 (or 0 for es_window) selects the built-in choice. */
 typedef struct aw_kernel_plan {
-    int32_t one_pass;   /* Darwin push and dcu kernels: push and deposit in one pass over a
-                           chunk whose window fits (1), or always in two passes (0)        */
+    int32_t one_pass;   /* fused particle kernels: push and deposit in one pass over a chunk
+                           whose window fits (1, the default), or always in two passes (0)  */
     int32_t tile;       /* two-pass Darwin kernels stage a gather tile of the chunk (1/0) */
-    int32_t es_window;  /* electrostatic push: rho window capacity in cells (> 0)         */
+    int32_t es_window;  /* electrostatic push in two passes: rho window capacity in cells  */
 } aw_kernel_plan;
 
 
