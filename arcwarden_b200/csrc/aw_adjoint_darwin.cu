@@ -210,7 +210,7 @@ struct PLoad {
 
 // Backward push: Boris transpose with the particle's own B (u1 = u + h e,
 // up = u1 + u1 x t, u2 = u1 + up x s, u3 = u2 + h e; t = h b, s = 2t / (1 + t^2)).
-__global__ void __launch_bounds__(256) k_dadj_push(PArgs a, float h, float dtx, float dty) {
+__global__ void __launch_bounds__(256, 4) k_dadj_push(PArgs a, float h, float dtx, float dty) {
     const long long n = a.n;
     const float* __restrict__ X = a.state();
     const float* __restrict__ gbp = a.gb_push();
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) k_dadj_push(PArgs a, float h, float dtx, 
 
 // Backward dcu deposit: g = G(ldcu); the scatter values (c g, c (g x u));
 // lu += c G(Bt) x g; lx += the deposit's and the gathers' position derivatives.
-__global__ void __launch_bounds__(256) k_dadj_dcu(PArgs a, const float* __restrict__ ldcu, double qm2oa) {
+__global__ void __launch_bounds__(256, 4) k_dadj_dcu(PArgs a, const float* __restrict__ ldcu, double qm2oa) {
     const long long n = a.n;
     const float* __restrict__ X = a.state();
     const float* __restrict__ gbd = a.gb_dcu();
