@@ -721,6 +721,18 @@ __device__ __forceinline__ void win1_flush(const int* __restrict__ s, const Win1
     }
 }
 
+// Whether a full chunk's sums may be expected to leave the int32 range: `top` is the
+// largest rms |coefficient| of a biased field in the last deposit, scaled. A single
+// pass that finds so only at its end (chunk_overflows1) has the whole chunk left for the
+// exact global path, 5 to 8 times the time of the two passes, which count carries; so
+// such chunks take those from the start. The scales bound the largest coefficient by
+// 2^22: a Maxwellian's rms is a fifth of its maximum or less (2048 x 2^22 / 5.6 = 1.5e9),
+// a cold beam's is almost the maximum (up to 8e9): 512 x 512, 256 per cell, drift
+// 0.24 over a spread of 0.07: 14.9 ms a step in the single pass, 2.7 in two.
+__device__ __forceinline__ bool expect_overflow1(float top, int cs) {
+    return top * static_cast<float>(cs) > 1.75e9f;
+}
+
 // True (block-uniformly) when some biased field's chunk sum may reach 2^31. Each
 // thread brings the largest of its fields' sums of cs^2 over its m fast
 // particles: sum |cs| + 1 <= sqrt(m l2) + m there (Cauchy), the sum over the
@@ -914,7 +926,9 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
 
     // ---- single pass: the particles do not move, so the window is the box of
     // their base cells plus the corner - the gather tile's box
-    if (A.one_pass) {
+    const float top = st->have_rms ? fmaxf(st->rms_dcu[0] * S[0], fmaxf(st->rms_dcu[1] * S[1], st->rms_dcu[2] * S[2]))
+                                   : 0.0f;
+    if (A.one_pass && !expect_overflow1(top, cs_)) {
         constexpr int P1 = 640, T1 = ((PC * win_planes(NF) - P1 * (NF + 1)) / 6) & ~3;     // 24 bytes per tile cell
         Box1 bx;
         Win1 w1;
@@ -1513,6 +1527,10 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     float S[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) S[f] = st->S_next[f];
+    float top = 0.0f;                             // (field 0 is carried exactly)
+    if (st->have_rms)
+#pragma unroll
+        for (int f = 1; f < NF; ++f) top = fmaxf(top, st->rms_src[f] * S[f]);
     const float2 Sp[4] = {make_float2(S[0], S[1]), make_float2(S[2], S[3]), make_float2(S[4], S[5]),
                           make_float2(S[6], S[7])};
     __shared__ __align__(16) int ends[4];
@@ -1525,7 +1543,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     ref_of(x0, y0, g, ir, jr);
 
     // ---- single pass -------------------------------------------------------
-    if (A.one_pass) {
+    if (A.one_pass && !expect_overflow1(top, cs_)) {
         constexpr int P1 = 384, T1 = ((PC * win_planes(NF) - P1 * (NF + 3)) / 6) & ~3;     // 24 bytes per tile cell
         // the cells a particle can cross in one step: twice the largest in-plane |u| of
         // the current state times dt/dx (one further cell for the rounding)
