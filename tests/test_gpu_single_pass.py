@@ -57,3 +57,41 @@ def test_single_pass_equals_two_passes(torch_cuda, aw, model, nx, ny, Lx, Ly, pp
             s.close()
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("ppc,vth", [(256, 0.01), (256, 0.05), (64, 0.01)])
+def test_cold_beams_keep_to_the_windows(torch_cuda, aw, ppc, vth):
+    """Two cold beams: every particle's coefficients are near the maximum, and a full
+    chunk's sums leave the int32 range. Such chunks take two passes from the start
+    (after the first step has measured the coefficients), not the exact global path,
+    with the same bits as the two-pass plan."""
+    nx, ny = 64, 32
+    n = nx * ny * ppc
+    rng = np.random.default_rng(ppc)
+    cell = np.repeat(np.arange(nx * ny), ppc // 2)
+    cell = np.concatenate([cell, cell])
+    beam = np.where(np.arange(n) < n // 2, 0.25, -0.25)
+    P = {"x": cell % nx + 0.999 * rng.random(n), "y": cell // nx + 0.999 * rng.random(n),
+         "ux": beam + rng.normal(0, vth, n), "uy": rng.normal(0, vth, n), "uz": rng.normal(0, vth, n),
+         "w": np.full(n, 1.0 / ppc)}
+    out = []
+    for one_pass in (0, 1):
+        s = Setup(torch_cuda, aw, nx, ny, float(nx), float(ny), n, 1, dt=0.05)
+        try:
+            s.ctx.set_kernel_plan(one_pass=one_pass)
+            for k in PARTICLE_KEYS:
+                s.put(k, P[k].astype(np.float32))
+            s.ctx.init()
+            s.ctx.run(0, 2)
+            slow = s.ctx.stats()["slow_deposits"]
+            s.ctx.run(2, 3)
+            assert s.ctx.stats()["slow_deposits"] - slow < n // 100
+            r = s.parts()
+            for k in ("rho", "Jx", "Jz", "Ex", "Ey", "Ez", "Bz"):
+                r[k] = s.grid(k)
+            assert s.ctx.error_word() == 0
+            out.append(r)
+        finally:
+            s.close()
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
