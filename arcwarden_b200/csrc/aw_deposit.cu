@@ -866,7 +866,7 @@ __device__ __forceinline__ void slow_pass_linear(const float* __restrict__ stage
         deposit_global<NF>(c.i0, c.j0, wv, cs, gacc, g);
         ++n;
     }
-    if (n) atomicAdd(&st->slow, static_cast<unsigned long long>(n));
+    count_slow(st, n);
 }
 
 // dcu scales: |coef_dcu (E + v x B)| <= |qm| coef_max (Emax + 2 Umax Bmax); in
@@ -1397,7 +1397,8 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
                     const float x = m.stage[s], y = m.stage[kChunk + s];
                     if (in_grid(x, y, g)) __stcs(p.cell + c0 + s, static_cast<int>(y) * g.nx + static_cast<int>(x));
                 }
-            if (nlist)
+            if (nlist) {
+                unsigned ns = 0;
                 for (int s = threadIdx.x; s < cnt; s += kThreads) {
                     if (!(slow[s >> 5] >> (s & 31) & 1u)) continue;
                     const float x = m.stage[s], y = m.stage[kChunk + s];
@@ -1406,8 +1407,10 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
                     const Cic c = cic(x, y);
                     const float wv[4] = {c.w0, c.w1, c.w2, c.w3};
                     deposit_global<1>(c.i0, c.j0, wv, cs, acc, g);
-                    atomicAdd(&st->slow, 1ull);
+                    ++ns;
                 }
+                count_slow(st, ns);
+            }
             if (threadIdx.x == 0) {
                 atomicAdd(&st->chunks, 1ull);
                 atomicAdd(&st->one_pass, 1ull);
@@ -2325,7 +2328,7 @@ __device__ __forceinline__ void yee_slow_pass(const float* __restrict__ stage, c
         });
         ++n;
     }
-    if (n) atomicAdd(&st->slow, static_cast<unsigned long long>(n));
+    count_slow(st, n);
 }
 
 __device__ __forceinline__ double yee_ramp(double t, double trmp, double toff) {
