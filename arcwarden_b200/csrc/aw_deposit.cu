@@ -70,15 +70,21 @@ constexpr int kRedInts = kThreads / 32 * (4 + 8);
 // The fused ES kernel: four CTAs per SM (56 KB each, at most 64 registers), so its
 // stage holds x y ux uy uz and not the weights: a chunk's weights are usually equal
 // (one species), and where they are not the kernel reads them from global memory.
-// stage | red | area, the area holding either the single pass's window of kEsP1
-// cells (4 planes), its gather tile of kEsT1 cells and the slow slots' bit map, or the
-// two-pass fallback's window (2 planes, up to kEsWinMax cells) and its slow list.
-// The ES path keeps the particle order, so a chunk covers cs / ppc consecutive cells
-// of the load order plus their drift.
+// stage | area | red, the area holding either the single pass's window of kEsP1 cells
+// (4 planes), its gather tile of kEsT1 cells and the slow slots' bit map, or, at its
+// end, the two-pass fallback's slow list. The fallback's window (2 planes) starts in
+// the stage's planes 3 and 4, which its first pass has read by then.
+// The ES path keeps the particle order and no run of it is re-sorted, so a chunk covers
+// cs / ppc consecutive cells of the load order plus their drift: at few particles per
+// cell whole grid rows and their spread (3472 cells: 13 rows of 256). A smaller window
+// takes more bands there and reaches the exact global path sooner. Steps 500 to 550 of a
+// 256 x 256 two-stream run (vth 0.05, drift 0.2), us a step with 1408 cells and with
+// these: at 8 per cell 119 and 62, at 16 per cell 115 and 71.
 constexpr int kEsP1 = 800, kEsT1 = 304;
 constexpr int kEsArea = kEsP1 * 4 * 4 + kEsT1 * 8 + kChunk / 8;
-constexpr int kEsWinMax = 1408;
-static_assert(kEsWinMax * 8 + kChunk * 2 <= kEsArea, "the fallback's window and list must fit the area");
+constexpr int kEsWindow = (2 * kChunk * 4 + kEsArea - kChunk * 2) / 8;
+constexpr int es_area(int wmax) { return wmax <= kEsWindow ? kEsArea : wmax * 8 + kChunk * 2 - 2 * kChunk * 4; }
+static_assert(es_area(kEsWindow) == kEsArea && kEsArea % 8 == 0 && kEsArea >= kChunk * 2, "window, list and area");
 // stage [np][kChunk] f32 | window [planes][wmax] i32 | red ints | slow list u16[kChunk]
 constexpr size_t win_offset(int np) { return static_cast<size_t>(np) * kChunk * 4; }
 constexpr size_t smem_bytes_w(int nf, int np, int wmax, int planes) {
@@ -86,8 +92,8 @@ constexpr size_t smem_bytes_w(int nf, int np, int wmax, int planes) {
            + kChunk * sizeof(unsigned short);
 }
 constexpr size_t smem_bytes(int nf, int np) { return smem_bytes_w(nf, np, wmax_cells(nf), win_planes(nf)); }
-constexpr size_t es_smem_bytes() { return win_offset(5) + kRedInts * sizeof(int) + kEsArea; }
-static_assert(4 * (es_smem_bytes() + 1024 + 400) <= 228 * 1024, "four ES CTAs per SM");
+constexpr size_t es_smem_bytes(int wmax) { return win_offset(5) + kRedInts * sizeof(int) + es_area(wmax); }
+static_assert(4 * (es_smem_bytes(kEsWindow) + 1024 + 400) <= 228 * 1024, "four ES CTAs per SM");
 
 struct Smem {
     float* stage;
@@ -1268,9 +1274,10 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     extern __shared__ __align__(16) unsigned char smem[];
     Smem m;
     m.stage = reinterpret_cast<float*>(smem);
-    m.red = reinterpret_cast<int*>(smem + win_offset(NIN));
-    m.win = m.red + kRedInts;
-    m.slow = reinterpret_cast<unsigned short*>(m.win + 2 * kEsWinMax);
+    m.win = reinterpret_cast<int*>(smem + win_offset(NIN - 2));
+    m.red = reinterpret_cast<int*>(smem + win_offset(NIN) + es_area(wmaxc));
+    m.slow = reinterpret_cast<unsigned short*>(m.red) - kChunk;
+    int* const area = reinterpret_cast<int*>(smem + win_offset(NIN));
     __shared__ unsigned long long bar;
     __shared__ int nlist;
     __shared__ double dsh[4 * (kThreads / 32)];
@@ -1342,12 +1349,12 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
             const bool wsame = wlo == whi;
             float w = __int_as_float(wlo);
             float cf0 = __double2float_rn(qoa * static_cast<double>(w));
-            float2* const tile = reinterpret_cast<float2*>(m.win + 4 * kEsP1);
+            float2* const tile = reinterpret_cast<float2*>(area + 4 * kEsP1);
             unsigned* const slow = reinterpret_cast<unsigned*>(tile + kEsT1);      // bit map of slots
             if (threadIdx.x < kChunk / 32) slow[threadIdx.x] = 0u;
             const int TW = bx.nI + 1;
             tile1_load_es<kEsT1>(tile, TW, bx, q, g);
-            win1_zero<4, kEsP1>(m.win, w1);
+            win1_zero<4, kEsP1>(area, w1);
             __syncthreads();
             const bool cells = pp.write_cell && p.cell;
 #pragma unroll 1
@@ -1379,7 +1386,7 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
                     const float cs[1] = {__fmul_rn(cf0, S1[0])};
                     const int di = win_col(static_cast<int>(x), w1.oi, g.nx), dj = win_col(static_cast<int>(y), w1.oj, g.ny);
                     if (fabsf(cs[0]) < kFastLim && di <= w1.W - 2 && dj <= w1.H - 2)
-                        win1_add<1, true, kEsP1>(m.win, w1, di, dj, x, y, cs);
+                        win1_add<1, true, kEsP1>(area, w1, di, dj, x, y, cs);
                     else { atomicOr(slow + (sl >> 5), 1u << (sl & 31)); nlist = 1; }
                 } else {
                     set_err(st, AW_DEV_OUT_OF_GRID);
@@ -1390,7 +1397,7 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
             const int pl[5] = {0, 1, 2, 3, 4};
             float* const dst[5] = {p.x, p.y, p.ux, p.uy, p.uz};
             bulk_store_planes<5>(m.stage, pl, dst, 5, c0, cnt, p.vec_ok != 0);
-            win1_flush<1, true, kEsP1>(m.win, w1, acc, g);
+            win1_flush<1, true, kEsP1>(area, w1, acc, g);
             if (cells)                        // the owning cells, from the staged new positions
 #pragma unroll 4
                 for (int s = threadIdx.x; s < cnt; s += kThreads) {
@@ -1946,8 +1953,8 @@ DcuArgs dcu_args(const Ctx& c, const float* gb, bool fused) {
     return a;
 }
 // Capacity of the two-pass fallback's window in cells (aw_kernel_plan::es_window;
-// results do not depend on it).
-int es_window(const Ctx& c) { return c.plan.es_window > 0 ? std::min(c.plan.es_window, kEsWinMax) : kEsWinMax; }
+// results do not depend on it; above kEsWindow three CTAs fit an SM instead of four).
+int es_window(const Ctx& c) { return c.plan.es_window > 0 ? c.plan.es_window : kEsWindow; }
 EsArgs es_args(const Ctx& c) {
     EsArgs a{};
     a.p = c.parts; a.g = c.geo; a.pp = push_params(c); a.gb = c.gb_es;
@@ -2518,7 +2525,7 @@ MultiPhase* multi_create(int kind, Ctx* const* runs, int nruns) {
         if (kind == kMultiEsPush) {
             const EsArgs a = es_args(*runs[r]);
             put(&a, sizeof a);
-            m->smem = es_smem_bytes();
+            m->smem = std::max(m->smem, es_smem_bytes(a.wmaxc));
         }
         else if (kind == kMultiDcu) { const DcuArgs a = dcu_args(*runs[r], runs[r]->gb_dcu, true); put(&a, sizeof a); }
         else { const EmArgs a = em_args(*runs[r]); put(&a, sizeof a); }
@@ -2576,7 +2583,7 @@ void launch_deposit_dcu(Ctx& c, const float* gb, bool fused) {
 
 void launch_push_deposit_es(Ctx& c) {
     if (c.parts.n == 0) return;
-    const size_t sh = es_smem_bytes();
+    const size_t sh = es_smem_bytes(es_window(c));
     const bool p2 = pow2_geo(c);
     const bool rec = c.rec_xy != nullptr;
     auto pick = [&](auto full) {

@@ -122,7 +122,8 @@ typedef struct aw_kernel_plan {
     int32_t one_pass;   /* fused particle kernels: push and deposit in one pass over a chunk
                            whose window fits (1, the default), or always in two passes (0)  */
     int32_t tile;       /* two-pass Darwin kernels stage a gather tile of the chunk (1/0) */
-    int32_t es_window;  /* electrostatic push in two passes: rho window capacity in cells  */
+    int32_t es_window;  /* electrostatic push in two passes: rho window capacity in cells,
+                           256..4096 (0: 3472; above that fewer chunks are resident)    */
 } aw_kernel_plan;
 
 
