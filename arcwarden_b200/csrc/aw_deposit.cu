@@ -82,7 +82,7 @@ constexpr int kRedInts = kThreads / 32 * (4 + 8);
 // these: at 8 per cell 119 and 62, at 16 per cell 115 and 71.
 constexpr int kEsP1 = 800, kEsT1 = 304;
 constexpr int kEsArea = kEsP1 * 4 * 4 + kEsT1 * 8 + kChunk / 8;
-constexpr int kEsWindow = (2 * kChunk * 4 + kEsArea - kChunk * 2) / 8;
+constexpr int kEsWindow = (2 * kChunk * 4 + kEsArea - kChunk * 2) / 8, kEsSmall = (kEsArea - kChunk * 2) / 8;
 constexpr int es_area(int wmax) { return wmax <= kEsWindow ? kEsArea : wmax * 8 + kChunk * 2 - 2 * kChunk * 4; }
 static_assert(es_area(kEsWindow) == kEsArea && kEsArea % 8 == 0 && kEsArea >= kChunk * 2, "window, list and area");
 // stage [np][kChunk] f32 | window [planes][wmax] i32 | red ints | slow list u16[kChunk]
@@ -1076,7 +1076,7 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     };
     float sq[NF] = {};
     float nval = 0.f;
-    auto stats = [&](const float (&a)[NS]) {
+    auto stats = [&](const float (&a)[NS], int = 0) {
         if (a[1] >= 0.0f) {
             const int ci = static_cast<int>(fabsf(a[0])), cj = static_cast<int>(a[1]);
             if (((ci + cj) & 7) == 0) {   // rms sample: the particles of one cell in 8, any order
@@ -1254,8 +1254,9 @@ __device__ __forceinline__ bool step_xy(float& x, float& y, float ux, float uy, 
 }
 
 // Fused ES step kernel. Single pass where the chunk's window fits (one read of the
-// staged particle, 7 shared atomics); else two passes through the stage: new x, y,
-// coefficient q w / (dx dy). Bound by instruction issue and by the latency of a
+// staged particle, 7 shared atomics); else two passes through the stage: new x (sign
+// set: no deposit - listed for the slow path, or no new position in the grid), y (< 0:
+// not pushed), ux uy uz, then the coefficient q w / (dx dy) in place of ux. Bound by instruction issue and by the latency of a
 // chunk's fixed phases (load, box, window, flush, sums): es256, 4.2 M particles, 390 ->
 // 250 instructions a particle, 73.7 -> 55.3 us (28 us of HBM time).
 struct EsArgs {
@@ -1330,6 +1331,12 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
         uxy = __ffma2_rn(Q, exy, uxy);
         ux = uxy.x; uy = uxy.y;
     };
+    auto weights_equal = [&] {                 // of the whole chunk: then wlo is the weight's bits
+        wlo = wred[0]; whi = wred[8];
+#pragma unroll
+        for (int k = 1; k < kThreads / 32; ++k) { wlo = min(wlo, wred[k]); whi = max(whi, wred[8 + k]); }
+        return wlo == whi;
+    };
     double ke = 0, px = 0, py = 0, pz = 0;
     float m0 = 0.f, m1 = 0.f;
     bool done = false;
@@ -1343,10 +1350,7 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
         if (mg > 0 && chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, kEsP1, mg, bx) &&
             window1<kEsP1>(w1, bx, mg, A.rep_need, g) && (bx.nI + 1) * (bx.nJ + 1) <= kEsT1) {
             done = true;
-            wlo = wred[0]; whi = wred[8];
-#pragma unroll
-            for (int k = 1; k < kThreads / 32; ++k) { wlo = min(wlo, wred[k]); whi = max(whi, wred[8 + k]); }
-            const bool wsame = wlo == whi;
+            const bool wsame = weights_equal();
             float w = __int_as_float(wlo);
             float cf0 = __double2float_rn(qoa * static_cast<double>(w));
             float2* const tile = reinterpret_cast<float2*>(area + 4 * kEsP1);
@@ -1431,6 +1435,7 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     if (!done) {
         int ir, jr;
         ref_of(x0, y0, g, ir, jr);
+        const bool wsame = weights_equal();
         BBox bb;
         float l1[NF] = {};
 #pragma unroll 2
@@ -1439,8 +1444,8 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
             const long long i = c0 + s;
             float x = m.stage[s], y = m.stage[kChunk + s];
             float ux = m.stage[2 * kChunk + s], uy = m.stage[3 * kChunk + s], uz = m.stage[4 * kChunk + s];
-            const float w = s < cnt ? __ldcs(p.w + i) : 0.0f;
-            float xs = -1.0f, cf0 = 0.0f;
+            const float w = wsame ? __int_as_float(wlo) : s < cnt ? __ldcs(p.w + i) : 0.0f;
+            float xs = -1.0f, ys = -1.0f;
             if (s < cnt) {
                 if (in_grid(x, y, g)) {
                     const Cic c = cic(x, y);
@@ -1456,32 +1461,59 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
                     m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy));
                     if (ok) {
                         bb.add(ci, cj, ir, jr, g);
-                        cf0 = __double2float_rn(qoa * static_cast<double>(w));
-                        const float cf[1] = {cf0};
+                        const float cf[1] = {__double2float_rn(qoa * static_cast<double>(w))};
                         float cs[1];
                         const bool fast = scale_fast<1>(cf, S1, cs, l1);
                         xs = __fadd_rn(x, 0.0f);
+                        ys = __fadd_rn(y, 0.0f);
                         if (!fast) { xs = -xs; list_slow(m.slow, &nlist, s); }
                     } else {
+                        ys = 0.0f;
                         set_err(st, AW_DEV_OUT_OF_GRID);
                     }
-                    const double dw = w, du = ux, dv = uy, dz = uz;
-                    ke += dw * (du * du + dv * dv + dz * dz);
-                    px += dw * du; py += dw * dv; pz += dw * dz;
                 } else {
                     set_err(st, AW_DEV_OUT_OF_GRID);
                 }
             }
             const int d = s;                     // in place: this thread's own slot
             m.stage[d] = xs;
-            m.stage[kChunk + d] = y;
-            m.stage[2 * kChunk + d] = cf0;
+            m.stage[kChunk + d] = ys;
+            m.stage[2 * kChunk + d] = ux; m.stage[3 * kChunk + d] = uy; m.stage[4 * kChunk + d] = uz;
         }
-        const Win wn = open_window<NF, T0>(bb, ir, jr, wmaxc, m, l1);
-        auto coef = [&](const float (&a)[NS], float (&cs)[NF]) {
-            cs[0] = __fmul_rn(a[2], S1[0]);
+        Win wn;
+        win_setup<NF, T0>(wn, bb.lo_i, bb.lo_j, bb.hi_i, bb.hi_j, ir, jr, wmaxc, m.red, l1);   // (syncs)
+        // The step's sums go over the slots each thread has in the single pass, in its
+        // order: the diagnostics don't depend on the path. The coefficient replaces ux.
+        double dw = __int_as_float(wlo);
+        float cf0 = __double2float_rn(qoa * dw);
+        auto sums = [&](int sl) {
+            float* const q5 = m.stage + sl;
+            if (!(q5[kChunk] >= 0.0f)) return;                // not pushed
+            if (!wsame) { dw = __ldg(p.w + c0 + sl); cf0 = __double2float_rn(qoa * dw); }
+            const double du = q5[2 * kChunk], dv = q5[3 * kChunk], dz = q5[4 * kChunk];
+            ke += dw * (du * du + dv * dv + dz * dz);
+            px += dw * du; py += dw * dv; pz += dw * dz;
+            q5[2 * kChunk] = cf0;
         };
-        window_pass<NF, NS, T0>(m.stage, m.win, wn, cs_, g, coef, acc);
+        auto coef = [&](const float (&a)[NS], float (&cs)[NF]) { cs[0] = __fmul_rn(a[2], S1[0]); };
+        if (wn.nb == 1 && wn.WH <= kEsSmall) {
+            // a small window fits the area behind the stage: deposit and sums together
+            // (375 x 225 at 50 per cell: 117.7 us a step, with the two apart 119.3)
+            wn.P = kEsSmall;
+            m.win = area;
+            win_zero<NF, T0>(m.win, wn);
+            __syncthreads();
+            window_particles<NF, NS, T0, false, 0>(
+                m.stage, m.win, wn, cs_, g, [&](const float (&)[NS], float (&cs)[NF]) { cs[0] = __fmul_rn(cf0, S1[0]); },
+                [&](const float (&)[NS], int sl) { sums(sl); });
+        } else {
+#pragma unroll 2
+            for (int k = 0; k < ppt; ++k) sums(sp.slot(k));
+            __syncthreads();
+            win_zero<NF, T0>(m.win, wn);
+            __syncthreads();
+            window_pass<NF, NS, T0>(m.stage, m.win, wn, cs_, g, coef, acc);
+        }
         close_window<NF, NS, T0>(m, wn, nlist, cs_, acc, g, st, coef);
     }
     // the in-plane |u| maxima bound the next step's moves (the single pass's margin)
@@ -1788,7 +1820,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     float2 sqp[4] = {};
     double ke = 0, px = 0, py = 0, pz = 0;
     float nval = 0.f;
-    auto stats = [&](const float (&a)[NS]) {
+    auto stats = [&](const float (&a)[NS], int = 0) {
         const double dw = a[2], du = a[3], dv = a[4], dz = a[5];
         ke += dw * (du * du + dv * dv + dz * dz);
         px += dw * du; py += dw * dv; pz += dw * dz;

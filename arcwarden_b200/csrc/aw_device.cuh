@@ -816,7 +816,7 @@ __device__ __forceinline__ void quant_bits(const float (&cs)[NF], const Cic2& c,
 // staged x has its sign bit set (invalid, or listed for the slow pass) are
 // skipped. PC: the plane stride when known at compile time (0: wn.P).
 struct NoHook {
-    template <int NS> __device__ __forceinline__ void operator()(const float (&)[NS]) const {}
+    template <int NS> __device__ __forceinline__ void operator()(const float (&)[NS], int) const {}
 };
 template <int NF, int NS, bool T0, bool TRACK_ALL, int PC, class CoefFn, class Hook = NoHook>
 __device__ __forceinline__ void window_particles(const float* __restrict__ stage, int* __restrict__ win,
@@ -832,7 +832,7 @@ __device__ __forceinline__ void window_particles(const float* __restrict__ stage
         float a[NS];
 #pragma unroll
         for (int f = 0; f < NS; ++f) a[f] = stage[f * kChunk + d];
-        hook(a);                                  // every slot, deposited or not
+        hook(a, d);                               // every slot, deposited or not
         if (__float_as_int(a[0]) < 0) continue;
         const Cic2 c = cic2(a[0], a[1]);
         float cs[NF];

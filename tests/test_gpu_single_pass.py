@@ -95,3 +95,33 @@ def test_cold_beams_keep_to_the_windows(torch_cuda, aw, ppc, vth):
             s.close()
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("model,nx,ny,Lx,Ly,ppc,weights", [c for c in CASES if c[0] == 0] + [CASES[4], CASES[7]])
+def test_diagnostics_do_not_depend_on_the_plan(torch_cuda, aw, model, nx, ny, Lx, Ly, ppc, weights):
+    """Every step's FP64 sums: each thread adds up the same particles in the same order
+    in one pass and in two."""
+    n = nx * ny * ppc - 3
+    rng = np.random.default_rng(nx * 100 + ny)
+    cell = np.repeat(np.arange(nx * ny), ppc)[:n]
+    edge = lambda v, top: np.minimum(v.astype(np.float32), np.nextafter(np.float32(top), np.float32(0)))  # noqa: E731
+    P = {"x": edge(cell % nx + rng.random(n), nx), "y": edge(cell // nx + rng.random(n), ny),
+         "ux": rng.normal(0, 0.3, n), "uy": rng.normal(0, 0.3, n), "uz": rng.normal(0, 0.2, n),
+         "w": np.full(n, Lx * Ly / (nx * ny) / ppc) * (1.0 if weights == "one" else rng.random(n))}
+    out = []
+    for one_pass in (0, 1):
+        s = Setup(torch_cuda, aw, nx, ny, Lx, Ly, n, model, dt=0.05, B0=(0.1, 0.0, 0.3))
+        try:
+            s.ctx.set_kernel_plan(one_pass=one_pass)
+            for k in PARTICLE_KEYS:
+                s.put(k, P[k].astype(np.float32))
+            s.ctx.init()
+            d = np.zeros((4, 8))
+            s.ctx.run_diag(0, 4, d.ctypes.data)
+            torch_cuda.cuda.synchronize()
+            assert s.ctx.error_word() == 0
+            out.append(d)
+        finally:
+            s.close()
+    assert np.abs(out[0][:, 0]).min() > 0
+    assert np.array_equal(out[0], out[1])
