@@ -613,6 +613,8 @@ int aw_particles_bind(aw_ctx* ctx, float* x, float* y, float* ux, float* uy, flo
         }
         c.npart_p = nb;
         AW_CUDA(cudaMemsetAsync(c.part_p, 0, sizeof(double) * 5 * nb, c.stream));
+        AW_CUDA(cudaMemsetAsync(c.part_c, 0, sizeof(float) * 9 * nb, c.stream));
+        AW_CUDA(cudaMemsetAsync(c.part_d, 0, sizeof(float) * 4 * nb, c.stream));
         c.pending_valid = false;
         c.inited = false;
         aw::drop_graph(c);

@@ -727,17 +727,44 @@ __device__ __forceinline__ void win1_flush(const int* __restrict__ s, const Win1
     }
 }
 
-// Whether a full chunk's sums may be expected to leave the int32 range: `top` is the
-// largest rms |coefficient| of a biased field in the last deposit, scaled. A single
-// pass that finds so only at its end (chunk_overflows1) has the whole chunk left for the
-// exact global path, 5 to 8 times the time of the two passes, which count carries; so
-// such chunks take those from the start. The scales bound the largest coefficient by
-// 2^22: a Maxwellian's rms is a fifth of its maximum or less (2048 x 2^22 / 5.6 = 1.5e9),
-// a cold beam's is almost the maximum (up to 8e9): 512 x 512, 256 per cell, drift
-// 0.24 over a spread of 0.07: 14.9 ms a step in the single pass, 2.7 in two.
-__device__ __forceinline__ bool expect_overflow1(float top, int cs) {
-    return top * static_cast<float>(cs) > 1.75e9f;
-}
+// Whether a chunk's sums may be expected to leave the int32 range: from the largest rms
+// |coefficient| of the biased fields first .. NF - 1, scaled, that this chunk's sample psq
+// had in the last deposit, or the whole run's where the sample has fewer than 64
+// particles (one fast particle in a few sent 512 x 1 chunks of 768 the long way: 52.6 ->
+// 54.1 us a step). A single pass that finds so only at its end (chunk_overflows1) is done
+// over in two passes, which count carries, so such chunks take those from the start.
+// The scales bound the largest coefficient by 2^22: a Maxwellian's rms is a fifth of its
+// maximum or less (2048 x 2^22 / 5.6 = 1.5e9), a cold beam's is almost the maximum (up to
+// 8e9). Asked of the chunk and not of the run, because a beam may be a part of the
+// particles, stored apart. 256 x 256 at 256 per cell, a tenth of them such a beam, us a
+// step: 897 the first and 694 the later ones when asked of the run and done over through
+// the exact global path, 628 and 635 like this (two passes for all: 803).
+// The second warp loads before the chunk does and sets `hot` after (the block's next
+// barrier publishes it): nothing waits for its loads.
+template <int NF>
+struct Expect1 {
+    bool have = false;
+    float n = 0.f, sq = 0.f, all = 0.f, s = 0.f;
+    template <class ScaleFn>
+    __device__ __forceinline__ Expect1(const DevState* st, const float* __restrict__ psq, const float* rms,
+                                       ScaleFn scale, int first, int chunk) {
+        const int f = static_cast<int>(threadIdx.x) - 32;
+        if (f < first || f >= NF) return;
+        have = st->have_rms != 0;
+        all = rms[f];
+        s = scale(f);
+        if (psq) {
+            const float* const q = psq + static_cast<size_t>(chunk) * (NF + 1);
+            n = q[NF]; sq = q[f];
+        }
+    }
+    __device__ __forceinline__ void set(int* hot, int cs) const {
+        if (threadIdx.x >> 5 != 1) return;
+        const float r = n >= 64.0f ? __fsqrt_rn(__fdividef(sq, n)) : all;
+        const bool over = __any_sync(0xffffffffu, have && r * s * static_cast<float>(cs) > 1.75e9f);
+        if (threadIdx.x == 32) *hot = over;
+    }
+};
 
 // True (block-uniformly) when some biased field's chunk sum may reach 2^31. Each
 // thread brings the largest of its fields' sums of cs^2 over its m fast
@@ -848,17 +875,15 @@ __device__ __forceinline__ void bulk_store_wait() {
     if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// Exact slow path of a single-pass chunk, from the linear stage: the listed
-// slots, or (redo: the window may have wrapped) every slot whose staged
-// position is in the grid. coef(s, cs) gives slot s's NF scaled coefficients.
+// Exact slow path of a single-pass chunk, from the linear stage: the listed slots whose
+// staged position is in the grid. coef(s, cs) gives slot s's NF scaled coefficients.
 template <int NF, class CoefFn>
 __device__ __forceinline__ void slow_pass_linear(const float* __restrict__ stage, const unsigned short* __restrict__ list,
-                                                 int nlist, bool redo, int cnt, unsigned long long* __restrict__ gacc,
+                                                 int nlist, unsigned long long* __restrict__ gacc,
                                                  const Geo& g, DevState* st, CoefFn coef) {
-    const int total = redo ? cnt : nlist;
     unsigned n = 0;
-    for (int k = threadIdx.x; k < total; k += kThreads) {
-        const int sl = redo ? k : static_cast<int>(list[k]);
+    for (int k = threadIdx.x; k < nlist; k += kThreads) {
+        const int sl = static_cast<int>(list[k]);
         const float x = stage[sl], y = stage[kChunk + sl];
         if (!in_grid(x, y, g)) continue;
         float cs[NF];
@@ -924,6 +949,8 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     if (chunk == 0 && threadIdx.x == 0) { st->S_dcu[0] = S[0]; st->S_dcu[1] = S[1]; st->S_dcu[2] = S[2]; }
     __shared__ __align__(16) int ends[4];
     if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
+    __shared__ int hot;
+    const Expect1<NF> expect(st, psq, st->rms_dcu, [&](int f) { return f == 0 ? S[0] : f == 1 ? S[1] : S[2]; }, 0, chunk);
     const ChunkSrc src{{p.x, p.y, p.w, p.ux, p.uy, p.uz}};
     float x0, y0;
     if (!load_chunk(m.stage, src, NIN, c0, cnt, p.vec_ok != 0, &bar, st, &x0, &y0)) return;
@@ -932,13 +959,12 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
 
     // ---- single pass: the particles do not move, so the window is the box of
     // their base cells plus the corner - the gather tile's box
-    const float top = st->have_rms ? fmaxf(st->rms_dcu[0] * S[0], fmaxf(st->rms_dcu[1] * S[1], st->rms_dcu[2] * S[2]))
-                                   : 0.0f;
-    if (A.one_pass && !expect_overflow1(top, cs_)) {
+    if (A.one_pass) {
+        expect.set(&hot, cs_);
         constexpr int P1 = 640, T1 = ((PC * win_planes(NF) - P1 * (NF + 1)) / 6) & ~3;     // 24 bytes per tile cell
         Box1 bx;
         Win1 w1;
-        if (chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, T1, 0, bx) && window1<P1>(w1, bx, 0, A.rep_need, g) &&
+        if (chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, T1, 0, bx) && !hot && window1<P1>(w1, bx, 0, A.rep_need, g) &&
             (bx.nI + 1) * (bx.nJ + 1) <= T1) {
             Tile1 tl;
             tile1_load<T1>(tl, reinterpret_cast<float*>(m.win + P1 * (NF + 1)), bx, gb, g);
@@ -984,28 +1010,34 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
                     list_slow(m.slow, &nlist, sl);
                 }
             }
-            const bool redo = chunk_overflows1(fmaxf(l2[0], fmaxf(l2[1], l2[2])), ppt, m.red);   // (its barrier ends the pass)
-            if (!redo) win1_flush<NF, false, P1>(m.win, w1, acc, g);
-            slow_pass_linear<NF>(m.stage, m.slow, nlist, redo, cnt, acc, g, st, [&](int sl, float (&cs)[NF]) {
-                float cf[NF];
-                const float x = m.stage[sl], y = m.stage[kChunk + sl];
-                coefs(sl, x, y, cic(x, y), cf);
+            // (its barrier ends the pass)
+            if (!chunk_overflows1(fmaxf(l2[0], fmaxf(l2[1], l2[2])), ppt, m.red)) {
+                win1_flush<NF, false, P1>(m.win, w1, acc, g);
+                slow_pass_linear<NF>(m.stage, m.slow, nlist, acc, g, st, [&](int sl, float (&cs)[NF]) {
+                    float cf[NF];
+                    const float x = m.stage[sl], y = m.stage[kChunk + sl];
+                    coefs(sl, x, y, cic(x, y), cf);
 #pragma unroll
-                for (int f = 0; f < NF; ++f) cs[f] = __fmul_rn(cf[f], S[f]);
-            });
-            if (threadIdx.x == 0) {
-                atomicAdd(&st->chunks, 1ull);
-                atomicAdd(&st->one_pass, 1ull);
-                if (redo) atomicAdd(&st->overflow, 1ull);
+                    for (int f = 0; f < NF; ++f) cs[f] = __fmul_rn(cf[f], S[f]);
+                });
+                if (threadIdx.x == 0) {
+                    atomicAdd(&st->chunks, 1ull);
+                    atomicAdd(&st->one_pass, 1ull);
+                }
+                if (psq) {
+                    block_sumsq_put<NF>(sq, nval, ssq);
+                    __syncthreads();
+                    block_sumsq_get<NF>(psq, ssq, chunk);
+                }
+                return;
             }
-            if (psq) {
-                block_sumsq_put<NF>(sq, nval, ssq);
-                __syncthreads();
-                block_sumsq_get<NF>(psq, ssq, chunk);
-            }
-            return;
+            // the window may have wrapped: the chunk over again in two passes (its stage
+            // is as it was loaded; the tile's bulk copies follow this window's accesses)
+            stage_fence();
         }
-        __syncthreads();           // the box scratch has been read
+        __syncthreads();           // the scratch has been read
+        if (threadIdx.x == 0) nlist = 0;
+        __syncthreads();
     }
 
     // ---- two passes --------------------------------------------------------
@@ -1569,15 +1601,13 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     float S[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) S[f] = st->S_next[f];
-    float top = 0.0f;                             // (field 0 is carried exactly)
-    if (st->have_rms)
-#pragma unroll
-        for (int f = 1; f < NF; ++f) top = fmaxf(top, st->rms_src[f] * S[f]);
     const float2 Sp[4] = {make_float2(S[0], S[1]), make_float2(S[2], S[3]), make_float2(S[4], S[5]),
                           make_float2(S[6], S[7])};
     __shared__ __align__(16) int ends[4];
     if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
     const float uxy_max = fmaxf(__uint_as_float(st->ucur_bits[0]), __uint_as_float(st->ucur_bits[1]));
+    __shared__ int hot;                           // (field 0 is carried exactly)
+    const Expect1<NF> expect(st, psq, st->rms_src, [&](int f) { return st->S_next[f]; }, 1, chunk);
     const ChunkSrc src{{p.x, p.y, p.w, p.ux, p.uy, p.uz}};
     float x0, y0;
     if (!load_chunk(m.stage, src, NS, c0, cnt, p.vec_ok != 0, &bar, st, &x0, &y0)) return;
@@ -1585,7 +1615,8 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     ref_of(x0, y0, g, ir, jr);
 
     // ---- single pass -------------------------------------------------------
-    if (A.one_pass && !expect_overflow1(top, cs_)) {
+    if (A.one_pass) {
+        expect.set(&hot, cs_);
         constexpr int P1 = 384, T1 = ((PC * win_planes(NF) - P1 * (NF + 3)) / 6) & ~3;     // 24 bytes per tile cell
         // the cells a particle can cross in one step: twice the largest in-plane |u| of
         // the current state times dt/dx (one further cell for the rounding)
@@ -1593,7 +1624,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
         const int mg = (dmv >= 0.0f && dmv < 8.0f) ? 1 + static_cast<int>(dmv) : -1;
         Box1 bx;
         Win1 w1;
-        if (mg > 0 && chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, P1, mg, bx) &&
+        if (mg > 0 && chunk_box<FULL>(m.stage, cs_, cnt, x0, y0, g, ends, m.red, P1, mg, bx) && !hot &&
             window1<P1>(w1, bx, mg, A.rep_need, g) && (bx.nI + 1) * (bx.nJ + 1) <= T1) {
             Tile1 tl;
             tile1_load<T1>(tl, reinterpret_cast<float*>(m.win + P1 * (NF + 3)), bx, gb, g);
@@ -1667,47 +1698,57 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
             float l2m = l2p[0].y;                                // field 0 is carried exactly (coarse planes)
 #pragma unroll
             for (int i = 1; i < 4; ++i) l2m = fmaxf(l2m, fmaxf(l2p[i].x, l2p[i].y));
-            const bool redo = chunk_overflows1(l2m, ppt, m.red);    // (its barrier ends the pass)
-            // the new state leaves by bulk copy (x y ux uy uz and the cells: stage planes 0 1 3 4 5 2)
-            const int pl[6] = {0, 1, 3, 4, 5, 2};
-            float* const dst[6] = {p.x, p.y, p.ux, p.uy, p.uz, reinterpret_cast<float*>(p.cell)};
-            bulk_store_planes<6>(m.stage, pl, dst, cells ? 6 : 5, c0, cnt, p.vec_ok != 0);
-            if (!redo) win1_flush<NF, true, P1>(m.win, w1, acc, g);
-            slow_pass_linear<NF>(m.stage, m.slow, nlist, redo, cnt, acc, g, st, [&](int sl, float (&cs)[NF]) {
-                float2 cp[4];
-                src_coefs8(__double2float_rn(qoa * static_cast<double>(p.w[c0 + sl])),
-                           m.stage[3 * kChunk + sl], m.stage[4 * kChunk + sl], m.stage[5 * kChunk + sl], cp);
+            // (its barrier ends the pass)
+            if (!chunk_overflows1(l2m, ppt, m.red)) {
+                // the new state leaves by bulk copy (x y ux uy uz and the cells: stage planes 0 1 3 4 5 2)
+                const int pl[6] = {0, 1, 3, 4, 5, 2};
+                float* const dst[6] = {p.x, p.y, p.ux, p.uy, p.uz, reinterpret_cast<float*>(p.cell)};
+                bulk_store_planes<6>(m.stage, pl, dst, cells ? 6 : 5, c0, cnt, p.vec_ok != 0);
+                win1_flush<NF, true, P1>(m.win, w1, acc, g);
+                slow_pass_linear<NF>(m.stage, m.slow, nlist, acc, g, st, [&](int sl, float (&cs)[NF]) {
+                    float2 cp[4];
+                    src_coefs8(__double2float_rn(qoa * static_cast<double>(p.w[c0 + sl])),
+                               m.stage[3 * kChunk + sl], m.stage[4 * kChunk + sl], m.stage[5 * kChunk + sl], cp);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 cc = __fmul2_rn(cp[i], Sp[i]);
-                    cs[2 * i] = cc.x; cs[2 * i + 1] = cc.y;
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 cc = __fmul2_rn(cp[i], Sp[i]);
+                        cs[2 * i] = cc.x; cs[2 * i + 1] = cc.y;
+                    }
+                });
+                if (threadIdx.x < 3) {
+                    unsigned mx = 0;
+                    for (int k = 0; k < kThreads / 32; ++k) mx = max(mx, umx[threadIdx.x][k]);
+                    atomicMax(&st->umax_bits[threadIdx.x], mx);
                 }
-            });
-            if (threadIdx.x < 3) {
-                unsigned mx = 0;
-                for (int k = 0; k < kThreads / 32; ++k) mx = max(mx, umx[threadIdx.x][k]);
-                atomicMax(&st->umax_bits[threadIdx.x], mx);
-            }
-            if (threadIdx.x == 0) {
-                atomicAdd(&st->chunks, 1ull);
-                atomicAdd(&st->one_pass, 1ull);
-                if (redo) atomicAdd(&st->overflow, 1ull);
-            }
-            const float sq[NF] = {sqp[0].x, sqp[0].y, sqp[1].x, sqp[1].y, sqp[2].x, sqp[2].y, sqp[3].x, sqp[3].y};
-            block_sumsq_put<NF>(sq, nval, ssq);
-            block_sum4_put(ke, px, py, pz, dsh);
-            __syncthreads();
-            block_sumsq_get<NF>(psq, ssq, chunk, 32);
-            block_sum4_get(part, dsh, chunk);
-            if (threadIdx.x == 0 && chunk == 0) {
+                if (threadIdx.x == 0) {
+                    atomicAdd(&st->chunks, 1ull);
+                    atomicAdd(&st->one_pass, 1ull);
+                }
+                const float sq[NF] = {sqp[0].x, sqp[0].y, sqp[1].x, sqp[1].y, sqp[2].x, sqp[2].y, sqp[3].x, sqp[3].y};
+                block_sumsq_put<NF>(sq, nval, ssq);
+                block_sum4_put(ke, px, py, pz, dsh);
+                __syncthreads();
+                block_sumsq_get<NF>(psq, ssq, chunk, 32);
+                block_sum4_get(part, dsh, chunk);
+                if (threadIdx.x == 0 && chunk == 0) {
 #pragma unroll
-                for (int f = 0; f < NF; ++f) st->S_pend[f] = S[f];
-                st->step += 1;
+                    for (int f = 0; f < NF; ++f) st->S_pend[f] = S[f];
+                    st->step += 1;
+                }
+                bulk_store_wait();
+                return;
             }
-            bulk_store_wait();
-            return;
+            // the window may have wrapped: the chunk over again in two passes, from its state
+            // in global memory, which is still the old one (the tile's bulk copies follow
+            // this window's accesses)
+#pragma unroll 1
+            for (int f = 0; f < NS; ++f)
+                for (int sl = threadIdx.x; sl < cnt; sl += kThreads) m.stage[f * kChunk + sl] = src.at(f)[c0 + sl];
+            stage_fence();
         }
-        __syncthreads();           // the box scratch has been read
+        __syncthreads();           // the scratch has been read
+        if (threadIdx.x == 0) nlist = 0;
+        __syncthreads();
     }
 
     // ---- two passes --------------------------------------------------------

@@ -125,3 +125,45 @@ def test_diagnostics_do_not_depend_on_the_plan(torch_cuda, aw, model, nx, ny, Lx
             s.close()
     assert np.abs(out[0][:, 0]).min() > 0
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nx,ny,ppc,part", [(128, 64, 256, 0.1), (128, 64, 256, 0.3), (64, 64, 64, 0.25)])
+def test_cold_minority_beam_keeps_to_the_windows(torch_cuda, aw, nx, ny, ppc, part):
+    """A cold beam that is a part of the particles, stored after a warm background: its
+    chunks' sums leave the int32 range while the run's rms says nothing of it. They are
+    done over in two passes, or take them from the start, with the two-pass plan's bits
+    and no more exact global deposits than it has: from the first step on."""
+    n, beam = nx * ny * ppc, int(part * ppc)
+    rng = np.random.default_rng(int(100 * part) + ppc)
+    cell = np.concatenate([np.repeat(np.arange(nx * ny), ppc - beam), np.repeat(np.arange(nx * ny), beam)])
+    cold = np.arange(n) >= n - beam * nx * ny
+    P = {"x": cell % nx + 0.999 * rng.random(n), "y": cell // nx + 0.999 * rng.random(n),
+         "ux": np.where(cold, 0.3 + rng.normal(0, 0.002, n), rng.normal(0, 0.03, n)),
+         "uy": np.where(cold, 0.25 + rng.normal(0, 0.002, n), rng.normal(0, 0.03, n)),
+         "uz": rng.normal(0, 0.03, n), "w": np.full(n, 1.0 / ppc)}
+    out = []
+    for one_pass in (0, 1):
+        s = Setup(torch_cuda, aw, nx, ny, float(nx), float(ny), n, 1, dt=0.05)
+        try:
+            s.ctx.set_kernel_plan(one_pass=one_pass)
+            for k in PARTICLE_KEYS:
+                s.put(k, P[k].astype(np.float32))
+            s.ctx.init()
+            slow, d = [s.ctx.stats()["slow_deposits"]], np.zeros((5, 8))
+            for k in range(5):
+                s.ctx.run_diag(k, 1, d[k:].ctypes.data)
+                torch_cuda.cuda.synchronize()
+                slow.append(s.ctx.stats()["slow_deposits"])
+            r = s.parts()
+            for k in ("rho", "Jx", "Jz", "Ex", "Ey", "Ez", "Bz"):
+                r[k] = s.grid(k)
+            assert s.ctx.error_word() == 0
+            r["diag"] = d
+            out.append((np.diff(slow), r, s.ctx.stats()))
+        finally:
+            s.close()
+    assert out[1][2]["one_pass_chunks"] > 0
+    # beyond the two-pass plan's: only particles that leave a single pass's window
+    assert (out[1][0] <= out[0][0] + n // 1000).all(), (out[0][0], out[1][0])
+    for k in out[0][1]:
+        assert np.array_equal(out[0][1][k], out[1][1][k]), k
