@@ -280,6 +280,22 @@ __device__ __forceinline__ void block_sumsq_get(float* __restrict__ psq, const f
     }
 }
 
+// JOINT kernels: the joint launches of an ensemble (k_*_multi). Runs that share a launch
+// fill the GPU together, so their chunks hold as many of a run's own chunks (part_cs
+// particles, chunk_size's choice for the run alone) as fit kChunk. Each thread still
+// goes over one own chunk after the other, over its slots of it, and the block's sums
+// end with each: the partials, and so the diagnostics and the coefficient rms, are
+// those of the run alone. Runs of 64 x 64 at 16 per cell, 48 together, us a step: with
+// own chunks of 256 391 (electrostatic) and 1000 (Darwin), like this 290 and 829.
+struct Own {
+    int cs, ppt, n, first;       // particles and iterations of one, how many here, the first's partial
+};
+template <bool JOINT>
+__device__ __forceinline__ Own own_chunks(int chunk, int cs, int cnt, int part_cs) {
+    if (!JOINT) return {cs, cs / kThreads, 1, chunk};
+    return {part_cs, part_cs / kThreads, (cnt + part_cs - 1) / part_cs, chunk * (cs / part_cs)};
+}
+
 // Running bounding box of wrapped cell offsets.
 struct BBox {
     int lo_i = 1 << 30, lo_j = 1 << 30, hi_i = -(1 << 30), hi_j = -(1 << 30);
@@ -746,17 +762,18 @@ struct Expect1 {
     bool have = false;
     float n = 0.f, sq = 0.f, all = 0.f, s = 0.f;
     template <class ScaleFn>
-    __device__ __forceinline__ Expect1(const DevState* st, const float* __restrict__ psq, const float* rms,
-                                       ScaleFn scale, int first, int chunk) {
+    __device__ __forceinline__ Expect1(const DevState* st, const float* psq, const float* rms, ScaleFn scale, int first,
+                                       const Own& own) {
         const int f = static_cast<int>(threadIdx.x) - 32;
         if (f < first || f >= NF) return;
         have = st->have_rms != 0;
         all = rms[f];
         s = scale(f);
-        if (psq) {
-            const float* const q = psq + static_cast<size_t>(chunk) * (NF + 1);
-            n = q[NF]; sq = q[f];
-        }
+        if (psq)
+            for (int k = 0; k < own.n; ++k) {
+                const float* const q = psq + static_cast<size_t>(own.first + k) * (NF + 1);
+                n += q[NF]; sq += q[f];
+            }
     }
     __device__ __forceinline__ void set(int* hot, int cs) const {
         if (threadIdx.x >> 5 != 1) return;
@@ -921,10 +938,10 @@ __device__ __forceinline__ void dcu_scales(const DevState* st, float abs_qm, boo
 // dcu deposit: input x y w ux uy uz; stage = x, y, ax, ay, az (scaled coefficients).
 struct DcuArgs {
     Parts p; Geo g; double qm2oa; float abs_qm; const float* gb; unsigned long long* acc; int wmaxc;
-    DevState* st; int use_rms; float* psq; int use_tile; int one_pass; int rep_need;
+    DevState* st; int use_rms; float* psq; int use_tile; int one_pass; int rep_need; int part_cs;
 };
 // FULL: chunks of kChunk particles (the trip counts are compile-time constants).
-template <bool FULL>
+template <bool FULL, bool JOINT>
 __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int chunk) {
     const Parts& p = A.p; const Geo& g = A.g;
     const double qm2oa = A.qm2oa; const float abs_qm = A.abs_qm;
@@ -943,14 +960,15 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
     const long long c0 = static_cast<long long>(chunk) * cs_;
     const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
     const int ppt = cs_ / kThreads;               // particles per thread
-    const Spread sp(cs_);
+    const Own own = own_chunks<JOINT>(chunk, cs_, cnt, A.part_cs);
+    const Spread sp(own.cs);
     float S[3];
     dcu_scales(st, abs_qm, use_rms != 0, S);
     if (chunk == 0 && threadIdx.x == 0) { st->S_dcu[0] = S[0]; st->S_dcu[1] = S[1]; st->S_dcu[2] = S[2]; }
     __shared__ __align__(16) int ends[4];
     if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
     __shared__ int hot;
-    const Expect1<NF> expect(st, psq, st->rms_dcu, [&](int f) { return f == 0 ? S[0] : f == 1 ? S[1] : S[2]; }, 0, chunk);
+    const Expect1<NF> expect(st, psq, st->rms_dcu, [&](int f) { return f == 0 ? S[0] : f == 1 ? S[1] : S[2]; }, 0, own);
     const ChunkSrc src{{p.x, p.y, p.w, p.ux, p.uy, p.uz}};
     float x0, y0;
     if (!load_chunk(m.stage, src, NIN, c0, cnt, p.vec_ok != 0, &bar, st, &x0, &y0)) return;
@@ -986,29 +1004,44 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
             };
             float l2[NF] = {}, sq[NF] = {};
             float nval = 0.f;
+            auto own_sums = [&](int o) {
+                if (!psq) return;
+                block_sumsq_put<NF>(sq, nval, ssq);
+                __syncthreads();
+                block_sumsq_get<NF>(psq, ssq, own.first + o);
+                if (!JOINT) return;
+                __syncthreads();
+#pragma unroll
+                for (int f = 0; f < NF; ++f) sq[f] = 0.f;
+                nval = 0.f;
+            };
 #pragma unroll 1
-            for (int k = 0; k < ppt; ++k) {
-                const int sl = sp.slot(k);
-                if (sl >= cnt) continue;
-                const float x = m.stage[sl], y = m.stage[kChunk + sl];
-                const Cic c = cic(x, y);
-                float cf[NF], cs[NF];
-                coefs(sl, x, y, c, cf);
+            for (int o = 0; o < own.n; ++o) {
+#pragma unroll 1
+                for (int k = 0; k < own.ppt; ++k) {
+                    const int sl = o * own.cs + sp.slot(k);
+                    if (sl >= cnt) continue;
+                    const float x = m.stage[sl], y = m.stage[kChunk + sl];
+                    const Cic c = cic(x, y);
+                    float cf[NF], cs[NF];
+                    coefs(sl, x, y, c, cf);
 #pragma unroll
-                for (int f = 0; f < NF; ++f) cs[f] = __fmul_rn(cf[f], S[f]);
-                if (((c.i0 + c.j0) & 7) == 0) {   // rms sample: the particles of one cell in 8, any order
+                    for (int f = 0; f < NF; ++f) cs[f] = __fmul_rn(cf[f], S[f]);
+                    if (((c.i0 + c.j0) & 7) == 0) {   // rms sample: the particles of one cell in 8, any order
 #pragma unroll
-                    for (int f = 0; f < NF; ++f) sq[f] = __fmaf_rn(cf[f], cf[f], sq[f]);
-                    nval += 1.0f;
+                        for (int f = 0; f < NF; ++f) sq[f] = __fmaf_rn(cf[f], cf[f], sq[f]);
+                        nval += 1.0f;
+                    }
+                    // (a NaN fails the test: fmaxf would drop it)
+                    if (fabsf(cs[0]) < kFastLim && fabsf(cs[1]) < kFastLim && fabsf(cs[2]) < kFastLim) {
+#pragma unroll
+                        for (int f = 0; f < NF; ++f) l2[f] = __fmaf_rn(cs[f], cs[f], l2[f]);
+                        win1_add<NF, false, P1>(m.win, w1, win_col(c.i0, w1.oi, g.nx), win_col(c.j0, w1.oj, g.ny), x, y, cs);
+                    } else {
+                        list_slow(m.slow, &nlist, sl);
+                    }
                 }
-                // (a NaN fails the test: fmaxf would drop it)
-                if (fabsf(cs[0]) < kFastLim && fabsf(cs[1]) < kFastLim && fabsf(cs[2]) < kFastLim) {
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) l2[f] = __fmaf_rn(cs[f], cs[f], l2[f]);
-                    win1_add<NF, false, P1>(m.win, w1, win_col(c.i0, w1.oi, g.nx), win_col(c.j0, w1.oj, g.ny), x, y, cs);
-                } else {
-                    list_slow(m.slow, &nlist, sl);
-                }
+                if (JOINT) own_sums(o);
             }
             // (its barrier ends the pass)
             if (!chunk_overflows1(fmaxf(l2[0], fmaxf(l2[1], l2[2])), ppt, m.red)) {
@@ -1024,11 +1057,7 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
                     atomicAdd(&st->chunks, 1ull);
                     atomicAdd(&st->one_pass, 1ull);
                 }
-                if (psq) {
-                    block_sumsq_put<NF>(sq, nval, ssq);
-                    __syncthreads();
-                    block_sumsq_get<NF>(psq, ssq, chunk);
-                }
+                if (!JOINT) own_sums(0);
                 return;
             }
             // the window may have wrapped: the chunk over again in two passes (its stage
@@ -1118,28 +1147,40 @@ __device__ __forceinline__ void deposit_dcu_chunk(const DcuArgs& A, const int ch
             }
         }
     };
-    if (wn.use && wn.nb == 1) {
+    auto own_sums = [&](int o) {
+        if (!psq) return;
+        block_sumsq_put<NF>(sq, nval, ssq);
+        __syncthreads();
+        block_sumsq_get<NF>(psq, ssq, own.first + o);
+        if (!JOINT) return;
+        __syncthreads();
+#pragma unroll
+        for (int f = 0; f < NF; ++f) sq[f] = 0.f;
+        nval = 0.f;
+    };
+    if (!JOINT && wn.use && wn.nb == 1) {
         if (wn.track_all) window_particles<NF, NS, T0, true, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
         else window_particles<NF, NS, T0, false, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
     } else {
 #pragma unroll 1
-        for (int k = 0; k < ppt; ++k) {
-            const int d = sp.slot(k);
-            float a[NS];
+        for (int o = 0; o < own.n; ++o) {
+#pragma unroll 1
+            for (int k = 0; k < own.ppt; ++k) {
+                const int d = o * own.cs + sp.slot(k);
+                float a[NS];
 #pragma unroll
-            for (int f = 0; f < NS; ++f) a[f] = m.stage[f * kChunk + d];
-            stats(a);
+                for (int f = 0; f < NS; ++f) a[f] = m.stage[f * kChunk + d];
+                stats(a);
+            }
+            if (JOINT) own_sums(o);
         }
         window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);   // bands (or the slow path alone)
     }
     close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
-    if (psq) {
-                block_sumsq_put<NF>(sq, nval, ssq);
-                __syncthreads();
-                block_sumsq_get<NF>(psq, ssq, chunk);
-            }}
+    if (!JOINT) own_sums(0);
+}
 template <bool FULL>
-__global__ void __launch_bounds__(kThreads, 3) k_deposit_dcu(DcuArgs A) { deposit_dcu_chunk<FULL>(A, blockIdx.x); }
+__global__ void __launch_bounds__(kThreads, 3) k_deposit_dcu(DcuArgs A) { deposit_dcu_chunk<FULL, false>(A, blockIdx.x); }
 
 // ---------------------------------------------------------------------------
 // Backward step A of the ES adjoint (the transpose of k_push_deposit_es's push
@@ -1295,9 +1336,9 @@ struct EsArgs {
     Parts p; Geo g; PushP pp; const float* gb; double qoa; unsigned long long* acc; int wmaxc;
     double* part; DevState* st;
     float* traj; const AdjDev* rec;   // trajectory recording (x_n, y_n into slot rec->rec_slot), or null
-    int one_pass, rep_need;
+    int one_pass, rep_need, part_cs;
 };
-template <bool POW2, bool FULL, bool RECORD = false>
+template <bool POW2, bool FULL, bool RECORD, bool JOINT>
 __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int chunk) {
     const Parts& p = A.p; const Geo& g = A.g; const PushP& pp = A.pp;
     const float* __restrict__ gb = A.gb; const double qoa = A.qoa; unsigned long long* __restrict__ acc = A.acc;
@@ -1320,7 +1361,8 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     const long long c0 = static_cast<long long>(chunk) * cs_;
     const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
     const int ppt = cs_ / kThreads;               // particles per thread
-    const Spread sp(cs_);
+    const Own own = own_chunks<JOINT>(chunk, cs_, cnt, A.part_cs);
+    const Spread sp(own.cs);
     const float S1[1] = {st->S_next[0]};
     __shared__ __align__(16) int ends[4];
     if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
@@ -1372,6 +1414,14 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     double ke = 0, px = 0, py = 0, pz = 0;
     float m0 = 0.f, m1 = 0.f;
     bool done = false;
+    auto own_sums = [&](int o) {
+        block_sum4_put(ke, px, py, pz, dsh);
+        __syncthreads();
+        block_sum4_get(part, dsh, own.first + o);
+        if (!JOINT) return;
+        __syncthreads();
+        ke = px = py = pz = 0.0;
+    };
 
     // ---- single pass -------------------------------------------------------
     if (A.one_pass) {
@@ -1394,39 +1444,43 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
             __syncthreads();
             const bool cells = pp.write_cell && p.cell;
 #pragma unroll 1
-            for (int k = 0; k < ppt; ++k) {
-                const int sl = sp.slot(k);
-                if (sl >= cnt) continue;
-                float x = m.stage[sl], y = m.stage[kChunk + sl];
-                float ux = m.stage[2 * kChunk + sl], uy = m.stage[3 * kChunk + sl], uz = m.stage[4 * kChunk + sl];
-                if (!wsame) {
-                    w = __ldg(p.w + c0 + sl);
-                    cf0 = __double2float_rn(qoa * static_cast<double>(w));
+            for (int o = 0; o < own.n; ++o) {
+#pragma unroll 1
+                for (int k = 0; k < own.ppt; ++k) {
+                    const int sl = o * own.cs + sp.slot(k);
+                    if (sl >= cnt) continue;
+                    float x = m.stage[sl], y = m.stage[kChunk + sl];
+                    float ux = m.stage[2 * kChunk + sl], uy = m.stage[3 * kChunk + sl], uz = m.stage[4 * kChunk + sl];
+                    if (!wsame) {
+                        w = __ldg(p.w + c0 + sl);
+                        cf0 = __double2float_rn(qoa * static_cast<double>(w));
+                    }
+                    {
+                        const Cic c = cic(x, y);
+                        int li = c.i0 - bx.i0, lj = c.j0 - bx.j0;
+                        if (li < 0) li += g.nx;
+                        if (lj < 0) lj += g.ny;
+                        const float2* e = tile + lj * TW + li;
+                        push(c, e[0], e[1], e[TW], e[TW + 1], ux, uy, uz);
+                    }
+                    const bool ok = step_xy<POW2>(x, y, ux, uy, pp, g);
+                    const double dw = w, du = ux, dv = uy, dz = uz;
+                    ke += dw * (du * du + dv * dv + dz * dz);
+                    px += dw * du; py += dw * dv; pz += dw * dz;
+                    m.stage[sl] = x; m.stage[kChunk + sl] = y;
+                    m.stage[2 * kChunk + sl] = ux; m.stage[3 * kChunk + sl] = uy; m.stage[4 * kChunk + sl] = uz;
+                    m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy));
+                    if (ok) {
+                        const float cs[1] = {__fmul_rn(cf0, S1[0])};
+                        const int di = win_col(static_cast<int>(x), w1.oi, g.nx), dj = win_col(static_cast<int>(y), w1.oj, g.ny);
+                        if (fabsf(cs[0]) < kFastLim && di <= w1.W - 2 && dj <= w1.H - 2)
+                            win1_add<1, true, kEsP1>(area, w1, di, dj, x, y, cs);
+                        else { atomicOr(slow + (sl >> 5), 1u << (sl & 31)); nlist = 1; }
+                    } else {
+                        set_err(st, AW_DEV_OUT_OF_GRID);
+                    }
                 }
-                {
-                    const Cic c = cic(x, y);
-                    int li = c.i0 - bx.i0, lj = c.j0 - bx.j0;
-                    if (li < 0) li += g.nx;
-                    if (lj < 0) lj += g.ny;
-                    const float2* e = tile + lj * TW + li;
-                    push(c, e[0], e[1], e[TW], e[TW + 1], ux, uy, uz);
-                }
-                const bool ok = step_xy<POW2>(x, y, ux, uy, pp, g);
-                const double dw = w, du = ux, dv = uy, dz = uz;
-                ke += dw * (du * du + dv * dv + dz * dz);
-                px += dw * du; py += dw * dv; pz += dw * dz;
-                m.stage[sl] = x; m.stage[kChunk + sl] = y;
-                m.stage[2 * kChunk + sl] = ux; m.stage[3 * kChunk + sl] = uy; m.stage[4 * kChunk + sl] = uz;
-                m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy));
-                if (ok) {
-                    const float cs[1] = {__fmul_rn(cf0, S1[0])};
-                    const int di = win_col(static_cast<int>(x), w1.oi, g.nx), dj = win_col(static_cast<int>(y), w1.oj, g.ny);
-                    if (fabsf(cs[0]) < kFastLim && di <= w1.W - 2 && dj <= w1.H - 2)
-                        win1_add<1, true, kEsP1>(area, w1, di, dj, x, y, cs);
-                    else { atomicOr(slow + (sl >> 5), 1u << (sl & 31)); nlist = 1; }
-                } else {
-                    set_err(st, AW_DEV_OUT_OF_GRID);
-                }
+                if (JOINT) own_sums(o);
             }
             stage_fence();
             __syncthreads();
@@ -1528,7 +1582,7 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
             q5[2 * kChunk] = cf0;
         };
         auto coef = [&](const float (&a)[NS], float (&cs)[NF]) { cs[0] = __fmul_rn(a[2], S1[0]); };
-        if (wn.nb == 1 && wn.WH <= kEsSmall) {
+        if (!JOINT && wn.nb == 1 && wn.WH <= kEsSmall) {
             // a small window fits the area behind the stage: deposit and sums together
             // (375 x 225 at 50 per cell: 117.7 us a step, with the two apart 119.3)
             wn.P = kEsSmall;
@@ -1539,8 +1593,12 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
                 m.stage, m.win, wn, cs_, g, [&](const float (&)[NS], float (&cs)[NF]) { cs[0] = __fmul_rn(cf0, S1[0]); },
                 [&](const float (&)[NS], int sl) { sums(sl); });
         } else {
+#pragma unroll 1
+            for (int o = 0; o < own.n; ++o) {
 #pragma unroll 2
-            for (int k = 0; k < ppt; ++k) sums(sp.slot(k));
+                for (int k = 0; k < own.ppt; ++k) sums(o * own.cs + sp.slot(k));
+                if (JOINT) own_sums(o);
+            }
             __syncthreads();
             win_zero<NF, T0>(m.win, wn);
             __syncthreads();
@@ -1555,9 +1613,8 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
         umx[0][threadIdx.x >> 5] = __float_as_uint(m0);
         umx[1][threadIdx.x >> 5] = __float_as_uint(m1);
     }
-    block_sum4_put(ke, px, py, pz, dsh);
-    __syncthreads();
-    block_sum4_get(part, dsh, chunk);
+    if (JOINT) __syncthreads();
+    else own_sums(0);
     if (threadIdx.x >= 32 && threadIdx.x < 34) {
         const int d = threadIdx.x - 32;
         unsigned mx = 0;
@@ -1568,15 +1625,15 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
 }
 template <bool POW2, bool FULL, bool RECORD>
 __global__ void __launch_bounds__(kThreads, 4) k_push_deposit_es(EsArgs A) {
-    push_deposit_es_chunk<POW2, FULL, RECORD>(A, blockIdx.x);
+    push_deposit_es_chunk<POW2, FULL, RECORD, false>(A, blockIdx.x);
 }
 
 // Fused Darwin step kernel: input x y w ux uy uz; stage = new x, y, coefficient, ux, uy, uz.
 struct EmArgs {
     Parts p; Geo g; PushP pp; const float* gb; double qoa; unsigned long long* acc; int wmaxc;
-    double* part; DevState* st; float* psq; int use_tile; int one_pass; int rep_need;
+    double* part; DevState* st; float* psq; int use_tile; int one_pass; int rep_need; int part_cs;
 };
-template <bool POW2, bool FULL>
+template <bool POW2, bool FULL, bool JOINT>
 __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int chunk) {
     const Parts& p = A.p; const Geo& g = A.g; const PushP& pp = A.pp;
     const float* __restrict__ gb = A.gb; const double qoa = A.qoa; unsigned long long* __restrict__ acc = A.acc;
@@ -1597,7 +1654,8 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     const long long c0 = static_cast<long long>(chunk) * cs_;
     const int cnt = static_cast<int>(min(static_cast<long long>(cs_), p.n - c0));
     const int ppt = cs_ / kThreads;               // particles per thread
-    const Spread sp(cs_);
+    const Own own = own_chunks<JOINT>(chunk, cs_, cnt, A.part_cs);
+    const Spread sp(own.cs);
     float S[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) S[f] = st->S_next[f];
@@ -1607,7 +1665,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
     if (threadIdx.x == 0) { nlist = 0; box_reset(ends); }
     const float uxy_max = fmaxf(__uint_as_float(st->ucur_bits[0]), __uint_as_float(st->ucur_bits[1]));
     __shared__ int hot;                           // (field 0 is carried exactly)
-    const Expect1<NF> expect(st, psq, st->rms_src, [&](int f) { return st->S_next[f]; }, 1, chunk);
+    const Expect1<NF> expect(st, psq, st->rms_src, [&](int f) { return st->S_next[f]; }, 1, own);
     const ChunkSrc src{{p.x, p.y, p.w, p.ux, p.uy, p.uz}};
     float x0, y0;
     if (!load_chunk(m.stage, src, NS, c0, cnt, p.vec_ok != 0, &bar, st, &x0, &y0)) return;
@@ -1634,57 +1692,75 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
             float2 l2p[4] = {}, sqp[4] = {};
             double ke = 0, px = 0, py = 0, pz = 0;
             float m0 = 0.f, m1 = 0.f, m2 = 0.f, nval = 0.f;
+            auto own_sums = [&](int o) {
+                const float sq[NF] = {sqp[0].x, sqp[0].y, sqp[1].x, sqp[1].y, sqp[2].x, sqp[2].y, sqp[3].x, sqp[3].y};
+                block_sumsq_put<NF>(sq, nval, ssq);
+                block_sum4_put(ke, px, py, pz, dsh);
+                __syncthreads();
+                block_sumsq_get<NF>(psq, ssq, own.first + o, 32);
+                block_sum4_get(part, dsh, own.first + o);
+                if (!JOINT) return;
+                __syncthreads();
+                ke = px = py = pz = 0.0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sqp[i] = make_float2(0.f, 0.f);
+                nval = 0.f;
+            };
 #pragma unroll 1
-            for (int k = 0; k < ppt; ++k) {
-                const int sl = sp.slot(k);
-                if (sl >= cnt) continue;
-                float x = m.stage[sl], y = m.stage[kChunk + sl];
-                const float w = m.stage[2 * kChunk + sl];
-                float2 uxy = make_float2(m.stage[3 * kChunk + sl], m.stage[4 * kChunk + sl]);
-                float uz = m.stage[5 * kChunk + sl];
-                {
-                    const EB2 eb = tile1_gather(tl, cic(x, y), g);
-                    boris_em2(uxy, uz, eb.exy, eb.ezbx.x, eb.ezbx.y, eb.byz, pp.qmh);
-                }
-                const float ux = uxy.x, uy = uxy.y;
-                bool ok = step_xy<POW2>(x, y, ux, uy, pp, g);
-                const double dw = w, du = ux, dv = uy, dz = uz;
-                ke += dw * (du * du + dv * dv + dz * dz);
-                px += dw * du; py += dw * dv; pz += dw * dz;
-                m.stage[sl] = x; m.stage[kChunk + sl] = y;
-                m.stage[3 * kChunk + sl] = ux; m.stage[4 * kChunk + sl] = uy; m.stage[5 * kChunk + sl] = uz;
-                m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy)); m2 = fmaxf(m2, fabsf(uz));
-                int cell;
-                if (ok) {
-                    const int ci = static_cast<int>(x), cj = static_cast<int>(y);
-                    cell = cj * g.nx + ci;
-                    float2 cp[4], csp[4];
-                    src_coefs8(__double2float_rn(qoa * dw), ux, uy, uz, cp);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) csp[i] = __fmul2_rn(cp[i], Sp[i]);
-                    if (((ci + cj) & 7) == 0) {   // rms sample: the particles of one cell in 8, any order
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) sqp[i] = __ffma2_rn(cp[i], cp[i], sqp[i]);
-                        nval += 1.0f;
+            for (int o = 0; o < own.n; ++o) {
+#pragma unroll 1
+                for (int k = 0; k < own.ppt; ++k) {
+                    const int sl = o * own.cs + sp.slot(k);
+                    if (sl >= cnt) continue;
+                    float x = m.stage[sl], y = m.stage[kChunk + sl];
+                    const float w = m.stage[2 * kChunk + sl];
+                    float2 uxy = make_float2(m.stage[3 * kChunk + sl], m.stage[4 * kChunk + sl]);
+                    float uz = m.stage[5 * kChunk + sl];
+                    {
+                        const EB2 eb = tile1_gather(tl, cic(x, y), g);
+                        boris_em2(uxy, uz, eb.exy, eb.ezbx.x, eb.ezbx.y, eb.byz, pp.qmh);
                     }
-                    bool fast = true;
+                    const float ux = uxy.x, uy = uxy.y;
+                    bool ok = step_xy<POW2>(x, y, ux, uy, pp, g);
+                    const double dw = w, du = ux, dv = uy, dz = uz;
+                    ke += dw * (du * du + dv * dv + dz * dz);
+                    px += dw * du; py += dw * dv; pz += dw * dz;
+                    m.stage[sl] = x; m.stage[kChunk + sl] = y;
+                    m.stage[3 * kChunk + sl] = ux; m.stage[4 * kChunk + sl] = uy; m.stage[5 * kChunk + sl] = uz;
+                    m0 = fmaxf(m0, fabsf(ux)); m1 = fmaxf(m1, fabsf(uy)); m2 = fmaxf(m2, fabsf(uz));
+                    int cell;
+                    if (ok) {
+                        const int ci = static_cast<int>(x), cj = static_cast<int>(y);
+                        cell = cj * g.nx + ci;
+                        float2 cp[4], csp[4];
+                        src_coefs8(__double2float_rn(qoa * dw), ux, uy, uz, cp);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) fast = fast && fabsf(csp[i].x) < kFastLim && fabsf(csp[i].y) < kFastLim;
-                    const int di = win_col(ci, w1.oi, g.nx), dj = win_col(cj, w1.oj, g.ny);
-                    if (fast && di <= w1.W - 2 && dj <= w1.H - 2) {
+                        for (int i = 0; i < 4; ++i) csp[i] = __fmul2_rn(cp[i], Sp[i]);
+                        if (((ci + cj) & 7) == 0) {   // rms sample: the particles of one cell in 8, any order
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) l2p[i] = __ffma2_rn(csp[i], csp[i], l2p[i]);
-                        const float cs[NF] = {csp[0].x, csp[0].y, csp[1].x, csp[1].y,
-                                              csp[2].x, csp[2].y, csp[3].x, csp[3].y};
-                        win1_add<NF, true, P1>(m.win, w1, di, dj, x, y, cs);
+                            for (int i = 0; i < 4; ++i) sqp[i] = __ffma2_rn(cp[i], cp[i], sqp[i]);
+                            nval += 1.0f;
+                        }
+                        bool fast = true;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) fast = fast && fabsf(csp[i].x) < kFastLim && fabsf(csp[i].y) < kFastLim;
+                        const int di = win_col(ci, w1.oi, g.nx), dj = win_col(cj, w1.oj, g.ny);
+                        if (fast && di <= w1.W - 2 && dj <= w1.H - 2) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) l2p[i] = __ffma2_rn(csp[i], csp[i], l2p[i]);
+                            const float cs[NF] = {csp[0].x, csp[0].y, csp[1].x, csp[1].y,
+                                                  csp[2].x, csp[2].y, csp[3].x, csp[3].y};
+                            win1_add<NF, true, P1>(m.win, w1, di, dj, x, y, cs);
+                        } else {
+                            list_slow(m.slow, &nlist, sl);
+                        }
                     } else {
-                        list_slow(m.slow, &nlist, sl);
+                        set_err(st, AW_DEV_OUT_OF_GRID);
+                        cell = cells ? p.cell[c0 + sl] : 0;          // stays as it is
                     }
-                } else {
-                    set_err(st, AW_DEV_OUT_OF_GRID);
-                    cell = cells ? p.cell[c0 + sl] : 0;          // stays as it is
+                    m.stage[2 * kChunk + sl] = __int_as_float(cell);  // w is read again from the caller's array
                 }
-                m.stage[2 * kChunk + sl] = __int_as_float(cell);  // w is read again from the caller's array
+                if (JOINT) own_sums(o);
             }
             m0 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m0)));
             m1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m1)));
@@ -1724,12 +1800,7 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
                     atomicAdd(&st->chunks, 1ull);
                     atomicAdd(&st->one_pass, 1ull);
                 }
-                const float sq[NF] = {sqp[0].x, sqp[0].y, sqp[1].x, sqp[1].y, sqp[2].x, sqp[2].y, sqp[3].x, sqp[3].y};
-                block_sumsq_put<NF>(sq, nval, ssq);
-                block_sum4_put(ke, px, py, pz, dsh);
-                __syncthreads();
-                block_sumsq_get<NF>(psq, ssq, chunk, 32);
-                block_sum4_get(part, dsh, chunk);
+                if (!JOINT) own_sums(0);
                 if (threadIdx.x == 0 && chunk == 0) {
 #pragma unroll
                     for (int f = 0; f < NF; ++f) st->S_pend[f] = S[f];
@@ -1876,37 +1947,51 @@ __device__ __forceinline__ void push_deposit_em_chunk(const EmArgs& A, const int
             }
         }
     };
-    if (wn.use && wn.nb == 1) {
+    auto own_sums = [&](int o) {
+        float sq[NF];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { sq[2 * i] = sqp[i].x; sq[2 * i + 1] = sqp[i].y; }
+        block_sumsq_put<NF>(sq, nval, ssq);
+        block_sum4_put(ke, px, py, pz, dsh);
+        __syncthreads();
+        block_sumsq_get<NF>(psq, ssq, own.first + o, 32);
+        block_sum4_get(part, dsh, own.first + o);
+        if (!JOINT) return;
+        __syncthreads();
+        ke = px = py = pz = 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sqp[i] = make_float2(0.f, 0.f);
+        nval = 0.f;
+    };
+    if (!JOINT && wn.use && wn.nb == 1) {
         if (wn.track_all) window_particles<NF, NS, T0, true, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
         else window_particles<NF, NS, T0, false, PC>(m.stage, m.win, wn, cs_, g, coef, stats);
     } else {
 #pragma unroll 1
-        for (int k = 0; k < ppt; ++k) {
-            const int d = sp.slot(k);
-            float a[NS];
+        for (int o = 0; o < own.n; ++o) {
+#pragma unroll 1
+            for (int k = 0; k < own.ppt; ++k) {
+                const int d = o * own.cs + sp.slot(k);
+                float a[NS];
 #pragma unroll
-            for (int f = 0; f < NS; ++f) a[f] = m.stage[f * kChunk + d];
-            stats(a);
+                for (int f = 0; f < NS; ++f) a[f] = m.stage[f * kChunk + d];
+                stats(a);
+            }
+            if (JOINT) own_sums(o);
         }
         window_pass<NF, NS, T0, PC>(m.stage, m.win, wn, cs_, g, coef, acc);   // bands (or the slow path alone)
     }
     close_window<NF, NS, T0, PC>(m, wn, nlist, cs_, acc, g, st, coef);
-    float sq[NF];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { sq[2 * i] = sqp[i].x; sq[2 * i + 1] = sqp[i].y; }
-    block_sumsq_put<NF>(sq, nval, ssq);
-    block_sum4_put(ke, px, py, pz, dsh);
-    __syncthreads();
-    block_sumsq_get<NF>(psq, ssq, chunk, 32);
-    block_sum4_get(part, dsh, chunk);
+    if (!JOINT) own_sums(0);
     if (threadIdx.x == 0 && chunk == 0) {
 #pragma unroll
         for (int f = 0; f < NF; ++f) st->S_pend[f] = S[f];
         st->step += 1;
-    }}
+    }
+}
 template <bool POW2, bool FULL>
 __global__ void __launch_bounds__(kThreads, 3) k_push_deposit_em(EmArgs A) {
-    push_deposit_em_chunk<POW2, FULL>(A, blockIdx.x);
+    push_deposit_em_chunk<POW2, FULL, false>(A, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1929,7 +2014,7 @@ k_deposit_dcu_multi(const DcuArgs* __restrict__ runs, const int* __restrict__ fi
     __shared__ int chunk;
     if (threadIdx.x == 0) { const int r = find_run(first, nruns); A = runs[r]; chunk = blockIdx.x - first[r]; }
     __syncthreads();
-    deposit_dcu_chunk<false>(A, chunk);
+    deposit_dcu_chunk<false, true>(A, chunk);
 }
 template <bool POW2>
 __global__ void __launch_bounds__(kThreads, 4)
@@ -1938,7 +2023,7 @@ k_push_deposit_es_multi(const EsArgs* __restrict__ runs, const int* __restrict__
     __shared__ int chunk;
     if (threadIdx.x == 0) { const int r = find_run(first, nruns); A = runs[r]; chunk = blockIdx.x - first[r]; }
     __syncthreads();
-    push_deposit_es_chunk<POW2, false>(A, chunk);
+    push_deposit_es_chunk<POW2, false, false, true>(A, chunk);
 }
 template <bool POW2>
 __global__ void __launch_bounds__(kThreads, 3)
@@ -1947,7 +2032,7 @@ k_push_deposit_em_multi(const EmArgs* __restrict__ runs, const int* __restrict__
     __shared__ int chunk;
     if (threadIdx.x == 0) { const int r = find_run(first, nruns); A = runs[r]; chunk = blockIdx.x - first[r]; }
     __syncthreads();
-    push_deposit_em_chunk<POW2, false>(A, chunk);
+    push_deposit_em_chunk<POW2, false, true>(A, chunk);
 }
 
 inline int nchunks(long long n, int cs) { return static_cast<int>(std::max<long long>(1, (n + cs - 1) / cs)); }
@@ -2007,15 +2092,21 @@ bool use_tile(const Ctx& c) {
 bool one_pass(const Ctx& c) { return c.plan.one_pass != 0; }
 // Window copies of the single pass: the lanes that meet in a cell, lanes sitting
 // 8 m particles apart (a power of two, at most 16).
-int rep_need(const Ctx& c) {
+int rep_need(const Ctx& c) {         // (of the run's own chunks, in joint launches too: Own)
     const double lanes = static_cast<double>(c.parts.n) / c.geo.ncell / (c.parts.cs / 32);
     int r = 1;
     while (r < 16 && r < lanes) r <<= 1;
     return r;
 }
-DcuArgs dcu_args(const Ctx& c, const float* gb, bool fused) {
+// The particles in chunks of a joint launch: as many own chunks as fit kChunk.
+Parts joint_parts(const Ctx& c) {
+    Parts p = c.parts;
+    p.cs *= kChunk / p.cs;
+    return p;
+}
+DcuArgs dcu_args(const Ctx& c, const float* gb, bool fused, bool joint = false) {
     DcuArgs a{};
-    a.p = c.parts; a.g = c.geo;
+    a.p = joint ? joint_parts(c) : c.parts; a.g = c.geo; a.part_cs = c.parts.cs;
     a.qm2oa = c.prm.qm * c.prm.qm / (c.geo.dx * c.geo.dy);
     a.abs_qm = static_cast<float>(std::fabs(c.prm.qm));
     a.gb = gb; a.acc = c.acc_dcu; a.wmaxc = wmax_cells(3); a.st = c.st;
@@ -2028,9 +2119,10 @@ DcuArgs dcu_args(const Ctx& c, const float* gb, bool fused) {
 // Capacity of the two-pass fallback's window in cells (aw_kernel_plan::es_window;
 // results do not depend on it; above kEsWindow three CTAs fit an SM instead of four).
 int es_window(const Ctx& c) { return c.plan.es_window > 0 ? c.plan.es_window : kEsWindow; }
-EsArgs es_args(const Ctx& c) {
+EsArgs es_args(const Ctx& c, bool joint = false) {
     EsArgs a{};
-    a.p = c.parts; a.g = c.geo; a.pp = push_params(c); a.gb = c.gb_es;
+    a.part_cs = c.parts.cs;
+    a.p = joint ? joint_parts(c) : c.parts; a.g = c.geo; a.pp = push_params(c); a.gb = c.gb_es;
     a.qoa = c.prm.qm / (c.geo.dx * c.geo.dy);
     a.acc = c.acc_src; a.wmaxc = es_window(c); a.part = c.part_p; a.st = c.st;
     a.traj = c.rec_xy; a.rec = c.rec_ad;
@@ -2038,9 +2130,10 @@ EsArgs es_args(const Ctx& c) {
     a.rep_need = rep_need(c);
     return a;
 }
-EmArgs em_args(const Ctx& c) {
+EmArgs em_args(const Ctx& c, bool joint = false) {
     EmArgs a{};
-    a.p = c.parts; a.g = c.geo; a.pp = push_params(c); a.gb = c.gb_push;
+    a.part_cs = c.parts.cs;
+    a.p = joint ? joint_parts(c) : c.parts; a.g = c.geo; a.pp = push_params(c); a.gb = c.gb_push;
     a.qoa = c.prm.qm / (c.geo.dx * c.geo.dy);
     a.acc = c.acc_src; a.wmaxc = wmax_cells(8); a.part = c.part_p; a.st = c.st; a.psq = c.part_c;
     a.use_tile = use_tile(c) ? 1 : 0;
@@ -2583,7 +2676,8 @@ MultiPhase* multi_create(int kind, Ctx* const* runs, int nruns) {
     m->kind = kind;
     m->nruns = nruns;
     std::vector<int> first(nruns + 1, 0);
-    for (int r = 0; r < nruns; ++r) first[r + 1] = first[r] + (runs[r]->parts.n > 0 ? nchunks(runs[r]->parts) : 0);
+    for (int r = 0; r < nruns; ++r)
+        first[r + 1] = first[r] + (runs[r]->parts.n > 0 ? nchunks(joint_parts(*runs[r])) : 0);
     m->nblocks = first[nruns];
     m->pow2 = pow2_geo(*runs[0]);
     for (int r = 1; r < nruns; ++r)
@@ -2596,12 +2690,12 @@ MultiPhase* multi_create(int kind, Ctx* const* runs, int nruns) {
     m->smem = kind == kMultiDcu ? smem_bytes(3, 6) : kind == kMultiEmPush ? smem_bytes(8, 6) : 0;
     for (int r = 0; r < nruns; ++r) {
         if (kind == kMultiEsPush) {
-            const EsArgs a = es_args(*runs[r]);
+            const EsArgs a = es_args(*runs[r], true);
             put(&a, sizeof a);
             m->smem = std::max(m->smem, es_smem_bytes(a.wmaxc));
         }
-        else if (kind == kMultiDcu) { const DcuArgs a = dcu_args(*runs[r], runs[r]->gb_dcu, true); put(&a, sizeof a); }
-        else { const EmArgs a = em_args(*runs[r]); put(&a, sizeof a); }
+        else if (kind == kMultiDcu) { const DcuArgs a = dcu_args(*runs[r], runs[r]->gb_dcu, true, true); put(&a, sizeof a); }
+        else { const EmArgs a = em_args(*runs[r], true); put(&a, sizeof a); }
     }
     bytes = host.size();
     try {

@@ -97,3 +97,43 @@ def test_ensemble_rejects_bad_specs(aw):
     specs[0].nspecies = 0
     with pytest.raises(aw.ArcError):
         aw.Ensemble(specs)
+
+
+@pytest.mark.parametrize("model", [0, 1])
+def test_members_of_every_chunk_size_equal_runs_alone(torch_cuda, aw, model):
+    """A run alone takes chunks of 256 to 2048 particles, by its own size; in an ensemble
+    the particle kernels take full ones and the sums go over the run's own: the same
+    bits in the state and the diagnostics, ragged counts and odd grids included, for
+    runs that share launches and runs with their own step."""
+    #        nx   ny  per beam
+    runs = [(50, 30, 5), (64, 64, 8), (64, 64, 33), (75, 64, 27), (128, 96, 21), (128, 64, 45), (256, 130, 16)]
+    beams = lambda ppc: [dict(ppc=ppc, density=0.5, uth=(0.05, 0.04, 0.06), ufl=(v, 0.02, 0.0)) for v in (0.2, -0.25)]  # noqa: E731
+    par = dict(dt=0.05, c=1.0, n0=1.0, B0=(0.1, 0.0, 0.4))
+    e = aw.Ensemble([aw.run_spec(model, nx, ny, float(nx), float(ny), beams(p), seed=k, **par)
+                     for k, (nx, ny, p) in enumerate(runs)])
+    try:
+        e.init()
+        e.run(3)
+        e.run(2)
+        torch_cuda.cuda.synchronize()
+        for k, (nx, ny, p) in enumerate(runs):
+            n = 2 * p * nx * ny
+            P = {q: torch_cuda.zeros(n, dtype=torch_cuda.float32, device="cuda:0") for q in PARTICLE_KEYS}
+            cell = torch_cuda.zeros(n, dtype=torch_cuda.int32, device="cuda:0")
+            ctx = aw.Context(nx, ny, float(nx), float(ny), model=model,
+                             stream=torch_cuda.cuda.current_stream().cuda_stream, **par)
+            try:
+                ctx.bind_particles(*(P[q] for q in PARTICLE_KEYS), cell)
+                ctx.load_species(beams(p), seed=k, noisy=True)
+                ctx.init()
+                ctx.run(0, 5)
+                torch_cuda.cuda.synchronize()
+                assert ctx.error_word() == 0
+                assert e.diag(k) == ctx.step_diag(), k
+                got = _ens_state(torch_cuda, e, k)
+                for q in got:
+                    assert np.array_equal(got[q], P[q].cpu().numpy()), (k, q)
+            finally:
+                ctx.close()
+    finally:
+        e.close()
