@@ -962,7 +962,7 @@ void launch_charge_ref(Ctx& c) {
 // ---- the three-kernel grid solves -------------------------------------------------
 struct GridFft {
     FftPlan px, py;
-    float2* tw = nullptr;              // [nx] then [ny]
+    double2* tw = nullptr;             // [nx] then [ny]
 };
 namespace {
 // Radices of n, or false when it has a factor the passes do not take.
@@ -975,6 +975,7 @@ bool make_fft_plan(FftPlan& p, int n) {
         const int r = m % 8 == 0 ? 8 : m % 4 == 0 ? 4 : m % 2 == 0 ? 2 : m % 3 == 0 ? 3 : m % 5 == 0 ? 5 : m % 7 == 0 ? 7 : 0;
         if (r == 0) return false;
         p.r[p.np] = r;
+        p.odd |= r & 1;
         p.rnb[p.np] = 1.0f / static_cast<float>(n / r);
         p.rl[p.np] = 1.0f / static_cast<float>(l);
         ++p.np;
@@ -993,7 +994,9 @@ GridFftArgs gf_args(const Ctx& c) {
 }
 int pairs_of(const Ctx& c) { return (c.geo.ny + 1) / 2; }
 constexpr size_t kGfSmem = 96 * 1024;         // two blocks per SM, beside their twiddles
-size_t tw_bytes(int n) { return static_cast<size_t>((n + 1) & ~1) * sizeof(float2); }
+size_t tw_bytes(const FftPlan& p) {
+    return static_cast<size_t>((p.n + 1) & ~1) * sizeof(float2) + (p.odd ? p.n * sizeof(double2) : 0);
+}
 // The most items (row pairs or columns) per block, up to `most`, that fit kGfSmem and
 // still give every SM a block: wider blocks read and write longer runs.
 int gf_batch(const Ctx& c, int total, int other_blocks, size_t bytes_each, int most) {
@@ -1010,7 +1013,7 @@ void launch_cols(Ctx& c, const cufftComplex* const* in, cufftComplex* out, const
     a.op = op;
     const size_t each = static_cast<size_t>(2) * std::max(Op::NI, Op::NO) * a.g.rsy * sizeof(float2);
     a.cols = gf_batch(c, c.sg.nkx, 1, each, 8);
-    const size_t sh = each * a.cols + tw_bytes(a.g.ny);
+    const size_t sh = each * a.cols + tw_bytes(a.g.py);
     opt_in_smem(reinterpret_cast<const void*>(k_cols<Op>), sh);
     k_cols<Op><<<(c.sg.nkx + a.cols - 1) / a.cols, kThreads, sh, c.stream>>>(a);
     AW_LAUNCH();
@@ -1023,17 +1026,17 @@ void gridfft_make(Ctx& c) {
     if (c.geo.ny < 48) return;
     FftPlan px, py;
     if (c.geo.nx < 2 || !make_fft_plan(px, c.geo.nx) || !make_fft_plan(py, c.geo.ny)) return;
-    std::vector<float2> tw;
+    std::vector<double2> tw;
     for (int n : {c.geo.nx, c.geo.ny})
         for (int k = 0; k < n; ++k) {
             const double a = -6.28318530717958647692 * k / n;
-            tw.push_back(make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a))));
+            tw.push_back(make_double2(std::cos(a), std::sin(a)));
         }
     std::unique_ptr<GridFft> f(new GridFft());
     f->px = px; f->py = py;
-    AW_CUDA(cudaMalloc(reinterpret_cast<void**>(&f->tw), tw.size() * sizeof(float2)));
+    AW_CUDA(cudaMalloc(reinterpret_cast<void**>(&f->tw), tw.size() * sizeof(double2)));
     c.gf = f.release();
-    AW_CUDA(cudaMemcpy(c.gf->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    AW_CUDA(cudaMemcpy(c.gf->tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice));
 }
 void gridfft_free(Ctx& c) {
     if (!c.gf) return;
@@ -1048,7 +1051,7 @@ void gridfft_rows_real(Ctx& c, const float* const* src, int nf, cufftComplex* ou
     a.out = out;
     const size_t each = static_cast<size_t>(2) * a.g.rsx * sizeof(float2);
     a.g.pr = gf_batch(c, pairs_of(c), nf, each, 4);
-    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
+    const size_t sh = each * a.g.pr + tw_bytes(a.g.px);
     opt_in_smem(reinterpret_cast<const void*>(k_rows_fwd), sh);
     k_rows_fwd<<<dim3((pairs_of(c) + a.g.pr - 1) / a.g.pr, nf), kThreads, sh, c.stream>>>(a);
     AW_LAUNCH();
@@ -1060,7 +1063,7 @@ void gridfft_rows_planes(Ctx& c, const cufftComplex* in, float* const* out, int 
     for (int f = 0; f < nf; ++f) a.out[f] = out[f];
     const size_t each = static_cast<size_t>(2) * a.g.rsx * sizeof(float2);
     a.g.pr = gf_batch(c, pairs_of(c), nf, each, 4);
-    const size_t sh = each * a.g.pr + tw_bytes(a.g.nx);
+    const size_t sh = each * a.g.pr + tw_bytes(a.g.px);
     opt_in_smem(reinterpret_cast<const void*>(k_rows_inv), sh);
     k_rows_inv<<<dim3((pairs_of(c) + a.g.pr - 1) / a.g.pr, nf), kThreads, sh, c.stream>>>(a);
     AW_LAUNCH();
