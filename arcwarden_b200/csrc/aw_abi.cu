@@ -1140,7 +1140,7 @@ int aw_tune_kernels(aw_ctx* ctx, int32_t trial_steps, aw_kernel_plan* chosen) {
         if (c.model == AW_MODEL_DARWIN)
             cands = {{0, 0, 0}, {0, 1, 0}, {1, 0, 0}, {1, 1, 0}};
         else if (c.model == AW_MODEL_ES)
-            cands = {{-1, -1, 1024}, {-1, -1, 2048}, {-1, -1, 3584}};
+            cands = {{1, -1, 3584}, {0, -1, 3584}};     // (smaller windows save nothing: kEsWindow)
         aw_kernel_plan best = c.plan;
         bool cached = false;
         {

@@ -70,21 +70,21 @@ constexpr int kRedInts = kThreads / 32 * (4 + 8);
 // The fused ES kernel: four CTAs per SM (56 KB each, at most 64 registers), so its
 // stage holds x y ux uy uz and not the weights: a chunk's weights are usually equal
 // (one species), and where they are not the kernel reads them from global memory.
-// stage | area | red, the area holding either the single pass's window of kEsP1 cells
-// (4 planes), its gather tile of kEsT1 cells and the slow slots' bit map, or, at its
-// end, the two-pass fallback's slow list. The fallback's window (2 planes) starts in
-// the stage's planes 3 and 4, which its first pass has read by then.
+// stage | area | red, the area holding the single pass's window of kEsP1 cells (4
+// planes), its gather tile of kEsT1 cells and the slow slots' bit map, or the end of the
+// two-pass fallback's window (2 planes), which starts in the stage's planes 3 and 4: its
+// first pass has read them by then. (Slow slots are marked in the stage there, no list.)
 // The ES path keeps the particle order and no run of it is re-sorted, so a chunk covers
 // cs / ppc consecutive cells of the load order plus their drift: at few particles per
-// cell whole grid rows and their spread (3472 cells: 13 rows of 256). A smaller window
+// cell whole grid rows and their spread (3984 cells: 15 rows of 256). A smaller window
 // takes more bands there and reaches the exact global path sooner. Steps 500 to 550 of a
 // 256 x 256 two-stream run (vth 0.05, drift 0.2), us a step with 1408 cells and with
-// these: at 8 per cell 119 and 62, at 16 per cell 115 and 71.
+// these: at 8 per cell 119 and 63, at 16 per cell 115 and 73.
 constexpr int kEsP1 = 800, kEsT1 = 304;
 constexpr int kEsArea = kEsP1 * 4 * 4 + kEsT1 * 8 + kChunk / 8;
-constexpr int kEsWindow = (2 * kChunk * 4 + kEsArea - kChunk * 2) / 8, kEsSmall = (kEsArea - kChunk * 2) / 8;
-constexpr int es_area(int wmax) { return wmax <= kEsWindow ? kEsArea : wmax * 8 + kChunk * 2 - 2 * kChunk * 4; }
-static_assert(es_area(kEsWindow) == kEsArea && kEsArea % 8 == 0 && kEsArea >= kChunk * 2, "window, list and area");
+constexpr int kEsWindow = (2 * kChunk * 4 + kEsArea) / 8, kEsSmall = kEsArea / 8;
+constexpr int es_area(int wmax) { return wmax <= kEsWindow ? kEsArea : wmax * 8 - 2 * kChunk * 4; }
+static_assert(es_area(kEsWindow) == kEsArea && kEsArea % 8 == 0, "window and area");
 // stage [np][kChunk] f32 | window [planes][wmax] i32 | red ints | slow list u16[kChunk]
 constexpr size_t win_offset(int np) { return static_cast<size_t>(np) * kChunk * 4; }
 constexpr size_t smem_bytes_w(int nf, int np, int wmax, int planes) {
@@ -1327,9 +1327,10 @@ __device__ __forceinline__ bool step_xy(float& x, float& y, float ux, float uy, 
 }
 
 // Fused ES step kernel. Single pass where the chunk's window fits (one read of the
-// staged particle, 7 shared atomics); else two passes through the stage: new x (sign
-// set: no deposit - listed for the slow path, or no new position in the grid), y (< 0:
-// not pushed), ux uy uz, then the coefficient q w / (dx dy) in place of ux. Bound by instruction issue and by the latency of a
+// staged particle, 7 shared atomics); else two passes through the stage: new x, y, ux uy
+// uz, then the coefficient q w / (dx dy) in place of ux. x with its sign set: not in the
+// window - for the slow path (y's sign clear), or no new position in the grid (y = -0),
+// or not pushed (y = -1). Bound by instruction issue and by the latency of a
 // chunk's fixed phases (load, box, window, flush, sums): es256, 4.2 M particles, 390 ->
 // 250 instructions a particle, 73.7 -> 55.3 us (28 us of HBM time).
 struct EsArgs {
@@ -1350,7 +1351,7 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
     m.stage = reinterpret_cast<float*>(smem);
     m.win = reinterpret_cast<int*>(smem + win_offset(NIN - 2));
     m.red = reinterpret_cast<int*>(smem + win_offset(NIN) + es_area(wmaxc));
-    m.slow = reinterpret_cast<unsigned short*>(m.red) - kChunk;
+    m.slow = nullptr;
     int* const area = reinterpret_cast<int*>(smem + win_offset(NIN));
     __shared__ unsigned long long bar;
     __shared__ int nlist;
@@ -1552,9 +1553,9 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
                         const bool fast = scale_fast<1>(cf, S1, cs, l1);
                         xs = __fadd_rn(x, 0.0f);
                         ys = __fadd_rn(y, 0.0f);
-                        if (!fast) { xs = -xs; list_slow(m.slow, &nlist, s); }
+                        if (!fast) { xs = -xs; nlist = 1; }
                     } else {
-                        ys = 0.0f;
+                        ys = -0.0f;
                         set_err(st, AW_DEV_OUT_OF_GRID);
                     }
                 } else {
@@ -1604,7 +1605,28 @@ __device__ __forceinline__ void push_deposit_es_chunk(const EsArgs& A, const int
             __syncthreads();
             window_pass<NF, NS, T0>(m.stage, m.win, wn, cs_, g, coef, acc);
         }
-        close_window<NF, NS, T0>(m, wn, nlist, cs_, acc, g, st, coef);
+        __syncthreads();
+        if (wn.nb == 1) win_flush<NF, T0>(m.win, wn, acc, g);
+        if (nlist || !wn.use) {                   // the exact slow path: the marked slots, or all
+            unsigned ns = 0;
+            for (int sl = threadIdx.x; sl < cnt; sl += kThreads) {
+                const float x = m.stage[sl], y = m.stage[kChunk + sl];
+                if (__float_as_int(y) < 0 || (wn.use && __float_as_int(x) >= 0)) continue;
+                const float a[NS] = {fabsf(x), y, m.stage[2 * kChunk + sl]};
+                float cs[NF];
+                coef(a, cs);
+                if (!isfinite(cs[0])) { set_err(st, AW_DEV_NONFINITE); continue; }
+                const Cic c = cic(a[0], y);
+                const float wv[4] = {c.w0, c.w1, c.w2, c.w3};
+                deposit_global<1>(c.i0, c.j0, wv, cs, acc, g);
+                ++ns;
+            }
+            count_slow(st, ns);
+        }
+        if (threadIdx.x == 0) {
+            atomicAdd(&st->chunks, 1ull);
+            if (!wn.use || wn.nb > 1) atomicAdd(&st->overflow, 1ull);
+        }
     }
     // the in-plane |u| maxima bound the next step's moves (the single pass's margin)
     m0 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m0)));

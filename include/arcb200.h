@@ -123,7 +123,7 @@ typedef struct aw_kernel_plan {
                            whose window fits (1, the default), or always in two passes (0)  */
     int32_t tile;       /* two-pass Darwin kernels stage a gather tile of the chunk (1/0) */
     int32_t es_window;  /* electrostatic push in two passes: rho window capacity in cells,
-                           256..4096 (0: 3472; above that fewer chunks are resident)    */
+                           256..4096 (0: 3984; above that fewer chunks are resident)    */
 } aw_kernel_plan;
 
 
@@ -247,7 +247,7 @@ int aw_get_kernel_plan(aw_ctx* ctx, aw_kernel_plan* plan);
  * with a fixed heuristic, include/pic/depositor.hpp:354-360 and
  * config.hpp:61-66). Call it with the particles bound and loaded, before
  * aw_init: every candidate plan (Darwin: single/two-pass x gather tile;
- * electrostatic: the rho window) runs init, 2 warm-up steps and `trial_steps`
+ * electrostatic: single/two-pass) runs init, 2 warm-up steps and `trial_steps`
  * timed steps from the same initial state, twice (the second round in reverse
  * order; each plan keeps its faster trial); the fastest is set (and written to
  * *chosen when not NULL). The particles are restored and the context is left
