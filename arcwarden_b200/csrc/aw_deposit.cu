@@ -746,15 +746,17 @@ __device__ __forceinline__ void win1_flush(const int* __restrict__ s, const Win1
 // Whether a chunk's sums may be expected to leave the int32 range: from the largest rms
 // |coefficient| of the biased fields first .. NF - 1, scaled, that this chunk's sample psq
 // had in the last deposit, or the whole run's where the sample has fewer than 64
-// particles (one fast particle in a few sent 512 x 1 chunks of 768 the long way: 52.6 ->
-// 54.1 us a step). A single pass that finds so only at its end (chunk_overflows1) is done
+// particles. A single pass that finds so only at its end (chunk_overflows1) is done
 // over in two passes, which count carries, so such chunks take those from the start.
 // The scales bound the largest coefficient by 2^22: a Maxwellian's rms is a fifth of its
-// maximum or less (2048 x 2^22 / 5.6 = 1.5e9), a cold beam's is almost the maximum (up to
-// 8e9). Asked of the chunk and not of the run, because a beam may be a part of the
-// particles, stored apart. 256 x 256 at 256 per cell, a tenth of them such a beam, us a
+// maximum or less (2048 x 2^22 / 5.6 = 1.5e9), a cold beam's is almost the maximum (3.4e9
+// to 8e9). The line between lies at 1.75e9, higher for a sample by what its few fast
+// particles may add (at 1.75e9 a warm 128 x 64 run at 256 per cell sent 46 of its 2048
+// chunks the long way for nothing, a 512 x 1 one lost 3%). Asked of
+// the chunk and not of the run, because a beam may be a part of the particles, stored
+// apart. 256 x 256 at 256 per cell, a tenth of them such a beam, us a
 // step: 897 the first and 694 the later ones when asked of the run and done over through
-// the exact global path, 628 and 635 like this (two passes for all: 803).
+// the exact global path, 637 and 645 like this (two passes for all: 803).
 // The second warp loads before the chunk does and sets `hot` after (the block's next
 // barrier publishes it): nothing waits for its loads.
 template <int NF>
@@ -777,8 +779,10 @@ struct Expect1 {
     }
     __device__ __forceinline__ void set(int* hot, int cs) const {
         if (threadIdx.x >> 5 != 1) return;
-        const float r = n >= 64.0f ? __fsqrt_rn(__fdividef(sq, n)) : all;
-        const bool over = __any_sync(0xffffffffu, have && r * s * static_cast<float>(cs) > 1.75e9f);
+        const bool local = n >= 64.0f;
+        const float r = local ? __fsqrt_rn(__fdividef(sq, n)) : all;
+        const float line = local ? 1.75e9f * (1.0f + 8.0f * rsqrtf(n)) : 1.75e9f;
+        const bool over = __any_sync(0xffffffffu, have && r * s * static_cast<float>(cs) > line);
         if (threadIdx.x == 32) *hot = over;
     }
 };
@@ -1332,7 +1336,7 @@ __device__ __forceinline__ bool step_xy(float& x, float& y, float ux, float uy, 
 // window - for the slow path (y's sign clear), or no new position in the grid (y = -0),
 // or not pushed (y = -1). Bound by instruction issue and by the latency of a
 // chunk's fixed phases (load, box, window, flush, sums): es256, 4.2 M particles, 390 ->
-// 250 instructions a particle, 73.7 -> 55.3 us (28 us of HBM time).
+// 279 instructions a particle, 73.7 -> 55.6 us (28 us of HBM time).
 struct EsArgs {
     Parts p; Geo g; PushP pp; const float* gb; double qoa; unsigned long long* acc; int wmaxc;
     double* part; DevState* st;

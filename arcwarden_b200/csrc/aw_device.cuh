@@ -685,7 +685,7 @@ struct ChunkSrc {
 
 // Load planes [0, np) of the chunk [c0, c0 + cnt) into stage[k * kChunk + s]
 // (linear layout). Bulk copies need 16-byte aligned addresses and sizes: the
-// arrays are 16-byte aligned when `vec`, chunk starts are multiples of 8 KB, and
+// arrays are 16-byte aligned when `vec`, chunk starts are multiples of 1 KB, and
 // the ragged tail (< 4 particles) and unaligned arrays use plain loads. Returns
 // false (block-uniformly) when the bounded wait gave up. Ends with a barrier;
 // *x0, *y0 receive the first particle's position (read before any overwrite).

@@ -15,13 +15,12 @@
 // step a particle crosses a cell edge, which a gradient shows.
 //
 // Two rows share one complex transform (z = a + i b, a and b of one field, so their
-// magnitudes are alike). The passes of radix 3, 5 and 7 are in double between the single
-// precision values in shared memory: all in single, the error of some sizes was above
-// the library transforms' (720 x 96 by a tenth). Between the kernels a field is stored transposed,
-// [k][j], so that the columns are contiguous and a block of PR row pairs reads and
-// writes 16 PR bytes at a time. The transforms are Stockham passes of radix 8, 4,
-// 2, 3, 5, 7 between two shared buffers, padded by one element in 16 so that a pass's
-// strided writes spread over the banks.
+// magnitudes are alike). Between the kernels a field is stored transposed, [k][j], so
+// that the columns are contiguous and a block of PR row pairs reads and writes 16 PR
+// bytes at a time. The transforms are Stockham passes of radix 8, 4, 2, 3, 5, 7 between
+// two shared buffers, padded by one element in 16 so that a pass's strided writes spread
+// over the banks. The passes of radix 3, 5 and 7 compute in double: all in single, the
+// error of some sizes was above the library transforms' (720 x 96 by a tenth).
 
 constexpr int kFftMax = 1024;          // longest row or column
 struct FftPlan {

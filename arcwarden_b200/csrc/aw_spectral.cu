@@ -16,8 +16,8 @@
 //                    kernels read, field maxima and FP64 energy partials.
 //   k_diag_reduce    fixed-order FP64 reduction of all partials (diagnostics.hpp).
 //
-// Scale folding is exact: nx*ny is a power of two for every grid this path is
-// run on, and multiplying by 2^-k commutes with FP32 rounding.
+// Where nx*ny is a power of two the scale folding is exact: multiplying by 2^-k commutes
+// with FP32 rounding. On other grids it is one more rounding of each mode.
 #include <cooperative_groups.h>
 #include "aw_internal.h"
 
@@ -793,11 +793,6 @@ struct YeeF {
     int nx, ny;
     float dxp, dyp, c2, dt;
 };
-__device__ __forceinline__ int yee_idx(int i, int j, int nx, int ny) {
-    i += (i < 0) * nx - (i >= nx) * nx;
-    j += (j < 0) * ny - (j >= ny) * ny;
-    return j * nx + i;
-}
 
 // B half step B -= dt2 curl E (k_faraday). With `begin` (the first launch of
 // a step) one thread also opens the step: t = step dt; the |u| maxima the last
