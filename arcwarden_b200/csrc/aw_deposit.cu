@@ -1336,7 +1336,7 @@ __device__ __forceinline__ bool step_xy(float& x, float& y, float ux, float uy, 
 // window - for the slow path (y's sign clear), or no new position in the grid (y = -0),
 // or not pushed (y = -1). Bound by instruction issue and by the latency of a
 // chunk's fixed phases (load, box, window, flush, sums): es256, 4.2 M particles, 390 ->
-// 279 instructions a particle, 73.7 -> 55.6 us (28 us of HBM time).
+// 279 instructions a particle, 69.2 -> 51.0 us a launch under ncu (28 us of HBM time).
 struct EsArgs {
     Parts p; Geo g; PushP pp; const float* gb; double qoa; unsigned long long* acc; int wmaxc;
     double* part; DevState* st;
