@@ -600,7 +600,7 @@ int aw_particles_bind(aw_ctx* ctx, float* x, float* y, float* ux, float* uy, flo
         auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
         c.parts.vec_ok = (al(x) && al(y) && al(ux) && al(uy) && al(uz) && al(w) && (!cell || al(cell))) ? 1 : 0;
         // resident CTAs of the particle kernels: four per SM (electrostatic), three (Darwin, Yee)
-        c.parts.cs = aw::chunk_size(n, (c.model == AW_MODEL_ES ? 4 : 3) * c.sms);
+        c.parts.cs = aw::chunk_size(n, (c.model == AW_MODEL_ES ? 4 : 3) * c.sms, true);
         const int nb = static_cast<int>(std::max<long long>(1, (n + c.parts.cs - 1) / c.parts.cs));
         if (nb > c.npart_p) {
             if (c.part_p) cudaFree(c.part_p);

@@ -84,23 +84,23 @@ struct PumpP {
 // iterations' worth of work that does not shrink with it (load latency, window
 // set-up, flush, sums): 1.05 M particles (512 full chunks on 444 slots) take 820
 // chunks of 1280, 65 k take 256 of 256 instead of 32 full ones (es 64x64: 2.56 ->
-// 2.22 ms). Full chunks stay where they cost at most a tenth more: their kernels have
-// constant trip counts, and a run with its own step in an ensemble, whose waves other
-// runs fill up, is better off (1.05 M electrostatic particles, chunks of 1792 and 2048:
-// alone 41.2 and 41.3 us a step at 64 per cell, 47.4 and 47.4 at 16; 16 such runs
-// together 338 and 310).
+// 2.22 ms). With `full`, a run's own particle kernels, full chunks stay where they cost
+// at most a tenth more: their kernels have constant trip counts, and a run with its own
+// step in an ensemble, whose waves other runs fill up, is better off (1.05 M
+// electrostatic particles, chunks of 1792 and 2048: alone 41.2 and 41.3 us a step at 64
+// per cell, 47.4 and 47.4 at 16; 16 such runs together 338 and 310).
 constexpr int kChunkFixed = 3;
-inline int chunk_size(long long n, int slots) {
+inline int chunk_size(long long n, int slots, bool full = false) {
     if (n >= 2LL * slots * kChunk) return kChunk;
     int best = kPPT;
-    long long cost = -1, full = 0;
+    long long cost = -1, most = 0;
     for (int m = kPPT; m >= 1; --m) {
         const long long chunks = (n + m * kThreads - 1) / (m * kThreads);
         const long long t = (chunks + slots - 1) / slots * (m + kChunkFixed);
-        if (m == kPPT) full = t;
+        if (m == kPPT) most = t;
         if (cost < 0 || t < cost) { cost = t; best = m; }
     }
-    return 10 * full <= 11 * cost ? kChunk : best * kThreads;
+    return full && 10 * most <= 11 * cost ? kChunk : best * kThreads;
 }
 
 struct Ctx {
